@@ -13,6 +13,7 @@
 #pragma once
 #include "common.cuh"
 #include "tree.cuh"
+#include "zq.cuh"
 
 namespace exafac {
 
@@ -108,6 +109,7 @@ struct Session {
     float* EmatF = nullptr;
     float* PhiPF = nullptr;
     BfsState bfs;
+    ZState zq;  // FP64 form: breadth-first draws (zq_sampler.cu)
 
     // nonzero-row tracking per factor (rows outside the list are zero)
     bool dense[kMaxModes] = {false};
@@ -183,6 +185,11 @@ int arls_leverage(Session& s, int k, bool all_rows, const double* pinv, cudaStre
 int arls_draw(Session& s, int n, int64_t J, const double* uni, const uint32_t* perms, cudaStream_t st);
 int sts_compute_M(Session& s, int n, cudaStream_t st);
 int sts_draw(Session& s, int n, int64_t J, const double* uni, cudaStream_t st);
+// The FP64 form's STS-CP draws, breadth first (zq_sampler.cu): every sample
+// that list [0 .. *count) does not name afterwards is drawn; the named ones are
+// left to the depth-first kernel.
+int sts_draw_zq(Session& s, int n, int64_t J, const double* uni, cudaStream_t st);
+bool sts_zq_wanted(int R, int64_t J);
 // The mixed forms' STS-CP draws, breadth first (bfs_sampler.cu).
 int sts_draw_bfs(Session& s, int n, int64_t J, const double* uni, cudaStream_t st);
 // Tensor-core descents (bfs_sampler.cu): used for R >= kTcMinRank.

@@ -524,19 +524,22 @@ struct StsModes {
 // R / (J h^T Phi h).  T = double: the reference's arithmetic on the FP64
 // trees and factors; T = float (mixed forms): the same descents on FP32
 // copies of the trees (summed in FP64, rounded once), factors, eigenvector
-// rows and Phi.
+// rows and Phi.  list != null: only the samples list[0 .. *list_count).
 template <typename T>
 __global__ void sts_draw_kernel(int N, int n, int R, int G, int S, int64_t J, StsModes<T> m, TreeShape et,
                                 const T* __restrict__ eigG, const T* __restrict__ E, const T* __restrict__ PhiP,
                                 const double* __restrict__ uni, uint32_t* __restrict__ samples,
-                                double* __restrict__ weights, DeviceStatus* status) {
+                                double* __restrict__ weights, DeviceStatus* status, const int32_t* __restrict__ list,
+                                const int32_t* __restrict__ list_count) {
     extern __shared__ __align__(16) unsigned char stsdyn[];
     const int P = node_stride<T>(R);  // node stride of the trees and of PhiP
     T *h, *sh, *q;
     int gi;
     const SampleGroup<T> grp = sample_group<T>(stsdyn, R, G, h, sh, q, gi);
     const int tg = grp.tg, nth = grp.nthreads();
-    for (int64_t i = (int64_t)blockIdx.x * S + gi; i < J; i += (int64_t)gridDim.x * S) {
+    const int64_t todo = list ? (int64_t)*list_count : J;
+    for (int64_t q0 = (int64_t)blockIdx.x * S + gi; q0 < todo; q0 += (int64_t)gridDim.x * S) {
+        const int64_t i = list ? (int64_t)list[q0] : q0;
         for (int r = tg; r < R; r += nth) h[r] = T(1);
         bool empty = false;  // a descent ended in a leaf of zero mass: weight 0
         grp.sync();
@@ -593,7 +596,8 @@ int sts_rebuild_tree(Session& s, int k, cudaStream_t st) {
 
 template <typename T>
 static int sts_draw_launch(Session& s, int n, int64_t J, const double* uni, const T* const* treeG, const T* const* U,
-                           const T* eigG, const T* E, const T* PhiP, cudaStream_t st) {
+                           const T* eigG, const T* E, const T* PhiP, const int32_t* list, const int32_t* list_count,
+                           cudaStream_t st) {
     const int N = s.N;
     StsModes<T> m;
     for (int k = 0; k < kMaxModes; k++) {
@@ -616,9 +620,9 @@ static int sts_draw_launch(Session& s, int n, int64_t J, const double* uni, cons
     const size_t smem = (size_t)S * sample_group_bytes(s.R, sizeof(T));
     if (smem > 48 * 1024)
         EXAFAC_CUDA_TRY(cudaFuncSetAttribute(sts_draw_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int64_t blocks = std::max<int64_t>(std::min<int64_t>(ceil_div(J, S), 152 * 32), 1);
+    const int64_t blocks = std::max<int64_t>(std::min<int64_t>(ceil_div(J, S), 152 * (list ? 2 : 32)), 1);
     sts_draw_kernel<T><<<(unsigned)blocks, S * G * 32, smem, st>>>(N, n, s.R, G, S, J, m, s.etree, eigG, E, PhiP, uni,
-                                                                   s.samples, s.weights, s.status);
+                                                                   s.samples, s.weights, s.status, list, list_count);
     count_launch();
     EXAFAC_CHECK_LAUNCH();
     return EXAFAC_OK;
@@ -632,7 +636,13 @@ int sts_draw(Session& s, int n, int64_t J, const double* uni, cudaStream_t st) {
             treeG[k] = k < s.N ? s.treeG[k] : nullptr;
             U[k] = k < s.N ? s.F.U[k] : nullptr;
         }
-        return sts_draw_launch<double>(s, n, J, uni, treeG, U, s.eigG, s.Emat, s.PhiP, st);
+        const int32_t *list = nullptr, *count = nullptr;
+        if (s.zq.xi && sts_zq_wanted(s.R, J)) {
+            EXAFAC_TRY(sts_draw_zq(s, n, J, uni, st));
+            list = s.zq.redo_list;
+            count = s.zq.redo_count;
+        }
+        return sts_draw_launch<double>(s, n, J, uni, treeG, U, s.eigG, s.Emat, s.PhiP, list, count, st);
     }
     return sts_draw_bfs(s, n, J, uni, st);
 }

@@ -1,0 +1,32 @@
+// Sample state of the breadth-first FP64 STS-CP draws (zq_sampler.cu), J_max
+// entries each unless stated.
+#pragma once
+#include "common.cuh"
+
+namespace exafac {
+
+struct ZState {
+    int64_t* xi = nullptr;      // J x (R rounded up to 4): the descent's vector, fixed point
+    double2* lh = nullptr;      // (low, high) of the current descent
+    double* rinv = nullptr;     // 1 / root mass (scaled units)
+    float2* err = nullptr;      // error bounds of (low, high)
+    float* e0 = nullptr;        // error bound of one mass over the root mass
+    float* n1 = nullptr;        // sum of |x'|
+    int32_t* ex = nullptr;      // exponent of the vector's largest entry
+    int64_t* node = nullptr;    // current node
+    int32_t* order[2] = {nullptr, nullptr};  // slot -> sample, ordered by node (ping-pong)
+    int32_t* v = nullptr;       // eigen-tree leaf
+    int32_t* pick = nullptr;    // row within the leaf, -1 while not placed
+    int32_t* redo = nullptr;    // marked for the depth-first kernel
+    int32_t* redo_list = nullptr;
+    int32_t* redo_count = nullptr;  // 1
+    uint32_t* mask = nullptr;   // 4 per tile of 128 slots: went left (or stayed)
+    int32_t* tcount = nullptr;  // per tile: flags set
+    int64_t* pref64 = nullptr;  // per tile: prefix of tcount (more tiles than shared memory takes)
+    int64_t* off[2] = {nullptr, nullptr};  // slot ranges of a level's nodes (ping-pong)
+    int32_t* tree_exp = nullptr;           // 2 N: exponent of each tree's root diagonal
+};
+
+void zq_carve(Arena& a, ZState& b, int R, int64_t J, int64_t widest, int trees);
+
+}  // namespace exafac

@@ -1,0 +1,1073 @@
+// STS-CP draws of the FP64 form, breadth first on the tensor cores
+// (STS_CP::KRPDrawSamples, sts_cp.hpp:203-300, and PartitionTree::PTSample,
+// partition_tree.hpp:204-380, at one rank), with the decisions of the
+// depth-first FP64 kernel (sts_draw_kernel<double>).
+//
+// The depth-first kernel evaluates every node mass x^T G x in FP64, about
+// R^2 / 2 FMAs each on a pipe that retires ~1.7 of them per clock per SM: 66 to
+// 82 % of an FP64 sweep.  A descent only uses a mass to decide d <= low + m_L
+// / m, so here the masses are formed from bf16 digits on the tensor cores
+// with an error that is bounded in advance, every decision whose distance
+// from its cutoff is within the bound (of both evaluations) marks its sample,
+// and the marked samples are drawn again, whole, by the depth-first kernel.
+// The others took the same branch at every node, so their rows are the same;
+// their weights are formed by the same FP64 code.  Samples and weights are
+// those of the depth-first kernel bit for bit.
+//
+// Digits.  A vector x (scaled by a power of two to |x'| < 2^6) is held in
+// fixed point (units of 2^-47, int64) and cut into balanced base-256 digits:
+// x' = x0 + xr, x0 = d0 + d1 2^-8 + d2 2^-16 + d3 2^-24, |xr| <= 2^-25; a node
+// (scaled by its tree's root diagonal, |A'| < 2^6) into six digits, the
+// remainder |Ar| <= 2^-41.  A digit has at most 8 significant bits, so d_i
+// 2^-8i is a bf16 value, a product of two digits and a sum of R <= 128 of
+// them per weight 2^-8s, s = i + j, are integers below 2^24 in that unit: the
+// FP32 accumulators of the tensor core hold every weight's sum exactly.  Per
+// 32 columns of the node and digit i of x, one MMA multiplies the stacked
+// node digits 0 .. 5 - i, whose results land on the accumulators of the
+// weights s = i .. 5.  With Y = x0 A (weights <= 5) the mass is
+//   q = sum_c Y_c (x0 + 2 xr)_c = x'^T A' x' - xr^T A' xr - (dropped weights),
+// the dot product in integers (GB300's FP64 pipe would take longer over it
+// than the tensor cores over the products).
+//
+// Error, in the scaled units (n1 = sum |x'_c|):
+//   dropped digits and remainders: |Y_c| error <= R 3.7 2^-34
+//   FP32 add of the weights 4 and 5 and its rounding to 2^-31: <= 1.5 2^-32
+//   xr^T A' xr <= R^2 2^-44
+//   the depth-first kernel's own rounding: <= 40 2^-53 |x'|^T |A'| |x'|
+//                                         <= n1 R 0.31 2^-34
+//   E = n1 (R 4.6 2^-34 + 1.7 2^-32) + R^2 2^-44
+// A cutoff low + q / m is then off by at most E / m for the root mass, E / m
+// for its own mass and E / m per earlier right turn.  The leaf's row is picked
+// from FP32 squares of dots with 30-bit x, with its own bound (zq_leaf_kernel).
+//
+// Measured (GB300), draws of a step: R = 64, J = 2^18, three 2000-row modes:
+// 55.8 -> 7.9 ms; R = 25, J = 65536: 4.3 -> 1.4 ms; about one sample in 1e4
+// is marked (the FP32 squares of the leaf stage), its depth-first draw 0.1 to
+// 0.5 ms a step (the latency of one sample).
+#include "engine.cuh"
+#include "prims.cuh"
+#include "umma.cuh"
+#include "zq.cuh"
+
+namespace exafac {
+
+constexpr int kZTile = 128;  // slots per tile (the MMA's M)
+constexpr int kZx = 4;       // digits of x
+constexpr int kZa = 6;       // digits of a node entry
+constexpr int kZu = 4;       // digits of a leaf row's entry
+constexpr int kZCols = 32;   // node columns (leaf rows) per chunk
+constexpr int64_t kZPrefSmem = 16384;  // tiles whose prefix fits in shared memory
+
+struct ZShape {
+    int Rk, nch;                 // K padded to 16, chunks of kZCols columns
+    uint32_t sbo, xs, bs;        // bytes of 8 rows, of one x digit (128 rows), of one chunk digit (32 rows)
+};
+__host__ __device__ inline ZShape z_shape(int R) {
+    ZShape z;
+    z.Rk = (R + 15) & ~15;
+    z.nch = (R + kZCols - 1) / kZCols;
+    z.sbo = (uint32_t)z.Rk * 16u;
+    z.xs = 16u * z.sbo;
+    z.bs = 4u * z.sbo;
+    return z;
+}
+static size_t z_smem(int R, int digits) {
+    const ZShape z = z_shape(R);
+    return (size_t)kZx * z.xs + (size_t)digits * z.bs + 128;
+}
+
+// kind::f16: D FP32, A and B bf16, both K-major.
+__host__ __device__ constexpr uint32_t umma_idesc_bf16(int M, int N) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                          uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+// Waits for the loads above; the registers pass through so that no use of
+// them moves before the wait.
+template <int S>
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[S][8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int s = 0; s < S; s++)
+        asm volatile("" : "+r"(r[s][0]), "+r"(r[s][1]), "+r"(r[s][2]), "+r"(r[s][3]), "+r"(r[s][4]), "+r"(r[s][5]),
+                     "+r"(r[s][6]), "+r"(r[s][7]));
+}
+
+// Biased exponent of |v| (0 for zero and subnormals, 2047 for inf and nan).
+__device__ __forceinline__ int bexp(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
+
+// v 2^(52 - (emax - 1023)) cut to an integer (toward zero): with |v| < 2^(emax
+// - 1022) this is v', scaled to below 2^6, in units of 2^-47.
+__device__ __forceinline__ long long fix47(double v, int emax) {
+    const long long b = __double_as_longlong(v);
+    const int e = (int)((b >> 52) & 0x7ff);
+    unsigned long long m = (unsigned long long)b & 0xfffffffffffffull;
+    if (e) m |= 1ull << 52;
+    const int s = max(max(emax, 1) - max(e, 1), 0);
+    m = s > 63 ? 0ull : m >> s;
+    return b < 0 ? -(long long)m : (long long)m;
+}
+
+// (byte idx of t - 128) 2^-8w as a float (exact).
+template <int W>
+__device__ __forceinline__ float digit_f(uint32_t t, uint32_t idx) {
+    constexpr float sc = W == 0 ? 1.0f : W == 1 ? 0x1p-8f : W == 2 ? 0x1p-16f : W == 3 ? 0x1p-24f
+                         : W == 4 ? 0x1p-32f : 0x1p-40f;
+    return fmaf(__uint_as_float(__byte_perm(t, 0x4B000000u, 0x7440u | idx)), sc, -8388736.0f * sc);
+}
+__device__ __forceinline__ float lead_f(int d) {  // |d| <= 128 as a float
+    return __int_as_float(0x4B400000 + d) - 12582912.0f;
+}
+// two exact bf16 values, given as floats, packed (lo in the low half)
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+    return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632u);
+}
+
+// Rows of the fixed-point vectors are padded with zeros to a multiple of 4
+// (32 bytes), so that a thread's eight values are two 32-byte loads: with
+// 8-byte loads of 32 different rows the level kernel took 3.3 times the
+// sectors from L2.
+__host__ __device__ __forceinline__ int z_row(int R) { return (R + 3) & ~3; }
+__device__ __forceinline__ void load_x4(const long long* p, long long (&v)[8], int at) {
+    asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(v[at]), "=l"(v[at + 1]), "=l"(v[at + 2]), "=l"(v[at + 3])
+                 : "l"(p));
+}
+__device__ __forceinline__ void load_x8(const long long* row, int k, int Rx, bool live, long long (&v)[8]) {
+#pragma unroll
+    for (int h = 0; h < 8; h += 4) {
+        if (live && k + h < Rx) {
+            load_x4(row + k + h, v, h);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; q++) v[h + q] = 0ll;
+        }
+    }
+}
+
+// The four digits of eight x values (fixed point) into the slices of the
+// operand, 16 bytes each.
+__device__ __forceinline__ void store_x_digits(unsigned char* dst, uint32_t xs, const long long (&X)[8]) {
+    uint32_t t[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) t[q] = (uint32_t)(int)((X[q] + (1ll << 22)) >> 23) + 0x808080u;
+    uint32_t o[kZx][4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const uint32_t a = t[2 * q], b = t[2 * q + 1];
+        o[0][q] = pack_bf16(lead_f((int)a >> 24), lead_f((int)b >> 24));
+        o[1][q] = pack_bf16(digit_f<1>(a, 2), digit_f<1>(b, 2));
+        o[2][q] = pack_bf16(digit_f<2>(a, 1), digit_f<2>(b, 1));
+        o[3][q] = pack_bf16(digit_f<3>(a, 0), digit_f<3>(b, 0));
+    }
+#pragma unroll
+    for (int d = 0; d < kZx; d++)
+        *reinterpret_cast<uint4*>(dst + d * xs) = make_uint4(o[d][0], o[d][1], o[d][2], o[d][3]);
+}
+
+// The digits of eight node entries (DG = 6: units down to 2^-40; 4: 2^-24).
+template <int DG>
+__device__ __forceinline__ void store_a_digits(unsigned char* dst, uint32_t bs, const double (&v)[8], int emax) {
+    uint32_t lo[8];
+    int hi[8];  // DG = 6: byte 4 of the biased value and the leading digit above it
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        const long long f = fix47(v[q], emax);
+        if (DG == 6) {
+            const long long t = ((f + 64) >> 7) + 0x8080808080ll;
+            lo[q] = (uint32_t)t;
+            hi[q] = (int)(t >> 32);
+        } else {
+            lo[q] = (uint32_t)(int)((f + (1ll << 22)) >> 23) + 0x808080u;
+            hi[q] = 0;
+        }
+    }
+    uint32_t o[DG][4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const uint32_t a = lo[2 * q], b = lo[2 * q + 1];
+        const int ah = hi[2 * q], bh = hi[2 * q + 1];
+        if (DG == 6) {
+            o[0][q] = pack_bf16(lead_f(ah >> 8), lead_f(bh >> 8));
+            o[1][q] = pack_bf16(digit_f<1>((uint32_t)ah, 0), digit_f<1>((uint32_t)bh, 0));
+            o[2][q] = pack_bf16(digit_f<2>(a, 3), digit_f<2>(b, 3));
+            o[3][q] = pack_bf16(digit_f<3>(a, 2), digit_f<3>(b, 2));
+            o[DG - 2][q] = pack_bf16(digit_f<4>(a, 1), digit_f<4>(b, 1));
+            o[DG - 1][q] = pack_bf16(digit_f<5>(a, 0), digit_f<5>(b, 0));
+        } else {
+            o[0][q] = pack_bf16(lead_f((int)a >> 24), lead_f((int)b >> 24));
+            o[1][q] = pack_bf16(digit_f<1>(a, 2), digit_f<1>(b, 2));
+            o[2][q] = pack_bf16(digit_f<2>(a, 1), digit_f<2>(b, 1));
+            o[3][q] = pack_bf16(digit_f<3>(a, 0), digit_f<3>(b, 0));
+        }
+    }
+#pragma unroll
+    for (int d = 0; d < DG; d++)
+        *reinterpret_cast<uint4*>(dst + d * bs) = make_uint4(o[d][0], o[d][1], o[d][2], o[d][3]);
+}
+
+// The tile's vectors xi[js[r]] as the A operand: rows past n and columns past
+// R zero.  The row runs fastest over the threads (conflict-free stores).
+__device__ __forceinline__ void stage_x(unsigned char* A, const long long* __restrict__ xi, const int32_t* js, int n,
+                                        int R, const ZShape& z) {
+    const int total = kZTile * (z.Rk / 8);
+    for (int e = threadIdx.x; e < total; e += blockDim.x) {
+        const int r = e & (kZTile - 1), k = 8 * (e / kZTile);
+        long long X[8];
+        load_x8(xi + (int64_t)js[r < n ? r : 0] * z_row(R), k, z_row(R), r < n, X);
+        store_x_digits(A + (uint32_t)(r >> 3) * z.sbo + (uint32_t)(k >> 3) * 128u + (uint32_t)(r & 7) * 16u, z.xs, X);
+    }
+}
+
+// Columns 32 ch .. + 31 of the packed node g as the B operand (digit j of
+// column c in row 32 j + c).
+__device__ __forceinline__ void expand_node(unsigned char* B, const double* __restrict__ g, const int* rs, int ch,
+                                            int R, int emax, const ZShape& z) {
+    const int total = kZCols * (z.Rk / 8);
+    for (int e = threadIdx.x; e < total; e += blockDim.x) {
+        const int c = e & (kZCols - 1), k = 8 * (e / kZCols);
+        const int col = ch * kZCols + c;
+        double v[8];
+        const int rc = col < R ? rs[col] : 0;
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            const int kk = k + q;
+            v[q] = (col < R && kk < R) ? __ldg(g + (kk >= col ? rc + (kk - col) : rs[kk] + (col - kk))) : 0.0;
+        }
+        store_a_digits<kZa>(B + (uint32_t)(c >> 3) * z.sbo + (uint32_t)(k >> 3) * 128u + (uint32_t)(c & 7) * 16u, z.bs,
+                            v, emax);
+    }
+}
+
+// Rows 32 ch .. + 31 of a leaf (its first rows live, else zero) as the B operand.
+__device__ __forceinline__ void expand_rows(unsigned char* B, const double* __restrict__ Ub, int ch, int rows, int R,
+                                            int emax, const ZShape& z) {
+    const int total = kZCols * (z.Rk / 8);
+    for (int e = threadIdx.x; e < total; e += blockDim.x) {
+        const int c = e & (kZCols - 1), k = 8 * (e / kZCols);
+        const int r = ch * kZCols + c;
+        double v[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) v[q] = (r < rows && k + q < R) ? __ldg(Ub + (int64_t)r * R + k + q) : 0.0;
+        store_a_digits<kZu>(B + (uint32_t)(c >> 3) * z.sbo + (uint32_t)(k >> 3) * 128u + (uint32_t)(c & 7) * 16u, z.bs,
+                            v, emax);
+    }
+}
+
+// One chunk's products, by one thread: weights s = i + j < DG in the TMEM
+// columns 32 s ..
+template <int DG>
+__device__ __forceinline__ void issue_chunk(uint32_t tmem, const unsigned char* A, const unsigned char* B,
+                                            const ZShape& z, uint64_t* bar) {
+    tc_fence_after();
+#pragma unroll
+    for (int i = 0; i < kZx; i++) {
+        const uint32_t idesc = umma_idesc_bf16(kZTile, kZCols * (DG - i));
+        for (int ks = 0; ks < z.Rk / 16; ks++)
+            umma_bf16(tmem + (uint32_t)(kZCols * i), umma_desc(A + i * z.xs + ks * 256, 128u, z.sbo),
+                      umma_desc(B + ks * 256, 128u, z.sbo), idesc, (i > 0 || ks > 0) ? 1u : 0u);
+    }
+    umma_commit(bar);
+}
+
+// Marks sample j for the depth-first kernel (once).
+__device__ __forceinline__ void z_mark(int32_t* redo, int32_t* list, int32_t* count, int32_t j) {
+    if (atomicExch(redo + j, 1) == 0) list[atomicAdd(count, 1)] = j;
+}
+
+// E of the header, in the scaled units.
+__device__ __forceinline__ double z_bound(float n1, int R) {
+    return (double)n1 * ((double)R * 4.6 * 0x1p-34 + 1.7 * 0x1p-32) + (double)R * (double)R * 0x1p-44;
+}
+
+// MODE 0: the root's mass of every sample (slot s holds sample s).
+// MODE 1: a level: the left child's mass and the branch.
+// MODE 2: the tail level: as MODE 1; samples already at a leaf stay.
+// The branch flags of a tile's slots go to mask[4 tile ..] and their count to
+// tcount[tile].
+template <int MODE, int NT>
+__global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
+    zq_level_kernel(int R, TreeShape t, const double* __restrict__ G, const int32_t* __restrict__ tree_exp, int64_t J,
+                    ZState b, const int32_t* __restrict__ order, const double* __restrict__ dv, DeviceStatus* status,
+                    uint32_t wait_polls) {
+    extern __shared__ __align__(128) unsigned char z_raw[];
+    constexpr int NG = NT / 128;        // threads per slot in the read-back
+    constexpr int CPT = kZCols / NG;    // columns of a chunk per thread
+    __shared__ int32_t cs[kZTile], js[kZTile];
+    __shared__ uint32_t rmask[4], fbits[4];
+    __shared__ long long part[NG][5][kZTile];
+    __shared__ uint32_t flag_sm[kZTile];
+    __shared__ int rs[kMaxRank];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t tmem_base;
+    __shared__ int abort_flag;
+    const ZShape z = z_shape(R);
+    unsigned char* A = z_raw + ((128u - (smem_u32(z_raw) & 127u)) & 127u);
+    unsigned char* B = A + kZx * z.xs;
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const int P = packed_size(R);
+    if (w == 0) tmem_alloc(&tmem_base, 256);
+    for (int a = tid; a < R; a += NT) rs[a] = packed_index(R, a, a);
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        fence_mbar_init();
+        abort_flag = 0;
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base;
+    const int emax = *tree_exp;
+    uint32_t phase = 0;
+    int64_t resident = -1;  // the node B holds (one-chunk ranks)
+    const int row = (w & 3) * 32 + lane, grp = w >> 2;
+    const int64_t ntiles = (J + kZTile - 1) / kZTile;
+    const int64_t per = (ntiles + gridDim.x - 1) / gridDim.x;
+    const int64_t t0 = (int64_t)blockIdx.x * per, t1 = min(ntiles, t0 + per);
+    const bool ok = emax < 2047;  // a tree with a non-finite root: every sample is marked at the root
+    int64_t tile = t0;
+    for (; tile < t1; tile++) {
+        const int64_t s0 = tile * kZTile;
+        const int n = (int)min((int64_t)kZTile, J - s0);
+        double low = 0.0, rinv = 0.0, d = 0.0;
+        float2 er = make_float2(0.f, 0.f);
+        float e0 = 0.f;
+        int ex = 0;
+        float n1 = 0.f;
+        if (tid < kZTile) {
+            int32_t j = 0, c = -1;
+            if (tid < n) {
+                j = order ? order[s0 + tid] : (int32_t)(s0 + tid);
+                c = MODE == 0 ? 0 : (int32_t)b.node[j];
+                ex = b.ex[j];
+                n1 = b.n1[j];
+                if (MODE != 0) {
+                    low = b.lh[j].x;
+                    rinv = b.rinv[j];
+                    er = b.err[j];
+                    e0 = b.e0[j];
+                    d = dv[j];
+                }
+            }
+            js[tid] = j;
+            cs[tid] = c;
+            flag_sm[tid] = 1u;
+            const int32_t up = __shfl_up_sync(0xffffffffu, c, 1);
+            // run starts: compared across the warps' borders below
+            const bool start = tid < n && lane != 0 && c != up;
+            const uint32_t m = __ballot_sync(0xffffffffu, start);
+            if (lane == 0) rmask[w] = m;
+        }
+        __syncthreads();
+        if (tid < 4) {
+            const int i = 32 * tid;
+            if (i < n && (i == 0 || cs[i] != cs[i - 1])) rmask[tid] |= 1u;
+        }
+        stage_x(A, reinterpret_cast<const long long*>(b.xi), js, n, R, z);
+        __syncthreads();
+        for (int i0 = 0; i0 < n;) {  // runs of equal node (uniform over the block)
+            const int32_t c = cs[i0];
+            int i1 = n;
+            for (int q = (i0 + 1) >> 5; q < 4; q++) {
+                uint32_t bits = rmask[q];
+                if (q == ((i0 + 1) >> 5)) bits &= ~0u << ((i0 + 1) & 31);
+                if (bits) {
+                    i1 = min(n, (q << 5) + __ffs(bits) - 1);
+                    break;
+                }
+            }
+            if (MODE == 2 && tree_is_leaf(t, c)) {  // stays: flag 1
+                i0 = i1;
+                continue;
+            }
+            const int64_t g = MODE == 0 ? 0 : 2 * (int64_t)c + 1;
+            long long aPh = 0, aPl = 0, aQh = 0, aQl = 0, aV = 0;
+            const long long* xrow = reinterpret_cast<const long long*>(b.xi) + (int64_t)js[row < n ? row : 0] * z_row(R);
+            for (int ch = 0; ch < z.nch; ch++) {
+                if (resident != g || z.nch > 1) {
+                    expand_node(B, G + g * P, rs, ch, R, emax, z);
+                    resident = g;
+                }
+                fence_proxy_async_smem();
+                tc_fence_before();
+                __syncthreads();
+                if (tid == 0) {
+                    issue_chunk<kZa>(tmem, A, B, z, &bar);
+                    if (!mbar_wait_limited(&bar, phase, wait_polls)) abort_flag = 1;
+                }
+                phase ^= 1u;
+                __syncthreads();
+                if (abort_flag) break;
+                tc_fence_after();
+#pragma unroll
+                for (int h = 0; h < CPT / 8; h++) {
+                    const int cc = grp * CPT + 8 * h;      // column within the chunk
+                    const int c0 = ch * kZCols + cc;
+                    uint32_t a[kZa][8];
+#pragma unroll
+                    for (int s = 0; s < kZa; s++)
+                        tmem_ld8_nowait(tmem + ((uint32_t)((w & 3) * 32) << 16) + (uint32_t)(kZCols * s + cc), a[s]);
+                    long long X[8];
+                    load_x8(xrow, c0, z_row(R), true, X);
+                    tmem_ld_wait<kZa>(a);
+#pragma unroll
+                    for (int q = 0; q < 8; q++) {
+                        const float a0 = __uint_as_float(a[0][q]), a1 = __uint_as_float(a[1][q]),
+                                    a2 = __uint_as_float(a[2][q]), a3 = __uint_as_float(a[3][q]),
+                                    a4 = __uint_as_float(a[4][q]), a5 = __uint_as_float(a[5][q]);
+                        // the weights' integers, by adding a power of two whose
+                        // ulp is the unit: n0 (1), n1 (2^-8), n2 (2^-16), and
+                        // weight 3 (2^-24) as a multiple of 2^-23 and a rest
+                        const int m0 = __float_as_int(a0 + 12582912.0f) - 0x4B400000;
+                        const int m1 = __float_as_int(a1 + 49152.0f) - 0x47400000;
+                        const int m2 = __float_as_int(a2 + 192.0f) - 0x43400000;
+                        const float f3 = a3 + 1.5f;
+                        const int m3 = __float_as_int(f3) - 0x3FC00000;
+                        const float v = (a3 - (f3 - 1.5f)) + (a4 + a5);
+                        const int V = __float_as_int(v + 0.005859375f) - 0x3BC00000;  // units of 2^-31
+                        const int Pn = m0 * 256 + m1;  // units of 2^-8
+                        const int Qn = m2 * 128 + m3;  // units of 2^-23
+                        const long long z4 = (X[q] + (1ll << 22)) >> 23;
+                        const long long wi = 2 * X[q] - (z4 << 23);  // x0 + 2 xr
+                        const int wh = (int)(wi >> 27), wl = (int)wi & 0x7ffffff;
+                        aPh += (long long)Pn * wh;
+                        aPl += (long long)Pn * wl;
+                        aQh += (long long)Qn * wh;
+                        aQl += (long long)Qn * wl;
+                        aV += (long long)V * wh;
+                    }
+                }
+                tc_fence_before();
+                if (ch + 1 < z.nch) __syncthreads();  // Y and B are free for the next chunk
+                tc_fence_after();
+            }
+            if (abort_flag) break;
+            part[grp][0][row] = aPh;
+            part[grp][1][row] = aPl;
+            part[grp][2][row] = aQh;
+            part[grp][3][row] = aQl;
+            part[grp][4][row] = aV;
+            __syncthreads();
+            if (tid >= i0 && tid < i1) {
+                long long s5[5];
+#pragma unroll
+                for (int u = 0; u < 5; u++) {
+                    s5[u] = part[0][u][tid];
+#pragma unroll
+                    for (int gq = 1; gq < NG; gq++) s5[u] += part[gq][u][tid];
+                }
+                // weights: P 2^-8, Q 2^-23, V 2^-31; wh 2^-20, wl 2^-47
+                const double q = (double)s5[0] * 0x1p-28 + (double)s5[1] * 0x1p-55 + (double)s5[2] * 0x1p-43 +
+                                 (double)s5[3] * 0x1p-70 + (double)s5[4] * 0x1p-51;
+                const int32_t j = js[tid];
+                if (MODE == 0) {
+                    const double E = z_bound(n1, R);
+                    const double e = E / q;
+                    const bool good = ok && ex < 2047 && q > 0.0 && e < 0x1p-10;
+                    b.rinv[j] = good ? 1.0 / q : 0.0;
+                    const float ef = __double2float_ru(e + 0x1p-50);
+                    b.e0[j] = good ? ef : 1.0f;
+                    b.err[j] = make_float2(good ? ef : 1.0f, good ? ef : 1.0f);
+                    if (!good) z_mark(b.redo, b.redo_list, b.redo_count, j);
+                } else {
+                    const double cutoff = low + q * rinv;
+                    const float ec = (er.x + e0) * 1.0001f + 0x1p-50f;
+                    const bool left = d <= cutoff;
+                    if (!(fabs(d - cutoff) > (double)ec)) z_mark(b.redo, b.redo_list, b.redo_count, j);
+                    b.node[j] = left ? 2 * (int64_t)c + 1 : 2 * (int64_t)c + 2;
+                    if (left) {
+                        b.lh[j].y = cutoff;
+                        b.err[j].y = ec;
+                    } else {
+                        b.lh[j].x = cutoff;
+                        b.err[j].x = ec;
+                    }
+                    flag_sm[tid] = left ? 1u : 0u;
+                }
+            }
+            __syncthreads();  // part, and Y and B for the next run
+            i0 = i1;
+        }
+        if (abort_flag) break;
+        if (MODE != 0) {
+            if (tid < kZTile) {
+                const uint32_t bits = __ballot_sync(0xffffffffu, tid < n && flag_sm[tid] != 0u);
+                if (lane == 0) {
+                    fbits[w] = bits;
+                    b.mask[4 * tile + w] = bits;
+                }
+            }
+            __syncthreads();
+            if (tid == 0)
+                b.tcount[tile] = __popc(fbits[0]) + __popc(fbits[1]) + __popc(fbits[2]) + __popc(fbits[3]);
+        }
+        __syncthreads();
+    }
+    __syncthreads();
+    if (abort_flag) {
+        // no flags for the tiles left out: the partition keeps their order
+        if (MODE != 0)
+            for (int64_t q = tile; q < t1; q++) {
+                if (tid < 4) b.mask[4 * q + tid] = 0u;
+                if (tid == 0) b.tcount[q] = 0;
+            }
+        if (tid == 0) {
+            report(status, EXAFAC_ERR_TIMEOUT, 23, blockIdx.x, 0);
+            mbar_wait_limited(&bar, phase ^ 1u, wait_polls);  // the MMAs in flight may still complete (bounded)
+        }
+        tc_fence_before();
+        __syncthreads();
+    }
+    if (w == 0) {
+        tc_fence_after();
+        tmem_dealloc(tmem, 256);
+    }
+}
+
+// The leaf stage: dots v_r = U_r . x of the leaf's rows from four digits of
+// each (weights <= 3), their FP32 squares' prefix in row order, and the row
+// whose range (before, before + v_r^2] holds frac x total, frac = (d - low) /
+// (high - low), when frac x total keeps a distance from both ends that
+// covers every error; otherwise the sample is marked.  In scaled units
+// (|x'|, |U'| < 2^6): a dot is off by at most e0 = R 5.2 2^-18 plus 2^-24 of
+// itself, so a prefix by 2 e0 sqrt(F total) + F e0^2 + 70 2^-24 total, and
+// frac by (err_low + err_high) / (high - low).
+template <int NT>
+__global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
+    zq_leaf_kernel(int R, TreeShape t, const double* __restrict__ G, const double* __restrict__ U, int64_t J, ZState b,
+                   const int32_t* __restrict__ order, const double* __restrict__ dv, int N, int col,
+                   uint32_t* __restrict__ samples, DeviceStatus* status, uint32_t wait_polls) {
+    extern __shared__ __align__(128) unsigned char z_raw[];
+    constexpr int NG = NT / 128;
+    constexpr int CPT = kZCols / NG;
+    constexpr int NS = (NT == 256 ? 2 : 4);  // chunks (leaf rows / 32) at most
+    __shared__ int32_t cs[kZTile], js[kZTile];
+    __shared__ float psum[NS * NG][kZTile];
+    __shared__ int diag_exp;
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t tmem_base;
+    __shared__ int abort_flag;
+    const ZShape z = z_shape(R);
+    unsigned char* A = z_raw + ((128u - (smem_u32(z_raw) & 127u)) & 127u);
+    unsigned char* B = A + kZx * z.xs;
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const int P = packed_size(R), F = (int)t.F;
+    const int nch = (F + kZCols - 1) / kZCols;
+    if (w == 0) tmem_alloc(&tmem_base, 128);
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        fence_mbar_init();
+        abort_flag = 0;
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base;
+    uint32_t phase = 0;
+    const int row = (w & 3) * 32 + lane, grp = w >> 2;
+    const int64_t ntiles = (J + kZTile - 1) / kZTile;
+    const int64_t per = (ntiles + gridDim.x - 1) / gridDim.x;
+    const int64_t t0 = (int64_t)blockIdx.x * per, t1 = min(ntiles, t0 + per);
+    for (int64_t tile = t0; tile < t1; tile++) {
+        const int64_t s0 = tile * kZTile;
+        const int n = (int)min((int64_t)kZTile, J - s0);
+        if (tid < kZTile) {
+            const int32_t j = tid < n ? (order ? order[s0 + tid] : (int32_t)(s0 + tid)) : 0;
+            js[tid] = j;
+            cs[tid] = tid < n ? (int32_t)b.node[j] : -1;
+        }
+        __syncthreads();
+        stage_x(A, reinterpret_cast<const long long*>(b.xi), js, n, R, z);
+        for (int i0 = 0; i0 < n;) {
+            const int32_t c = cs[i0];
+            int i1 = i0 + 1;
+            while (i1 < n && cs[i1] == c) i1++;
+            if (!tree_is_leaf(t, c)) {  // only after a wait that ran out: not placed
+                if (tid >= i0 && tid < i1) {
+                    z_mark(b.redo, b.redo_list, b.redo_count, js[tid]);
+                    samples[(int64_t)js[tid] * N + col] = 0u;
+                }
+                i0 = i1;
+                continue;
+            }
+            const int64_t leaf = tree_leaf_idx(t, c);
+            const int rows = (int)min((int64_t)F, t.n - leaf * F);
+            const double* Ub = U + leaf * F * R;
+            // |U_rj| <= sqrt(G_jj) of the leaf's Gram: the rows' common exponent
+            if (tid < 32) {
+                int e = 0;
+                for (int a = lane; a < R; a += 32) e = max(e, bexp(__ldg(G + (int64_t)c * P + packed_index(R, a, a))));
+                e = __reduce_max_sync(0xffffffffu, e);
+                // max G_jj < 2^(e - 1022): |U| < 2^ceil((e - 1022) / 2); one more for rounding
+                if (lane == 0) diag_exp = e >= 2047 ? 2047 : ((e - 1022 + 2047) >> 1) - 1023 + 1 + 1022;
+            }
+            __syncthreads();
+            const int emax = diag_exp;
+            float y[NS][CPT];
+#pragma unroll
+            for (int ch = 0; ch < NS; ch++) {
+                if (ch < nch) {
+                    expand_rows(B, Ub, ch, rows, R, emax, z);
+                    fence_proxy_async_smem();
+                    tc_fence_before();
+                    __syncthreads();
+                    if (tid == 0) {
+                        issue_chunk<kZu>(tmem, A, B, z, &bar);
+                        if (!mbar_wait_limited(&bar, phase, wait_polls)) abort_flag = 1;
+                    }
+                    phase ^= 1u;
+                    __syncthreads();
+                    tc_fence_after();
+                    float ps = 0.0f;
+#pragma unroll
+                    for (int h = 0; h < CPT / 8; h++) {
+                        uint32_t a[kZu][8];
+#pragma unroll
+                        for (int s = 0; s < kZu; s++)
+                            tmem_ld8_nowait(tmem + ((uint32_t)((w & 3) * 32) << 16) +
+                                                (uint32_t)(kZCols * s + grp * CPT + 8 * h), a[s]);
+                        tmem_ld_wait<kZu>(a);
+#pragma unroll
+                        for (int q = 0; q < 8; q++) {
+                            const float v = __uint_as_float(a[0][q]) +
+                                            (__uint_as_float(a[1][q]) +
+                                             (__uint_as_float(a[2][q]) + __uint_as_float(a[3][q])));
+                            y[ch][8 * h + q] = v * v;
+                            ps += v * v;
+                        }
+                    }
+                    psum[ch * NG + grp][row] = ps;
+                    tc_fence_before();
+                    __syncthreads();
+                    tc_fence_after();
+                    if (abort_flag) break;
+                } else {
+#pragma unroll
+                    for (int q = 0; q < CPT; q++) y[ch][q] = 0.0f;
+                }
+            }
+            if (abort_flag) break;
+            if (row >= i0 && row < i1) {
+                const int32_t j = js[row];
+                float total = 0.0f;
+                for (int s = 0; s < nch * NG; s++) total += psum[s][row];
+                const double2 lh = b.lh[j];
+                const float2 er = b.err[j];
+                const double width = lh.y - lh.x;
+                const float rw = (float)(1.0 / width);
+                const float frac = (float)((dv[j] - lh.x) / width);
+                const float thr = frac * total;
+                const float de = (er.x + er.y + 0x1p-49f) * rw * total * 1.001f;
+                const float ev = (float)R * 5.2f * 0x1p-18f;
+                const float delta = 1.01f * (de + 2.0f * ev * sqrtf((float)F * total) + (float)F * ev * ev +
+                                             70.0f * 0x1p-24f * total);
+                // every thread of the slot looks for the row in its slices
+                bool found = false;
+                float before = 0.0f;
+                int at = 0;
+#pragma unroll
+                for (int ch = 0; ch < NS; ch++) {
+                    if (ch < nch) {
+                        for (int gq = 0; gq < NG; gq++) {
+                            const float ps = psum[ch * NG + gq][row];
+                            if (gq == grp) {
+                                float pre = before;
+#pragma unroll
+                                for (int q = 0; q < CPT; q++) {
+                                    const float nx = pre + y[ch][q];
+                                    const int r = ch * kZCols + grp * CPT + q;
+                                    if (!found && r < rows && thr < nx - delta && (r == 0 || thr > pre + delta)) {
+                                        found = true;
+                                        at = r;
+                                    }
+                                    pre = nx;
+                                }
+                            }
+                            before += ps;
+                        }
+                    }
+                }
+                // delta is a finite number only if every input was; a sample
+                // that no thread places is marked
+                if (found && width > 0.0 && total > 0.0f && delta < total && emax < 2047)
+                    b.pick[j] = at;
+            }
+            __syncthreads();
+            if (tid >= i0 && tid < i1) {
+                const int32_t j = js[tid];
+                const int p = b.pick[j];
+                if (p < 0) z_mark(b.redo, b.redo_list, b.redo_count, j);
+                samples[(int64_t)j * N + col] = (uint32_t)(leaf * F + max(p, 0));
+            }
+            __syncthreads();
+            i0 = i1;
+        }
+        if (abort_flag) break;
+        __syncthreads();
+    }
+    __syncthreads();
+    if (abort_flag) {
+        if (tid == 0) {
+            report(status, EXAFAC_ERR_TIMEOUT, 24, blockIdx.x, 0);
+            mbar_wait_limited(&bar, phase ^ 1u, wait_polls);
+        }
+        tc_fence_before();
+        __syncthreads();
+    }
+    if (w == 0) {
+        tc_fence_after();
+        tmem_dealloc(tmem, 128);
+    }
+}
+
+// Exclusive prefix of the tiles' counts in a block's shared memory.
+__device__ __forceinline__ void tile_prefix(const int32_t* __restrict__ tcount, int ntiles, int32_t* pref) {
+    __shared__ int32_t wsum[32];
+    const int nt = blockDim.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int32_t carry = 0;
+    for (int base = 0; base < ntiles; base += 4 * nt) {
+        int32_t v[4], s = 0;
+        const int i = base + 4 * threadIdx.x;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            v[q] = i + q < ntiles ? __ldg(tcount + i + q) : 0;
+            s += v[q];
+        }
+        int32_t inc = s;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += u;
+        }
+        if (lane == 31) wsum[w] = inc;
+        __syncthreads();
+        int32_t pre = carry + inc - s, all = 0;
+        for (int q = 0; q < (nt >> 5); q++) {
+            if (q < w) pre += wsum[q];
+            all += wsum[q];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (i + q < ntiles) pref[i + q] = pre;
+            pre += v[q];
+        }
+        carry += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) pref[ntiles] = carry;
+    __syncthreads();
+}
+
+// The stable partition after a level in one launch: SL(s), the flags set
+// before slot s, is the tile's prefix plus the bits below s of its mask.
+// Within its parent's slot range a slot whose flag is set (went left, or
+// stayed at a leaf) keeps its order among those, before the others; the
+// children's slot ranges follow (coff, when another level does).  Every block
+// forms the tiles' prefix in shared memory (up to kZPrefSmem tiles), or reads
+// pref64 (more).  lb: the parents' first node index, nl their number.
+__global__ void __launch_bounds__(512)
+    zq_partition_kernel(int64_t J, int ntiles, const uint32_t* __restrict__ mask, const int32_t* __restrict__ tcount,
+                        const int64_t* __restrict__ pref64, int64_t lb, int64_t nl, const int32_t* __restrict__ order,
+                        const int64_t* __restrict__ node, const int64_t* __restrict__ off,
+                        int32_t* __restrict__ order2, int64_t* __restrict__ coff) {
+    extern __shared__ int32_t z_pref[];
+    if (!pref64) tile_prefix(tcount, ntiles, z_pref);
+    auto SL = [&](int64_t s) -> int64_t {
+        const int64_t tile = s >> 7;
+        int64_t v = pref64 ? pref64[tile] : (int64_t)z_pref[tile];
+        const int in = (int)(s & 127);
+        if (in) {
+            const uint32_t* m = mask + 4 * tile;
+            for (int q = 0; q < (in >> 5); q++) v += __popc(__ldg(m + q));
+            if (in & 31) v += __popc(__ldg(m + (in >> 5)) & ((1u << (in & 31)) - 1u));
+        }
+        return v;
+    };
+    const int64_t step = (int64_t)gridDim.x * blockDim.x, first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (int64_t s = first; s < J; s += step) {
+        const int32_t j = order ? order[s] : (int32_t)s;
+        const int64_t c = node[j];
+        const int64_t i = (c >= lb + nl ? (c - 1) / 2 : c) - lb;
+        if (i < 0 || i >= nl) {  // only after a wait that ran out
+            order2[s] = j;
+            continue;
+        }
+        const int64_t start = off[i], end = off[i + 1];
+        const int64_t at0 = SL(start), at = SL(s);
+        const bool fl = (__ldg(mask + 4 * (s >> 7) + ((s & 127) >> 5)) >> (s & 31)) & 1u;
+        const int64_t before = at - at0;
+        const int64_t pos = fl ? start + before : start + (SL(end) - at0) + ((s - start) - before);
+        if (pos >= 0 && pos < J) order2[pos] = j;
+    }
+    if (coff)
+        for (int64_t i = first; i < nl; i += step) {
+            const int64_t start = off[i], end = off[i + 1];
+            coff[2 * i] = start;
+            coff[2 * i + 1] = start + (SL(end) - SL(start));
+            if (i == 0) coff[2 * nl] = J;
+        }
+}
+
+// Largest diagonal exponent of a tree's root, plus one (the entries of the
+// tree's nodes are bounded by their diagonals, those by the root's; one more
+// bit for rounding).
+__global__ void zq_tree_exp_kernel(int R, const double* __restrict__ root, int32_t* __restrict__ out) {
+    int e = 0;
+    for (int a = threadIdx.x; a < R; a += 32) e = max(e, bexp(root[packed_index(R, a, a)]));
+    e = __reduce_max_sync(0xffffffffu, e);
+    if (threadIdx.x == 0) *out = e >= 2047 ? 2047 : e + 1;
+}
+
+// The vector of the next descent in fixed point, a warp per sample, and the
+// sample's state at the root.
+// KIND 0: h = 1.  KIND 1: x = h * E[v].  KIND 2: h *= U[row], x = h.
+template <int KIND>
+__global__ void zq_vector_kernel(int R, int64_t J, double* __restrict__ h, const double* __restrict__ M,
+                                 const uint32_t* __restrict__ samples, int N, int col, int64_t rows, ZState b,
+                                 DeviceStatus* status) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t j = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < J; j += nw) {
+        double x[4];
+        int64_t r = 0;
+        if (KIND != 0) {
+            r = KIND == 1 ? (int64_t)b.v[j] : (int64_t)samples[j * N + col];
+            if (r < 0 || r >= rows) {  // as the depth-first kernel: report, take the last row
+                if (lane == 0) report(status, EXAFAC_ERR_DEVICE, KIND, r, rows);
+                r = rows - 1;
+            }
+        }
+        int e = 0;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int c = lane + 32 * q;
+            x[q] = 0.0;
+            if (c < R) {
+                if (KIND == 0) x[q] = 1.0;
+                else x[q] = h[j * R + c] * __ldg(M + r * R + c);
+                if (KIND != 1) h[j * R + c] = x[q];
+                e = max(e, bexp(x[q]));
+            }
+        }
+        e = __reduce_max_sync(0xffffffffu, e);
+        float n1 = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int c = lane + 32 * q;
+            if (c < z_row(R)) {  // (x is zero past R)
+                const long long f = e < 2047 ? fix47(x[q], e) : 0ll;
+                reinterpret_cast<long long*>(b.xi)[j * z_row(R) + c] = f;
+                n1 += (float)((int)(llabs(f) >> 24) + 1) * 0x1p-23f;
+            }
+        }
+        n1 = warp_sum(n1);
+        if (lane == 0) {
+            b.ex[j] = e;
+            b.n1[j] = 1.001f * n1;
+            b.node[j] = 0;
+            b.lh[j] = make_double2(0.0, 1.0);
+            b.pick[j] = -1;
+            if (KIND == 0) b.redo[j] = 0;
+            if (KIND == 0 && j == 0) *b.redo_count = 0;
+            if (j == 0) {
+                b.off[0][0] = 0;
+                b.off[0][1] = J;
+            }
+        }
+    }
+}
+
+// The eigen tree's leaves: the leaf's index (F = 1).
+__global__ void zq_leaf1_kernel(TreeShape t, int64_t J, ZState b, int N, int col, uint32_t* __restrict__ samples) {
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < J; j += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t v = tree_leaf_idx(t, b.node[j]);
+        samples[j * N + col] = (uint32_t)v;
+        b.v[j] = (int32_t)v;
+    }
+}
+
+// Weight = R / (J h^T Phi h): the depth-first kernel's quadratic form, a group
+// of warps per sample.
+__global__ void zq_weight_kernel(int R, int Gw, int S, int64_t J, const double* __restrict__ hs,
+                                 const double* __restrict__ PhiP, double* __restrict__ weights) {
+    extern __shared__ __align__(16) unsigned char z_wdyn[];
+    double *h, *unused, *q;
+    int gi;
+    const SampleGroup<double> grp = sample_group<double>(z_wdyn, R, Gw, h, unused, q, gi);
+    for (int64_t i = (int64_t)blockIdx.x * S + gi; i < J; i += (int64_t)gridDim.x * S) {
+        for (int r = grp.tg; r < R; r += grp.nthreads()) h[r] = hs[i * R + r];
+        grp.sync();
+        grp.build_z(R, h);
+        const double hq = grp.quad(packed_size(R), PhiP);
+        if (grp.tg == 0) weights[i] = hq > 0.0 ? (double)R / (hq * (double)J) : 0.0;
+        grp.sync();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Host side
+// ---------------------------------------------------------------------------
+
+// A level of the breadth-first form is two launches whatever J (about 8 us),
+// and the marked samples' pass takes the latency of one depth-first draw; the
+// depth-first kernel takes J R (R + 1) / 2 FMAs per level over the whole chip.
+// 2^22 of them is the size from which the breadth-first form was no slower.
+bool sts_zq_wanted(int R, int64_t J) { return J * (int64_t)packed_size(R) >= (1ll << 22); }
+
+void zq_carve(Arena& a, ZState& b, int R, int64_t J, int64_t widest, int trees) {
+    b.xi = a.take<int64_t>(J * z_row(R));
+    b.lh = a.take<double2>(J);
+    b.rinv = a.take<double>(J);
+    b.err = a.take<float2>(J);
+    b.e0 = a.take<float>(J);
+    b.n1 = a.take<float>(J);
+    b.ex = a.take<int32_t>(J);
+    b.node = a.take<int64_t>(J);
+    b.order[0] = a.take<int32_t>(J);
+    b.order[1] = a.take<int32_t>(J);
+    b.v = a.take<int32_t>(J);
+    b.pick = a.take<int32_t>(J);
+    b.redo = a.take<int32_t>(J);
+    b.redo_list = a.take<int32_t>(J);
+    b.redo_count = a.take<int32_t>(1);
+    b.mask = a.take<uint32_t>(4 * ceil_div(J, kZTile));
+    b.tcount = a.take<int32_t>(ceil_div(J, kZTile) + 4);
+    b.pref64 = a.take<int64_t>(ceil_div(J, kZTile) + 1);
+    b.off[0] = a.take<int64_t>(2 * widest + 2);
+    b.off[1] = a.take<int64_t>(2 * widest + 2);
+    b.tree_exp = a.take<int32_t>(trees);
+}
+
+static unsigned z_grid(int64_t work) {
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(work, 256), 152 * 16));
+}
+
+template <int MODE, int NT>
+static int z_level(Session& s, const TreeShape& t, const double* G, const int32_t* ex, int64_t J, const int32_t* order,
+                   const double* dv, cudaStream_t st) {
+    const size_t smem = z_smem(s.R, kZa);
+    EXAFAC_CUDA_TRY(cudaFuncSetAttribute(zq_level_kernel<MODE, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem));
+    const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(J, kZTile), NT == 256 ? 304 : 152);
+    zq_level_kernel<MODE, NT><<<blocks, NT, smem, st>>>(s.R, t, G, ex, J, s.zq, order, dv, s.status,
+                                                        s.wait_polls ? s.wait_polls : kSpinLimit);
+    count_launch();
+    return EXAFAC_OK;
+}
+template <int MODE>
+static int z_level_any(Session& s, const TreeShape& t, const double* G, const int32_t* ex, int64_t J,
+                       const int32_t* order, const double* dv, cudaStream_t st) {
+    return s.R <= 64 ? z_level<MODE, 256>(s, t, G, ex, J, order, dv, st)
+                     : z_level<MODE, 512>(s, t, G, ex, J, order, dv, st);
+}
+
+// One descent of every sample; the vectors and the root state are in place.
+static int z_descend(Session& s, const TreeShape& t, const double* G, const double* U, const double* dv, int64_t J,
+                     int col, int tree, cudaStream_t st) {
+    ZState& b = s.zq;
+    const int R = s.R;
+    int32_t* ex = b.tree_exp + tree;
+    zq_tree_exp_kernel<<<1, 32, 0, st>>>(R, G, ex);
+    count_launch();
+    EXAFAC_TRY(z_level_any<0>(s, t, G, ex, J, nullptr, dv, st));
+    const int64_t ntiles = ceil_div(J, kZTile);
+    const bool in_smem = ntiles <= kZPrefSmem;
+    const size_t psm = in_smem ? sizeof(int32_t) * (ntiles + 1) : 0;
+    if (psm > 48 * 1024)
+        EXAFAC_CUDA_TRY(
+            cudaFuncSetAttribute(zq_partition_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
+    const bool tail = t.node_count > t.nodes_upto_lfill;
+    const int32_t* order = nullptr;
+    int oi = 0, cur = 0;
+    int64_t lb = 0, nl = 1;
+    for (int64_t lvl = 0; lvl <= t.lfill_level; lvl++) {
+        const bool is_tail = lvl == t.lfill_level;
+        if (is_tail && !tail) break;
+        if (is_tail) EXAFAC_TRY(z_level_any<2>(s, t, G, ex, J, order, dv, st));
+        else EXAFAC_TRY(z_level_any<1>(s, t, G, ex, J, order, dv, st));
+        if (is_tail && t.F <= 1) break;  // the leaf index needs no order
+        if (!in_smem)
+            EXAFAC_TRY(scan_exclusive_u32_to_i64(reinterpret_cast<const uint32_t*>(b.tcount), b.pref64, ntiles,
+                                                 b.pref64 + ntiles, s.scan_sc, st));
+        zq_partition_kernel<<<(unsigned)std::min<int64_t>(ceil_div(J, 512), 152 * 2), 512, psm, st>>>(
+            J, (int)ntiles, b.mask, b.tcount, in_smem ? nullptr : b.pref64, lb, nl, order, b.node, b.off[oi],
+            b.order[cur], is_tail ? nullptr : b.off[oi ^ 1]);
+        count_launch();
+        order = b.order[cur];
+        cur ^= 1;
+        oi ^= 1;
+        lb = 2 * lb + 1;
+        nl *= 2;
+    }
+    if (t.F <= 1) {
+        zq_leaf1_kernel<<<z_grid(J), 256, 0, st>>>(t, J, b, s.N, col, s.samples);
+    } else {
+        const size_t smem = z_smem(R, kZu);
+        const uint32_t polls = s.wait_polls ? s.wait_polls : kSpinLimit;
+        const int64_t tiles = ceil_div(J, kZTile);
+        if (R <= 64) {
+            EXAFAC_CUDA_TRY(cudaFuncSetAttribute(zq_leaf_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)smem));
+            zq_leaf_kernel<256><<<(unsigned)std::min<int64_t>(tiles, 304), 256, smem, st>>>(
+                R, t, G, U, J, b, order, dv, s.N, col, s.samples, s.status, polls);
+        } else {
+            EXAFAC_CUDA_TRY(cudaFuncSetAttribute(zq_leaf_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)smem));
+            zq_leaf_kernel<512><<<(unsigned)std::min<int64_t>(tiles, 152), 512, smem, st>>>(
+                R, t, G, U, J, b, order, dv, s.N, col, s.samples, s.status, polls);
+        }
+    }
+    count_launch();
+    EXAFAC_CHECK_LAUNCH();
+    return EXAFAC_OK;
+}
+
+int sts_draw_zq(Session& s, int n, int64_t J, const double* uni, cudaStream_t st) {
+    const int N = s.N, R = s.R, P = s.P;
+    ZState& b = s.zq;
+    double* h = s.D;  // J x R; the design rows are formed after the draw
+    const unsigned vgrid = z_grid(J * 32);
+    zq_vector_kernel<0><<<vgrid, 256, 0, st>>>(R, J, h, nullptr, nullptr, N, 0, 0, b, s.status);
+    count_launch();
+    for (int k = 0; k < N; k++) {
+        if (k == n) continue;
+        int nx = k + 1;
+        if (nx == n) nx++;
+        if (nx > N) nx = N;
+        // eigen tree of mode k, driven by h: v, then x = h * E_next[v]
+        EXAFAC_TRY(z_descend(s, s.etree, s.eigG + (int64_t)k * s.etree.node_count * P, nullptr,
+                             uni + ((int64_t)k * 2 + 0) * J, J, n, 2 * k, st));
+        zq_vector_kernel<1><<<vgrid, 256, 0, st>>>(R, J, h, s.Emat + (int64_t)nx * R * R, s.samples, N, n, R, b,
+                                                   s.status);
+        count_launch();
+        // row tree of mode k, driven by x: the row, then h *= U_k[row]
+        EXAFAC_TRY(z_descend(s, s.rtree[k], s.treeG[k], s.F.U[k], uni + ((int64_t)k * 2 + 1) * J, J, k, 2 * k + 1, st));
+        zq_vector_kernel<2><<<vgrid, 256, 0, st>>>(R, J, h, s.F.U[k], s.samples, N, k, s.dims[k], b, s.status);
+        count_launch();
+    }
+    int Gw, S;
+    sample_group_shape(R, sizeof(double), Gw, S);
+    const size_t smem = (size_t)S * sample_group_bytes(R, sizeof(double));
+    if (smem > 48 * 1024)
+        EXAFAC_CUDA_TRY(cudaFuncSetAttribute(zq_weight_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int64_t blocks = std::max<int64_t>(std::min<int64_t>(ceil_div(J, S), 152 * 32), 1);
+    zq_weight_kernel<<<(unsigned)blocks, S * Gw * 32, smem, st>>>(R, Gw, S, J, h, s.PhiP, s.weights);
+    count_launch();
+    EXAFAC_CHECK_LAUNCH();
+    return EXAFAC_OK;
+}
+
+}  // namespace exafac
