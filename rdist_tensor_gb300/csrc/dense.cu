@@ -4,6 +4,8 @@
 // sts_cp.hpp:110-176) of the reference.
 #include "dense.cuh"
 
+#include <utility>
+
 namespace exafac {
 
 // Round-robin ("circle") pairing of Re = even(R) indices: in round t, pair 0
@@ -24,16 +26,13 @@ __device__ __forceinline__ void rr_pair(int t, int i, int m, int& p, int& q) {
     }
 }
 
-// Jacobi on the symmetric matrix whose upper triangle is A (row-major R x R).
+// Cyclic Jacobi on the symmetric matrix whose upper triangle is A (row-major
+// R x R): jacobi_init, then jacobi_sweeps.
 // Shared: a[Re*Re] (the working matrix), rot[Re/2] cosines and sines.
 // vt (global, Re*Re) holds V^T: vt[i*Re + r] = component r of eigenvector i.
-__device__ void jacobi_block(int R, const double* __restrict__ A, double* a, double* vt, double* rc, double* rs,
-                             int* flag) {
+__device__ void jacobi_init(int R, const double* __restrict__ A, double* a, double* vt) {
     const int Re = R + (R & 1);
-    const int m = Re - 1;
-    const int npairs = Re / 2;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    for (int e = tid; e < Re * Re; e += nt) {
+    for (int e = threadIdx.x; e < Re * Re; e += blockDim.x) {
         int i = e / Re, j = e % Re;
         double v = 0.0;
         if (i < R && j < R) v = (i <= j) ? A[i * R + j] : A[j * R + i];
@@ -41,10 +40,34 @@ __device__ void jacobi_block(int R, const double* __restrict__ A, double* a, dou
         vt[e] = (i == j && i < R) ? 1.0 : 0.0;
     }
     __syncthreads();
+}
+
+// Rotate unless a_pq is negligible relative to the diagonal (Demmel-Veselic
+// criterion, tol = R * eps).
+__device__ __forceinline__ bool jacobi_rotates(int R, double apq, double app, double aqq) {
+    return apq != 0.0 && fabs(apq) > (double)R * 2.220446049250313e-16 * sqrt(fabs(app * aqq));
+}
+
+// Sweeps until no pair rotates.  A sweep starts by looking at every pair at
+// once, so a matrix that is already diagonal (the end of every call, and the
+// usual start after syev_refine) costs one pass instead of Re - 1 rounds.
+__device__ void jacobi_sweeps(int R, double* a, double* vt, double* rc, double* rs, int* flag) {
+    const int Re = R + (R & 1);
+    const int m = Re - 1;
+    const int npairs = Re / 2;
+    const int tid = threadIdx.x, nt = blockDim.x;
     if (R == 1) return;
     for (int sweep = 0; sweep < 60; sweep++) {
         if (tid == 0) *flag = 0;
         __syncthreads();
+        bool any = false;
+        for (int e = tid; e < R * R && !any; e += nt) {
+            const int i = e / R, j = e % R;
+            any = i < j && jacobi_rotates(R, a[i * Re + j], a[i * Re + i], a[j * Re + j]);
+        }
+        if (any) *flag = 1;
+        __syncthreads();
+        if (*flag == 0) break;
         for (int t = 0; t < m; t++) {
             // Rotation angles (Golub & Van Loan, sym.schur2).
             for (int i = tid; i < npairs; i += nt) {
@@ -54,9 +77,7 @@ __device__ void jacobi_block(int R, const double* __restrict__ A, double* a, dou
                 if (q < R) {
                     double apq = a[p * Re + q];
                     double app = a[p * Re + p], aqq = a[q * Re + q];
-                    // Rotate unless a_pq is negligible relative to the
-                    // diagonal (Demmel-Veselic criterion, tol = R * eps).
-                    if (apq != 0.0 && fabs(apq) > (double)R * 2.220446049250313e-16 * sqrt(fabs(app * aqq))) {
+                    if (jacobi_rotates(R, apq, app, aqq)) {
                         double tau = (aqq - app) / (2.0 * apq);
                         double tt;
                         if (fabs(tau) > 1e150) {
@@ -66,7 +87,6 @@ __device__ void jacobi_block(int R, const double* __restrict__ A, double* a, dou
                         }
                         c = 1.0 / sqrt(1.0 + tt * tt);
                         s = tt * c;
-                        *flag = 1;
                     }
                 }
                 rc[i] = c;
@@ -103,8 +123,6 @@ __device__ void jacobi_block(int R, const double* __restrict__ A, double* a, dou
             }
             __syncthreads();
         }
-        if (*flag == 0) break;
-        __syncthreads();
     }
 }
 
@@ -130,31 +148,39 @@ __device__ void ascending_ranks(int R, const double* a, int Re, int* rank) {
 // Outputs (any may be null):
 //   V[u*R + v]    eigenvector v (ascending eigenvalues), lam[v]
 //   pinv          sum over lam_v > tol of v v^T / lam_v  (full symmetric)
-__device__ void syev_block(int R, const double* __restrict__ A, double* V, double* lam, double* pinv, double tol,
-                           double* vt, double* smem) {
+struct SyevSmem {
+    double *a, *rc, *rs;
+    int *rank, *order, *flag;
+};
+__device__ __forceinline__ SyevSmem syev_smem(int R, double* smem) {
     const int Re = R + (R & 1);
-    double* a = smem;
-    double* rc = a + Re * Re;
-    double* rs = rc + Re / 2 + 1;
-    int* rank = reinterpret_cast<int*>(rs + Re / 2 + 1);
-    int* order = rank + Re;
-    int* flag = order + Re;
-    const int b = 0;
-    const int64_t v_stride = 0;
-    jacobi_block(R, A, a, vt, rc, rs, flag);
+    SyevSmem m;
+    m.a = smem;
+    m.rc = m.a + Re * Re;
+    m.rs = m.rc + Re / 2 + 1;
+    m.rank = reinterpret_cast<int*>(m.rs + Re / 2 + 1);
+    m.order = m.rank + Re;
+    m.flag = m.order + Re;
+    return m;
+}
+
+// The outputs from the diagonalised m.a and the rows of vt.
+__device__ void syev_outputs(int R, const SyevSmem& m, const double* vt, double* V, double* lam, double* pinv,
+                             double tol) {
+    const int Re = R + (R & 1);
     __syncthreads();
-    ascending_ranks(R, a, Re, rank);
+    ascending_ranks(R, m.a, Re, m.rank);
     __syncthreads();
-    for (int i = threadIdx.x; i < R; i += blockDim.x) order[rank[i]] = i;
+    for (int i = threadIdx.x; i < R; i += blockDim.x) m.order[m.rank[i]] = i;
     __syncthreads();
     if (V) {
         for (int e = threadIdx.x; e < R * R; e += blockDim.x) {
             int i = e / R, u = e % R;  // eigenvector i (original slot), component u
-            V[b * v_stride + u * R + rank[i]] = vt[i * Re + u];
+            V[u * R + m.rank[i]] = vt[i * Re + u];
         }
     }
     if (lam) {
-        for (int i = threadIdx.x; i < R; i += blockDim.x) lam[b * R + rank[i]] = a[i * Re + i];
+        for (int i = threadIdx.x; i < R; i += blockDim.x) lam[m.rank[i]] = m.a[i * Re + i];
     }
     if (pinv) {
         // Sum over eigen-pairs in ascending eigenvalue order, as
@@ -163,16 +189,24 @@ __device__ void syev_block(int R, const double* __restrict__ A, double* V, doubl
             int r1 = e / R, r2 = e % R;
             double acc = 0.0;
             for (int k = 0; k < R; k++) {
-                int i = order[k];
-                double l = a[i * Re + i];
+                int i = m.order[k];
+                double l = m.a[i * Re + i];
                 if (l > tol) {
                     double s = 1.0 / sqrt(l);
                     acc += (vt[i * Re + r1] * s) * (vt[i * Re + r2] * s);
                 }
             }
-            pinv[b * (int64_t)R * R + e] = acc;
+            pinv[e] = acc;
         }
     }
+}
+
+__device__ void syev_block(int R, const double* __restrict__ A, double* V, double* lam, double* pinv, double tol,
+                           double* vt, double* smem) {
+    const SyevSmem m = syev_smem(R, smem);
+    jacobi_init(R, A, m.a, vt);
+    jacobi_sweeps(R, m.a, vt, m.rc, m.rs, m.flag);
+    syev_outputs(R, m, vt, V, lam, pinv, tol);
 }
 
 // One CTA per matrix (matrix b at A + b * a_stride).
@@ -183,6 +217,355 @@ __global__ void syev_kernel(int R, const double* __restrict__ A, int64_t a_strid
     const int b = blockIdx.x;
     syev_block(R, A + b * a_stride, V ? V + b * v_stride : nullptr, lam ? lam + (int64_t)b * R : nullptr,
                pinv ? pinv + (int64_t)b * R * R : nullptr, tol, vt_scratch + (int64_t)b * Re * Re, smem);
+}
+
+// ---------------------------------------------------------------------------
+// Eigendecomposition of the FP64 form's sampling matrices: an FP32 Jacobi
+// start, refined in FP64.
+//
+// The FP64 Jacobi takes ~10 sweeps of ~6 R^3 FP64 operations on one SM (GB300
+// retires ~1.7 of them per clock per SM): 0.87 / 5.2 / 19 ms a call at R = 25 /
+// 64 / 100, which was 15 to 52 % of an FP64 STS-CP sweep.  Here
+//   1. jacobi32_kernel: the sweeps in FP32 (shared memory, one CTA a matrix);
+//   2. kRefineSteps refinement steps of the eigenvector matrix X in FP64
+//      (Ogita and Aishima, "Iterative refinement for symmetric eigenvalue
+//      decomposition", 2018): with S = X^T A X, G = X^T X, r = I - G,
+//      lambda_i = S_ii / G_ii, X <- X + X E, E_ij = (S_ij + lambda_j r_ij) /
+//      (lambda_j - lambda_i), or r_ij / 2 on the diagonal and where the
+//      quotient is no small rotation (equal eigenvalues).  S is taken
+//      symmetric (its upper triangle), which keeps E_ij + E_ji = r_ij to
+//      rounding and so X orthonormal.  The error squares per step; the
+//      products run on R blocks.  Where a quotient is no small rotation in
+//      the first step (eigenvalues closer than FP32 resolves beside the
+//      largest), that step is a second FP32 Jacobi, on S less those pairs'
+//      mean eigenvalue, whose block FP64 has resolved by then: E = V - I;
+//   3. syev_finish_kernel: the FP64 Jacobi sweeps on S with X as the start,
+//      so the result meets the same convergence criterion whatever the steps
+//      left (a cluster, eigenvalues below FP32's resolution), then the sorted
+//      outputs.  X that is not orthonormal to 4 R eps, or a value that is not
+//      finite, starts the sweeps from A as before.
+// Measured (GB300, a batch of 3, launches included): R = 25 / 64 / 100 / 128:
+// 0.24 / 0.69 / 2.2 / 2.9 ms (the FP64 sweeps alone 0.88 / 5.2 / 17.6 / 35.9),
+// |A v - lambda v| <= 6e-16 |A| against 5e-15 .. 3e-14, a 92-fold near-null
+// cluster at R = 100 11 against 26 ms.
+// ---------------------------------------------------------------------------
+constexpr int kRefineSteps = 4;
+constexpr int kJacobi32MaxSweeps = 10;
+
+// Cyclic Jacobi in FP32 on the full symmetric matrix a (Re x Re, shared), v
+// (Re x Re, shared) <- V^T (row i = eigenvector i).  A pair rotates while
+// |a_pq| > max(2^-22 sqrt|a_pp a_qq|, floor).  A round's rotations act on
+// disjoint pairs, so the two-sided update is independent 2 x 2 blocks.
+struct Jacobi32Smem {
+    float2 cs[kMaxRank / 2];
+    int2 pq[kMaxRank / 2];
+    int flag;
+};
+__device__ __forceinline__ bool jacobi32_rotates(float apq, float app, float aqq, float floor) {
+    return fabsf(apq) > fmaxf(0x1p-22f * sqrtf(fabsf(app) * fabsf(aqq)), floor);
+}
+__device__ void jacobi32_block(int R, float* a, float* v, float floor, Jacobi32Smem* sm) {
+    const int Re = R + (R & 1), m = Re - 1, np = Re / 2, ld = Re;
+    const int tid = threadIdx.x, nt = blockDim.x;
+    for (int e = tid; e < Re * Re; e += nt) v[e] = e / Re == e % Re ? 1.0f : 0.0f;
+    __syncthreads();
+    for (int sweep = 0; sweep < kJacobi32MaxSweeps && R > 1; sweep++) {
+        if (tid == 0) sm->flag = 0;
+        __syncthreads();
+        bool any = false;  // a look at every pair: a converged matrix ends here
+        for (int i = tid >> 5; i < R && !any; i += nt >> 5)
+            for (int j = i + 1 + (tid & 31); j < R; j += 32)
+                any = any || jacobi32_rotates(a[i * ld + j], a[i * ld + i], a[j * ld + j], floor);
+        if (any) sm->flag = 1;
+        __syncthreads();
+        if (!sm->flag) break;
+        for (int t = 0; t < m; t++) {
+            if (tid < np) {
+                int p, q;
+                rr_pair(t, tid, m, p, q);
+                float c = 1.0f, s = 0.0f;
+                const float apq = a[p * ld + q], app = a[p * ld + p], aqq = a[q * ld + q];
+                if (q < R && jacobi32_rotates(apq, app, aqq, floor)) {
+                    const float tau = (aqq - app) / (2.0f * apq);
+                    const float tt = copysignf(1.0f, tau) / (fabsf(tau) + sqrtf(fmaf(tau, tau, 1.0f)));
+                    c = rsqrtf(fmaf(tt, tt, 1.0f));
+                    s = tt * c;
+                }
+                sm->cs[tid] = make_float2(c, s);
+                sm->pq[tid] = make_int2(p, q);
+            }
+            __syncthreads();
+            // the 2 x 2 blocks J_i^T a_ij J_j, and the rows of V^T: a warp per
+            // pair i, its lanes along j and along the row
+            for (int i = tid >> 5; i < np; i += nt >> 5) {
+                const float2 ri = sm->cs[i];
+                const int2 pi = sm->pq[i];
+                float* rp = a + pi.x * ld;
+                float* rq = a + pi.y * ld;
+                for (int j = tid & 31; j < np; j += 32) {
+                    const float2 rj = sm->cs[j];
+                    if (ri.y == 0.0f && rj.y == 0.0f) continue;
+                    const int2 pj = sm->pq[j];
+                    const float pp = rp[pj.x], pqv = rp[pj.y], qp = rq[pj.x], qq = rq[pj.y];
+                    const float l0 = ri.x * pp - ri.y * qp, l1 = ri.x * pqv - ri.y * qq;
+                    const float m0 = ri.y * pp + ri.x * qp, m1 = ri.y * pqv + ri.x * qq;
+                    rp[pj.x] = rj.x * l0 - rj.y * l1;
+                    rp[pj.y] = rj.y * l0 + rj.x * l1;
+                    rq[pj.x] = rj.x * m0 - rj.y * m1;
+                    rq[pj.y] = rj.y * m0 + rj.x * m1;
+                }
+                if (ri.y == 0.0f) continue;
+                float* vp = v + pi.x * ld;
+                float* vq = v + pi.y * ld;
+                for (int r = tid & 31; r < Re; r += 32) {
+                    const float x = vp[r], y = vq[r];
+                    vp[r] = ri.x * x - ri.y * y;
+                    vq[r] = ri.y * x + ri.x * y;
+                }
+            }
+            __syncthreads();
+        }
+        __syncthreads();  // flag is read by everyone before the next sweep clears it
+    }
+    __syncthreads();
+}
+
+// The power of two that brings mx into [1, 2); 0 when there is none to speak of.
+__device__ __forceinline__ double scale_of(double mx) {
+    const int ex = ((__double2hiint(mx) >> 20) & 0x7ff) - 1023;
+    return (mx > 0.0 && isfinite(mx) && ex > -1000) ? scalbn(1.0, -ex) : 0.0;
+}
+__device__ double block_sum(double x, double* red) {  // red: 32 doubles, added in warp order
+    __syncthreads();
+    x = warp_sum(x);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = x;
+    __syncthreads();
+    x = 0.0;
+    for (int q = 0; q < (int)(blockDim.x >> 5); q++) x += red[q];
+    return x;
+}
+__device__ double block_max(double mx, double* red) {
+    __syncthreads();
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    mx = 0.0;
+    for (int q = 0; q < (int)(blockDim.x >> 5); q++) mx = fmax(mx, red[q]);
+    return mx;
+}
+
+__global__ void __launch_bounds__(512) jacobi32_kernel(int R, const double* __restrict__ A, int64_t a_stride,
+                                                       double* __restrict__ X, double* __restrict__ As,
+                                                       int64_t scratch_stride) {
+    extern __shared__ float j32[];
+    __shared__ Jacobi32Smem sm;
+    __shared__ double red[32];
+    const int Re = R + (R & 1);
+    const int tid = threadIdx.x, nt = blockDim.x;
+    float* a = j32;
+    float* v = a + Re * Re;
+    A += blockIdx.x * a_stride;
+    X += blockIdx.x * scratch_stride;
+    As += blockIdx.x * scratch_stride;
+    // less the mean eigenvalue: a cluster near it keeps FP32's resolution
+    double tr = 0.0;
+    for (int i = 0; i < R; i++) tr += A[i * R + i];
+    const double mu = tr / R;
+    double mx = 0.0;
+    for (int e = tid; e < R * R; e += nt) {
+        const int i = e / R, j = e % R;
+        const double x = i <= j ? A[i * R + j] : A[j * R + i];
+        As[e] = x;
+        mx = fmax(mx, fabs(i == j ? x - mu : x));
+    }
+    const double sc = scale_of(block_max(mx, red));
+    for (int e = tid; e < Re * Re; e += nt) {
+        const int i = e / Re, j = e % Re;
+        double x = 0.0;
+        if (i < R && j < R) x = (i <= j ? A[i * R + j] : A[j * R + i]) - (i == j ? mu : 0.0);
+        a[e] = (float)(x * sc);
+    }
+    __syncthreads();
+    jacobi32_block(R, a, v, 0x1p-22f, &sm);
+    for (int e = tid; e < R * R; e += nt) X[e] = (double)v[(e % R) * Re + e / R];  // column j = eigenvector j
+}
+
+// Sum of x[k] y[k * stride], four chains (a dependent FP64 add takes ~64 cycles).
+__device__ __forceinline__ double dot4(const double* x, const double* __restrict__ y, int stride, int n) {
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    int k = 0;
+    for (; k + 3 < n; k += 4) {
+        s0 = fma(x[k], y[(int64_t)k * stride], s0);
+        s1 = fma(x[k + 1], y[(int64_t)(k + 1) * stride], s1);
+        s2 = fma(x[k + 2], y[(int64_t)(k + 2) * stride], s2);
+        s3 = fma(x[k + 3], y[(int64_t)(k + 3) * stride], s3);
+    }
+    for (; k < n; k++) s0 = fma(x[k], y[(int64_t)k * stride], s0);
+    return (s0 + s1) + (s2 + s3);
+}
+
+// Row i (blockIdx.x) of S = X^T A X and G = X^T X of matrix blockIdx.y.
+__global__ void __launch_bounds__(128) refine_forms_kernel(int R, const double* __restrict__ As,
+                                                           const double* __restrict__ X, double* __restrict__ S,
+                                                           double* __restrict__ G, int64_t scratch_stride) {
+    __shared__ double xi[kMaxRank], ti[kMaxRank];
+    pdl_wait();
+    pdl_trigger();
+    const int i = blockIdx.x, j = threadIdx.x;
+    const int64_t o = (int64_t)blockIdx.y * scratch_stride;
+    if (j < R) xi[j] = X[o + (int64_t)j * R + i];
+    __syncthreads();
+    if (j < R) ti[j] = dot4(xi, As + o + j, R, R);
+    __syncthreads();
+    if (j < R) {
+        S[o + (int64_t)i * R + j] = dot4(ti, X + o + j, R, R);
+        G[o + (int64_t)i * R + j] = dot4(xi, X + o + j, R, R);
+    }
+}
+
+// (S_ij + lambda_j r_ij, lambda_j - lambda_i) of the upper triangle's S, and
+// the larger numerator of (i, j) and (j, i), so that both take the same branch.
+__device__ __forceinline__ double3 refine_quotient(int R, const double* S, const double* G, int i, int j) {
+    const double li = S[i * R + i] / G[i * R + i], lj = S[j * R + j] / G[j * R + j];
+    const double sij = i <= j ? S[i * R + j] : S[j * R + i];
+    const double g = G[i * R + j];
+    return make_double3(sij - lj * g, lj - li, fmax(fabs(sij - lj * g), fabs(sij - li * g)));
+}
+// A quotient that is a small rotation, and one that says something: between
+// close eigenvalues (lmax: the largest) a numerator at the rounding of S
+// would turn X by noise / gap in every step, whose square X's orthonormality
+// loses again; those pairs are left to the Jacobi sweeps.
+__device__ __forceinline__ bool small_rotation(double3 q, double lmax) {
+    return q.z < 0x1p-5 * fabs(q.y) && (q.z > 0x1p-48 * lmax || fabs(q.y) > 0x1p-23 * lmax);
+}
+
+__global__ void __launch_bounds__(128) refine_e_kernel(int R, const double* __restrict__ S,
+                                                       const double* __restrict__ G, double* __restrict__ E,
+                                                       int64_t scratch_stride) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ double red[32];
+    const int i = blockIdx.x, j = threadIdx.x;
+    const int64_t o = (int64_t)blockIdx.y * scratch_stride;
+    const double lmax = block_max(j < R ? fabs(S[o + j * R + j]) : 0.0, red);
+    if (j >= R) return;
+    double e = 0.5 * ((i == j ? 1.0 : 0.0) - G[o + i * R + j]);
+    if (i != j) {
+        const double3 q = refine_quotient(R, S + o, G + o, i, j);
+        if (small_rotation(q, lmax)) e = q.x / q.y;
+    }
+    E[o + i * R + j] = e;
+}
+
+// The first step's E, a CTA per matrix.
+__global__ void __launch_bounds__(512) refine_first_kernel(int R, const double* __restrict__ S,
+                                                           const double* __restrict__ G, double* __restrict__ E,
+                                                           int64_t scratch_stride) {
+    extern __shared__ float j32[];
+    __shared__ Jacobi32Smem sm;
+    __shared__ double red[32];
+    __shared__ int second;
+    pdl_wait();
+    const int Re = R + (R & 1);
+    const int tid = threadIdx.x, nt = blockDim.x;
+    S += blockIdx.x * scratch_stride;
+    G += blockIdx.x * scratch_stride;
+    E += blockIdx.x * scratch_stride;
+    if (tid == 0) second = 0;
+    __syncthreads();
+    // the pairs whose rotation is not small: how many, their mean eigenvalue
+    // and the spread among them
+    const double lmax = block_max(tid < R ? fabs(S[tid * R + tid]) : 0.0, red);
+    double cnt = 0.0, mean = 0.0, spread = 0.0;
+    for (int e = tid; e < R * R; e += nt) {
+        const int i = e / R, j = e % R;
+        double v = 0.5 * ((i == j ? 1.0 : 0.0) - G[e]);
+        if (i != j) {
+            const double3 q = refine_quotient(R, S, G, i, j);
+            if (small_rotation(q, lmax)) {
+                v = q.x / q.y;
+            } else if (i < j && jacobi_rotates(R, S[e], S[i * R + i], S[j * R + j])) {
+                cnt += 1.0;
+                mean += 0.5 * (S[i * R + i] + S[j * R + j]);
+                spread = fmax(spread, fmax(fabs(q.y), fabs(S[e])));
+            }
+        }
+        E[e] = v;
+    }
+    if (cnt > 0.0) second = 1;
+    __syncthreads();
+    if (!second) return;
+    cnt = block_sum(cnt, red);
+    mean = block_sum(mean, red) / cnt;
+    spread = block_max(spread, red);
+    double mx = 0.0;
+    for (int e = tid; e < R * R; e += nt) {
+        const int i = e / R, j = e % R;
+        mx = fmax(mx, fabs(i == j ? S[e] - mean : S[i <= j ? e : j * R + i]));
+    }
+    const double sc = scale_of(block_max(mx, red));
+    if (sc == 0.0) return;
+    float* a = j32;
+    float* v = a + Re * Re;
+    for (int e = tid; e < Re * Re; e += nt) {
+        const int i = e / Re, j = e % Re;
+        double x = 0.0;
+        if (i < R && j < R) x = (i <= j ? S[i * R + j] : S[j * R + i]) - (i == j ? mean : 0.0);
+        a[e] = (float)(x * sc);
+    }
+    __syncthreads();
+    jacobi32_block(R, a, v, (float)(0x1p-22 * spread * sc), &sm);
+    for (int e = tid; e < R * R; e += nt) {
+        const int i = e / R, j = e % R;
+        E[e] = (double)v[j * Re + i] - (i == j ? 1.0 : 0.0);
+    }
+}
+
+// Row c (blockIdx.x) of X + X E.
+__global__ void __launch_bounds__(128) refine_update_kernel(int R, const double* __restrict__ X,
+                                                            const double* __restrict__ E, double* __restrict__ Xn,
+                                                            int64_t scratch_stride) {
+    __shared__ double xr[kMaxRank];
+    pdl_wait();
+    pdl_trigger();
+    const int c = blockIdx.x, j = threadIdx.x;
+    const int64_t o = (int64_t)blockIdx.y * scratch_stride;
+    if (j < R) xr[j] = X[o + (int64_t)c * R + j];
+    __syncthreads();
+    if (j < R) Xn[o + (int64_t)c * R + j] = xr[j] + dot4(xr, E + o + j, R, R);
+}
+
+__global__ void __launch_bounds__(512) syev_finish_kernel(int R, const double* __restrict__ A, int64_t a_stride,
+                                                          const double* __restrict__ X, const double* __restrict__ S,
+                                                          const double* __restrict__ G, int64_t scratch_stride,
+                                                          double* V, double* lam, int64_t v_stride, double* vt) {
+    extern __shared__ double smem[];
+    __shared__ int bad;
+    pdl_wait();
+    const int Re = R + (R & 1);
+    const int64_t b = blockIdx.x, o = b * scratch_stride;
+    const SyevSmem m = syev_smem(R, smem);
+    vt += b * Re * Re;
+    if (threadIdx.x == 0) bad = 0;
+    __syncthreads();
+    for (int e = threadIdx.x; e < Re * Re; e += blockDim.x) {
+        const int i = e / Re, j = e % Re;
+        double s = 0.0, x = 0.0;
+        if (i < R && j < R) {
+            s = S[o + (i <= j ? i * R + j : j * R + i)];
+            x = X[o + (int64_t)j * R + i];
+            if (!isfinite(s) || !(fabs(G[o + i * R + j] - (i == j ? 1.0 : 0.0)) < 4.0 * R * 2.220446049250313e-16))
+                bad = 1;
+        }
+        m.a[e] = s;
+        vt[i * Re + j] = x;  // row i = eigenvector i
+    }
+    __syncthreads();
+    const bool restart = bad != 0;
+    __syncthreads();
+    if (restart) jacobi_init(R, A + b * a_stride, m.a, vt);
+    jacobi_sweeps(R, m.a, vt, m.rc, m.rs, m.flag);
+    syev_outputs(R, m, vt, V + b * v_stride, lam + b * R, nullptr, 0.0);
 }
 
 // Symmetric pseudo-inverse, fast path: Cholesky A = L L^T, L^{-1} by
@@ -797,6 +1180,53 @@ int launch_syev(int R, const double* A, int64_t a_stride, int batch, double* V, 
     }
     int threads = R <= 32 ? 256 : 512;
     syev_kernel<<<batch, threads, smem, stream>>>(R, A, a_stride, V, lam, v_stride, pinv, tol, vt_scratch); count_launch();
+    EXAFAC_CHECK_LAUNCH();
+    return EXAFAC_OK;
+}
+
+// X, its successor, A in full, S, G and E of each matrix.
+size_t syev_refine_doubles(int R, int batch) { return (size_t)batch * 6 * R * R; }
+
+int launch_syev_refined(int R, const double* A, int64_t a_stride, int batch, double* V, double* lam, int64_t v_stride,
+                        double* vt_scratch, double* scratch, cudaStream_t stream) {
+    const int Re = R + (R & 1);
+    const int64_t R2 = (int64_t)R * R, ss = 6 * R2;
+    double *X = scratch, *Xn = X + R2, *As = Xn + R2, *S = As + R2, *G = S + R2, *E = G + R2;
+    const size_t jsm = sizeof(float) * 2 * (size_t)Re * Re;
+    if (jsm > 48 * 1024) {
+        EXAFAC_CUDA_TRY(cudaFuncSetAttribute(jacobi32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jsm));
+        EXAFAC_CUDA_TRY(
+            cudaFuncSetAttribute(refine_first_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jsm));
+    }
+    jacobi32_kernel<<<batch, R <= 32 ? 256 : 512, jsm, stream>>>(R, A, a_stride, X, As, ss);
+    count_launch();
+    const dim3 grid((unsigned)R, (unsigned)batch);
+    for (int it = 0; it <= kRefineSteps; it++) {
+        EXAFAC_CUDA_TRY(launch_dependent(refine_forms_kernel, grid, 128, 0, stream, R, (const double*)As,
+                                         (const double*)X, S, G, ss));
+        count_launch();
+        if (it == kRefineSteps) break;
+        if (it == 0) {
+            EXAFAC_CUDA_TRY(launch_dependent(refine_first_kernel, (unsigned)batch, R <= 32 ? 256 : 512, jsm, stream, R,
+                                             (const double*)S, (const double*)G, E, ss));
+        } else {
+            EXAFAC_CUDA_TRY(launch_dependent(refine_e_kernel, grid, 128, 0, stream, R, (const double*)S,
+                                             (const double*)G, E, ss));
+        }
+        count_launch();
+        EXAFAC_CUDA_TRY(launch_dependent(refine_update_kernel, grid, 128, 0, stream, R, (const double*)X,
+                                         (const double*)E, Xn, ss));
+        count_launch();
+        std::swap(X, Xn);
+    }
+    const size_t smem = syev_smem_bytes(R);
+    if (smem > 48 * 1024)
+        EXAFAC_CUDA_TRY(
+            cudaFuncSetAttribute(syev_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    EXAFAC_CUDA_TRY(launch_dependent(syev_finish_kernel, (unsigned)batch, R <= 32 ? 256 : 512, smem, stream, R, A,
+                                     a_stride, (const double*)X, (const double*)S, (const double*)G, ss, V, lam,
+                                     v_stride, vt_scratch));
+    count_launch();
     EXAFAC_CHECK_LAUNCH();
     return EXAFAC_OK;
 }

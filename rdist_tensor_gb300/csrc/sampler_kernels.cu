@@ -319,7 +319,7 @@ static int narrow_nodes(const double* in, float* out, int R, int64_t nodes, cuda
 // the factor Grams over the modes != n; chain[n] is cleared.
 __global__ void sts_chain_kernel(int N, int n, int R, const double* __restrict__ gram, double* __restrict__ chain) {
     const int R2 = R * R;
-    for (int e = threadIdx.x; e < R2; e += blockDim.x) {
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < R2; e += gridDim.x * blockDim.x) {
         double last = 1.0;
         for (int k = N - 1; k >= 0; k--) {
             if (k == n) {
@@ -334,32 +334,31 @@ __global__ void sts_chain_kernel(int N, int n, int R, const double* __restrict__
 
 // computeM part 2 (sts_cp.hpp:118-153): W[:, R-1-v] = v-th eigenvector /
 // sqrt(lambda_v) (dropped at lambda_v <= 1e-8), Phi = W W^T, the rows of W^T
-// become E[N], and chain[k] *= Phi for k >= 1.
-__global__ void sts_phi_kernel(int N, int n, int R, const double* __restrict__ V0, const double* __restrict__ L0,
-                               double* __restrict__ chain, double* __restrict__ E, double* __restrict__ Phi,
-                               double* __restrict__ PhiP) {
-    extern __shared__ double W[];
-    const int R2 = R * R;
-    for (int e = threadIdx.x; e < R2; e += blockDim.x) {
-        int u = e / R, v = e % R;
-        double lam = L0[v];
-        W[u * R + (R - 1 - v)] = lam > 1e-8 ? V0[u * R + v] / sqrt(lam) : 0.0;
-    }
+// become E[N], and chain[k] *= Phi for k >= 1.  sts_w_kernel, then a block
+// per row a of Phi (on one SM the R^3 FP64 FMAs took 0.18 / 0.37 ms at R = 64
+// / 100); entry (a, b) and (b, a) are the same sum of the same products.
+__global__ void sts_w_kernel(int N, int R, const double* __restrict__ V0, const double* __restrict__ L0,
+                             double* __restrict__ E) {
+    const int v = blockIdx.x;
+    const double lam = L0[v];
+    double* EN = E + (int64_t)N * R * R + (int64_t)(R - 1 - v) * R;
+    for (int u = threadIdx.x; u < R; u += blockDim.x) EN[u] = lam > 1e-8 ? V0[u * R + v] / sqrt(lam) : 0.0;
+}
+
+__global__ void sts_phi_kernel(int N, int n, int R, const double* __restrict__ E, double* __restrict__ chain,
+                               double* __restrict__ Phi, double* __restrict__ PhiP) {
+    __shared__ double wa[kMaxRank];  // row a of W
+    const int a = blockIdx.x, R2 = R * R;
+    const double* EN = E + (int64_t)N * R2;
+    for (int v = threadIdx.x; v < R; v += blockDim.x) wa[v] = EN[v * R + a];
     __syncthreads();
-    for (int e = threadIdx.x; e < R2; e += blockDim.x) {
-        int a = e / R, b = e % R;
-        E[(int64_t)N * R2 + a * R + b] = W[b * R + a];
+    for (int b = threadIdx.x; b < R; b += blockDim.x) {
         double acc = 0.0;
-        for (int v = 0; v < R; v++) acc = fma(W[a * R + v], W[b * R + v], acc);
-        Phi[e] = acc;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < R2; e += blockDim.x) {
-        int a = e / R, b = e % R;
-        double p = Phi[a <= b ? a * R + b : b * R + a];
-        if (a <= b) PhiP[packed_index(R, a, b)] = p;
+        for (int v = 0; v < R; v++) acc = fma(wa[v], EN[v * R + b], acc);
+        Phi[a * R + b] = acc;
+        if (a <= b) PhiP[packed_index(R, a, b)] = acc;
         for (int k = N - 1; k > 0; k--)
-            if (k != n) chain[(int64_t)k * R2 + e] *= p;
+            if (k != n) chain[(int64_t)k * R2 + a * R + b] *= acc;
     }
 }
 
@@ -367,14 +366,11 @@ __global__ void sts_phi_kernel(int N, int n, int R, const double* __restrict__ V
 // eigenvector of chain[k] (k = 1..N-1, k != n).
 __global__ void sts_emat_kernel(int N, int n, int R, const double* __restrict__ V, const double* __restrict__ L,
                                 double* __restrict__ E) {
-    const int R2 = R * R;
-    for (int k = 1; k < N; k++) {
-        if (k == n) continue;
-        for (int e = threadIdx.x; e < R2; e += blockDim.x) {
-            int v = e / R, u = e % R;
-            E[(int64_t)k * R2 + v * R + u] = V[(int64_t)k * R2 + u * R + v] * sqrt(L[(int64_t)k * R + v]);
-        }
-    }
+    const int64_t k = blockIdx.y + 1, R2 = (int64_t)R * R;
+    const int v = blockIdx.x;
+    if (k == n) return;
+    const double s = sqrt(L[k * R + v]);
+    for (int u = threadIdx.x; u < R; u += blockDim.x) E[k * R2 + v * R + u] = V[k * R2 + u * R + v] * s;
 }
 
 // Eigen tree of each sampled mode k (sts_cp.hpp:179-187): PartitionTree over
@@ -474,24 +470,22 @@ static int build_eigen_trees(Session& s, int n, cudaStream_t st) {
 static int sts_eigen_factors(Session& s, int n, cudaStream_t st) {
     const int N = s.N, R = s.R, R2 = R * R;
     const int first = (n == 0) ? 1 : 0;
-    EXAFAC_TRY(launch_syev(R, s.chain + (int64_t)first * R2, 0, 1, s.eigV, s.eigL, 0, nullptr, 0.0, s.vt, st));
-    const size_t phi_smem = sizeof(double) * R2;
-    if (phi_smem > 48 * 1024)
-        EXAFAC_CUDA_TRY(cudaFuncSetAttribute(sts_phi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)phi_smem));
-    sts_phi_kernel<<<1, 256, phi_smem, st>>>(N, n, R, s.eigV, s.eigL, s.chain, s.Emat, s.Phi, s.PhiP); count_launch();
+    EXAFAC_TRY(launch_syev_refined(R, s.chain + (int64_t)first * R2, 0, 1, s.eigV, s.eigL, 0, s.vt, s.eigscr, st));
+    sts_w_kernel<<<R, 64, 0, st>>>(N, R, s.eigV, s.eigL, s.Emat); count_launch();
+    sts_phi_kernel<<<R, 128, 0, st>>>(N, n, R, s.Emat, s.chain, s.Phi, s.PhiP); count_launch();
     EXAFAC_CHECK_LAUNCH();
     if (N > 1) {
         // matrices 1..N-1 (chain[n] was cleared, its decomposition is trivial)
-        EXAFAC_TRY(launch_syev(R, s.chain + R2, R2, N - 1, s.eigV + R2, s.eigL + R, R2, nullptr, 0.0, s.vt, st));
+        EXAFAC_TRY(launch_syev_refined(R, s.chain + R2, R2, N - 1, s.eigV + R2, s.eigL + R, R2, s.vt, s.eigscr, st));
+        sts_emat_kernel<<<dim3(R, N - 1), 64, 0, st>>>(N, n, R, s.eigV, s.eigL, s.Emat); count_launch();
     }
-    sts_emat_kernel<<<1, 256, 0, st>>>(N, n, R, s.eigV, s.eigL, s.Emat); count_launch();
     EXAFAC_CHECK_LAUNCH();
     return EXAFAC_OK;
 }
 
 int sts_compute_M(Session& s, int n, cudaStream_t st) {
     const int N = s.N, R = s.R, R2 = R * R;
-    sts_chain_kernel<<<1, 256, 0, st>>>(N, n, R, s.gram, s.chain); count_launch();
+    sts_chain_kernel<<<(unsigned)ceil_div(R2, 128), 128, 0, st>>>(N, n, R, s.gram, s.chain); count_launch();
     EXAFAC_CHECK_LAUNCH();
     if (s.cfg.precision != EXAFAC_PREC_FP64) {
         // the mixed forms: Cholesky factors (the same row distribution)

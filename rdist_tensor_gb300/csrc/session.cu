@@ -81,7 +81,10 @@ static void carve(Session& s) {
             b.off[1] = a.take<int64_t>(2 * widest + 2);
             b.v = a.take<int32_t>(J);
             b.empty = a.take<int32_t>(J);
-        } else if (sts_zq_wanted(R, J)) {
+        } else {
+            s.eigscr = a.take<double>((int64_t)syev_refine_doubles(R, std::max(N - 1, 1)));
+        }
+        if (s.cfg.precision == EXAFAC_PREC_FP64 && sts_zq_wanted(R, J)) {
             int64_t widest = std::max<int64_t>(s.etree.leaf_count, 1);
             for (int k = 0; k < N; k++) widest = std::max<int64_t>(widest, s.rtree[k].leaf_count);
             zq_carve(a, s.zq, R, J, widest, 2 * N);
