@@ -20,11 +20,13 @@ struct ZState {
     int32_t* redo = nullptr;    // marked for the depth-first kernel
     int32_t* redo_list = nullptr;
     int32_t* redo_count = nullptr;  // 1
-    uint32_t* mask = nullptr;   // 4 per tile of 128 slots: went left (or stayed)
-    int32_t* tcount = nullptr;  // per tile: flags set
+    // of two consecutive levels (ping-pong), per tile of 128 slots:
+    uint32_t* mask[2] = {nullptr, nullptr};   // 4 words: went left (or stayed)
+    int32_t* tcount[2] = {nullptr, nullptr};  // flags set
+    int32_t* truns[2] = {nullptr, nullptr};   // runs of equal node, less one
     int64_t* pref64 = nullptr;  // per tile: prefix of tcount (more tiles than shared memory takes)
     int64_t* off[2] = {nullptr, nullptr};  // slot ranges of a level's nodes (ping-pong)
-    int32_t* tree_exp = nullptr;           // 2 N: exponent of each tree's root diagonal
+    int32_t* tree_exp = nullptr;           // 2 N + 1: exponent of each tree's root diagonal, and Phi's
 };
 
 void zq_carve(Arena& a, ZState& b, int R, int64_t J, int64_t widest, int trees);

@@ -10,9 +10,9 @@
 // with an error that is bounded in advance, every decision whose distance
 // from its cutoff is within the bound (of both evaluations) marks its sample,
 // and the marked samples are drawn again, whole, by the depth-first kernel.
-// The others took the same branch at every node, so their rows are the same;
-// their weights are formed by the same FP64 code.  Samples and weights are
-// those of the depth-first kernel bit for bit.
+// The others took the same branch at every node, so their rows are the same.
+// Their weights come from the same kind of products with enough digits to be
+// below FP64's rounding (zq_weight_kernel).
 //
 // Digits.  A vector x (scaled by a power of two to |x'| < 2^6) is held in
 // fixed point (units of 2^-47, int64) and cut into balanced base-256 digits:
@@ -121,11 +121,34 @@ __device__ __forceinline__ long long fix47(double v, int emax) {
     return b < 0 ? -(long long)m : (long long)m;
 }
 
+// The same rounded to nearest (the vectors: their weights take the mass to
+// FP64's own accuracy).
+__device__ __forceinline__ long long fix47_rn(double v, int emax) {
+    const long long b = __double_as_longlong(v);
+    const int e = (int)((b >> 52) & 0x7ff);
+    unsigned long long m = (unsigned long long)b & 0xfffffffffffffull;
+    if (e) m |= 1ull << 52;
+    const int s = max(max(emax, 1) - max(e, 1), 0);
+    m = s > 60 ? 0ull : (s > 0 ? (m + (1ull << (s - 1))) >> s : m);
+    return b < 0 ? -(long long)m : (long long)m;
+}
+
+// v' in units of 2^-56 (toward zero).
+__device__ __forceinline__ long long fix56(double v, int emax) {
+    const long long b = __double_as_longlong(v);
+    const int e = (int)((b >> 52) & 0x7ff);
+    unsigned long long m = (unsigned long long)b & 0xfffffffffffffull;
+    if (e) m |= 1ull << 52;
+    const int s = max(max(emax, 1) - max(e, 1), 0);
+    m = s > 63 ? 0ull : (m << 9) >> s;
+    return b < 0 ? -(long long)m : (long long)m;
+}
+
 // (byte idx of t - 128) 2^-8w as a float (exact).
 template <int W>
 __device__ __forceinline__ float digit_f(uint32_t t, uint32_t idx) {
     constexpr float sc = W == 0 ? 1.0f : W == 1 ? 0x1p-8f : W == 2 ? 0x1p-16f : W == 3 ? 0x1p-24f
-                         : W == 4 ? 0x1p-32f : 0x1p-40f;
+                         : W == 4 ? 0x1p-32f : W == 5 ? 0x1p-40f : W == 6 ? 0x1p-48f : 0x1p-56f;
     return fmaf(__uint_as_float(__byte_perm(t, 0x4B000000u, 0x7440u | idx)), sc, -8388736.0f * sc);
 }
 __device__ __forceinline__ float lead_f(int d) {  // |d| <= 128 as a float
@@ -293,36 +316,163 @@ __device__ __forceinline__ double z_bound(float n1, int R) {
     return (double)n1 * ((double)R * 4.6 * 0x1p-34 + 1.7 * 0x1p-32) + (double)R * (double)R * 0x1p-44;
 }
 
+// The block's share of a level's runs.  A run (consecutive slots of one tile
+// at the same node) costs its node's expansion and products whatever its
+// length, and the runs are spread unevenly over the tiles (skewed modes: the
+// tiles of the rare rows hold up to 128), so every block takes the same number
+// of runs: runs [first, first + count) in slot order, found from the per-tile
+// run counts.  With equal numbers of tiles the slowest block took 3.9 ms on a
+// tail level of a Zipf mode, with equal numbers of runs 0.2 ms.
+struct ZShare {
+    int64_t tile;   // first tile
+    int run;        // first run within it
+    int64_t count;  // runs
+};
+template <int NT>
+__device__ __forceinline__ ZShare z_share(const int32_t* __restrict__ truns, int64_t ntiles) {
+    __shared__ long long wsum[NT / 32];
+    __shared__ long long found[2];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int64_t per = (ntiles + NT - 1) / NT;
+    const int64_t a = min(ntiles, per * tid), e = min(ntiles, a + per);
+    long long sum = e - a;
+    for (int64_t q = a; q < e; q++) sum += __ldg(truns + q);
+    long long inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long u = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += u;
+    }
+    if (lane == 31) wsum[w] = inc;
+    if (tid == 0) {
+        found[0] = ntiles;
+        found[1] = 0;
+    }
+    __syncthreads();
+    long long before = inc - sum, total = 0;
+    for (int q = 0; q < NT / 32; q++) {
+        if (q < w) before += wsum[q];
+        total += wsum[q];
+    }
+    const long long first = total * blockIdx.x / gridDim.x, last = total * (blockIdx.x + 1) / gridDim.x;
+    if (first >= before && first < before + sum) {
+        long long at = before;
+        for (int64_t q = a; q < e; q++) {
+            const long long r = 1 + __ldg(truns + q);
+            if (first < at + r) {
+                found[0] = q;
+                found[1] = first - at;
+                break;
+            }
+            at += r;
+        }
+    }
+    __syncthreads();
+    ZShare s;
+    s.tile = found[0];
+    s.run = (int)found[1];
+    s.count = last - first;
+    return s;
+}
+
+// Run starts of the tile's nodes cs[0 .. n) as a bit mask (threads < 128;
+// cs[-1] differs); two block barriers.
+__device__ __forceinline__ void z_run_mask(const int32_t* cs, int n, uint32_t* rmask) {
+    const int tid = threadIdx.x;
+    __syncthreads();
+    if (tid < kZTile) {
+        const bool start = tid < n && (tid == 0 || cs[tid] != cs[tid - 1]);
+        const uint32_t m = __ballot_sync(0xffffffffu, start);
+        if ((tid & 31) == 0) rmask[tid >> 5] = m;
+    }
+    __syncthreads();
+}
+__device__ __forceinline__ int z_run_end(const uint32_t* rmask, int i0, int n) {
+    for (int q = (i0 + 1) >> 5; q < 4; q++) {
+        uint32_t bits = rmask[q];
+        if (q == ((i0 + 1) >> 5)) bits &= ~0u << ((i0 + 1) & 31);
+        if (bits) return min(n, (q << 5) + __ffs(bits) - 1);
+    }
+    return n;
+}
+
+// One chunk's read-back, columns c0 .. c0 + 7 of the node: the five integer
+// sums of Y_c (x0 + 2 xr)_c.
+struct ZSums {
+    long long Ph, Pl, Qh, Ql, V;
+};
+__device__ __forceinline__ void z_dot8(uint32_t taddr, const long long* xrow, int c0, int Rx, ZSums& s) {
+    uint32_t a[kZa][8];
+#pragma unroll
+    for (int q = 0; q < kZa; q++) tmem_ld8_nowait(taddr + (uint32_t)(kZCols * q), a[q]);
+    long long X[8];
+    load_x8(xrow, c0, Rx, true, X);
+    tmem_ld_wait<kZa>(a);
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        const float a0 = __uint_as_float(a[0][q]), a1 = __uint_as_float(a[1][q]), a2 = __uint_as_float(a[2][q]),
+                    a3 = __uint_as_float(a[3][q]), a4 = __uint_as_float(a[4][q]), a5 = __uint_as_float(a[5][q]);
+        // the weights' integers, by adding a power of two whose ulp is the
+        // unit: n0 (1), n1 (2^-8), n2 (2^-16), and weight 3 (2^-24) as a
+        // multiple of 2^-23 and a rest
+        const int m0 = __float_as_int(a0 + 12582912.0f) - 0x4B400000;
+        const int m1 = __float_as_int(a1 + 49152.0f) - 0x47400000;
+        const int m2 = __float_as_int(a2 + 192.0f) - 0x43400000;
+        const float f3 = a3 + 1.5f;
+        const int m3 = __float_as_int(f3) - 0x3FC00000;
+        const float v = (a3 - (f3 - 1.5f)) + (a4 + a5);
+        const int V = __float_as_int(v + 0.005859375f) - 0x3BC00000;  // units of 2^-31
+        const int Pn = m0 * 256 + m1;                                  // units of 2^-8
+        const int Qn = m2 * 128 + m3;                                  // units of 2^-23
+        const long long z4 = (X[q] + (1ll << 22)) >> 23;
+        const long long wi = 2 * X[q] - (z4 << 23);  // x0 + 2 xr
+        const int wh = (int)(wi >> 27), wl = (int)wi & 0x7ffffff;
+        s.Ph += (long long)Pn * wh;
+        s.Pl += (long long)Pn * wl;
+        s.Qh += (long long)Qn * wh;
+        s.Ql += (long long)Qn * wl;
+        s.V += (long long)V * wh;
+    }
+}
+
 // MODE 0: the root's mass of every sample (slot s holds sample s).
 // MODE 1: a level: the left child's mass and the branch.
 // MODE 2: the tail level: as MODE 1; samples already at a leaf stay.
-// The branch flags of a tile's slots go to mask[4 tile ..] and their count to
-// tcount[tile].
+// The branch flags of a tile's slots are set in mask[p], their count added to
+// tcount[p] (both zero before); truns[p] holds the runs per tile less one,
+// truns[p ^ 1] is cleared for the partition that follows.
+// NT = 512 (R > 64, one block per SM): a chunk's products run beside the
+// previous chunk's read-back (two accumulator sets), and beside the next
+// chunk's expansion when a second node buffer fits (nb = 2).
 template <int MODE, int NT>
 __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
-    zq_level_kernel(int R, TreeShape t, const double* __restrict__ G, const int32_t* __restrict__ tree_exp, int64_t J,
-                    ZState b, const int32_t* __restrict__ order, const double* __restrict__ dv, DeviceStatus* status,
-                    uint32_t wait_polls) {
+    zq_level_kernel(int R, int nb, TreeShape t, const double* __restrict__ G, const int32_t* __restrict__ tree_exp,
+                    int64_t J, ZState b, int p, const int32_t* __restrict__ order, const double* __restrict__ dv,
+                    DeviceStatus* status, uint32_t wait_polls) {
     extern __shared__ __align__(128) unsigned char z_raw[];
     constexpr int NG = NT / 128;        // threads per slot in the read-back
     constexpr int CPT = kZCols / NG;    // columns of a chunk per thread
+    constexpr bool kPipe = NT == 512;
+    constexpr uint32_t kTmem = kPipe ? 512 : 256;
     __shared__ int32_t cs[kZTile], js[kZTile];
-    __shared__ uint32_t rmask[4], fbits[4];
+    __shared__ uint32_t rmask[4];
     __shared__ long long part[NG][5][kZTile];
-    __shared__ uint32_t flag_sm[kZTile];
+    __shared__ int32_t flag_sm[kZTile];  // -1: not this block's, 0 right, 1 left (or stays)
     __shared__ int rs[kMaxRank];
-    __shared__ __align__(8) uint64_t bar;
+    __shared__ __align__(8) uint64_t bars[2];
     __shared__ uint32_t tmem_base;
     __shared__ int abort_flag;
     const ZShape z = z_shape(R);
+    const int Rx = z_row(R);
     unsigned char* A = z_raw + ((128u - (smem_u32(z_raw) & 127u)) & 127u);
-    unsigned char* B = A + kZx * z.xs;
+    unsigned char* Bb[2] = {A + kZx * z.xs, A + kZx * z.xs + (nb - 1) * kZa * z.bs};
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const int P = packed_size(R);
-    if (w == 0) tmem_alloc(&tmem_base, 256);
+    if (w == 0) tmem_alloc(&tmem_base, kTmem);
     for (int a = tid; a < R; a += NT) rs[a] = packed_index(R, a, a);
     if (tid == 0) {
-        mbar_init(&bar, 1);
+        mbar_init(&bars[0], 1);
+        mbar_init(&bars[1], 1);
         fence_mbar_init();
         abort_flag = 0;
     }
@@ -331,22 +481,34 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
     tc_fence_after();
     const uint32_t tmem = tmem_base;
     const int emax = *tree_exp;
-    uint32_t phase = 0;
+    uint32_t phase[2] = {0, 0};
     int64_t resident = -1;  // the node B holds (one-chunk ranks)
     const int row = (w & 3) * 32 + lane, grp = w >> 2;
+    const uint32_t lane_base = tmem + ((uint32_t)((w & 3) * 32) << 16);
     const int64_t ntiles = (J + kZTile - 1) / kZTile;
-    const int64_t per = (ntiles + gridDim.x - 1) / gridDim.x;
-    const int64_t t0 = (int64_t)blockIdx.x * per, t1 = min(ntiles, t0 + per);
+    ZShare sh;
+    if (MODE == 0) {
+        sh.tile = ntiles * blockIdx.x / gridDim.x;
+        sh.run = 0;
+        sh.count = ntiles * (blockIdx.x + 1) / gridDim.x - sh.tile;
+    } else {
+        sh = z_share<NT>(b.truns[p], ntiles);
+        for (int64_t q = (int64_t)blockIdx.x * NT + tid; q < ntiles; q += (int64_t)gridDim.x * NT) b.truns[p ^ 1][q] = 0;
+    }
     const bool ok = emax < 2047;  // a tree with a non-finite root: every sample is marked at the root
-    int64_t tile = t0;
-    for (; tile < t1; tile++) {
-        const int64_t s0 = tile * kZTile;
+    // the chunk's products are done (every thread); a wait that ran out raises abort_flag
+    auto wait = [&](int q) {
+        if (!mbar_wait_limited(&bars[q], phase[q], wait_polls)) abort_flag = 1;
+        phase[q] ^= 1u;
+        tc_fence_after();
+    };
+    for (; sh.count > 0 && sh.tile < ntiles; sh.tile++, sh.run = 0) {
+        const int64_t s0 = sh.tile * kZTile;
         const int n = (int)min((int64_t)kZTile, J - s0);
         double low = 0.0, rinv = 0.0, d = 0.0;
         float2 er = make_float2(0.f, 0.f);
-        float e0 = 0.f;
+        float e0 = 0.f, n1 = 0.f;
         int ex = 0;
-        float n1 = 0.f;
         if (tid < kZTile) {
             int32_t j = 0, c = -1;
             if (tid < n) {
@@ -364,103 +526,70 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
             }
             js[tid] = j;
             cs[tid] = c;
-            flag_sm[tid] = 1u;
-            const int32_t up = __shfl_up_sync(0xffffffffu, c, 1);
-            // run starts: compared across the warps' borders below
-            const bool start = tid < n && lane != 0 && c != up;
-            const uint32_t m = __ballot_sync(0xffffffffu, start);
-            if (lane == 0) rmask[w] = m;
+            flag_sm[tid] = -1;
         }
-        __syncthreads();
-        if (tid < 4) {
-            const int i = 32 * tid;
-            if (i < n && (i == 0 || cs[i] != cs[i - 1])) rmask[tid] |= 1u;
-        }
+        z_run_mask(cs, n, rmask);
         stage_x(A, reinterpret_cast<const long long*>(b.xi), js, n, R, z);
-        __syncthreads();
-        for (int i0 = 0; i0 < n;) {  // runs of equal node (uniform over the block)
+        int i0 = 0;
+        for (int q = 0; q < sh.run && i0 < n; q++) i0 = z_run_end(rmask, i0, n);
+        for (; i0 < n && sh.count > 0; sh.count--) {  // runs of equal node (uniform over the block)
             const int32_t c = cs[i0];
-            int i1 = n;
-            for (int q = (i0 + 1) >> 5; q < 4; q++) {
-                uint32_t bits = rmask[q];
-                if (q == ((i0 + 1) >> 5)) bits &= ~0u << ((i0 + 1) & 31);
-                if (bits) {
-                    i1 = min(n, (q << 5) + __ffs(bits) - 1);
-                    break;
-                }
-            }
-            if (MODE == 2 && tree_is_leaf(t, c)) {  // stays: flag 1
+            const int i1 = z_run_end(rmask, i0, n);
+            if (MODE == 2 && tree_is_leaf(t, c)) {  // stays
+                if (tid >= i0 && tid < i1) flag_sm[tid] = 1;
                 i0 = i1;
                 continue;
             }
             const int64_t g = MODE == 0 ? 0 : 2 * (int64_t)c + 1;
-            long long aPh = 0, aPl = 0, aQh = 0, aQl = 0, aV = 0;
-            const long long* xrow = reinterpret_cast<const long long*>(b.xi) + (int64_t)js[row < n ? row : 0] * z_row(R);
+            ZSums sum = {0, 0, 0, 0, 0};
+            const long long* xrow = reinterpret_cast<const long long*>(b.xi) + (int64_t)js[row < n ? row : 0] * Rx;
+            if (resident != g || z.nch > 1) expand_node(Bb[0], G + g * P, rs, 0, R, emax, z);
+            resident = g;
+            fence_proxy_async_smem();
+            tc_fence_before();
+            __syncthreads();
+            if (tid == 0) issue_chunk<kZa>(tmem, A, Bb[0], z, &bars[0]);
             for (int ch = 0; ch < z.nch; ch++) {
-                if (resident != g || z.nch > 1) {
-                    expand_node(B, G + g * P, rs, ch, R, emax, z);
-                    resident = g;
-                }
-                fence_proxy_async_smem();
-                tc_fence_before();
-                __syncthreads();
-                if (tid == 0) {
-                    issue_chunk<kZa>(tmem, A, B, z, &bar);
-                    if (!mbar_wait_limited(&bar, phase, wait_polls)) abort_flag = 1;
-                }
-                phase ^= 1u;
-                __syncthreads();
-                if (abort_flag) break;
-                tc_fence_after();
+                const int cur = kPipe ? ch & 1 : 0;
+                const bool more = ch + 1 < z.nch;
+                const uint32_t acc = lane_base + (uint32_t)(cur * 256 + grp * CPT);
+                if (kPipe) {
+                    if (more) {
+                        if (nb == 1) wait(cur);
+                        expand_node(Bb[(ch + 1) & (nb - 1)], G + g * P, rs, ch + 1, R, emax, z);
+                        fence_proxy_async_smem();
+                        tc_fence_before();
+                        __syncthreads();
+                        if (tid == 0)
+                            issue_chunk<kZa>(tmem + (uint32_t)((cur ^ 1) * 256), A, Bb[(ch + 1) & (nb - 1)], z,
+                                             &bars[cur ^ 1]);
+                    }
+                    if (nb == 2 || !more) wait(cur);
 #pragma unroll
-                for (int h = 0; h < CPT / 8; h++) {
-                    const int cc = grp * CPT + 8 * h;      // column within the chunk
-                    const int c0 = ch * kZCols + cc;
-                    uint32_t a[kZa][8];
+                    for (int h = 0; h < CPT / 8; h++)
+                        z_dot8(acc + 8 * h, xrow, ch * kZCols + grp * CPT + 8 * h, Rx, sum);
+                } else {
+                    wait(0);
 #pragma unroll
-                    for (int s = 0; s < kZa; s++)
-                        tmem_ld8_nowait(tmem + ((uint32_t)((w & 3) * 32) << 16) + (uint32_t)(kZCols * s + cc), a[s]);
-                    long long X[8];
-                    load_x8(xrow, c0, z_row(R), true, X);
-                    tmem_ld_wait<kZa>(a);
-#pragma unroll
-                    for (int q = 0; q < 8; q++) {
-                        const float a0 = __uint_as_float(a[0][q]), a1 = __uint_as_float(a[1][q]),
-                                    a2 = __uint_as_float(a[2][q]), a3 = __uint_as_float(a[3][q]),
-                                    a4 = __uint_as_float(a[4][q]), a5 = __uint_as_float(a[5][q]);
-                        // the weights' integers, by adding a power of two whose
-                        // ulp is the unit: n0 (1), n1 (2^-8), n2 (2^-16), and
-                        // weight 3 (2^-24) as a multiple of 2^-23 and a rest
-                        const int m0 = __float_as_int(a0 + 12582912.0f) - 0x4B400000;
-                        const int m1 = __float_as_int(a1 + 49152.0f) - 0x47400000;
-                        const int m2 = __float_as_int(a2 + 192.0f) - 0x43400000;
-                        const float f3 = a3 + 1.5f;
-                        const int m3 = __float_as_int(f3) - 0x3FC00000;
-                        const float v = (a3 - (f3 - 1.5f)) + (a4 + a5);
-                        const int V = __float_as_int(v + 0.005859375f) - 0x3BC00000;  // units of 2^-31
-                        const int Pn = m0 * 256 + m1;  // units of 2^-8
-                        const int Qn = m2 * 128 + m3;  // units of 2^-23
-                        const long long z4 = (X[q] + (1ll << 22)) >> 23;
-                        const long long wi = 2 * X[q] - (z4 << 23);  // x0 + 2 xr
-                        const int wh = (int)(wi >> 27), wl = (int)wi & 0x7ffffff;
-                        aPh += (long long)Pn * wh;
-                        aPl += (long long)Pn * wl;
-                        aQh += (long long)Qn * wh;
-                        aQl += (long long)Qn * wl;
-                        aV += (long long)V * wh;
+                    for (int h = 0; h < CPT / 8; h++)
+                        z_dot8(acc + 8 * h, xrow, ch * kZCols + grp * CPT + 8 * h, Rx, sum);
+                    if (more) {
+                        expand_node(Bb[0], G + g * P, rs, ch + 1, R, emax, z);
+                        fence_proxy_async_smem();
+                        tc_fence_before();
+                        __syncthreads();
+                        if (tid == 0) issue_chunk<kZa>(tmem, A, Bb[0], z, &bars[0]);
                     }
                 }
-                tc_fence_before();
-                if (ch + 1 < z.nch) __syncthreads();  // Y and B are free for the next chunk
-                tc_fence_after();
             }
-            if (abort_flag) break;
-            part[grp][0][row] = aPh;
-            part[grp][1][row] = aPl;
-            part[grp][2][row] = aQh;
-            part[grp][3][row] = aQl;
-            part[grp][4][row] = aV;
+            part[grp][0][row] = sum.Ph;
+            part[grp][1][row] = sum.Pl;
+            part[grp][2][row] = sum.Qh;
+            part[grp][3][row] = sum.Ql;
+            part[grp][4][row] = sum.V;
+            tc_fence_before();
             __syncthreads();
+            if (abort_flag) break;
             if (tid >= i0 && tid < i1) {
                 long long s5[5];
 #pragma unroll
@@ -495,45 +624,35 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
                         b.lh[j].x = cutoff;
                         b.err[j].x = ec;
                     }
-                    flag_sm[tid] = left ? 1u : 0u;
+                    flag_sm[tid] = left ? 1 : 0;
                 }
             }
-            __syncthreads();  // part, and Y and B for the next run
+            __syncthreads();  // part, and the accumulators and node buffers for the next run
             i0 = i1;
         }
         if (abort_flag) break;
-        if (MODE != 0) {
-            if (tid < kZTile) {
-                const uint32_t bits = __ballot_sync(0xffffffffu, tid < n && flag_sm[tid] != 0u);
-                if (lane == 0) {
-                    fbits[w] = bits;
-                    b.mask[4 * tile + w] = bits;
-                }
+        __syncthreads();
+        if (MODE != 0 && tid < kZTile) {
+            const uint32_t bits = __ballot_sync(0xffffffffu, flag_sm[tid] > 0);
+            if (lane == 0 && bits) {
+                atomicOr(b.mask[p] + 4 * sh.tile + w, bits);
+                atomicAdd(b.tcount[p] + sh.tile, __popc(bits));
             }
-            __syncthreads();
-            if (tid == 0)
-                b.tcount[tile] = __popc(fbits[0]) + __popc(fbits[1]) + __popc(fbits[2]) + __popc(fbits[3]);
         }
         __syncthreads();
     }
     __syncthreads();
-    if (abort_flag) {
-        // no flags for the tiles left out: the partition keeps their order
-        if (MODE != 0)
-            for (int64_t q = tile; q < t1; q++) {
-                if (tid < 4) b.mask[4 * q + tid] = 0u;
-                if (tid == 0) b.tcount[q] = 0;
-            }
-        if (tid == 0) {
-            report(status, EXAFAC_ERR_TIMEOUT, 23, blockIdx.x, 0);
-            mbar_wait_limited(&bar, phase ^ 1u, wait_polls);  // the MMAs in flight may still complete (bounded)
-        }
+    if (abort_flag) {  // the tiles left out keep clear flags: the partition keeps their order
+        if (tid == 0) report(status, EXAFAC_ERR_TIMEOUT, 23, blockIdx.x, 0);
+        // the MMAs in flight may still complete (bounded)
+        if (tid == 0) mbar_wait_limited(&bars[0], phase[0] ^ 1u, wait_polls);
+        if (tid == 32) mbar_wait_limited(&bars[1], phase[1] ^ 1u, wait_polls);
         tc_fence_before();
         __syncthreads();
     }
     if (w == 0) {
         tc_fence_after();
-        tmem_dealloc(tmem, 256);
+        tmem_dealloc(tmem, kTmem);
     }
 }
 
@@ -548,13 +667,14 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
 template <int NT>
 __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
     zq_leaf_kernel(int R, TreeShape t, const double* __restrict__ G, const double* __restrict__ U, int64_t J, ZState b,
-                   const int32_t* __restrict__ order, const double* __restrict__ dv, int N, int col,
+                   int p, const int32_t* __restrict__ order, const double* __restrict__ dv, int N, int col,
                    uint32_t* __restrict__ samples, DeviceStatus* status, uint32_t wait_polls) {
     extern __shared__ __align__(128) unsigned char z_raw[];
     constexpr int NG = NT / 128;
     constexpr int CPT = kZCols / NG;
     constexpr int NS = (NT == 256 ? 2 : 4);  // chunks (leaf rows / 32) at most
     __shared__ int32_t cs[kZTile], js[kZTile];
+    __shared__ uint32_t rmask[4];
     __shared__ float psum[NS * NG][kZTile];
     __shared__ int diag_exp;
     __shared__ __align__(8) uint64_t bar;
@@ -579,22 +699,22 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
     uint32_t phase = 0;
     const int row = (w & 3) * 32 + lane, grp = w >> 2;
     const int64_t ntiles = (J + kZTile - 1) / kZTile;
-    const int64_t per = (ntiles + gridDim.x - 1) / gridDim.x;
-    const int64_t t0 = (int64_t)blockIdx.x * per, t1 = min(ntiles, t0 + per);
-    for (int64_t tile = t0; tile < t1; tile++) {
-        const int64_t s0 = tile * kZTile;
+    ZShare sh = z_share<NT>(b.truns[p], ntiles);
+    for (; sh.count > 0 && sh.tile < ntiles; sh.tile++, sh.run = 0) {
+        const int64_t s0 = sh.tile * kZTile;
         const int n = (int)min((int64_t)kZTile, J - s0);
         if (tid < kZTile) {
             const int32_t j = tid < n ? (order ? order[s0 + tid] : (int32_t)(s0 + tid)) : 0;
             js[tid] = j;
             cs[tid] = tid < n ? (int32_t)b.node[j] : -1;
         }
-        __syncthreads();
+        z_run_mask(cs, n, rmask);
         stage_x(A, reinterpret_cast<const long long*>(b.xi), js, n, R, z);
-        for (int i0 = 0; i0 < n;) {
+        int i0 = 0;
+        for (int q = 0; q < sh.run && i0 < n; q++) i0 = z_run_end(rmask, i0, n);
+        for (; i0 < n && sh.count > 0; sh.count--) {
             const int32_t c = cs[i0];
-            int i1 = i0 + 1;
-            while (i1 < n && cs[i1] == c) i1++;
+            const int i1 = z_run_end(rmask, i0, n);
             if (!tree_is_leaf(t, c)) {  // only after a wait that ran out: not placed
                 if (tid >= i0 && tid < i1) {
                     z_mark(b.redo, b.redo_list, b.redo_count, js[tid]);
@@ -624,12 +744,9 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
                     fence_proxy_async_smem();
                     tc_fence_before();
                     __syncthreads();
-                    if (tid == 0) {
-                        issue_chunk<kZu>(tmem, A, B, z, &bar);
-                        if (!mbar_wait_limited(&bar, phase, wait_polls)) abort_flag = 1;
-                    }
+                    if (tid == 0) issue_chunk<kZu>(tmem, A, B, z, &bar);
+                    if (!mbar_wait_limited(&bar, phase, wait_polls)) abort_flag = 1;
                     phase ^= 1u;
-                    __syncthreads();
                     tc_fence_after();
                     float ps = 0.0f;
 #pragma unroll
@@ -652,7 +769,6 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
                     psum[ch * NG + grp][row] = ps;
                     tc_fence_before();
                     __syncthreads();
-                    tc_fence_after();
                     if (abort_flag) break;
                 } else {
 #pragma unroll
@@ -708,15 +824,14 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
             __syncthreads();
             if (tid >= i0 && tid < i1) {
                 const int32_t j = js[tid];
-                const int p = b.pick[j];
-                if (p < 0) z_mark(b.redo, b.redo_list, b.redo_count, j);
-                samples[(int64_t)j * N + col] = (uint32_t)(leaf * F + max(p, 0));
+                const int at = b.pick[j];
+                if (at < 0) z_mark(b.redo, b.redo_list, b.redo_count, j);
+                samples[(int64_t)j * N + col] = (uint32_t)(leaf * F + max(at, 0));
             }
-            __syncthreads();
             i0 = i1;
         }
-        if (abort_flag) break;
         __syncthreads();
+        if (abort_flag) break;
     }
     __syncthreads();
     if (abort_flag) {
@@ -775,12 +890,14 @@ __device__ __forceinline__ void tile_prefix(const int32_t* __restrict__ tcount, 
 // before slot s, is the tile's prefix plus the bits below s of its mask.
 // Within its parent's slot range a slot whose flag is set (went left, or
 // stayed at a leaf) keeps its order among those, before the others; the
-// children's slot ranges follow (coff, when another level does).  Every block
+// children's slot ranges (coff) and their runs per tile follow, and the next
+// level's flags are cleared.  Every block
 // forms the tiles' prefix in shared memory (up to kZPrefSmem tiles), or reads
 // pref64 (more).  lb: the parents' first node index, nl their number.
 __global__ void __launch_bounds__(512)
     zq_partition_kernel(int64_t J, int ntiles, const uint32_t* __restrict__ mask, const int32_t* __restrict__ tcount,
-                        const int64_t* __restrict__ pref64, int64_t lb, int64_t nl, const int32_t* __restrict__ order,
+                        uint32_t* __restrict__ mask_next, int32_t* __restrict__ tcount_next,
+                        int32_t* __restrict__ truns_next, const int64_t* __restrict__ pref64, int64_t lb, int64_t nl, const int32_t* __restrict__ order,
                         const int64_t* __restrict__ node, const int64_t* __restrict__ off,
                         int32_t* __restrict__ order2, int64_t* __restrict__ coff) {
     extern __shared__ int32_t z_pref[];
@@ -812,13 +929,20 @@ __global__ void __launch_bounds__(512)
         const int64_t pos = fl ? start + before : start + (SL(end) - at0) + ((s - start) - before);
         if (pos >= 0 && pos < J) order2[pos] = j;
     }
-    if (coff)
-        for (int64_t i = first; i < nl; i += step) {
-            const int64_t start = off[i], end = off[i + 1];
-            coff[2 * i] = start;
-            coff[2 * i + 1] = start + (SL(end) - SL(start));
-            if (i == 0) coff[2 * nl] = J;
-        }
+    for (int64_t i = first; i < nl; i += step) {
+        const int64_t start = off[i], end = off[i + 1];
+        const int64_t mid = start + (SL(end) - SL(start));
+        coff[2 * i] = start;
+        coff[2 * i + 1] = mid;
+        if (i == 0) coff[2 * nl] = J;
+        // a child that begins inside a tile begins one more run there
+        if (mid > start && (start & 127)) atomicAdd(truns_next + (start >> 7), 1);
+        if (end > mid && (mid & 127)) atomicAdd(truns_next + (mid >> 7), 1);
+    }
+    for (int64_t q = first; q < ntiles; q += step) {
+        reinterpret_cast<uint4*>(mask_next)[q] = make_uint4(0u, 0u, 0u, 0u);
+        tcount_next[q] = 0;
+    }
 }
 
 // Largest diagonal exponent of a tree's root, plus one (the entries of the
@@ -868,7 +992,7 @@ __global__ void zq_vector_kernel(int R, int64_t J, double* __restrict__ h, const
         for (int q = 0; q < 4; q++) {
             const int c = lane + 32 * q;
             if (c < z_row(R)) {  // (x is zero past R)
-                const long long f = e < 2047 ? fix47(x[q], e) : 0ll;
+                const long long f = e < 2047 ? fix47_rn(x[q], e) : 0ll;
                 reinterpret_cast<long long*>(b.xi)[j * z_row(R) + c] = f;
                 n1 += (float)((int)(llabs(f) >> 24) + 1) * 0x1p-23f;
             }
@@ -882,6 +1006,12 @@ __global__ void zq_vector_kernel(int R, int64_t J, double* __restrict__ h, const
             b.pick[j] = -1;
             if (KIND == 0) b.redo[j] = 0;
             if (KIND == 0 && j == 0) *b.redo_count = 0;
+            if ((j & 127) == 0) {
+                const int64_t tile = j >> 7;
+                reinterpret_cast<uint4*>(b.mask[0])[tile] = make_uint4(0u, 0u, 0u, 0u);
+                b.tcount[0][tile] = 0;
+                b.truns[0][tile] = 0;
+            }
             if (j == 0) {
                 b.off[0][0] = 0;
                 b.off[0][1] = J;
@@ -899,21 +1029,236 @@ __global__ void zq_leaf1_kernel(TreeShape t, int64_t J, ZState b, int N, int col
     }
 }
 
-// Weight = R / (J h^T Phi h): the depth-first kernel's quadratic form, a group
-// of warps per sample.
-__global__ void zq_weight_kernel(int R, int Gw, int S, int64_t J, const double* __restrict__ hs,
-                                 const double* __restrict__ PhiP, double* __restrict__ weights) {
-    extern __shared__ __align__(16) unsigned char z_wdyn[];
-    double *h, *unused, *q;
-    int gi;
-    const SampleGroup<double> grp = sample_group<double>(z_wdyn, R, Gw, h, unused, q, gi);
-    for (int64_t i = (int64_t)blockIdx.x * S + gi; i < J; i += (int64_t)gridDim.x * S) {
-        for (int r = grp.tg; r < R; r += grp.nthreads()) h[r] = hs[i * R + r];
-        grp.sync();
-        grp.build_z(R, h);
-        const double hq = grp.quad(packed_size(R), PhiP);
-        if (grp.tg == 0) weights[i] = hq > 0.0 ? (double)R / (hq * (double)J) : 0.0;
-        grp.sync();
+// ---- the weights R / (J h^T Phi h)
+//
+// The same products with five digits of h and eight of Phi (weights <= 7, in
+// chunks of 16 columns): the dropped part is below R 4 2^-50 of n1 in the
+// scaled units, under FP64's rounding of the depth-first sum, whose R^2 / 2
+// products and sums per sample took 3.1 ms at R = 64, J = 2^18.  A sample
+// whose form is not positive, not finite, or cancels (the bound above 2^-45 of
+// it) is marked.
+constexpr int kWx = 5, kWa = 8, kWCols = 16;
+
+static size_t zw_smem(int R) {
+    const ZShape z = z_shape(R);
+    return (size_t)kWx * z.xs + (size_t)kWa * 2 * z.sbo + 128;
+}
+
+__device__ __forceinline__ void tmem_ld4_nowait(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr)
+                 : "memory");
+}
+
+template <int NT>
+__global__ void __launch_bounds__(NT, 1)
+    zq_weight_kernel(int R, int64_t J, ZState b, const double* __restrict__ PhiP, const int32_t* __restrict__ phi_exp,
+                     double* __restrict__ weights, DeviceStatus* status, uint32_t wait_polls) {
+    extern __shared__ __align__(128) unsigned char z_raw[];
+    constexpr int NG = NT / 128;
+    constexpr int CPT = kWCols / NG;  // columns per thread: 8 or 4, in groups of 4
+    __shared__ long long part[NG][7][kZTile];
+    __shared__ int rs[kMaxRank];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t tmem_base;
+    __shared__ int abort_flag;
+    const ZShape z = z_shape(R);
+    const int Rx = z_row(R);
+    const uint32_t bs = 2u * z.sbo;  // one digit of 16 columns
+    unsigned char* A = z_raw + ((128u - (smem_u32(z_raw) & 127u)) & 127u);
+    unsigned char* B = A + kWx * z.xs;
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    if (w == 0) tmem_alloc(&tmem_base, 128);
+    for (int a = tid; a < R; a += NT) rs[a] = packed_index(R, a, a);
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        fence_mbar_init();
+        abort_flag = 0;
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base;
+    const int emax = *phi_exp;
+    uint32_t phase = 0;
+    const int row = (w & 3) * 32 + lane, grp = w >> 2;
+    const int nch = (R + kWCols - 1) / kWCols;
+    const int64_t ntiles = (J + kZTile - 1) / kZTile;
+    const long long* xi = reinterpret_cast<const long long*>(b.xi);
+    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int64_t s0 = tile * kZTile;
+        const int n = (int)min((int64_t)kZTile, J - s0);
+        for (int e = tid; e < kZTile * (z.Rk / 8); e += NT) {  // h, the row fastest
+            const int r = e & (kZTile - 1), k = 8 * (e / kZTile);
+            long long X[8];
+            load_x8(xi + (s0 + (r < n ? r : 0)) * Rx, k, Rx, r < n, X);
+            uint32_t lo[8];
+            int hi[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const long long t = ((X[q] + (1ll << 14)) >> 15) + 0x80808080ll;  // units of 2^-32
+                lo[q] = (uint32_t)t;
+                hi[q] = (int)(t >> 32);
+            }
+            uint32_t o[kWx][4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const uint32_t u = lo[2 * q], v = lo[2 * q + 1];
+                o[0][q] = pack_bf16(lead_f(hi[2 * q]), lead_f(hi[2 * q + 1]));
+                o[1][q] = pack_bf16(digit_f<1>(u, 3), digit_f<1>(v, 3));
+                o[2][q] = pack_bf16(digit_f<2>(u, 2), digit_f<2>(v, 2));
+                o[3][q] = pack_bf16(digit_f<3>(u, 1), digit_f<3>(v, 1));
+                o[4][q] = pack_bf16(digit_f<4>(u, 0), digit_f<4>(v, 0));
+            }
+            unsigned char* dst = A + (uint32_t)(r >> 3) * z.sbo + (uint32_t)(k >> 3) * 128u + (uint32_t)(r & 7) * 16u;
+#pragma unroll
+            for (int d = 0; d < kWx; d++)
+                *reinterpret_cast<uint4*>(dst + d * z.xs) = make_uint4(o[d][0], o[d][1], o[d][2], o[d][3]);
+        }
+        long long sum[7] = {0, 0, 0, 0, 0, 0, 0};  // P, Q, T times the high and low parts of x0 + 2 xr, W times the high
+        const long long* xrow = xi + (s0 + (row < n ? row : 0)) * Rx;
+        for (int ch = 0; ch < nch; ch++) {
+            for (int e = tid; e < kWCols * (z.Rk / 8); e += NT) {  // Phi's columns, the column fastest
+                const int c = e & (kWCols - 1), k = 8 * (e / kWCols);
+                const int col = ch * kWCols + c;
+                const int rc = col < R ? rs[col] : 0;
+                uint32_t lo[8], hi[8];
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    const int kk = k + q;
+                    const double v =
+                        (col < R && kk < R) ? __ldg(PhiP + (kk >= col ? rc + (kk - col) : rs[kk] + (col - kk))) : 0.0;
+                    const long long t = fix56(v, emax) + 0x80808080808080ll;  // eight digits
+                    lo[q] = (uint32_t)t;
+                    hi[q] = (uint32_t)(t >> 32);
+                }
+                uint32_t o[kWa][4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const uint32_t u = lo[2 * q], v = lo[2 * q + 1], uh = hi[2 * q], vh = hi[2 * q + 1];
+                    o[0][q] = pack_bf16(lead_f((int)uh >> 24), lead_f((int)vh >> 24));
+                    o[1][q] = pack_bf16(digit_f<1>(uh, 2), digit_f<1>(vh, 2));
+                    o[2][q] = pack_bf16(digit_f<2>(uh, 1), digit_f<2>(vh, 1));
+                    o[3][q] = pack_bf16(digit_f<3>(uh, 0), digit_f<3>(vh, 0));
+                    o[4][q] = pack_bf16(digit_f<4>(u, 3), digit_f<4>(v, 3));
+                    o[5][q] = pack_bf16(digit_f<5>(u, 2), digit_f<5>(v, 2));
+                    o[6][q] = pack_bf16(digit_f<6>(u, 1), digit_f<6>(v, 1));
+                    o[7][q] = pack_bf16(digit_f<7>(u, 0), digit_f<7>(v, 0));
+                }
+                unsigned char* dst = B + (uint32_t)(c >> 3) * z.sbo + (uint32_t)(k >> 3) * 128u + (uint32_t)(c & 7) * 16u;
+#pragma unroll
+                for (int d = 0; d < kWa; d++)
+                    *reinterpret_cast<uint4*>(dst + d * bs) = make_uint4(o[d][0], o[d][1], o[d][2], o[d][3]);
+            }
+            fence_proxy_async_smem();
+            tc_fence_before();
+            __syncthreads();
+            if (tid == 0) {
+                tc_fence_after();
+#pragma unroll
+                for (int i = 0; i < kWx; i++) {
+                    const uint32_t idesc = umma_idesc_bf16(kZTile, kWCols * (kWa - i));
+                    for (int ks = 0; ks < z.Rk / 16; ks++)
+                        umma_bf16(tmem + (uint32_t)(kWCols * i), umma_desc(A + i * z.xs + ks * 256, 128u, z.sbo),
+                                  umma_desc(B + ks * 256, 128u, z.sbo), idesc, (i > 0 || ks > 0) ? 1u : 0u);
+                }
+                umma_commit(&bar);
+            }
+            if (!mbar_wait_limited(&bar, phase, wait_polls)) abort_flag = 1;
+            phase ^= 1u;
+            tc_fence_after();
+#pragma unroll
+            for (int h = 0; h < CPT / 4; h++) {
+                const int cc = grp * CPT + 4 * h;
+                uint32_t a[kWa][4];
+#pragma unroll
+                for (int q = 0; q < kWa; q++)
+                    tmem_ld4_nowait(tmem + ((uint32_t)((w & 3) * 32) << 16) + (uint32_t)(kWCols * q + cc), a[q]);
+                long long X[4] = {0, 0, 0, 0};
+                if (ch * kWCols + cc < Rx)
+                    asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+                                 : "=l"(X[0]), "=l"(X[1]), "=l"(X[2]), "=l"(X[3])
+                                 : "l"(xrow + ch * kWCols + cc));
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int q = 0; q < kWa; q++)
+                    asm volatile("" : "+r"(a[q][0]), "+r"(a[q][1]), "+r"(a[q][2]), "+r"(a[q][3]));
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    float f[kWa];
+#pragma unroll
+                    for (int u = 0; u < kWa; u++) f[u] = __uint_as_float(a[u][q]);
+                    // integers of the weights 0, 1, 2; weight 3 to 2^-23, weight
+                    // 4 to 2^-30; their (exact) rests with weight 5 to 2^-38;
+                    // that rest with the weights 6 and 7 to 2^-46
+                    const int m0 = __float_as_int(f[0] + 12582912.0f) - 0x4B400000;
+                    const int m1 = __float_as_int(f[1] + 49152.0f) - 0x47400000;
+                    const int m2 = __float_as_int(f[2] + 192.0f) - 0x43400000;
+                    const float t3 = f[3] + 1.5f;
+                    const int m3 = __float_as_int(t3) - 0x3FC00000;
+                    const float t4 = f[4] + 0x1.8p-7f;
+                    const int m4 = __float_as_int(t4) - 0x3C400000;
+                    const float g5 = ((f[3] - (t3 - 1.5f)) + (f[4] - (t4 - 0x1.8p-7f))) + f[5];
+                    const float t5 = g5 + 0x1.8p-15f;
+                    const int m5 = __float_as_int(t5) - 0x38400000;
+                    const float g6 = (g5 - (t5 - 0x1.8p-15f)) + (f[6] + f[7]);
+                    const int W = __float_as_int(g6 + 0x1.8p-23f) - 0x34400000;
+                    const int Pn = m0 * 256 + m1, Qn = m2 * 128 + m3, Tn = m4 * 256 + m5;
+                    const long long z5 = (X[q] + (1ll << 14)) >> 15;
+                    const long long wi = 2 * X[q] - (z5 << 15);
+                    const int wh = (int)(wi >> 27), wl = (int)wi & 0x7ffffff;
+                    sum[0] += (long long)Pn * wh;
+                    sum[1] += (long long)Pn * wl;
+                    sum[2] += (long long)Qn * wh;
+                    sum[3] += (long long)Qn * wl;
+                    sum[4] += (long long)Tn * wh;
+                    sum[5] += (long long)Tn * wl;
+                    sum[6] += (long long)W * wh;
+                }
+            }
+            tc_fence_before();
+            __syncthreads();  // the accumulators and B are free for the next chunk
+            if (abort_flag) break;
+        }
+        if (abort_flag) break;
+#pragma unroll
+        for (int u = 0; u < 7; u++) part[grp][u][row] = sum[u];
+        __syncthreads();
+        if (tid < n) {
+            long long s6[7];
+#pragma unroll
+            for (int u = 0; u < 7; u++) {
+                s6[u] = part[0][u][tid];
+#pragma unroll
+                for (int gq = 1; gq < NG; gq++) s6[u] += part[gq][u][tid];
+            }
+            // P 2^-8, Q 2^-23, T 2^-38, W 2^-46; the parts of x0 + 2 xr 2^-20, 2^-47
+            const double q = (((double)s6[5] * 0x1p-85 + (double)s6[6] * 0x1p-66) + (double)s6[4] * 0x1p-58) +
+                             (((double)s6[3] * 0x1p-70 + (double)s6[1] * 0x1p-55) +
+                              ((double)s6[2] * 0x1p-43 + (double)s6[0] * 0x1p-28));
+            const int64_t j = s0 + tid;
+            const int ex = b.ex[j];
+            const bool good = q > 0.0 && ex < 2047 && emax < 2047 &&
+                              (double)b.n1[j] * (double)R * 0x1p-48 + (double)R * (double)R * 0x1p-57 < q * 0x1p-45;
+            const double hq = scalbn(q, 2 * ex + emax - 3084);
+            weights[j] = good ? (double)R / (hq * (double)J) : 0.0;
+            if (!good) z_mark(b.redo, b.redo_list, b.redo_count, (int32_t)j);
+        }
+        __syncthreads();
+    }
+    __syncthreads();
+    if (abort_flag) {
+        if (tid == 0) {
+            report(status, EXAFAC_ERR_TIMEOUT, 25, blockIdx.x, 0);
+            mbar_wait_limited(&bar, phase ^ 1u, wait_polls);
+        }
+        tc_fence_before();
+        __syncthreads();
+    }
+    if (w == 0) {
+        tc_fence_after();
+        tmem_dealloc(tmem, 128);
     }
 }
 
@@ -943,12 +1288,15 @@ void zq_carve(Arena& a, ZState& b, int R, int64_t J, int64_t widest, int trees) 
     b.redo = a.take<int32_t>(J);
     b.redo_list = a.take<int32_t>(J);
     b.redo_count = a.take<int32_t>(1);
-    b.mask = a.take<uint32_t>(4 * ceil_div(J, kZTile));
-    b.tcount = a.take<int32_t>(ceil_div(J, kZTile) + 4);
+    for (int q = 0; q < 2; q++) {
+        b.mask[q] = a.take<uint32_t>(4 * ceil_div(J, kZTile));
+        b.tcount[q] = a.take<int32_t>(ceil_div(J, kZTile) + 4);
+        b.truns[q] = a.take<int32_t>(ceil_div(J, kZTile) + 4);
+    }
     b.pref64 = a.take<int64_t>(ceil_div(J, kZTile) + 1);
     b.off[0] = a.take<int64_t>(2 * widest + 2);
     b.off[1] = a.take<int64_t>(2 * widest + 2);
-    b.tree_exp = a.take<int32_t>(trees);
+    b.tree_exp = a.take<int32_t>(trees + 1);
 }
 
 static unsigned z_grid(int64_t work) {
@@ -956,33 +1304,47 @@ static unsigned z_grid(int64_t work) {
 }
 
 template <int MODE, int NT>
-static int z_level(Session& s, const TreeShape& t, const double* G, const int32_t* ex, int64_t J, const int32_t* order,
-                   const double* dv, cudaStream_t st) {
-    const size_t smem = z_smem(s.R, kZa);
+static int z_level(Session& s, const TreeShape& t, const double* G, const int32_t* ex, int64_t J, int p,
+                   const int32_t* order, const double* dv, cudaStream_t st) {
+    // a second node buffer where one block per SM runs and it fits beside the
+    // 22 KB of static shared memory
+    const size_t two = z_smem(s.R, 2 * kZa);
+    const int nb = NT == 512 && two <= 200 * 1024 ? 2 : 1;
+    const size_t smem = nb == 2 ? two : z_smem(s.R, kZa);
     EXAFAC_CUDA_TRY(cudaFuncSetAttribute(zq_level_kernel<MODE, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem));
     const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(J, kZTile), NT == 256 ? 304 : 152);
-    zq_level_kernel<MODE, NT><<<blocks, NT, smem, st>>>(s.R, t, G, ex, J, s.zq, order, dv, s.status,
+    zq_level_kernel<MODE, NT><<<blocks, NT, smem, st>>>(s.R, nb, t, G, ex, J, s.zq, p, order, dv, s.status,
                                                         s.wait_polls ? s.wait_polls : kSpinLimit);
     count_launch();
     return EXAFAC_OK;
 }
 template <int MODE>
-static int z_level_any(Session& s, const TreeShape& t, const double* G, const int32_t* ex, int64_t J,
+static int z_level_any(Session& s, const TreeShape& t, const double* G, const int32_t* ex, int64_t J, int p,
                        const int32_t* order, const double* dv, cudaStream_t st) {
-    return s.R <= 64 ? z_level<MODE, 256>(s, t, G, ex, J, order, dv, st)
-                     : z_level<MODE, 512>(s, t, G, ex, J, order, dv, st);
+    return s.R <= 64 ? z_level<MODE, 256>(s, t, G, ex, J, p, order, dv, st)
+                     : z_level<MODE, 512>(s, t, G, ex, J, p, order, dv, st);
+}
+template <int NT>
+static int z_leaf(Session& s, const TreeShape& t, const double* G, const double* U, int64_t J, int p,
+                  const int32_t* order, const double* dv, int col, cudaStream_t st) {
+    const size_t smem = z_smem(s.R, kZu);
+    EXAFAC_CUDA_TRY(cudaFuncSetAttribute(zq_leaf_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(J, kZTile), NT == 256 ? 304 : 152);
+    zq_leaf_kernel<NT><<<blocks, NT, smem, st>>>(s.R, t, G, U, J, s.zq, p, order, dv, s.N, col, s.samples, s.status,
+                                                 s.wait_polls ? s.wait_polls : kSpinLimit);
+    count_launch();
+    return EXAFAC_OK;
 }
 
 // One descent of every sample; the vectors and the root state are in place.
 static int z_descend(Session& s, const TreeShape& t, const double* G, const double* U, const double* dv, int64_t J,
                      int col, int tree, cudaStream_t st) {
     ZState& b = s.zq;
-    const int R = s.R;
     int32_t* ex = b.tree_exp + tree;
-    zq_tree_exp_kernel<<<1, 32, 0, st>>>(R, G, ex);
+    zq_tree_exp_kernel<<<1, 32, 0, st>>>(s.R, G, ex);
     count_launch();
-    EXAFAC_TRY(z_level_any<0>(s, t, G, ex, J, nullptr, dv, st));
+    EXAFAC_TRY(z_level_any<0>(s, t, G, ex, J, 0, nullptr, dv, st));
     const int64_t ntiles = ceil_div(J, kZTile);
     const bool in_smem = ntiles <= kZPrefSmem;
     const size_t psm = in_smem ? sizeof(int32_t) * (ntiles + 1) : 0;
@@ -991,46 +1353,34 @@ static int z_descend(Session& s, const TreeShape& t, const double* G, const doub
             cudaFuncSetAttribute(zq_partition_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
     const bool tail = t.node_count > t.nodes_upto_lfill;
     const int32_t* order = nullptr;
-    int oi = 0, cur = 0;
+    int p = 0;  // parity of the level
     int64_t lb = 0, nl = 1;
     for (int64_t lvl = 0; lvl <= t.lfill_level; lvl++) {
         const bool is_tail = lvl == t.lfill_level;
         if (is_tail && !tail) break;
-        if (is_tail) EXAFAC_TRY(z_level_any<2>(s, t, G, ex, J, order, dv, st));
-        else EXAFAC_TRY(z_level_any<1>(s, t, G, ex, J, order, dv, st));
+        if (is_tail) EXAFAC_TRY(z_level_any<2>(s, t, G, ex, J, p, order, dv, st));
+        else EXAFAC_TRY(z_level_any<1>(s, t, G, ex, J, p, order, dv, st));
         if (is_tail && t.F <= 1) break;  // the leaf index needs no order
         if (!in_smem)
-            EXAFAC_TRY(scan_exclusive_u32_to_i64(reinterpret_cast<const uint32_t*>(b.tcount), b.pref64, ntiles,
+            EXAFAC_TRY(scan_exclusive_u32_to_i64(reinterpret_cast<const uint32_t*>(b.tcount[p]), b.pref64, ntiles,
                                                  b.pref64 + ntiles, s.scan_sc, st));
         zq_partition_kernel<<<(unsigned)std::min<int64_t>(ceil_div(J, 512), 152 * 2), 512, psm, st>>>(
-            J, (int)ntiles, b.mask, b.tcount, in_smem ? nullptr : b.pref64, lb, nl, order, b.node, b.off[oi],
-            b.order[cur], is_tail ? nullptr : b.off[oi ^ 1]);
+            J, (int)ntiles, b.mask[p], b.tcount[p], b.mask[p ^ 1], b.tcount[p ^ 1], b.truns[p ^ 1],
+            in_smem ? nullptr : b.pref64, lb, nl, order, b.node, b.off[p], b.order[p], b.off[p ^ 1]);
         count_launch();
-        order = b.order[cur];
-        cur ^= 1;
-        oi ^= 1;
+        order = b.order[p];
+        p ^= 1;
         lb = 2 * lb + 1;
         nl *= 2;
     }
     if (t.F <= 1) {
         zq_leaf1_kernel<<<z_grid(J), 256, 0, st>>>(t, J, b, s.N, col, s.samples);
+        count_launch();
+    } else if (s.R <= 64) {
+        EXAFAC_TRY(z_leaf<256>(s, t, G, U, J, p, order, dv, col, st));
     } else {
-        const size_t smem = z_smem(R, kZu);
-        const uint32_t polls = s.wait_polls ? s.wait_polls : kSpinLimit;
-        const int64_t tiles = ceil_div(J, kZTile);
-        if (R <= 64) {
-            EXAFAC_CUDA_TRY(cudaFuncSetAttribute(zq_leaf_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)smem));
-            zq_leaf_kernel<256><<<(unsigned)std::min<int64_t>(tiles, 304), 256, smem, st>>>(
-                R, t, G, U, J, b, order, dv, s.N, col, s.samples, s.status, polls);
-        } else {
-            EXAFAC_CUDA_TRY(cudaFuncSetAttribute(zq_leaf_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)smem));
-            zq_leaf_kernel<512><<<(unsigned)std::min<int64_t>(tiles, 152), 512, smem, st>>>(
-                R, t, G, U, J, b, order, dv, s.N, col, s.samples, s.status, polls);
-        }
+        EXAFAC_TRY(z_leaf<512>(s, t, G, U, J, p, order, dv, col, st));
     }
-    count_launch();
     EXAFAC_CHECK_LAUNCH();
     return EXAFAC_OK;
 }
@@ -1058,13 +1408,14 @@ int sts_draw_zq(Session& s, int n, int64_t J, const double* uni, cudaStream_t st
         zq_vector_kernel<2><<<vgrid, 256, 0, st>>>(R, J, h, s.F.U[k], s.samples, N, k, s.dims[k], b, s.status);
         count_launch();
     }
-    int Gw, S;
-    sample_group_shape(R, sizeof(double), Gw, S);
-    const size_t smem = (size_t)S * sample_group_bytes(R, sizeof(double));
-    if (smem > 48 * 1024)
-        EXAFAC_CUDA_TRY(cudaFuncSetAttribute(zq_weight_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int64_t blocks = std::max<int64_t>(std::min<int64_t>(ceil_div(J, S), 152 * 32), 1);
-    zq_weight_kernel<<<(unsigned)blocks, S * Gw * 32, smem, st>>>(R, Gw, S, J, h, s.PhiP, s.weights);
+    zq_tree_exp_kernel<<<1, 32, 0, st>>>(R, s.PhiP, b.tree_exp + 2 * N);
+    count_launch();
+    const size_t smem = zw_smem(R);
+    const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(J, kZTile), 152);
+    EXAFAC_CUDA_TRY(
+        cudaFuncSetAttribute(zq_weight_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    zq_weight_kernel<512><<<blocks, 512, smem, st>>>(R, J, b, s.PhiP, b.tree_exp + 2 * N, s.weights, s.status,
+                                                     s.wait_polls ? s.wait_polls : kSpinLimit);
     count_launch();
     EXAFAC_CHECK_LAUNCH();
     return EXAFAC_OK;
