@@ -114,13 +114,22 @@ __global__ void __launch_bounds__(256) segreduce_kernel(int R, const int64_t* __
 // sampled reduction, so the sums have a fixed order.  Lane l holds columns
 // l + 32 b, b < CB; a lane loads one nonzero's value and coordinates per
 // group of 32, and the factor rows of 8 nonzeros are gathered before their
-// FMAs.  Carries use a stride of 32 CB doubles per chunk.
+// FMAs.  Bound by the FP64 pipe (N - 2 multiplies and an FMA per nonzero and
+// column; products rounded in integer arithmetic instead took 1.8 times as
+// long).  Carries use a stride of 32 CB doubles per chunk.
+// The factors off the updated mode, in mode order, and their coordinate
+// columns (the kernel's loop over them knows its first at compile time).
+struct OffModes {
+    const double* U[kMaxModes - 1];
+    int col[kMaxModes - 1];
+};
+
 template <int CB>
-__global__ void __launch_bounds__(256) exact_segreduce_kernel(int N, int n, int R, const int64_t* __restrict__ counters,
+__global__ void __launch_bounds__(256) exact_segreduce_kernel(int N, int R, OffModes o, const int64_t* __restrict__ counters,
                                                               int64_t cap, const uint32_t* __restrict__ keys,
                                                               const uint32_t* __restrict__ pay,
                                                               const uint32_t* __restrict__ idx,
-                                                              const double* __restrict__ vals, FactorPtrs f,
+                                                              const double* __restrict__ vals,
                                                               double* __restrict__ M, double* __restrict__ carry_first,
                                                               double* __restrict__ carry_last,
                                                               uint32_t* __restrict__ carry_row) {
@@ -146,17 +155,17 @@ __global__ void __launch_bounds__(256) exact_segreduce_kernel(int N, int n, int 
         for (int b = 0; b < CB; b++) acc[b] = 0.0;
         for (int64_t g = cs; g < ce; g += 32) {
             const int nn = (int)min((int64_t)32, ce - g);
-            uint32_t hr = kNoRow, mi[kMaxModes];
+            uint32_t hr = kNoRow, mi[kMaxModes - 1];
             double hv = 0.0;
 #pragma unroll
-            for (int k = 0; k < kMaxModes; k++) mi[k] = 0;
+            for (int k = 0; k < kMaxModes - 1; k++) mi[k] = 0;
             if (lane < nn) {
                 hr = keys[g + lane];
                 const uint32_t i = pay[g + lane];
                 hv = vals[i];
 #pragma unroll
-                for (int k = 0; k < kMaxModes; k++)
-                    if (k < N) mi[k] = idx[(int64_t)i * N + k];
+                for (int k = 0; k < kMaxModes - 1; k++)
+                    if (k < N - 1) mi[k] = idx[(int64_t)i * N + o.col[k]];
             }
             uint32_t up = __shfl_up_sync(full, hr, 1);
             if (lane == 0) up = cur;
@@ -168,13 +177,16 @@ __global__ void __launch_bounds__(256) exact_segreduce_kernel(int N, int n, int 
 #pragma unroll
                     for (int b = 0; b < CB; b++) prod[u][b] = 1.0;
 #pragma unroll
-                    for (int k = 0; k < kMaxModes; k++) {
-                        if (k < N && k != n) {
+                    for (int k = 0; k < kMaxModes - 1; k++) {
+                        if (k < N - 1) {
                             const int64_t row = __shfl_sync(full, mi[k], t0 + u);
 #pragma unroll
                             for (int b = 0; b < CB; b++) {
                                 const int col = lane + 32 * b;
-                                if (col < R && t0 + u < nn) prod[u][b] *= f.U[k][row * R + col];
+                                if (col < R && t0 + u < nn) {
+                                    const double x = o.U[k][row * R + col];
+                                    prod[u][b] = k == 0 ? x : prod[u][b] * x;
+                                }
                             }
                         }
                     }
@@ -219,10 +231,10 @@ __global__ void __launch_bounds__(256) exact_segreduce_kernel(int N, int n, int 
 }
 
 template <int CB>
-static void launch_exact_mttkrp(Session& s, int n, double* M, FactorPtrs f, cudaStream_t st) {
+static void launch_exact_mttkrp(Session& s, const OffModes& o, double* M, cudaStream_t st) {
     const int hb = 152 * 8;
-    exact_segreduce_kernel<CB><<<hb, 256, 0, st>>>(s.N, n, s.R, s.counters, s.nnz, s.key_sorted, s.pay_sorted, s.idx,
-                                                   s.vals, f, M, s.carry_first, s.carry_last, s.carry_row);
+    exact_segreduce_kernel<CB><<<hb, 256, 0, st>>>(s.N, s.R, o, s.counters, s.nnz, s.key_sorted, s.pay_sorted, s.idx,
+                                                   s.vals, M, s.carry_first, s.carry_last, s.carry_row);
     count_launch();
     segfix_kernel<double, kSegChunk, CB><<<hb, 256, 0, st>>>(s.R, s.R, s.counters, s.nnz, s.carry_row, nullptr,
                                                              nullptr, s.key_sorted, s.carry_first, s.carry_last, M);
@@ -232,13 +244,17 @@ static void launch_exact_mttkrp(Session& s, int n, double* M, FactorPtrs f, cuda
 int exact_mttkrp(Session& s, int n, double* M, cudaStream_t st) {
     EXAFAC_CUDA_TRY(cudaMemsetAsync(M, 0, sizeof(double) * s.dims[n] * s.R, st));
     EXAFAC_TRY(nonzeros_by_row(s, n, st));
-    FactorPtrs f;
-    for (int k = 0; k < kMaxModes; k++) f.U[k] = k < s.N ? s.F.U[k] : nullptr;
+    OffModes o = {};
+    for (int k = 0, q = 0; k < s.N; k++) {
+        if (k == n) continue;
+        o.U[q] = s.F.U[k];
+        o.col[q++] = k;
+    }
     const int cb = (s.R + 31) / 32;
-    if (cb == 1) launch_exact_mttkrp<1>(s, n, M, f, st);
-    else if (cb == 2) launch_exact_mttkrp<2>(s, n, M, f, st);
-    else if (cb == 3) launch_exact_mttkrp<3>(s, n, M, f, st);
-    else launch_exact_mttkrp<4>(s, n, M, f, st);
+    if (cb == 1) launch_exact_mttkrp<1>(s, o, M, st);
+    else if (cb == 2) launch_exact_mttkrp<2>(s, o, M, st);
+    else if (cb == 3) launch_exact_mttkrp<3>(s, o, M, st);
+    else launch_exact_mttkrp<4>(s, o, M, st);
     EXAFAC_CHECK_LAUNCH();
     return EXAFAC_OK;
 }

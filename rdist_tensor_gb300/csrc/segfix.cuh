@@ -7,13 +7,15 @@
 namespace exafac {
 
 constexpr uint32_t kNoRow = 0xffffffffu;  // rows are < 2^32 - 1
+constexpr int kLongSpan = 256;             // chunks from which an FP64 row takes a whole block
+constexpr int kMaxLongSpans = 64;          // of them kept per block; more are summed by their warps
 
 // Crossing rows, one warp per chunk c0 whose last row continues: the row's
 // carries carry_last[c0] + sum over c in (c0, c1] of carry_first[c], c1 the
 // last chunk that starts inside the row: the chunk of the row's last hit,
 // seg_start[carry_seg[c0] + 1] - 1, when the run starts are given (one load
 // however long the row); otherwise the chunks that do form a prefix of c0+1,
-// c0+2, ..., found 32 at a time by ballot.  Spans of up to 32 chunks
+// c0+2, ..., whose end is searched.  Spans of up to 32 chunks
 // (almost every row): lane = column, chunks summed in order.  Longer spans
 // (the hot rows): lane l sums chunks c0+1+l, c0+1+l+32, ... over all 32 padded
 // columns, then a butterfly reduce-scatter leaves column l's total in lane l.
@@ -35,6 +37,13 @@ __global__ void __launch_bounds__(256) segfix_kernel(int R, int ldm, const int64
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const unsigned full = 0xffffffffu;
+    constexpr bool kBlockSpans = sizeof(TA) == 8;
+    __shared__ int nlong;
+    __shared__ int64_t longs[kBlockSpans ? kMaxLongSpans : 1][2];
+    if (kBlockSpans) {
+        if (threadIdx.x == 0) nlong = 0;
+        __syncthreads();
+    }
     for (int64_t c0 = warp; c0 < nchunks; c0 += nwarps) {
         const uint32_t row = carry_row[c0];
         if (row == kNoRow) continue;
@@ -43,13 +52,18 @@ __global__ void __launch_bounds__(256) segfix_kernel(int R, int ldm, const int64
         if (seg_start) {
             c1 = (min(seg_start[out + 1], H) - 1) / kChunk;
         } else {
-            for (int64_t b = c0 + 1;; b += 32) {
-                const int64_t m = b + lane;
-                const bool on = m < nchunks && keys[m * kChunk] == row;
-                const unsigned bal = __ballot_sync(full, on);
-                c1 = b + __popc(bal) - 1;
-                if (bal != full) break;
+            // the last chunk that starts inside the row: the keys ascend, so a
+            // 32-way search (a row of 1e6 nonzeros spans 8000 chunks)
+            int64_t lo = c0, hi = nchunks;  // keys[lo kChunk ..] on (or c0), hi off (or the end)
+            while (hi - lo > 1) {
+                const int64_t step = (hi - lo + 31) / 32;
+                const int64_t m = lo + (lane + 1) * step;
+                const bool on = m < hi && keys[m * kChunk] == row;
+                const int cnt = __popc(__ballot_sync(full, on));
+                hi = min(hi, lo + (cnt + 1) * step);
+                lo += cnt * step;
             }
+            c1 = lo;
         }
         // Columns R .. ldm - 1 of a padded FP32 row are written as zeros: the
         // solve reads whole rows, and the row's memory holds whatever the
@@ -68,6 +82,18 @@ __global__ void __launch_bounds__(256) segfix_kernel(int R, int ldm, const int64
                 Mc[out * ldm + col] = v;
             }
             continue;
+        }
+        if (kBlockSpans && c1 - c0 > kLongSpan) {  // a hot row: left to the whole block, below
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&nlong, 1);
+            at = __shfl_sync(full, at, 0);
+            if (at < kMaxLongSpans) {
+                if (lane == 0) {
+                    longs[at][0] = c0;
+                    longs[at][1] = c1;
+                }
+                continue;
+            }
         }
         for (int cb = 0; cb < CB; cb++) {
             TA acc[32];
@@ -91,6 +117,45 @@ __global__ void __launch_bounds__(256) segfix_kernel(int R, int ldm, const int64
             const int col = 32 * cb + lane;
             if (col < R) Mc[out * ldm + col] = carry_last[c0 * (32 * CB) + col] + acc[0];
             else if (col < ldm) Mc[out * ldm + col] = TA(0);
+        }
+    }
+    if (!kBlockSpans) return;
+    // FP64 spans of more than kLongSpan chunks (rows of thousands of hits), by
+    // the whole block: warp w sums the chunks c0 + 1 + w, + 8, ... with lane =
+    // column, the warps' sums are added in warp order (one warp took 0.9 ms
+    // over the hottest row of 1e7 Zipf nonzeros, the block 0.05)
+    __syncthreads();
+    __shared__ TA wsum[8][32];
+    const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int todo = min(nlong, kMaxLongSpans);
+    for (int q = 0; q < todo; q++) {
+        const int64_t c0 = longs[q][0], c1 = longs[q][1];
+        const int64_t out = carry_seg ? (int64_t)carry_seg[c0] : (int64_t)carry_row[c0];
+        for (int cb = 0; cb < CB; cb++) {
+            TA s[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) s[k] = TA(0);
+            int64_t m = c0 + 1 + w;
+            for (; m + 7 * nw <= c1; m += 8 * nw) {
+                TA v[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) v[k] = carry_first[(m + k * nw) * (32 * CB) + 32 * cb + lane];
+#pragma unroll
+                for (int k = 0; k < 8; k++) s[k] += v[k];
+            }
+            for (; m <= c1; m += nw) s[0] += carry_first[m * (32 * CB) + 32 * cb + lane];
+            wsum[w][lane] = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+            __syncthreads();
+            const int col = 32 * cb + lane;
+            if (w == 0 && col < ldm) {
+                TA v = TA(0);
+                if (col < R) {
+                    v = carry_last[c0 * (32 * CB) + col];
+                    for (int k = 0; k < nw; k++) v += wsum[k][lane];
+                }
+                Mc[out * ldm + col] = v;
+            }
+            __syncthreads();
         }
     }
 }

@@ -901,28 +901,76 @@ int zero_old_rows(Session& s, int n, cudaStream_t st) {
 // sparse_tensor.hpp:288-356, sort_lookup.hpp:377-438): sum over nonzeros of
 // x^2 - 2 x m(x) with m(x) = sum_u sigma_u prod_{k>=1} U_k[i_k,u] * U_0[i_0,u].
 // ---------------------------------------------------------------------------
-__global__ void fit_kernel(int N, int R, int64_t nnz, const uint32_t* __restrict__ idx, const double* __restrict__ vals,
-                           FactorPtrs f, const double* __restrict__ sigma, double* __restrict__ part) {
-    __shared__ double red[256];
-    double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t* c = idx + i * N;
-        double value = 0.0;
-        for (int u = 0; u < R; u++) {
-            double p = sigma[u];
-            for (int k = 1; k < N; k++) p *= f.U[k][(int64_t)c[k] * R + u];
-            value += p * f.U[0][(int64_t)c[0] * R + u];
+// Warp per nonzero, lane = column (CB column blocks): sum_nz x m = sum_u
+// sigma_u sum_nz x prod_k U_k[i_k, u], so a lane keeps its columns' sums over
+// all of the warp's nonzeros and no sum over the lanes is needed before the
+// end.  The factor rows are read whole (256 bytes per 32 columns); N FP64
+// operations per nonzero and column.
+constexpr int kFitBatch = 4;  // nonzeros whose rows are in flight together
+
+template <int CB>
+__global__ void __launch_bounds__(256) fit_kernel(int N, int R, int64_t nnz, const uint32_t* __restrict__ idx,
+                                                  const double* __restrict__ vals, FactorPtrs f,
+                                                  const double* __restrict__ sigma, double* __restrict__ part) {
+    __shared__ double red[8];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    double acc[CB], xx = 0.0;
+#pragma unroll
+    for (int b = 0; b < CB; b++) acc[b] = 0.0;
+    for (int64_t base = warp * 32; base < nnz; base += nwarps * 32) {
+        const int n = (int)min((int64_t)32, nnz - base);
+        uint32_t mi[kMaxModes];
+        double x = 0.0;
+#pragma unroll
+        for (int k = 0; k < kMaxModes; k++) mi[k] = 0;
+        if (lane < n) {
+            x = vals[base + lane];
+#pragma unroll
+            for (int k = 0; k < kMaxModes; k++)
+                if (k < N) mi[k] = idx[(base + lane) * N + k];
         }
-        const double x = vals[i];
-        acc += x * x - 2 * value * x;
+        xx = fma(x, x, xx);
+        for (int t0 = 0; t0 < n; t0 += kFitBatch) {
+            double p[kFitBatch][CB];
+#pragma unroll
+            for (int u = 0; u < kFitBatch; u++) {
+#pragma unroll
+                for (int k = 0; k < kMaxModes; k++) {
+                    if (k < N) {
+                        const int64_t row = __shfl_sync(0xffffffffu, mi[k], t0 + u);
+#pragma unroll
+                        for (int b = 0; b < CB; b++) {
+                            const int col = lane + 32 * b;
+                            const double y = (col < R && t0 + u < n) ? f.U[k][row * R + col] : 0.0;
+                            p[u][b] = k == 0 ? y : p[u][b] * y;
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kFitBatch; u++) {
+                const double v = __shfl_sync(0xffffffffu, x, t0 + u);
+#pragma unroll
+                for (int b = 0; b < CB; b++) acc[b] = fma(p[u][b], v, acc[b]);
+            }
+        }
     }
-    red[threadIdx.x] = acc;
+    double s = 0.0;
+#pragma unroll
+    for (int b = 0; b < CB; b++) {
+        const int col = lane + 32 * b;
+        if (col < R) s = fma(sigma[col], acc[b], s);
+    }
+    s = warp_sum(xx - 2.0 * s);
+    if (lane == 0) red[w] = s;
     __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-        __syncthreads();
+    if (threadIdx.x == 0) {
+        double a = 0.0;
+        for (int q = 0; q < 8; q++) a += red[q];
+        part[blockIdx.x] = a;
     }
-    if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
 
 __global__ void sum_kernel(const double* __restrict__ part, int n, double* __restrict__ out) {
@@ -940,7 +988,9 @@ __global__ void sum_kernel(const double* __restrict__ part, int n, double* __res
 
 int fit_residual(Session& s, double* out_dev, cudaStream_t st) {
     const int blocks = 152 * 8;
-    fit_kernel<<<blocks, 256, 0, st>>>(s.N, s.R, s.nnz, s.idx, s.vals, factor_ptrs(s), s.F.sigma, s.fitpart); count_launch();
+    const int cb = (s.R + 31) / 32;
+    auto kernel = cb == 1 ? fit_kernel<1> : cb == 2 ? fit_kernel<2> : cb == 3 ? fit_kernel<3> : fit_kernel<4>;
+    kernel<<<blocks, 256, 0, st>>>(s.N, s.R, s.nnz, s.idx, s.vals, factor_ptrs(s), s.F.sigma, s.fitpart); count_launch();
     sum_kernel<<<1, 256, 0, st>>>(s.fitpart, blocks, out_dev); count_launch();
     EXAFAC_CHECK_LAUNCH();
     return EXAFAC_OK;
