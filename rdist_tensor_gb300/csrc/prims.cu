@@ -274,8 +274,10 @@ int scan_cdf_f64(const double* in, double* out, int64_t n, double* total, void* 
 // ---------------------------------------------------------------------------
 // Radix sort
 // ---------------------------------------------------------------------------
-constexpr int kRadixThreads = 256;
-constexpr int kRadixItems = 16;
+// 512 threads of 8 items: with 256 of 16 the keys, payloads and ranks took 137
+// registers a thread and one block filled an SM.
+constexpr int kRadixThreads = 512;
+constexpr int kRadixItems = 8;
 constexpr int kRadixTile = kRadixThreads * kRadixItems;  // 4096
 constexpr int kRadixWarps = kRadixThreads / 32;
 
@@ -301,51 +303,91 @@ __global__ void radix_hist_kernel(const uint64_t* __restrict__ lo, const uint64_
     for (int d = threadIdx.x; d < 256; d += blockDim.x) hist[(int64_t)d * nb + blockIdx.x] = cnt[d];
 }
 
-__global__ void radix_scatter_kernel(const uint64_t* __restrict__ lo, const uint64_t* __restrict__ hi,
-                                     const uint32_t* __restrict__ pay, int64_t n, int shift,
-                                     const int64_t* __restrict__ offsets, int64_t nb, uint64_t* __restrict__ lo_out,
-                                     uint64_t* __restrict__ hi_out, uint32_t* __restrict__ pay_out) {
+// The stable scatter of one digit.  A tile's items are ranked warp by warp
+// (match + per-warp counters), put in digit order in shared memory, and
+// written from there, so that a warp's global writes run along the digits'
+// pieces: written straight from the ranks, each lane to its own digit, a pass
+// over 2e7 items took 0.34 ms, this form 0.16.
+template <bool HI>
+static constexpr size_t radix_smem() { return (size_t)kRadixTile * (HI ? 20 : 12); }
+
+template <bool HI>
+__global__ void __launch_bounds__(kRadixThreads, 2) radix_scatter_kernel(
+    const uint64_t* __restrict__ lo, const uint64_t* __restrict__ hi, const uint32_t* __restrict__ pay, int64_t n,
+    int shift, const int64_t* __restrict__ offsets, int64_t nb, uint64_t* __restrict__ lo_out,
+    uint64_t* __restrict__ hi_out, uint32_t* __restrict__ pay_out) {
+    extern __shared__ __align__(16) unsigned char rx_dyn[];
+    uint64_t* slo = reinterpret_cast<uint64_t*>(rx_dyn);
+    uint64_t* shi = slo + kRadixTile;  // HI only
+    uint32_t* spay = reinterpret_cast<uint32_t*>(rx_dyn + (size_t)kRadixTile * (HI ? 16 : 8));
     __shared__ uint32_t whist[kRadixWarps][256];
+    __shared__ uint32_t tstart[256];
+    __shared__ int64_t gbase[256];  // where the tile's digit begins in the output, less tstart
+    __shared__ uint32_t red[33];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int i = threadIdx.x; i < kRadixWarps * 256; i += blockDim.x) (&whist[0][0])[i] = 0;
+    const int64_t tile0 = (int64_t)blockIdx.x * kRadixTile;
+    const int64_t base = tile0 + (int64_t)w * 32 * kRadixItems;
+    uint64_t klo[kRadixItems], khi[HI ? kRadixItems : 1];
+    uint32_t pp[kRadixItems], rk[kRadixItems];
+#pragma unroll
+    for (int r = 0; r < kRadixItems; r++) {  // all loads in flight before the first use
+        const int64_t g = base + r * 32 + lane;
+        const bool on = g < n;
+        klo[r] = on ? lo[g] : 0ull;
+        if (HI) khi[r] = on ? hi[g] : 0ull;
+        pp[r] = on ? pay[g] : 0u;
+    }
     __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * kRadixTile + (int64_t)w * 32 * kRadixItems;
-    unsigned dg[kRadixItems];
-    uint32_t rk[kRadixItems];
     const unsigned lt = (1u << lane) - 1u;
 #pragma unroll
     for (int r = 0; r < kRadixItems; r++) {
-        int64_t g = base + r * 32 + lane;
-        unsigned d = 256;
-        if (g < n) d = digit_of(lo[g], hi ? hi[g] : 0ull, shift);
-        unsigned mask = __match_any_sync(0xffffffffu, d);
-        uint32_t before = (d < 256) ? whist[w][d] : 0u;
+        const unsigned d = base + r * 32 + lane < n ? digit_of(klo[r], HI ? khi[r] : 0ull, shift) : 256u;
+        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        const uint32_t before = d < 256 ? whist[w][d] : 0u;
         __syncwarp();
-        if (d < 256 && (mask & lt) == 0) whist[w][d] = before + __popc(mask);
+        if (d < 256 && (peers & lt) == 0) whist[w][d] = before + __popc(peers);
         __syncwarp();
-        dg[r] = d;
-        rk[r] = before + __popc(mask & lt);
+        rk[r] = before + __popc(peers & lt);
     }
     __syncthreads();
-    for (int d = threadIdx.x; d < 256; d += blockDim.x) {
+    {
+        const int d = threadIdx.x;
+        const int64_t off = d < 256 ? offsets[(int64_t)d * nb + blockIdx.x] : 0;
         uint32_t run = 0;
-        for (int ww = 0; ww < kRadixWarps; ww++) {
-            uint32_t c = whist[ww][d];
-            whist[ww][d] = run;
-            run += c;
+        if (d < 256) {
+            for (int ww = 0; ww < kRadixWarps; ww++) {
+                const uint32_t c = whist[ww][d];
+                whist[ww][d] = run;
+                run += c;
+            }
+        }
+        uint32_t total;
+        const uint32_t ts = block_exclusive_scan(run, red, &total);
+        if (d < 256) {
+            tstart[d] = ts;
+            gbase[d] = off - (int64_t)ts;
         }
     }
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < kRadixItems; r++) {
-        int64_t g = base + r * 32 + lane;
-        unsigned d = dg[r];
-        if (d < 256) {
-            int64_t pos = offsets[(int64_t)d * nb + blockIdx.x] + whist[w][d] + rk[r];
-            lo_out[pos] = lo[g];
-            if (hi) hi_out[pos] = hi[g];
-            pay_out[pos] = pay[g];
+        if (base + r * 32 + lane < n) {
+            const unsigned d = digit_of(klo[r], HI ? khi[r] : 0ull, shift);
+            const uint32_t l = tstart[d] + whist[w][d] + rk[r];
+            slo[l] = klo[r];
+            if (HI) shi[l] = khi[r];
+            spay[l] = pp[r];
         }
+    }
+    __syncthreads();
+    const int nvalid = (int)min((int64_t)kRadixTile, n - tile0);
+    for (int i = threadIdx.x; i < nvalid; i += kRadixThreads) {
+        const uint64_t kl = slo[i], kh = HI ? shi[i] : 0ull;
+        const int64_t pos = gbase[digit_of(kl, kh, shift)] + i;
+        lo_out[pos] = kl;
+        if (HI) hi_out[pos] = kh;
+        pay_out[pos] = spay[i];
     }
 }
 
@@ -377,20 +419,27 @@ int radix_sort_pairs(int64_t count, int bits, int kw, const uint64_t* lo_in, con
         EXAFAC_CUDA_TRY(cudaMemcpyAsync(pay_out, pay_in, sizeof(uint32_t) * count, cudaMemcpyDeviceToDevice, s));
         return EXAFAC_OK;
     }
+    EXAFAC_CUDA_TRY(cudaFuncSetAttribute(radix_scatter_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)radix_smem<true>()));
+    EXAFAC_CUDA_TRY(cudaFuncSetAttribute(radix_scatter_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)radix_smem<false>()));
     for (int p = 0; p < passes; p++) {
-        const bool last = (p == passes - 1);
         // Destination alternates so the final pass lands in *_out.
         const bool to_out = ((passes - 1 - p) % 2) == 0;
         uint64_t* dlo = to_out ? lo_out : lo_tmp;
         uint64_t* dhi = to_out ? hi_out : hi_tmp;
         uint32_t* dp = to_out ? pay_out : pay_tmp;
-        (void)last;
         radix_hist_kernel<<<(unsigned)nb, kRadixThreads, 0, s>>>(src_lo, has_hi ? src_hi : nullptr, count, p * 8, hist,
                                                                  nb); count_launch();
         EXAFAC_CHECK_LAUNCH();
         EXAFAC_TRY(scan_exclusive_u32_to_i64(hist, offs, 256 * nb, nullptr, scan_sc, s));
-        radix_scatter_kernel<<<(unsigned)nb, kRadixThreads, 0, s>>>(src_lo, has_hi ? src_hi : nullptr, src_p, count,
-                                                                    p * 8, offs, nb, dlo, dhi, dp); count_launch();
+        if (has_hi)
+            radix_scatter_kernel<true><<<(unsigned)nb, kRadixThreads, radix_smem<true>(), s>>>(
+                src_lo, src_hi, src_p, count, p * 8, offs, nb, dlo, dhi, dp);
+        else
+            radix_scatter_kernel<false><<<(unsigned)nb, kRadixThreads, radix_smem<false>(), s>>>(
+                src_lo, nullptr, src_p, count, p * 8, offs, nb, dlo, nullptr, dp);
+        count_launch();
         EXAFAC_CHECK_LAUNCH();
         src_lo = dlo;
         src_hi = dhi;
