@@ -939,6 +939,17 @@ __global__ void __launch_bounds__(kSmallPinvThreads)
 // sessions' scratch holds (N + 1) R^2).
 __device__ __forceinline__ int tri(int i, int j) { return i * (i + 1) / 2 + j; }
 
+// a / b from y ~ 1 / b: the quotient's exact residual, multiplied back
+// (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990): the correctly rounded a / b when y is the
+// rounded reciprocal, and for a y within an ulp of it unless a / b lies within
+// 2^-52 ulp of a midpoint.  Three dependent FP64 operations (~64 cycles each)
+// where the division itself takes some 700 cycles.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+    const double q = a * y;
+    return fma(fma(-q, b, a), y, q);
+}
+
 // Sums with four independent FP64 accumulators (a dependent FP64 operation
 // takes ~64 cycles on GB300, so one chain of R FMAs is latency-bound).
 // sub_dot: s0 - sum_{t in [t0, t1)} L(i, t) Li(t, c); gram_dot: sum_{k in
@@ -1062,6 +1073,226 @@ __global__ void spd_pinv_packed_kernel(int R, const double* __restrict__ A, doub
     if (refine) newton_refine_global(R, A, out, vt_scratch);
 }
 
+// ---------------------------------------------------------------------------
+// The Cholesky inverse of one matrix over many blocks (32 < R <= 128), the same
+// operations in the same order as the one-block kernels above (and so the same
+// bits), spread where they are independent:
+//   chol_factor_kernel   one CTA: L, every element in a register of its owner
+//                        (a step: the pivot column's owners divide, all owners
+//                        of later columns take one FMA)
+//   chol_columns_kernel  a block per column of L^{-1}, its rows' sums in the
+//                        threads, one finished row per step
+//   chol_gram_kernel     a block per row of L^{-T} L^{-1}
+// then the acceptance test with the Jacobi fallback in one CTA, and the Newton
+// step a block per row.  On one SM the FP64 pipe's ~1.8 operations per clock
+// and the ~64 cycles of each dependent one made them 0.13 / 0.25 / 0.87 ms at
+// R = 45 / 64 / 128; split, the factor takes 0.075 / 0.106 / 0.33 ms (a square
+// root and an FMA deep per column, so still latency), the columns 0.013 /
+// 0.027 / 0.052 and the products and the test 0.013 each.  kFour: L^{-1} and
+// the products summed in four chains (sub_dot, gram_dot), as the packed
+// kernels do.  At R <= 32 the small kernels' one launch is the shorter.
+// ---------------------------------------------------------------------------
+struct CholScratch {
+    double *Lp, *Li, *T, *fro;
+    int* rank;
+};
+__host__ __device__ inline CholScratch chol_scratch(double* p, int R) {
+    CholScratch c;
+    c.Lp = p;
+    c.Li = c.Lp + R * (R + 1) / 2;
+    c.T = c.Li + R * R;
+    c.fro = c.T + R * R;
+    c.rank = reinterpret_cast<int*>(c.fro + R);
+    return c;
+}
+size_t chol_scratch_doubles(int R) { return (size_t)R * (R + 1) / 2 + 2 * (size_t)R * R + R + 8; }
+
+constexpr int kFactorThreads = 512;
+
+template <int EPT>
+__global__ void __launch_bounds__(kFactorThreads) chol_factor_kernel(int R, const double* __restrict__ A,
+                                                                     double* __restrict__ scr) {
+    __shared__ double colv[2][kMaxRank];  // the pivot column (scaled), ping-pong
+    __shared__ double diag[2][3];         // the pivot, its square root and the root's reciprocal
+    pdl_wait();
+    pdl_trigger();
+    const CholScratch c = chol_scratch(scr, R);
+    const int tid = threadIdx.x, P = R * (R + 1) / 2;
+    // element e of the lower triangle by columns: column j holds rows j .. R - 1
+    double v[EPT];
+    int ij[EPT];  // i | j << 16; j = 0xffff: none
+#pragma unroll
+    for (int m = 0; m < EPT; m++) {
+        const int e = tid + m * kFactorThreads;
+        int j = 0, start = 0;
+        while (j < R - 1 && e >= start + (R - j)) {
+            start += R - j;
+            j++;
+        }
+        const int i = j + (e - start);
+        ij[m] = e < P ? (i | (j << 16)) : (0xffff << 16);
+        v[m] = e < P ? A[j * R + i] : 0.0;  // upper triangle of A
+    }
+    int rank = R;
+    for (int k = 0; k < R; k++) {
+        double* col = colv[k & 1];
+#pragma unroll
+        for (int m = 0; m < EPT; m++)
+            if (ij[m] == (k | (k << 16))) {  // its owner alone, two independent chains
+                diag[k & 1][0] = v[m];
+                diag[k & 1][1] = sqrt(v[m]);
+                diag[k & 1][2] = rsqrt(v[m]);
+            }
+        __syncthreads();
+        const double d = diag[k & 1][0], lkk = diag[k & 1][1], y = diag[k & 1][2];
+        const long long bits = __double_as_longlong(d);
+        if (!(bits > 0 && bits < 0x7ff0000000000000ll)) {  // not a positive finite number: the same in every thread
+            rank = k;
+            break;
+        }
+#pragma unroll
+        for (int m = 0; m < EPT; m++) {
+            if ((ij[m] >> 16) == k) {
+                const int i = ij[m] & 0xffff;
+                v[m] = i == k ? lkk : div_by(v[m], lkk, y);
+                col[i] = v[m];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < EPT; m++) {
+            const int i = ij[m] & 0xffff, j = ij[m] >> 16;
+            if (j > k && j < R) v[m] -= col[i] * col[j];
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < EPT; m++)
+        if ((ij[m] >> 16) < R) c.Lp[tri(ij[m] & 0xffff, ij[m] >> 16)] = v[m];
+    if (tid == 0) *c.rank = rank;
+}
+
+template <bool kFour>
+__global__ void __launch_bounds__(kMaxRank) chol_columns_kernel(int R, double* __restrict__ scr) {
+    __shared__ double val[2];
+    pdl_wait();
+    pdl_trigger();
+    const CholScratch s = chol_scratch(scr, R);
+    if (*s.rank != R) return;
+    const int c = blockIdx.x, i = threadIdx.x;
+    double a0 = i == c ? 1.0 : 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+    const bool row = i < R && i >= c;
+    const double lii = row ? s.Lp[tri(i, i)] : 1.0, yii = 1.0 / lii;
+    const int four = (i - c) & ~3;  // terms in whole groups of four
+    double next = row && i > c ? s.Lp[tri(i, c)] : 0.0;  // L(i, t), one step ahead
+    if (i < R && i < c) s.Li[i * R + c] = 0.0;
+    for (int t = c; t < R; t++) {
+        if (i == t) {
+            const double x = div_by(kFour ? (a0 + a1) + (a2 + a3) : a0, lii, yii);
+            val[t & 1] = x;
+            s.Li[t * R + c] = x;
+        }
+        const double l = next;
+        if (row && i > t + 1) next = s.Lp[tri(i, t + 1)];
+        __syncthreads();
+        if (row && i > t) {
+            const double x = val[t & 1];
+            const int q = kFour && t - c < four ? (t - c) & 3 : 0;
+            if (q == 0) a0 -= l * x;
+            else if (q == 1) a1 -= l * x;
+            else if (q == 2) a2 -= l * x;
+            else a3 -= l * x;
+        }
+    }
+}
+
+template <bool kFour>
+__global__ void __launch_bounds__(kMaxRank) chol_gram_kernel(int R, double* __restrict__ scr, double* __restrict__ out) {
+    __shared__ double la[kMaxRank];  // column a of L^{-1}
+    __shared__ double red[4];
+    pdl_wait();
+    pdl_trigger();
+    const CholScratch s = chol_scratch(scr, R);
+    if (*s.rank != R) return;
+    const int a = blockIdx.x, b = threadIdx.x;
+    if (b < R) la[b] = b >= a ? s.Li[b * R + a] : 0.0;
+    __syncthreads();
+    double part = 0.0;
+    if (b >= a && b < R) {
+        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+        int k = b;
+        if (kFour) {
+            for (; k + 3 < R; k += 4) {
+                s0 = fma(la[k], s.Li[k * R + b], s0);
+                s1 = fma(la[k + 1], s.Li[(k + 1) * R + b], s1);
+                s2 = fma(la[k + 2], s.Li[(k + 2) * R + b], s2);
+                s3 = fma(la[k + 3], s.Li[(k + 3) * R + b], s3);
+            }
+        }
+        for (; k < R; k++) s0 = fma(la[k], s.Li[k * R + b], s0);
+        const double acc = kFour ? (s0 + s1) + (s2 + s3) : s0;
+        out[a * R + b] = acc;
+        out[b * R + a] = acc;
+        part = (a == b ? 1.0 : 2.0) * (acc * acc);
+    }
+    part = warp_sum(part);
+    if ((b & 31) == 0) red[b >> 5] = part;
+    __syncthreads();
+    if (b == 0) s.fro[a] = (red[0] + red[1]) + (red[2] + red[3]);
+}
+
+// 1 / ||A^{-1}||_F > 10 tol, a lower bound of the smallest eigenvalue (every
+// thread the same); false when the factorisation stopped.
+__device__ bool chol_accepted(int R, const CholScratch& s, double tol) {
+    if (*s.rank != R) return false;
+    double fro = 0.0;
+    for (int a = 0; a < R; a++) fro += s.fro[a];
+    return isfinite(fro) && 1.0 / sqrt(fro) > 10.0 * tol;
+}
+
+// The pseudo-inverse's fallback: one CTA, which returns at once when the
+// Cholesky inverse stands.
+__global__ void __launch_bounds__(512) chol_accept_kernel(int R, const double* __restrict__ A, double* __restrict__ out,
+                                                          double tol, double* __restrict__ scr, double* vt) {
+    extern __shared__ double smem[];
+    __shared__ int stands;
+    pdl_wait();
+    const CholScratch s = chol_scratch(scr, R);
+    if (threadIdx.x < 32) {
+        const bool yes = chol_accepted(R, s, tol);
+        if (threadIdx.x == 0) stands = yes;
+    }
+    __syncthreads();
+    if (stands) return;
+    syev_block(R, A, nullptr, nullptr, out, tol, vt, smem);
+}
+
+// newton_refine over R blocks: T = A X, then X = 2X - X T.
+__global__ void __launch_bounds__(kMaxRank) newton_ax_kernel(int R, const double* __restrict__ A,
+                                                             const double* __restrict__ X, double* __restrict__ scr) {
+    __shared__ double arow[kMaxRank];
+    pdl_wait();
+    const CholScratch s = chol_scratch(scr, R);
+    const int i = blockIdx.x, j = threadIdx.x;
+    if (j < R) arow[j] = i <= j ? A[i * R + j] : A[j * R + i];
+    __syncthreads();
+    if (j >= R) return;
+    double acc = 0.0;
+    for (int k = 0; k < R; k++) acc = fma(arow[k], X[k * R + j], acc);
+    s.T[i * R + j] = acc;
+}
+__global__ void __launch_bounds__(kMaxRank) newton_out_kernel(int R, double* __restrict__ X, double* __restrict__ scr) {
+    __shared__ double xrow[kMaxRank];
+    pdl_wait();
+    const CholScratch s = chol_scratch(scr, R);
+    const int i = blockIdx.x, j = threadIdx.x;
+    if (j < R) xrow[j] = X[i * R + j];
+    __syncthreads();
+    if (j >= R) return;
+    double acc = 0.0;
+    for (int k = 0; k < R; k++) acc = fma(xrow[k], s.T[k * R + j], acc);
+    X[i * R + j] = 2.0 * xrow[j] - acc;
+}
+
 // The Newton step X <- X + X (I - A X) (= 2X - X A X, the fixed point a
 // pseudo-inverse) for the packed path, spread over R blocks of one row each
 // in FP64: T = I - A X (A's upper triangle read), then X += X T.  On one SM
@@ -1104,8 +1335,42 @@ size_t pinv_smem_bytes(int R) {
     return std::max(chol_smem_bytes(R), jac);
 }
 
+// L, L^{-1} (scr) and out = A^{-1} where the factorisation goes through.
+static int launch_chol_inverse(int R, const double* A, double* out, bool four, double* scr, cudaStream_t st) {
+    auto factor = R <= 64 ? chol_factor_kernel<5> : R <= 96 ? chol_factor_kernel<10> : chol_factor_kernel<17>;
+    factor<<<1, kFactorThreads, 0, st>>>(R, A, scr);
+    EXAFAC_CUDA_TRY(launch_dependent(four ? chol_columns_kernel<true> : chol_columns_kernel<false>, R, kMaxRank, 0, st, R,
+                                     scr));
+    EXAFAC_CUDA_TRY(launch_dependent(four ? chol_gram_kernel<true> : chol_gram_kernel<false>, R, kMaxRank, 0, st, R, scr,
+                                     out));
+    add_launches(3);
+    return EXAFAC_OK;
+}
+
+// scr (chol_scratch_doubles(R)): the split kernels; null: one CTA.
 static int launch_pinv_impl(int R, const double* A, double* out, double tol, double* vt_scratch, int refine,
-                            cudaStream_t stream) {
+                            cudaStream_t stream, double* scr = nullptr) {
+    if (R > kSmallPinvMaxR && scr) {
+        const bool four = chol_smem_bytes(R) > kPinvSmemCap;
+        EXAFAC_TRY(launch_chol_inverse(R, A, out, four, scr, stream));
+        const size_t smem = syev_smem_bytes(R);
+        if (smem > 48 * 1024)
+            EXAFAC_CUDA_TRY(
+                cudaFuncSetAttribute(chol_accept_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        EXAFAC_CUDA_TRY(launch_dependent(chol_accept_kernel, 1, 512, smem, stream, R, A, out, tol, scr, vt_scratch));
+        count_launch();
+        if (refine && four) {
+            newton_residual_kernel<<<R, 128, 0, stream>>>(R, A, out, chol_scratch(scr, R).T);
+            newton_update_kernel<<<R, 128, 0, stream>>>(R, chol_scratch(scr, R).T, out);
+            add_launches(2);
+        } else if (refine) {
+            EXAFAC_CUDA_TRY(launch_dependent(newton_ax_kernel, R, kMaxRank, 0, stream, R, A, (const double*)out, scr));
+            EXAFAC_CUDA_TRY(launch_dependent(newton_out_kernel, R, kMaxRank, 0, stream, R, out, scr));
+            add_launches(2);
+        }
+        EXAFAC_CHECK_LAUNCH();
+        return EXAFAC_OK;
+    }
     if (R <= kSmallPinvMaxR) {
         const size_t smem = std::max(syev_smem_bytes(R), chol_smem_bytes(R));
         spd_pinv_small_kernel<<<1, kSmallPinvThreads, smem, stream>>>(R, A, out, tol, vt_scratch, refine);
@@ -1138,12 +1403,13 @@ static int launch_pinv_impl(int R, const double* A, double* out, double tol, dou
     return EXAFAC_OK;
 }
 
-int launch_pinv(int R, const double* A, double* out, double tol, double* vt_scratch, cudaStream_t stream) {
-    return launch_pinv_impl(R, A, out, tol, vt_scratch, 0, stream);
+int launch_pinv(int R, const double* A, double* out, double tol, double* vt_scratch, cudaStream_t stream, double* scr) {
+    return launch_pinv_impl(R, A, out, tol, vt_scratch, 0, stream, scr);
 }
 
-int launch_pinv_refined(int R, const double* A, double* out, double tol, double* vt_scratch, cudaStream_t stream) {
-    return launch_pinv_impl(R, A, out, tol, vt_scratch, 1, stream);
+int launch_pinv_refined(int R, const double* A, double* out, double tol, double* vt_scratch, cudaStream_t stream,
+                        double* scr) {
+    return launch_pinv_impl(R, A, out, tol, vt_scratch, 1, stream, scr);
 }
 
 int launch_sigma_pinv_f32(int R, const double* ugram, double* sigma, double* ngram, int* degenerate, double* out,
@@ -1154,12 +1420,6 @@ int launch_sigma_pinv_f32(int R, const double* ugram, double* sigma, double* ngr
     count_launch();
     EXAFAC_CHECK_LAUNCH();
     return EXAFAC_OK;
-}
-
-int launch_pinv_leverage_f32(int R, const double* A, double* out, double tol, double* vt_scratch,
-                             cudaStream_t stream) {
-    if (R > kSmallPinvMaxR) return launch_pinv_impl(R, A, out, tol, vt_scratch, 0, stream);
-    return launch_pinv_impl(R, A, out, tol, vt_scratch, 2, stream);
 }
 
 size_t syev_smem_bytes(int R) {
@@ -1245,13 +1505,13 @@ int launch_syev_refined(int R, const double* A, int64_t a_stride, int batch, dou
 // Cholesky factors: about R^3 / 3 FP64 FMAs each, against some ten Jacobi
 // sweeps of about 5 R^3.
 //
-// sts_phi_chol_kernel (one CTA): A = chain[first] (the Hadamard product of
-// every Gram but mode n's) = L L^T, Phi = A^{-1} = L^{-T} L^{-1}, taken when
-// lambda_min >= 1 / ||A^{-1}||_F > 10 tol (as the Cholesky pseudo-inverse
-// above); the rows of L^{-1} are a factor of Phi and become E[N].  Otherwise
-// the CTA computes the Jacobi eigendecomposition and the reference's
-// W = V Lambda^{-1/2} (eigenvalues <= tol dropped).  Then chain[k] *= Phi
-// for k >= 1, k != n.
+// A = chain[first] (the Hadamard product of every Gram but mode n's) = L L^T,
+// Phi = A^{-1} = L^{-T} L^{-1} (launch_chol_inverse), taken when lambda_min >=
+// 1 / ||A^{-1}||_F > 10 tol (as the Cholesky pseudo-inverse above); the rows
+// of L^{-1} are a factor of Phi and become E[N].  Otherwise
+// sts_phi_accept_kernel (one CTA) computes the Jacobi eigendecomposition and
+// the reference's W = V Lambda^{-1/2} (eigenvalues <= tol dropped).  Then
+// chain[k] *= Phi for k >= 1, k != n.
 //
 // sts_chain_chol_kernel (one CTA per k = 1..N-1, k != n): the pivoted
 // Cholesky P^T chain[k] P = L L^T (largest remaining diagonal first; stops
@@ -1261,85 +1521,80 @@ int launch_syev_refined(int R, const double* A, int64_t a_stride, int batch, dou
 // ---------------------------------------------------------------------------
 
 // Right-looking Cholesky of the packed lower triangle L (tri(i, j), j <= i),
-// in place.  piv != nullptr: symmetric pivoting on the largest remaining
-// diagonal (piv[j] = the original index at position j), stopping when it is
-// <= stop; *rank = the number of columns factored.  piv == nullptr: stops at
-// a pivot that is not a positive finite number, *rank = its position.
-// col: R doubles of shared scratch.  Every thread returns the same *rank.
-__device__ void chol_packed_block(int R, double* L, int* piv, double stop, double* col, int* rank) {
+// in place, with symmetric pivoting on the largest remaining diagonal (piv[j] =
+// the original index at position j), stopping when it is <= stop; *rank = the
+// number of columns factored.  col: R doubles of shared scratch.  Every thread
+// returns the same *rank.
+__device__ void chol_pivoted_block(int R, double* L, int* piv, double stop, double* col, int* rank) {
     __shared__ int s_p;
     __shared__ int s_stop;
+    __shared__ double s_d, s_root[2];  // the pivot, its square root and the root's reciprocal
     const int tid = threadIdx.x, nt = blockDim.x;
-    if (piv)
-        for (int i = tid; i < R; i += nt) piv[i] = i;
+    for (int i = tid; i < R; i += nt) piv[i] = i;
     if (tid == 0) s_stop = R;
     __syncthreads();
     for (int k = 0; k < R; k++) {
-        if (piv) {
-            if (tid < 32) {  // warp 0: the largest remaining diagonal (first index on ties)
-                double best = -1.0;
-                int bi = k;
-                for (int i = k + tid; i < R; i += 32) {
-                    const double d = L[tri(i, i)];
-                    if (d > best) {
-                        best = d;
-                        bi = i;
-                    }
-                }
-                for (int o = 16; o > 0; o >>= 1) {
-                    const double ob = __shfl_down_sync(0xffffffffu, best, o);
-                    const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-                    if (ob > best || (ob == best && oi < bi)) {
-                        best = ob;
-                        bi = oi;
-                    }
-                }
-                if (tid == 0) {
-                    s_p = bi;
-                    if (!(best > stop)) s_stop = k;
+        if (tid < 32) {  // warp 0: the largest remaining diagonal (first index on ties)
+            // positive doubles order as their bits: integer compares, off the FP64 pipe
+            unsigned long long best = 0;
+            int bi = k;
+            for (int i = k + tid; i < R; i += 32) {
+                const long long d = __double_as_longlong(L[tri(i, i)]);
+                const unsigned long long v = d > 0 && d <= 0x7ff0000000000000ll ? (unsigned long long)d : 0ull;
+                if (v > best) {
+                    best = v;
+                    bi = i;
                 }
             }
-            __syncthreads();
-            if (s_stop == k) break;
-            const int p = s_p;
-            if (p != k) {  // swap rows and columns k and p (disjoint element pairs)
-                for (int j = tid; j < R; j += nt) {
-                    double *x = nullptr, *y = nullptr;
-                    if (j < k) {
-                        x = &L[tri(k, j)];
-                        y = &L[tri(p, j)];
-                    } else if (j == k) {
-                        x = &L[tri(k, k)];
-                        y = &L[tri(p, p)];
-                    } else if (j < p) {
-                        x = &L[tri(j, k)];
-                        y = &L[tri(p, j)];
-                    } else if (j > p) {
-                        x = &L[tri(j, k)];
-                        y = &L[tri(j, p)];
-                    }
-                    if (x) {
-                        const double t = *x;
-                        *x = *y;
-                        *y = t;
-                    }
-                }
-                if (tid == 0) {
-                    const int t = piv[k];
-                    piv[k] = piv[p];
-                    piv[p] = t;
-                }
-            }
-            __syncthreads();
-        } else {
-            const double d = L[tri(k, k)];
-            if (!(d > 0.0) || !isfinite(d)) {  // the same in every thread
-                if (tid == 0) s_stop = k;
-                break;
+            const uint32_t hi = __reduce_max_sync(0xffffffffu, (uint32_t)(best >> 32));
+            const uint32_t mylo = (uint32_t)(best >> 32) == hi ? (uint32_t)best : 0u;
+            const uint32_t lo = __reduce_max_sync(0xffffffffu, mylo);
+            const unsigned long long top = ((unsigned long long)hi << 32) | lo;
+            const int at = (int)__reduce_min_sync(0xffffffffu, best == top ? (uint32_t)bi : 0xffffu);
+            if (tid == 0) {
+                s_p = at;
+                s_d = __longlong_as_double((long long)top);
+                if (!(__longlong_as_double((long long)top) > stop)) s_stop = k;
             }
         }
-        const double lkk = sqrt(L[tri(k, k)]);
-        for (int i = k + 1 + tid; i < R; i += nt) col[i] = L[tri(i, k)] / lkk;
+        __syncthreads();
+        if (s_stop == k) break;
+        const int p = s_p;
+        if (tid == nt - 1) {  // beside the swap (the diagonal entry to be at k moves meanwhile)
+            s_root[0] = sqrt(s_d);
+            s_root[1] = rsqrt(s_d);
+        }
+        if (p != k) {  // swap rows and columns k and p (disjoint element pairs)
+            for (int j = tid; j < R; j += nt) {
+                double *x = nullptr, *y = nullptr;
+                if (j < k) {
+                    x = &L[tri(k, j)];
+                    y = &L[tri(p, j)];
+                } else if (j == k) {
+                    x = &L[tri(k, k)];
+                    y = &L[tri(p, p)];
+                } else if (j < p) {
+                    x = &L[tri(j, k)];
+                    y = &L[tri(p, j)];
+                } else if (j > p) {
+                    x = &L[tri(j, k)];
+                    y = &L[tri(j, p)];
+                }
+                if (x) {
+                    const double t = *x;
+                    *x = *y;
+                    *y = t;
+                }
+            }
+            if (tid == 0) {
+                const int t = piv[k];
+                piv[k] = piv[p];
+                piv[p] = t;
+            }
+        }
+        __syncthreads();
+        const double lkk = s_root[0], rkk = s_root[1];
+        for (int i = k + 1 + tid; i < R; i += nt) col[i] = div_by(L[tri(i, k)], lkk, rkk);
         __syncthreads();
         if (tid == 0) L[tri(k, k)] = lkk;
         {  // the trailing lower triangle: a warp per row, its lanes along the row
@@ -1360,81 +1615,56 @@ __device__ void chol_packed_block(int R, double* L, int* piv, double stop, doubl
     *rank = s_stop;
 }
 
-__global__ void sts_phi_chol_kernel(int N, int n, int R, int first, double tol, double* __restrict__ chain,
-                                    double* __restrict__ E, double* __restrict__ Phi, double* __restrict__ PhiP,
-                                    double* __restrict__ V, double* __restrict__ lam, double* __restrict__ vt) {
+// After launch_chol_inverse: E[N] and Phi stand, or one CTA computes them from
+// the Jacobi eigendecomposition.
+__global__ void __launch_bounds__(512) sts_phi_accept_kernel(int N, int R, const double* __restrict__ A, double tol,
+                                                             double* __restrict__ E, double* __restrict__ Phi,
+                                                             double* __restrict__ V, double* __restrict__ lam,
+                                                             double* __restrict__ vt, double* __restrict__ scr) {
     extern __shared__ double smem[];
-    __shared__ double fro_w[32];
-    __shared__ double col[kMaxRank];
-    const int P = R * (R + 1) / 2, R2 = R * R;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    double* L = smem;
-    double* Li = smem + P;
-    const double* A = chain + (int64_t)first * R2;
+    __shared__ int stands;
+    pdl_wait();
+    const CholScratch s = chol_scratch(scr, R);
+    const int R2 = R * R, tid = threadIdx.x, nt = blockDim.x;
     double* EN = E + (int64_t)N * R2;
-    for (int i = tid >> 5; i < R; i += nt >> 5)  // a warp per row of the packed lower triangle
-        for (int j = tid & 31; j <= i; j += 32) {
-            L[tri(i, j)] = A[j * R + i];  // upper triangle of A
-            Li[tri(i, j)] = 0.0;
-        }
-    __syncthreads();
-    int rank;
-    chol_packed_block(R, L, nullptr, 0.0, col, &rank);
-    bool ok = rank == R;
-    if (ok) {
-        for (int c = tid; c < R; c += nt) {  // L^{-1}, column c by forward substitution
-            for (int i = c; i < R; i++) {
-                const double s = sub_dot(L, Li, i, c, c, i, (i == c) ? 1.0 : 0.0);
-                Li[tri(i, c)] = s / L[tri(i, i)];
-            }
-        }
-        __syncthreads();
-        double part = 0.0;
-        for (int e = tid; e < R2; e += nt) {  // Phi = L^{-T} L^{-1}: (a, b), a <= b, once and mirrored
-            const int a = e / R, b = e % R;
-            if (a > b) continue;
-            const double acc = gram_dot(Li, a, b, b, R);
-            Phi[a * R + b] = acc;
-            Phi[b * R + a] = acc;
-            part += (a == b ? 1.0 : 2.0) * (acc * acc);
-        }
-        part = warp_sum(part);
-        if ((tid & 31) == 0) fro_w[tid >> 5] = part;
-        __syncthreads();
-        double fro = 0.0;
-        for (int q = 0; q < (nt + 31) / 32; q++) fro += fro_w[q];
-        ok = isfinite(fro) && 1.0 / sqrt(fro) > 10.0 * tol;  // the same in every thread
-        if (ok)
-            for (int e = tid; e < R2; e += nt) {  // E[N] row v = row v of L^{-1}
-                const int v = e / R, u = e % R;
-                EN[e] = u <= v ? Li[tri(v, u)] : 0.0;
-            }
+    if (tid < 32) {
+        const bool yes = chol_accepted(R, s, tol);
+        if (tid == 0) stands = yes;
     }
     __syncthreads();
-    if (!ok) {  // Jacobi: W[:, R-1-v] = eigenvector v / sqrt(lambda_v), lambda_v > tol
-        syev_block(R, A, V, lam, nullptr, tol, vt, smem);
-        __syncthreads();
-        for (int e = tid; e < R2; e += nt) {
-            const int a = e / R, b = e % R;
-            const int v = R - 1 - a;
-            EN[e] = lam[v] > tol ? V[b * R + v] / sqrt(lam[v]) : 0.0;
-        }
-        __syncthreads();
-        for (int e = tid; e < R2; e += nt) {
-            const int a = e / R, b = e % R;
-            double acc = 0.0;
-            for (int w = 0; w < R; w++) acc = fma(EN[w * R + a], EN[w * R + b], acc);
-            Phi[e] = acc;
-        }
+    if (stands) return;
+    // Jacobi: W[:, R-1-v] = eigenvector v / sqrt(lambda_v), lambda_v > tol
+    syev_block(R, A, V, lam, nullptr, tol, vt, smem);
+    __syncthreads();
+    for (int e = tid; e < R2; e += nt) {
+        const int a = e / R, b = e % R;
+        const int v = R - 1 - a;
+        EN[e] = lam[v] > tol ? V[b * R + v] / sqrt(lam[v]) : 0.0;
     }
     __syncthreads();
     for (int e = tid; e < R2; e += nt) {
         const int a = e / R, b = e % R;
-        const double p = Phi[a <= b ? a * R + b : b * R + a];
-        if (a <= b) PhiP[a * R - a * (a - 1) / 2 + (b - a)] = p;  // packed upper triangle, rows in order
-        for (int k = N - 1; k > 0; k--)
-            if (k != n) chain[(int64_t)k * R2 + e] *= p;
+        double acc = 0.0;
+        for (int w = 0; w < R; w++) acc = fma(EN[w * R + a], EN[w * R + b], acc);
+        Phi[e] = acc;
     }
+    if (tid == 0) *s.rank = -1;  // E[N] is written
+}
+
+// Row a: E[N] row a = row a of L^{-1} (when it stands), the packed Phi, and
+// chain[k] *= Phi for k >= 1, k != n.
+__global__ void __launch_bounds__(kMaxRank) sts_phi_rows_kernel(int N, int n, int R, double* __restrict__ chain,
+                                                                double* __restrict__ E, const double* __restrict__ Phi,
+                                                                double* __restrict__ PhiP, double* __restrict__ scr) {
+    pdl_wait();
+    const CholScratch s = chol_scratch(scr, R);
+    const int R2 = R * R, a = blockIdx.x, b = threadIdx.x;
+    if (b >= R) return;
+    if (*s.rank != -1) E[(int64_t)N * R2 + a * R + b] = b <= a ? s.Li[a * R + b] : 0.0;
+    const double p = Phi[a <= b ? a * R + b : b * R + a];
+    if (a <= b) PhiP[a * R - a * (a - 1) / 2 + (b - a)] = p;  // packed upper triangle, rows in order
+    for (int k = N - 1; k > 0; k--)
+        if (k != n) chain[(int64_t)k * R2 + a * R + b] *= p;
 }
 
 __global__ void sts_chain_chol_kernel(int N, int n, int R, const double* __restrict__ chain, double* __restrict__ E) {
@@ -1459,24 +1689,26 @@ __global__ void sts_chain_chol_kernel(int N, int n, int R, const double* __restr
     double dmax = 0.0;
     for (int q = 0; q < (nt + 31) / 32; q++) dmax = fmax(dmax, dmax_w[q]);
     int rank;
-    chol_packed_block(R, L, piv, (double)R * 2.220446049250313e-16 * dmax, col, &rank);
+    chol_pivoted_block(R, L, piv, (double)R * 2.220446049250313e-16 * dmax, col, &rank);
     for (int e = tid; e < R2; e += nt) {  // E[k][v][piv[i]] = L[i][v]
         const int v = e / R, i = e % R;
         Ek[v * R + piv[i]] = (v < rank && i >= v) ? L[tri(i, v)] : 0.0;
     }
 }
 
-size_t sts_factor_smem_bytes(int R) {
-    return std::max(sizeof(double) * 2 * (size_t)(R * (R + 1) / 2), syev_smem_bytes(R));
-}
-
 int launch_sts_factors_chol(int N, int n, int R, double tol, double* chain, double* E, double* Phi, double* PhiP,
-                            double* V, double* lam, double* vt, cudaStream_t stream) {
-    const size_t smem = sts_factor_smem_bytes(R);
-    EXAFAC_CUDA_TRY(cudaFuncSetAttribute(sts_phi_chol_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                            double* V, double* lam, double* vt, double* scr, cudaStream_t stream) {
     const int first = (n == 0) ? 1 : 0;
-    sts_phi_chol_kernel<<<1, 512, smem, stream>>>(N, n, R, first, tol, chain, E, Phi, PhiP, V, lam, vt);
-    count_launch();
+    const double* A = chain + (int64_t)first * R * R;
+    EXAFAC_TRY(launch_chol_inverse(R, A, Phi, true, scr, stream));
+    const size_t smem = syev_smem_bytes(R);
+    if (smem > 48 * 1024)
+        EXAFAC_CUDA_TRY(
+            cudaFuncSetAttribute(sts_phi_accept_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    EXAFAC_CUDA_TRY(launch_dependent(sts_phi_accept_kernel, 1, 512, smem, stream, N, R, A, tol, E, Phi, V, lam, vt, scr));
+    EXAFAC_CUDA_TRY(launch_dependent(sts_phi_rows_kernel, R, kMaxRank, 0, stream, N, n, R, chain, E, (const double*)Phi,
+                                     PhiP, scr));
+    add_launches(2);
     const size_t fsm = sizeof(double) * (size_t)(R * (R + 1) / 2);
     if (fsm > 48 * 1024)
         EXAFAC_CUDA_TRY(

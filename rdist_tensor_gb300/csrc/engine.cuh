@@ -101,6 +101,7 @@ struct Session {
     double* Phi = nullptr;     // R x R (full)
     double* PhiP = nullptr;    // packed
     double* vt = nullptr;      // Jacobi scratch, N+1 matrices
+    double* cholscr = nullptr; // Cholesky inverses (launch_pinv, launch_sts_factors_chol)
     double* eigscr = nullptr;  // FP64 form: scratch of the refined eigendecompositions
     // FP32 copies the mixed forms' STS-CP descents read (rounded from the FP64
     // arrays after every change): row trees, factors, eigen trees, E, Phi

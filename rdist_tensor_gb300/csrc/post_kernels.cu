@@ -986,7 +986,7 @@ static int normalize_typed(Session& s, int n, bool arls, cudaStream_t st) {
     const int R = s.R;
     EXAFAC_TRY(gram_reduce_to(s, kSolveBlocks, s.ugram, st));
     EXAFAC_TRY(sigma_and_gram(s, st));
-    if (arls) EXAFAC_TRY(launch_pinv(R, s.ngram, s.upinv, 1e-11, s.vt, st));
+    if (arls) EXAFAC_TRY(launch_pinv(R, s.ngram, s.upinv, 1e-11, s.vt, st, s.cholscr));
     normlev_kernel<TA><<<grid_capped(s.dims[n], kNormWarps * 32), kNormWarps * 32, 0, st>>>(
         R, s.counters, s.touched, s.F.sigma, arls ? s.upinv : nullptr, reinterpret_cast<int*>(s.counters + 6),
         s.F.U[n], arls ? s.scores[n] : nullptr, s.scores_c);

@@ -489,7 +489,7 @@ int sts_compute_M(Session& s, int n, cudaStream_t st) {
     EXAFAC_CHECK_LAUNCH();
     if (s.cfg.precision != EXAFAC_PREC_FP64) {
         // the mixed forms: Cholesky factors (the same row distribution)
-        EXAFAC_TRY(launch_sts_factors_chol(N, n, R, 1e-8, s.chain, s.Emat, s.Phi, s.PhiP, s.eigV, s.eigL, s.vt, st));
+        EXAFAC_TRY(launch_sts_factors_chol(N, n, R, 1e-8, s.chain, s.Emat, s.Phi, s.PhiP, s.eigV, s.eigL, s.vt, s.cholscr, st));
     } else {
         EXAFAC_TRY(sts_eigen_factors(s, n, st));
     }

@@ -99,6 +99,7 @@ static void carve(Session& s) {
     s.Phi = a.take<double>(R2);
     s.PhiP = a.take<double>(P);
     s.vt = a.take<double>((int64_t)syev_scratch_doubles(R, N + 1));
+    s.cholscr = a.take<double>((int64_t)chol_scratch_doubles(R));
     for (int k = 0; k < N; k++) s.nzrows[k] = a.take<uint32_t>(s.dims[k]);
     s.nzcount = a.take<int64_t>(N);
     s.uni = a.take<double>((int64_t)N * 2 * J);
@@ -218,7 +219,7 @@ static int refresh_sampler(Session& s, int k, bool all_rows, cudaStream_t st) {
     EXAFAC_CUDA_TRY(cudaMemcpyAsync(s.gram + (int64_t)k * R * R, s.ngram, sizeof(double) * R * R,
                                     cudaMemcpyDeviceToDevice, st));
     if (s.cfg.sampler == EXAFAC_SAMPLER_CP_ARLS_LEV) {
-        EXAFAC_TRY(launch_pinv(R, s.ngram, s.upinv, 1e-11, s.vt, st));
+        EXAFAC_TRY(launch_pinv(R, s.ngram, s.upinv, 1e-11, s.vt, st, s.cholscr));
         if (all_rows) EXAFAC_CUDA_TRY(cudaMemsetAsync(s.scores[k], 0, sizeof(double) * s.dims[k], st));
         EXAFAC_TRY(arls_leverage(s, k, all_rows, s.upinv, st));
         EXAFAC_TRY(arls_build_cdf(s, k, nullptr, nullptr, st));
@@ -664,7 +665,7 @@ extern "C" int exafac_als_exact_step(exafac_als_t h, int32_t n, void* stream) {
     const int R = s.R;
     EXAFAC_TRY(all_grams(s, st));
     EXAFAC_TRY(chain_gram(s, n, s.dgram, st));
-    EXAFAC_TRY(launch_pinv(R, s.dgram, s.dpinv, 1e-11, s.vt, st));
+    EXAFAC_TRY(launch_pinv(R, s.dgram, s.dpinv, 1e-11, s.vt, st, s.cholscr));
     EXAFAC_TRY(exact_mttkrp(s, n, s.Mexact, st));
     EXAFAC_TRY(matmul_rows_sym(s, s.Mexact, s.dpinv, s.F.U[n], s.dims[n], st));
     EXAFAC_TRY(normalize_factor(s, n, true, st));

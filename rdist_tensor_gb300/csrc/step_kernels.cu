@@ -625,8 +625,8 @@ int design_gram(Session& s, int n, int64_t J, cudaStream_t st) {
 // (common.h:405-443, eigenvalue cut 1e-11); the mixed forms add one Newton
 // step X <- X (2I - G X) on the FP32-accumulated Gram.
 int design_pinv(Session& s, cudaStream_t st) {
-    if (s.cfg.precision != EXAFAC_PREC_FP64) return launch_pinv_refined(s.R, s.dgram, s.dpinv, 1e-11, s.vt, st);
-    return launch_pinv(s.R, s.dgram, s.dpinv, 1e-11, s.vt, st);
+    if (s.cfg.precision != EXAFAC_PREC_FP64) return launch_pinv_refined(s.R, s.dgram, s.dpinv, 1e-11, s.vt, st, s.cholscr);
+    return launch_pinv(s.R, s.dgram, s.dpinv, 1e-11, s.vt, st, s.cholscr);
 }
 
 // ---------------------------------------------------------------------------

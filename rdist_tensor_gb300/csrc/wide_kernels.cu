@@ -449,7 +449,7 @@ static int wide_normalize(Session& s, int n, bool arls, cudaStream_t st) {
     const int R = s.R;
     EXAFAC_TRY(gram_reduce_to(s, kWideSolveBlocks, s.ugram, st));
     EXAFAC_TRY(sigma_and_gram(s, st));
-    if (arls) EXAFAC_TRY(launch_pinv(R, s.ngram, s.upinv, 1e-11, s.vt, st));
+    if (arls) EXAFAC_TRY(launch_pinv(R, s.ngram, s.upinv, 1e-11, s.vt, st, s.cholscr));
     constexpr int RP = 32 * CB;
     const size_t smem = sizeof(double) * ((arls ? (size_t)RP * RP : 0) + (size_t)kWideWarps * RP);
     EXAFAC_CUDA_TRY(
