@@ -295,6 +295,27 @@ int exafac_cp_sampled_adjoint(int32_t N, int32_t R, const int64_t* dims_host, in
                               const void* grad_m_dev, const void* const* factors_dev, void* const* grads_dev,
                               int32_t dtype, int32_t* status_dev, void* stream);
 
+/* The weighted loss over the sampled entries and its derivative in each model
+ * value, in one launch: *loss_dev = sum_j w[j] f(x[j], m[j]) and deriv[j] =
+ * w[j] df/dm(x[j], m[j]) with m as exafac_cp_sampled_model gives it and f the
+ * Poisson (m - x log(m + 1e-10)), Bernoulli-odds (log(m + 1) - x log(m +
+ * 1e-10)) or Gaussian ((x - m)^2) loss.  Terms are in `dtype`, their sum in
+ * FP64.  J >= 1.  scratch_dev: EXAFAC_LOSS_SCRATCH_BYTES, 8-byte aligned, no
+ * initial contents, one per stream in flight. */
+enum { EXAFAC_LOSS_POISSON = 0, EXAFAC_LOSS_BERNOULLI = 1, EXAFAC_LOSS_GAUSSIAN = 2 };
+enum { EXAFAC_LOSS_BLOCKS = 2432, EXAFAC_LOSS_SCRATCH_BYTES = 8 * (EXAFAC_LOSS_BLOCKS + 1) };
+int exafac_cp_sampled_loss(int32_t kind, int32_t N, int32_t R, const int64_t* dims_host, int64_t J,
+                           const int32_t* idx_dev, const void* x_dev, const void* w_dev,
+                           const void* const* factors_dev, void* deriv_dev, void* loss_dev, void* scratch_dev,
+                           int32_t dtype, int32_t* status_dev, void* stream);
+
+/* exafac_cp_sampled_adjoint into grads that it zeroes first (dims[n] x R each;
+ * null entries are skipped), every grad_m[j] multiplied by the device scalar
+ * *scale_dev when that is not null.  J >= 1. */
+int exafac_cp_sampled_gradient(int32_t N, int32_t R, const int64_t* dims_host, int64_t J, const int32_t* idx_dev,
+                               const void* grad_m_dev, const void* scale_dev, const void* const* factors_dev,
+                               void* const* grads_dev, int32_t dtype, int32_t* status_dev, void* stream);
+
 /* Stratified entry sample: J_nz nonzeros drawn uniformly with replacement
  * (value x, weight nnz / J_nz) followed by J_z uniform coordinates taken as
  * zeros (value 0, weight (prod dims - nnz) / J_z); Philox4x32-10 keyed by

@@ -81,6 +81,8 @@ SIGNATURES = {
                                              ctypes.POINTER(_P)]),
     "exafac_cp_sampled_model": (ctypes.c_int, [_I32, _I32, _P, _I64, _P, _P, _P, _I32, _P, _P]),
     "exafac_cp_sampled_adjoint": (ctypes.c_int, [_I32, _I32, _P, _I64, _P, _P, _P, _P, _I32, _P, _P]),
+    "exafac_cp_sampled_loss": (ctypes.c_int, [_I32, _I32, _I32, _P, _I64, _P, _P, _P, _P, _P, _P, _P, _I32, _P, _P]),
+    "exafac_cp_sampled_gradient": (ctypes.c_int, [_I32, _I32, _P, _I64, _P, _P, _P, _P, _P, _I32, _P, _P]),
     "exafac_gcp_sample_entries": (ctypes.c_int, [_I32, _P, _I64, _P, _P, _I64, _I64, ctypes.c_uint64,
                                                  ctypes.c_uint64, _P, _P, _P, _I32, _P]),
     "exafac_adam_step": (ctypes.c_int, [_I32, _P, _P, _P, _P, _P, _I32, ctypes.c_double, ctypes.c_double,

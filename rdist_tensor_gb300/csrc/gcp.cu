@@ -4,10 +4,11 @@
 // nearest relatives are execute_exact_mttkrp (sort_lookup.hpp:440-495) and
 // the zero-sampling fit estimate of exafac/low_rank_tensor.py:110-184.
 //
-//   model     m_j = sum_r prod_k U_k[i_jk, r]                 warp per entry
-//   adjoint   G_n[i_jn, :] += g_j * prod_{k != n} U_k[i_jk, :]  warp per entry,
-//             every mode from one load of the entry's N factor rows; the
-//             Khatri-Rao rows are recomputed here, never stored
+//   model     m_j = sum_r prod_k U_k[i_jk, r], a group of lanes per entry
+//   loss      sum_j w_j f(x_j, m_j) and w_j df/dm in the model's pass
+//   adjoint   G_n[i_jn, :] += g_j * prod_{k != n} U_k[i_jk, :], a group of
+//             lanes per entry, every mode from one load of the entry's N
+//             factor rows; the Khatri-Rao rows are recomputed here, never stored
 //   sampler   J_nz nonzeros uniformly (weight nnz / J_nz) and J_z coordinates
 //             uniformly (value 0, weight (prod dims - nnz) / J_z), Philox
 //   adam      one Adam step over all factors in one launch, fused with the
@@ -32,80 +33,232 @@ struct Dims {
     int64_t d[kMaxModes];
 };
 
-// Loads the entry's coordinates (lane k holds mode k) and checks them against
-// the mode sizes; an entry with an out-of-range coordinate is skipped and
-// flagged in *status (when given).
+// V consecutive elements, one 16-byte access when V * sizeof(T) == 16.
+template <typename T, int V>
+struct alignas(V * sizeof(T)) Pack {
+    T v[V];
+};
+
+// The lanes of a warp that share an entry: a power of two, at least R / V of
+// them up to the whole warp.  A factor row of 32 floats is 8 lanes' 16-byte
+// loads, so a warp holds four entries in flight where a lane per column held
+// one (J = 2^17 entries, R = 32, FP32: model 40 -> XXX us, adjoint 72 -> XXX).
+static int entry_lanes(int R, int V) {
+    int L = 1;
+    while (L < 32 && L * V < R) L <<= 1;
+    return L;
+}
+
+// The entry's coordinates, checked against the mode sizes; an entry with an
+// out-of-range coordinate is skipped and flagged in *status (when given).
+template <int M>
 __device__ __forceinline__ bool load_entry(int N, const Dims& dims, const int32_t* __restrict__ idx, int64_t j,
-                                           int64_t (&rows)[kMaxModes], int* status) {
-    const int lane = threadIdx.x & 31;
-    const int32_t my = lane < N ? idx[j * N + lane] : 0;
-    const bool bad = lane < N && (my < 0 || (int64_t)my >= dims.d[lane]);
-    if (__any_sync(0xffffffffu, bad)) {
-        if (lane == 0 && status) atomicExch(status, 1);
-        return false;
-    }
+                                           int32_t (&rows)[M], int* status) {
+    bool ok = true;
 #pragma unroll
-    for (int k = 0; k < kMaxModes; k++) rows[k] = __shfl_sync(0xffffffffu, my, k);
-    return true;
+    for (int k = 0; k < M; k++) {
+        rows[k] = k < N ? __ldg(&idx[j * N + k]) : 0;
+        if (k < N && (rows[k] < 0 || (int64_t)rows[k] >= dims.d[k])) ok = false;
+    }
+    if (!ok && status) atomicExch(status, 1);
+    return ok;
 }
 
-__device__ __forceinline__ double warp_sum_any(double v) { return warp_sum(v); }
-__device__ __forceinline__ float warp_sum_any(float v) { return warp_sum(v); }
+// The kernels take the modes as a compile-time bound M (4, or 8 above four
+// modes): the unrolled loops then hold no registers for modes that are not
+// there (adjoint, 16-byte accesses: 40 against 80).
+//
+// The model value of entry j over the L lanes that share it (every lane of the
+// warp calls; dead lanes pass live = false): the same sum on each of them.
+template <typename T, int V, int M>
+__device__ __forceinline__ T entry_model(int N, int R, const Dims& dims, int64_t j, bool live, int L, int gl,
+                                         const int32_t* __restrict__ idx, const PtrsT<const T>& f, int* status) {
+    int32_t rows[M];
+    T acc = 0;
+    if (live && load_entry(N, dims, idx, j, rows, status)) {
+        for (int c = gl * V; c < R; c += L * V) {
+            Pack<T, V> p;
+#pragma unroll
+            for (int v = 0; v < V; v++) p.v[v] = T(1);
+#pragma unroll
+            for (int k = 0; k < M; k++)
+                if (k < N) {
+                    const Pack<T, V> u = *reinterpret_cast<const Pack<T, V>*>(&f.p[k][(int64_t)rows[k] * R + c]);
+#pragma unroll
+                    for (int v = 0; v < V; v++) p.v[v] *= u.v[v];
+                }
+            if constexpr (V == 4)  // the pairwise order of a lane per column
+                acc += (p.v[0] + p.v[1]) + (p.v[2] + p.v[3]);
+            else if constexpr (V == 2)
+                acc += p.v[0] + p.v[1];
+            else
+                acc += p.v[0];
+        }
+    }
+    for (int o = L >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    return acc;
+}
 
-template <typename T>
-__global__ void cp_model_kernel(int N, int R, Dims dims, int64_t J, const int32_t* __restrict__ idx,
-                                PtrsT<const T> f, T* __restrict__ m, int* status) {
-    const int lane = threadIdx.x & 31;
+template <typename T, int V, int M>
+__global__ void __launch_bounds__(256) cp_model_kernel(int N, int R, int L, Dims dims, int64_t J,
+                                                       const int32_t* __restrict__ idx, PtrsT<const T> f,
+                                                       T* __restrict__ m, int* status) {
+    const int lane = threadIdx.x & 31, G = 32 / L, gl = lane & (L - 1);
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t j = warp; j < J; j += nwarps) {
-        int64_t rows[kMaxModes];
-        if (!load_entry(N, dims, idx, j, rows, status)) {
-            if (lane == 0) m[j] = T(0);
-            continue;
-        }
-        T acc = 0;
-        for (int c = lane; c < R; c += 32) {
-            T p = 1;
-#pragma unroll
-            for (int k = 0; k < kMaxModes; k++)
-                if (k < N) p *= f.p[k][rows[k] * R + c];
-            acc += p;
-        }
-        acc = warp_sum_any(acc);
-        if (lane == 0) m[j] = acc;
+    for (int64_t j0 = warp * G; j0 < J; j0 += nwarps * G) {
+        const int64_t j = j0 + lane / L;
+        const T v = entry_model<T, V, M>(N, R, dims, j, j < J, L, gl, idx, f, status);
+        if (gl == 0 && j < J) m[j] = v;
     }
 }
 
+// The losses f(x, m) and their derivatives in m (Hong, Kolda, Duersch, Table
+// 2.1), the operations torch's autograd does on the same expressions.
+constexpr double kLossEps = 1e-10;
 template <typename T>
-__global__ void cp_adjoint_kernel(int N, int R, Dims dims, int64_t J, const int32_t* __restrict__ idx,
-                                  const T* __restrict__ gm, PtrsT<const T> f, PtrsT<T> g, int* status) {
-    const int lane = threadIdx.x & 31;
+__device__ __forceinline__ void loss_term(int kind, T x, T w, T m, T& term, T& d) {
+    if (kind == EXAFAC_LOSS_GAUSSIAN) {
+        const T r = x - m;
+        term = w * (r * r);
+        d = -(w * (T(2) * r));
+        return;
+    }
+    const T me = m + (T)kLossEps;
+    const T lg = log(me);
+    if (kind == EXAFAC_LOSS_POISSON) {
+        term = w * (m - x * lg);
+        d = w - (w * x) / me;
+    } else {
+        const T m1 = m + T(1);
+        term = w * (log(m1) - x * lg);
+        d = w / m1 - (w * x) / me;
+    }
+}
+
+// The weighted loss over the sampled entries and its derivative in each model
+// value, in one pass: no model values, loss values or derivatives of the steps
+// between go through memory, where torch's elementwise kernels took ten
+// launches (FP32, J = 2^17: model 40 us and 45 us of those; 29 us together).  Terms are summed in FP64: each thread its own, the block's in a
+// fixed tree, and the last block to finish (partial[0 .. grid) written, a
+// ticket taken) adds the blocks' sums in order, so the sum does not depend on
+// the schedule.
+template <typename T, int V, int M>
+__global__ void __launch_bounds__(256) cp_loss_kernel(int kind, int N, int R, int L, Dims dims, int64_t J,
+                                                      const int32_t* __restrict__ idx, const T* __restrict__ x,
+                                                      const T* __restrict__ w, PtrsT<const T> f, T* __restrict__ d,
+                                                      T* __restrict__ loss, double* __restrict__ partial, int* ticket,
+                                                      int* status) {
+    __shared__ double red[8];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, G = 32 / L, gl = lane & (L - 1);
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t j = warp; j < J; j += nwarps) {
-        const T gj = gm[j];
-        if (gj == T(0)) continue;  // uniform across the warp
-        int64_t rows[kMaxModes];
+    double sum = 0.0;
+    for (int64_t j0 = warp * G; j0 < J; j0 += nwarps * G) {
+        const int64_t j = j0 + lane / L;
+        const bool own = gl == 0 && j < J;
+        const T xj = own ? x[j] : T(0), wj = own ? w[j] : T(0);
+        const T m = entry_model<T, V, M>(N, R, dims, j, j < J, L, gl, idx, f, status);
+        if (own) {
+            T term, dj;
+            loss_term<T>(kind, xj, wj, m, term, dj);
+            d[j] = dj;
+            sum += (double)term;
+        }
+    }
+    sum = warp_sum(sum);
+    if (lane == 0) red[wid] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (int i = 0; i < 8; i++) s += red[i];
+        partial[blockIdx.x] = s;
+        __threadfence();
+        last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double s = 0.0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += 256) s += __ldcg(&partial[i]);
+    s = warp_sum(s);
+    if (lane == 0) red[wid] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int i = 0; i < 8; i++) t += red[i];
+        *loss = (T)t;
+    }
+}
+
+// Adds V consecutive elements to device memory: one 16-byte reduction for four
+// floats, an element at a time otherwise (there is no wider FP64 form).
+template <typename T, int V>
+__device__ __forceinline__ void add_pack(T* at, const Pack<T, V>& p) {
+    if constexpr (std::is_same<T, float>::value && V == 4) {
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(__cvta_generic_to_global(at)), "f"(p.v[0]),
+                     "f"(p.v[1]), "f"(p.v[2]), "f"(p.v[3])
+                     : "memory");
+    } else {
+#pragma unroll
+        for (int v = 0; v < V; v++) atomicAdd(at + v, p.v[v]);
+    }
+}
+
+// scale: a device scalar multiplied into every gm[j], or null.
+template <typename T, int V, int M>
+__global__ void __launch_bounds__(256) cp_adjoint_kernel(int N, int R, int L, Dims dims, int64_t J,
+                                                         const int32_t* __restrict__ idx, const T* __restrict__ gm,
+                                                         const T* __restrict__ scale, PtrsT<const T> f, PtrsT<T> g,
+                                                         int* status) {
+    const int lane = threadIdx.x & 31, G = 32 / L, gl = lane & (L - 1);
+    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const T sc = scale ? *scale : T(1);
+    for (int64_t j = warp * G + lane / L; j < J; j += nwarps * G) {
+        const T gj = scale ? gm[j] * sc : gm[j];
+        if (gj == T(0)) continue;
+        int32_t rows[M];
         if (!load_entry(N, dims, idx, j, rows, status)) continue;
-        for (int c = lane; c < R; c += 32) {
-            T v[kMaxModes];
+        for (int c = gl * V; c < R; c += L * V) {
+            Pack<T, V> v[M];
 #pragma unroll
-            for (int k = 0; k < kMaxModes; k++) v[k] = k < N ? f.p[k][rows[k] * R + c] : T(1);
+            for (int k = 0; k < M; k++)
+                if (k < N) v[k] = *reinterpret_cast<const Pack<T, V>*>(&f.p[k][(int64_t)rows[k] * R + c]);
 #pragma unroll
-            for (int n = 0; n < kMaxModes; n++) {
+            for (int n = 0; n < M; n++) {
                 if (n < N && g.p[n]) {
-                    T p = gj;
+                    Pack<T, V> p;
 #pragma unroll
-                    for (int k = 0; k < kMaxModes; k++)
-                        if (k < N && k != n) p *= v[k];
-                    atomicAdd(&g.p[n][rows[n] * R + c], p);
+                    for (int e = 0; e < V; e++) p.v[e] = gj;
+#pragma unroll
+                    for (int k = 0; k < M; k++)
+                        if (k < N && k != n)
+#pragma unroll
+                            for (int e = 0; e < V; e++) p.v[e] *= v[k].v[e];
+                    add_pack<T, V>(&g.p[n][(int64_t)rows[n] * R + c], p);
                 }
             }
         }
     }
 }
 
+// Zeroes up to kMaxModes device arrays in one launch (16-byte stores where the
+// array starts on a 16-byte boundary); lengths in 4-byte words.
+struct ZeroList {
+    uint32_t* p[kMaxModes];
+    int64_t words[kMaxModes];
+};
+__global__ void __launch_bounds__(256) zero_list_kernel(int count, ZeroList z) {
+    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int t = 0; t < count; t++) {
+        const int64_t nv = ((uintptr_t)z.p[t] & 15u) ? 0 : z.words[t] >> 2;
+        for (int64_t i = tid; i < nv; i += stride) reinterpret_cast<uint4*>(z.p[t])[i] = make_uint4(0, 0, 0, 0);
+        for (int64_t i = nv * 4 + tid; i < z.words[t]; i += stride) z.p[t][i] = 0u;
+    }
+}
 
 template <typename T>
 __global__ void gcp_sample_kernel(int N, Dims dims, int64_t nnz, const int32_t* __restrict__ nz_idx,
@@ -169,8 +322,12 @@ __device__ __forceinline__ void adam_elem(T& p, T g, T& m, T& v, const AdamCoef<
     if (c.project && p < c.lower) p = c.lower;
 }
 
-template <typename T, bool VEC>
+// V elements per access (16 bytes when every base is 16-byte aligned); bound by
+// DRAM: 64 million FP32 parameters in 0.29 ms, 6.3 TB/s.  A block per
+// contiguous tile instead of the grid-stride loop was slower (0.32 ms).
+template <typename T, int V>
 __global__ void __launch_bounds__(256) adam_step_kernel(int count, AdamTensors ts, AdamCoef<T> c) {
+    using P = Pack<T, V>;
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int t = 0; t < count; t++) {
@@ -178,32 +335,21 @@ __global__ void __launch_bounds__(256) adam_step_kernel(int count, AdamTensors t
         const T* __restrict__ g = static_cast<const T*>(ts.g[t]);
         T* __restrict__ m = static_cast<T*>(ts.m[t]);
         T* __restrict__ v = static_cast<T*>(ts.v[t]);
-        const int64_t n = ts.n[t];
-        int64_t done = 0;
-        if constexpr (VEC) {  // float4 body; every base is 16-byte aligned
-            const int64_t nv = n >> 2;
-            for (int64_t i = tid; i < nv; i += stride) {
-                float4 P = reinterpret_cast<float4*>(p)[i];
-                const float4 G = g ? reinterpret_cast<const float4*>(g)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-                float4 M = reinterpret_cast<float4*>(m)[i];
-                float4 V = reinterpret_cast<float4*>(v)[i];
-                adam_elem(P.x, G.x, M.x, V.x, c);
-                adam_elem(P.y, G.y, M.y, V.y, c);
-                adam_elem(P.z, G.z, M.z, V.z, c);
-                adam_elem(P.w, G.w, M.w, V.w, c);
-                reinterpret_cast<float4*>(p)[i] = P;
-                reinterpret_cast<float4*>(m)[i] = M;
-                reinterpret_cast<float4*>(v)[i] = V;
-            }
-            done = nv << 2;
+        const int64_t n = ts.n[t], nv = n / V;
+        for (int64_t i = tid; i < nv; i += stride) {
+            P a = reinterpret_cast<P*>(p)[i], b = reinterpret_cast<P*>(m)[i], d = reinterpret_cast<P*>(v)[i], e;
+            if (g)
+                e = reinterpret_cast<const P*>(g)[i];
+            else
+#pragma unroll
+                for (int u = 0; u < V; u++) e.v[u] = T(0);
+#pragma unroll
+            for (int u = 0; u < V; u++) adam_elem(a.v[u], e.v[u], b.v[u], d.v[u], c);
+            reinterpret_cast<P*>(p)[i] = a;
+            reinterpret_cast<P*>(m)[i] = b;
+            reinterpret_cast<P*>(v)[i] = d;
         }
-        for (int64_t i = done + tid; i < n; i += stride) {
-            T P = p[i], M = m[i], V = v[i];
-            adam_elem(P, g ? g[i] : T(0), M, V, c);
-            p[i] = P;
-            m[i] = M;
-            v[i] = V;
-        }
+        for (int64_t i = nv * V + tid; i < n; i += stride) adam_elem(p[i], g ? g[i] : T(0), m[i], v[i], c);
     }
 }
 
@@ -229,6 +375,68 @@ static int dims_arg(int N, const int64_t* dims, Dims* d) {
     return EXAFAC_OK;
 }
 
+// 16-byte accesses need rows that are a multiple of 16 bytes and bases on a
+// 16-byte boundary.
+static bool packable(int R, int N, const void* const* a, const void* const* b, int dtype) {
+    if ((int64_t)R * (dtype == EXAFAC_DTYPE_F32 ? 4 : 8) % 16) return false;
+    for (int k = 0; k < N; k++) {
+        if ((uintptr_t)a[k] & 15u) return false;
+        if (b && ((uintptr_t)b[k] & 15u)) return false;
+    }
+    return true;
+}
+
+template <typename T>
+static PtrsT<T> ptrs_of(int N, const void* const* a) {
+    PtrsT<T> f{};
+    for (int k = 0; k < N; k++) f.p[k] = static_cast<T*>(const_cast<void*>(a[k]));
+    return f;
+}
+
+template <typename T, int V, int M>
+static void launch_model(int N, int R, const Dims& d, int64_t J, const int32_t* idx, const void* const* factors,
+                         void* m, int* status, cudaStream_t st) {
+    const int L = entry_lanes(R, V);
+    cp_model_kernel<T, V, M><<<grid_for(J, 8 * (32 / L)), 256, 0, st>>>(N, R, L, d, J, idx, ptrs_of<const T>(N, factors),
+                                                                    static_cast<T*>(m), status);
+}
+
+template <typename T, int V, int M>
+static void launch_adjoint(int N, int R, const Dims& d, int64_t J, const int32_t* idx, const void* gm,
+                           const void* scale, const void* const* factors, void* const* grads, int* status,
+                           cudaStream_t st) {
+    const int L = entry_lanes(R, V);
+    cp_adjoint_kernel<T, V, M><<<grid_for(J, 8 * (32 / L)), 256, 0, st>>>(
+        N, R, L, d, J, idx, static_cast<const T*>(gm), static_cast<const T*>(scale), ptrs_of<const T>(N, factors),
+        ptrs_of<T>(N, grads), status);
+}
+
+template <typename T, int V, int M>
+static void launch_loss(int kind, int N, int R, const Dims& d, int64_t J, const int32_t* idx, const void* x,
+                        const void* w, const void* const* factors, void* deriv, void* loss, double* partial,
+                        int* ticket, int* status, cudaStream_t st) {
+    const int L = entry_lanes(R, V);
+    cp_loss_kernel<T, V, M><<<std::min<int>(grid_for(J, 8 * (32 / L)), EXAFAC_LOSS_BLOCKS), 256, 0, st>>>(
+        kind, N, R, L, d, J, idx, static_cast<const T*>(x), static_cast<const T*>(w), ptrs_of<const T>(N, factors),
+        static_cast<T*>(deriv), static_cast<T*>(loss), partial, ticket, status);
+}
+
+#define GCP_DISPATCH_MODES(fn, T, V, ...) (N <= 4 ? fn<T, V, 4> : fn<T, V, kMaxModes>)(__VA_ARGS__)
+#define GCP_DISPATCH(fn, pack, ...)                           \
+    do {                                                      \
+        const bool p_ = (pack);                               \
+        if (dtype == EXAFAC_DTYPE_F32) {                      \
+            if (p_)                                           \
+                GCP_DISPATCH_MODES(fn, float, 4, __VA_ARGS__); \
+            else                                              \
+                GCP_DISPATCH_MODES(fn, float, 1, __VA_ARGS__); \
+        } else if (p_) {                                      \
+            GCP_DISPATCH_MODES(fn, double, 2, __VA_ARGS__);   \
+        } else {                                              \
+            GCP_DISPATCH_MODES(fn, double, 1, __VA_ARGS__);   \
+        }                                                     \
+    } while (0)
+
 extern "C" int exafac_cp_sampled_model(int32_t N, int32_t R, const int64_t* dims, int64_t J, const int32_t* idx,
                                        const void* const* factors, void* m_out, int32_t dtype, int32_t* status,
                                        void* stream) {
@@ -242,16 +450,7 @@ extern "C" int exafac_cp_sampled_model(int32_t N, int32_t R, const int64_t* dims
     EXAFAC_ARG(idx && factors && m_out, "null argument");
     for (int k = 0; k < N; k++) EXAFAC_ARG(factors[k] != nullptr, "null factor matrix");
     cudaStream_t st = (cudaStream_t)stream;
-    const int grid = grid_for(J, 8);
-    if (dtype == EXAFAC_DTYPE_F32) {
-        PtrsT<const float> f{};
-        for (int k = 0; k < N; k++) f.p[k] = static_cast<const float*>(factors[k]);
-        cp_model_kernel<float><<<grid, 256, 0, st>>>(N, R, d, J, idx, f, static_cast<float*>(m_out), status);
-    } else {
-        PtrsT<const double> f{};
-        for (int k = 0; k < N; k++) f.p[k] = static_cast<const double*>(factors[k]);
-        cp_model_kernel<double><<<grid, 256, 0, st>>>(N, R, d, J, idx, f, static_cast<double*>(m_out), status);
-    }
+    GCP_DISPATCH(launch_model, packable(R, N, factors, nullptr, dtype), N, R, d, J, idx, factors, m_out, status, st);
     count_launch();
     EXAFAC_CHECK_LAUNCH();
     return EXAFAC_OK;
@@ -270,26 +469,64 @@ extern "C" int exafac_cp_sampled_adjoint(int32_t N, int32_t R, const int64_t* di
     EXAFAC_ARG(idx && grad_m && factors && grads, "null argument");
     for (int k = 0; k < N; k++) EXAFAC_ARG(factors[k] != nullptr, "null factor matrix");
     cudaStream_t st = (cudaStream_t)stream;
-    const int grid = grid_for(J, 8);
-    if (dtype == EXAFAC_DTYPE_F32) {
-        PtrsT<const float> f{};
-        PtrsT<float> g{};
-        for (int k = 0; k < N; k++) {
-            f.p[k] = static_cast<const float*>(factors[k]);
-            g.p[k] = static_cast<float*>(grads[k]);
+    GCP_DISPATCH(launch_adjoint, packable(R, N, factors, grads, dtype), N, R, d, J, idx, grad_m, nullptr, factors,
+                 grads, status, st);
+    count_launch();
+    EXAFAC_CHECK_LAUNCH();
+    return EXAFAC_OK;
+}
+
+extern "C" int exafac_cp_sampled_loss(int32_t kind, int32_t N, int32_t R, const int64_t* dims, int64_t J,
+                                      const int32_t* idx, const void* x, const void* w, const void* const* factors,
+                                      void* deriv_out, void* loss_out, void* scratch, int32_t dtype, int32_t* status,
+                                      void* stream) {
+    EXAFAC_ARG(kind >= EXAFAC_LOSS_POISSON && kind <= EXAFAC_LOSS_GAUSSIAN, "unknown loss");
+    EXAFAC_ARG(N >= 1 && N <= kMaxModes, "N must be in [1, 8]");
+    EXAFAC_ARG(R >= 1, "R must be >= 1");
+    EXAFAC_ARG(J >= 1, "J must be >= 1");
+    GCP_DTYPE_ARG(dtype);
+    Dims d;
+    EXAFAC_TRY(dims_arg(N, dims, &d));
+    EXAFAC_ARG(idx && x && w && factors && deriv_out && loss_out && scratch, "null argument");
+    EXAFAC_ARG(((uintptr_t)scratch & 7u) == 0, "scratch must be 8-byte aligned");
+    for (int k = 0; k < N; k++) EXAFAC_ARG(factors[k] != nullptr, "null factor matrix");
+    cudaStream_t st = (cudaStream_t)stream;
+    double* partial = static_cast<double*>(scratch) + 1;
+    int* ticket = static_cast<int*>(scratch);
+    EXAFAC_CUDA_TRY(cudaMemsetAsync(ticket, 0, sizeof(int), st));
+    GCP_DISPATCH(launch_loss, packable(R, N, factors, nullptr, dtype), kind, N, R, d, J, idx, x, w, factors,
+                 deriv_out, loss_out, partial, ticket, status, st);
+    count_launch();
+    EXAFAC_CHECK_LAUNCH();
+    return EXAFAC_OK;
+}
+
+extern "C" int exafac_cp_sampled_gradient(int32_t N, int32_t R, const int64_t* dims, int64_t J, const int32_t* idx,
+                                          const void* grad_m, const void* scale, const void* const* factors,
+                                          void* const* grads, int32_t dtype, int32_t* status, void* stream) {
+    EXAFAC_ARG(N >= 1 && N <= kMaxModes, "N must be in [1, 8]");
+    EXAFAC_ARG(R >= 1, "R must be >= 1");
+    EXAFAC_ARG(J >= 1, "J must be >= 1");
+    GCP_DTYPE_ARG(dtype);
+    Dims d;
+    EXAFAC_TRY(dims_arg(N, dims, &d));
+    EXAFAC_ARG(idx && grad_m && factors && grads, "null argument");
+    for (int k = 0; k < N; k++) EXAFAC_ARG(factors[k] != nullptr, "null factor matrix");
+    cudaStream_t st = (cudaStream_t)stream;
+    ZeroList z{};
+    int count = 0;
+    int64_t most = 0;
+    for (int k = 0; k < N; k++)
+        if (grads[k]) {
+            z.p[count] = static_cast<uint32_t*>(grads[k]);
+            z.words[count] = dims[k] * R * (dtype == EXAFAC_DTYPE_F32 ? 1 : 2);
+            most = std::max(most, z.words[count++]);
         }
-        cp_adjoint_kernel<float><<<grid, 256, 0, st>>>(N, R, d, J, idx, static_cast<const float*>(grad_m), f, g,
-                                                       status);
-    } else {
-        PtrsT<const double> f{};
-        PtrsT<double> g{};
-        for (int k = 0; k < N; k++) {
-            f.p[k] = static_cast<const double*>(factors[k]);
-            g.p[k] = static_cast<double*>(grads[k]);
-        }
-        cp_adjoint_kernel<double><<<grid, 256, 0, st>>>(N, R, d, J, idx, static_cast<const double*>(grad_m), f, g,
-                                                        status);
-    }
+    if (count == 0) return EXAFAC_OK;
+    zero_list_kernel<<<grid_for(most / 4 + 1, 256), 256, 0, st>>>(count, z);
+    count_launch();
+    GCP_DISPATCH(launch_adjoint, packable(R, N, factors, grads, dtype), N, R, d, J, idx, grad_m, scale, factors,
+                 grads, status, st);
     count_launch();
     EXAFAC_CHECK_LAUNCH();
     return EXAFAC_OK;
@@ -338,14 +575,12 @@ static void launch_adam(int count, const AdamTensors& ts, int64_t total, double 
     c.eps = (T)eps;
     c.lower = (T)lower;
     c.project = project;
-    const int grid = grid_for(vec ? (total + 3) / 4 : total, 256);
-    if constexpr (std::is_same<T, float>::value) {
-        if (vec) {
-            adam_step_kernel<float, true><<<grid, 256, 0, st>>>(count, ts, c);
-            return;
-        }
-    }
-    adam_step_kernel<T, false><<<grid, 256, 0, st>>>(count, ts, c);
+    constexpr int V = 16 / sizeof(T);
+    const int grid = grid_for(vec ? (total + V - 1) / V : total, 256);
+    if (vec)
+        adam_step_kernel<T, V><<<grid, 256, 0, st>>>(count, ts, c);
+    else
+        adam_step_kernel<T, 1><<<grid, 256, 0, st>>>(count, ts, c);
 }
 
 extern "C" int exafac_adam_step(int32_t count, void* const* params, const void* const* grads, void* const* exp_avg,
@@ -361,7 +596,7 @@ extern "C" int exafac_adam_step(int32_t count, void* const* params, const void* 
     EXAFAC_ARG(params && exp_avg && exp_avg_sq && numel, "null argument");
     AdamTensors ts{};
     int64_t total = 0;
-    bool vec = dtype == EXAFAC_DTYPE_F32;
+    bool vec = true;  // 16-byte accesses
     for (int t = 0; t < count; t++) {
         EXAFAC_ARG(numel[t] >= 0, "element counts must be >= 0");
         EXAFAC_ARG(numel[t] == 0 || (params[t] && exp_avg[t] && exp_avg_sq[t]), "null parameter or moment");
@@ -379,7 +614,7 @@ extern "C" int exafac_adam_step(int32_t count, void* const* params, const void* 
     if (dtype == EXAFAC_DTYPE_F32)
         launch_adam<float>(count, ts, total, lr, beta1, beta2, eps, step, project, lower, vec, st);
     else
-        launch_adam<double>(count, ts, total, lr, beta1, beta2, eps, step, project, lower, false, st);
+        launch_adam<double>(count, ts, total, lr, beta1, beta2, eps, step, project, lower, vec, st);
     count_launch();
     EXAFAC_CHECK_LAUNCH();
     return EXAFAC_OK;

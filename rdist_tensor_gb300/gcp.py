@@ -9,7 +9,8 @@ the factors instead of stored.  A loss on the sampled entries (Poisson,
 Bernoulli or Gaussian) written in torch then gives gradient-based GCP
 (Hong, Kolda and Duersch, "Generalized canonical polyadic tensor
 decomposition", SIAM Review 2020) driven by the stratified sampler
-``exafac_gcp_sample_entries``.
+``exafac_gcp_sample_entries``.  A step's own objective takes the model, the
+loss and its derivative in one kernel (``SampledLoss``).
 
 This part has no counterpart in the reference; its nearest relatives there
 are execute_exact_mttkrp (exafac/cpp_ext/sort_lookup.hpp:440-495) and the
@@ -26,6 +27,8 @@ import torch
 from . import _lib
 
 _DTYPES = {torch.float32: 0, torch.float64: 1}
+_LOSSES = {"poisson": 0, "bernoulli": 1, "gaussian": 2}
+_LOSS_SCRATCH = 2432 + 1  # doubles: EXAFAC_LOSS_SCRATCH_BYTES of the C header
 EPS = 1e-10
 
 
@@ -87,6 +90,42 @@ class SampledCPModel(torch.autograd.Function):
                   ctypes.c_void_p(gm.data_ptr()), _ptrs(factors), _ptrs(grads), _DTYPES[dt],
                   ctypes.c_void_p(ctx.status.data_ptr()), _stream())
         return (None, *grads)
+
+
+class SampledLoss(torch.autograd.Function):
+    """f = SampledLoss.apply(kind, idx, x, w, *factors): the weighted loss over
+    the sampled entries, ``(w * loss_values(kind, x, sampled_model(idx,
+    factors))).sum()`` for x and w of the factors' dtype that need no
+    gradient, with the model, the loss and its derivative in one kernel and
+    the sum in FP64 (``exafac_cp_sampled_loss``); backward is the sampled
+    MTTKRP of the derivatives (``exafac_cp_sampled_gradient``)."""
+
+    @staticmethod
+    def forward(ctx, kind: str, idx: torch.Tensor, x: torch.Tensor, w: torch.Tensor,
+                *factors: torch.Tensor) -> torch.Tensor:
+        dt, R = _check(idx, factors)
+        N, J = len(factors), idx.shape[0]
+        d = torch.empty_like(x)
+        loss = torch.empty((), dtype=dt, device=idx.device)
+        scratch = torch.empty(_LOSS_SCRATCH, dtype=torch.float64, device=idx.device)
+        _lib.call("exafac_cp_sampled_loss", _LOSSES[kind], N, R, _dims_arg([U.shape[0] for U in factors]), J,
+                  ctypes.c_void_p(idx.data_ptr()), ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(w.data_ptr()),
+                  _ptrs(factors), ctypes.c_void_p(d.data_ptr()), ctypes.c_void_p(loss.data_ptr()),
+                  ctypes.c_void_p(scratch.data_ptr()), _DTYPES[dt], None, _stream())
+        ctx.save_for_backward(idx, d, *factors)
+        return loss
+
+    @staticmethod
+    def backward(ctx, grad: torch.Tensor):
+        idx, d, *factors = ctx.saved_tensors
+        dt, R = _check(idx, factors)
+        N, J = len(factors), idx.shape[0]
+        grads = [torch.empty_like(U) if ctx.needs_input_grad[4 + k] else None for k, U in enumerate(factors)]
+        grad = grad.to(dt)
+        _lib.call("exafac_cp_sampled_gradient", N, R, _dims_arg([U.shape[0] for U in factors]), J,
+                  ctypes.c_void_p(idx.data_ptr()), ctypes.c_void_p(d.data_ptr()), ctypes.c_void_p(grad.data_ptr()),
+                  _ptrs(factors), _ptrs(grads), _DTYPES[dt], None, _stream())
+        return (None, None, None, None, *grads)
 
 
 def sampled_model(idx: torch.Tensor, factors: Sequence[torch.Tensor]) -> torch.Tensor:
@@ -214,6 +253,19 @@ class GCP:
         m = sampled_model(idx, self.factors)
         return (w * loss_values(self.loss, x, m)).sum()
 
+    def _step_objective(self, idx, x, w) -> torch.Tensor:
+        """``objective`` of a step's own sample: the fused loss (3 launches
+        forward and backward where the torch expression takes 19) when the
+        sample and the objective are this class's and the sample's type is the
+        factors'; an overridden objective or sampler, an empty sample and an
+        unknown loss take the expression."""
+        cls = type(self)
+        own = (cls.objective is GCP.objective and cls.step_sample is GCP.step_sample
+               and "objective" not in self.__dict__ and "step_sample" not in self.__dict__)
+        if own and self.loss in _LOSSES and idx.shape[0] > 0 and x.dtype == self.factors[0].dtype:
+            return SampledLoss.apply(self.loss, idx, x, w, *self.factors)
+        return self.objective(idx, x, w)
+
     def step_sample(self, J_nz: int, J_z: int):
         out = sample_entries(self.idx, self.vals, self.dims, J_nz, J_z, self.seed, self.counter)
         self.counter += 1
@@ -238,8 +290,11 @@ class GCP:
         opt = self.optimizer(lr)
         idx, x, w = self.step_sample(J_nz, J_z)
         opt.zero_grad(set_to_none=True)
-        f = self.objective(idx, x, w)
-        f.backward()
+        f = self._step_objective(idx, x, w)
+        # on this thread: the hand-over to the engine's device thread and back
+        # was 0.2 ms of a small step's 0.35 ms
+        with torch.autograd.grad_mode.set_multithreading_enabled(False):
+            f.backward()
         opt.step()
         return f.detach()
 
