@@ -614,7 +614,7 @@ static int sts_draw_launch(Session& s, int n, int64_t J, const double* uni, cons
     const size_t smem = (size_t)S * sample_group_bytes(s.R, sizeof(T));
     if (smem > 48 * 1024)
         EXAFAC_CUDA_TRY(cudaFuncSetAttribute(sts_draw_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int64_t blocks = std::max<int64_t>(std::min<int64_t>(ceil_div(J, S), 152 * (list ? 2 : 32)), 1);
+    const int64_t blocks = std::max<int64_t>(std::min<int64_t>(ceil_div(J, S), 152 * (list ? 4 : 32)), 1);
     sts_draw_kernel<T><<<(unsigned)blocks, S * G * 32, smem, st>>>(N, n, s.R, G, S, J, m, s.etree, eigG, E, PhiP, uni,
                                                                    s.samples, s.weights, s.status, list, list_count);
     count_launch();

@@ -38,12 +38,11 @@
 //   E = n1 (R 4.6 2^-34 + 1.7 2^-32) + R^2 2^-44
 // A cutoff low + q / m is then off by at most E / m for the root mass, E / m
 // for its own mass and E / m per earlier right turn.  The leaf's row is picked
-// from FP32 squares of dots with 30-bit x, with its own bound (zq_leaf_kernel).
+// from FP32 squares of dots with 30-bit x, with its own bound (zq_leaf_kernel),
+// and from FP64 dots where that bound leaves it open (zq_place_kernel).
 //
 // Measured (GB300), draws of a step: R = 64, J = 2^18, three 2000-row modes:
-// 55.8 -> 7.9 ms; R = 25, J = 65536: 4.3 -> 1.4 ms; about one sample in 1e4
-// is marked (the FP32 squares of the leaf stage), its depth-first draw 0.1 to
-// 0.5 ms a step (the latency of one sample).
+// 55.8 -> 7.9 ms; R = 25, J = 65536: 4.3 -> 1.4 ms.
 #include "engine.cuh"
 #include "prims.cuh"
 #include "umma.cuh"
@@ -656,11 +655,16 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
     }
 }
 
+// The common exponent of a leaf's rows from the largest of its Gram's diagonal
+// exponents: max G_jj < 2^(e - 1022), |U| < 2^ceil((e - 1022) / 2); one more
+// for rounding.
+__device__ __forceinline__ int z_leaf_exp(int e) { return e >= 2047 ? 2047 : ((e - 1022 + 2047) >> 1) - 1023 + 1 + 1022; }
+
 // The leaf stage: dots v_r = U_r . x of the leaf's rows from four digits of
 // each (weights <= 3), their FP32 squares' prefix in row order, and the row
 // whose range (before, before + v_r^2] holds frac x total, frac = (d - low) /
 // (high - low), when frac x total keeps a distance from both ends that
-// covers every error; otherwise the sample is marked.  In scaled units
+// covers every error; otherwise the sample is listed for zq_place_kernel.  In scaled units
 // (|x'|, |U'| < 2^6): a dot is off by at most e0 = R 5.2 2^-18 plus 2^-24 of
 // itself, so a prefix by 2 e0 sqrt(F total) + F e0^2 + 70 2^-24 total, and
 // frac by (err_low + err_high) / (high - low).
@@ -731,8 +735,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
                 int e = 0;
                 for (int a = lane; a < R; a += 32) e = max(e, bexp(__ldg(G + (int64_t)c * P + packed_index(R, a, a))));
                 e = __reduce_max_sync(0xffffffffu, e);
-                // max G_jj < 2^(e - 1022): |U| < 2^ceil((e - 1022) / 2); one more for rounding
-                if (lane == 0) diag_exp = e >= 2047 ? 2047 : ((e - 1022 + 2047) >> 1) - 1023 + 1 + 1022;
+                if (lane == 0) diag_exp = z_leaf_exp(e);
             }
             __syncthreads();
             const int emax = diag_exp;
@@ -817,7 +820,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
                     }
                 }
                 // delta is a finite number only if every input was; a sample
-                // that no thread places is marked
+                // that no thread places is left to zq_place_kernel
                 if (found && width > 0.0 && total > 0.0f && delta < total && emax < 2047)
                     b.pick[j] = at;
             }
@@ -825,7 +828,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
             if (tid >= i0 && tid < i1) {
                 const int32_t j = js[tid];
                 const int at = b.pick[j];
-                if (at < 0) z_mark(b.redo, b.redo_list, b.redo_count, j);
+                if (at < 0) b.near_list[atomicAdd(b.near_count, 1)] = j;  // zq_place_kernel
                 samples[(int64_t)j * N + col] = (uint32_t)(leaf * F + max(at, 0));
             }
             i0 = i1;
@@ -845,6 +848,93 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
     if (w == 0) {
         tc_fence_after();
         tmem_dealloc(tmem, 128);
+    }
+}
+
+// The listed samples' rows (three to twelve in a thousand: the FP32 squares'
+// rounding), a block per sample in turn: the leaf's dots, squares and prefix
+// in FP64 from the fixed-point vector, eight lanes per row.  In scaled units a
+// dot, and the depth-first kernel's own, is off by at most e1 = R (2^-42 +
+// 2^-45 n1) (the vector's rounding, the two sums'), a prefix by 2 e1 sqrt(F
+// total) + F e1^2 + F 2^-50 total, frac as in zq_leaf_kernel.  A sample that
+// is still within the bound is marked.  Drawing the listed samples again depth
+// first took 0.46 ms a step at R = 64, J = 2^18 and 1.8 ms at R = 100, J =
+// 100003, four modes.
+constexpr int kPlaceThreads = 256;
+__global__ void __launch_bounds__(kPlaceThreads)
+    zq_place_kernel(int R, TreeShape t, const double* __restrict__ G, const double* __restrict__ U, ZState b,
+                    const double* __restrict__ dv, int N, int col, uint32_t* __restrict__ samples) {
+    __shared__ double xs[kMaxRank], sq[kMaxLeafRows];
+    __shared__ int diag_exp;
+    const int tid = threadIdx.x, lane = tid & 31, P = packed_size(R), F = (int)t.F;
+    const int count = *b.near_count;
+    for (int q = blockIdx.x; q < count; q += gridDim.x) {
+        const int32_t j = b.near_list[q];
+        const int64_t c = b.node[j];
+        const int64_t leaf = tree_leaf_idx(t, c);
+        const int rows = (int)min((int64_t)F, t.n - leaf * F);
+        const double* Ub = U + leaf * F * R;
+        if (tid < 32) {
+            int e = 0;
+            for (int a = lane; a < R; a += 32) e = max(e, bexp(__ldg(G + c * P + packed_index(R, a, a))));
+            e = __reduce_max_sync(0xffffffffu, e);
+            if (lane == 0) diag_exp = z_leaf_exp(e);
+        }
+        const long long* X = reinterpret_cast<const long long*>(b.xi) + (int64_t)j * z_row(R);
+        for (int a = tid; a < R; a += kPlaceThreads) xs[a] = (double)X[a] * 0x1p-47;
+        __syncthreads();
+        const int emax = diag_exp;
+        const double scale = scalbn(1.0, max(min(1028 - emax, 1000), -1000));
+        for (int r0 = 0; r0 < F; r0 += kPlaceThreads / 8) {
+            const int r = r0 + (tid >> 3);
+            double v = 0.0;
+            if (r < rows)
+                for (int a = tid & 7; a < R; a += 8) v = fma(__ldg(Ub + (int64_t)r * R + a), xs[a], v);
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            v *= scale;
+            if ((tid & 7) == 0 && r < F) sq[r] = v * v;
+        }
+        __syncthreads();
+        if (tid < 32) {
+            double incl[4], own[4], total = 0.0;
+#pragma unroll
+            for (int blk = 0; blk < 4; blk++) {
+                const int r = 32 * blk + lane;
+                double v = r < F ? sq[r] : 0.0;
+                own[blk] = v;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const double u = __shfl_up_sync(0xffffffffu, v, o);
+                    if (lane >= o) v += u;
+                }
+                incl[blk] = total + v;
+                total += __shfl_sync(0xffffffffu, v, 31);
+            }
+            const double2 lh = b.lh[j];
+            const float2 er = b.err[j];
+            const double width = lh.y - lh.x;
+            const double thr = (dv[j] - lh.x) / width * total;
+            const double de = 1.001 * ((double)er.x + (double)er.y + 0x1p-49) / width * total;
+            const double e1 = (double)R * (0x1p-42 + (double)b.n1[j] * 0x1p-45);
+            const double delta =
+                1.01 * (de + 2.0 * e1 * sqrt((double)F * total) + (double)F * e1 * e1 + (double)F * 0x1p-50 * total);
+            const bool usable = width > 0.0 && total > 0.0 && delta < total && emax < 2047 && emax > 28;
+            int at = -1;
+#pragma unroll
+            for (int blk = 0; blk < 4; blk++) {
+                const int r = 32 * blk + lane;
+                const bool hit = usable && r < rows && thr < incl[blk] - delta &&
+                                 (r == 0 || thr > (incl[blk] - own[blk]) + delta);
+                const unsigned mask = __ballot_sync(0xffffffffu, hit);
+                if (at < 0 && mask) at = 32 * blk + __ffs(mask) - 1;
+            }
+            if (lane == 0) {
+                if (at < 0) z_mark(b.redo, b.redo_list, b.redo_count, j);
+                else samples[(int64_t)j * N + col] = (uint32_t)(leaf * F + at);
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -1006,6 +1096,7 @@ __global__ void zq_vector_kernel(int R, int64_t J, double* __restrict__ h, const
             b.pick[j] = -1;
             if (KIND == 0) b.redo[j] = 0;
             if (KIND == 0 && j == 0) *b.redo_count = 0;
+            if (j == 0) *b.near_count = 0;
             if ((j & 127) == 0) {
                 const int64_t tile = j >> 7;
                 reinterpret_cast<uint4*>(b.mask[0])[tile] = make_uint4(0u, 0u, 0u, 0u);
@@ -1288,6 +1379,8 @@ void zq_carve(Arena& a, ZState& b, int R, int64_t J, int64_t widest, int trees) 
     b.redo = a.take<int32_t>(J);
     b.redo_list = a.take<int32_t>(J);
     b.redo_count = a.take<int32_t>(1);
+    b.near_list = a.take<int32_t>(J);
+    b.near_count = a.take<int32_t>(1);
     for (int q = 0; q < 2; q++) {
         b.mask[q] = a.take<uint32_t>(4 * ceil_div(J, kZTile));
         b.tcount[q] = a.take<int32_t>(ceil_div(J, kZTile) + 4);
@@ -1348,7 +1441,7 @@ static int z_descend(Session& s, const TreeShape& t, const double* G, const doub
     const int64_t ntiles = ceil_div(J, kZTile);
     const bool in_smem = ntiles <= kZPrefSmem;
     const size_t psm = in_smem ? sizeof(int32_t) * (ntiles + 1) : 0;
-    if (psm > 48 * 1024)
+    if (psm > 40 * 1024)  // (the 48 KB of a launch without it include the static part)
         EXAFAC_CUDA_TRY(
             cudaFuncSetAttribute(zq_partition_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
     const bool tail = t.node_count > t.nodes_upto_lfill;
@@ -1380,6 +1473,11 @@ static int z_descend(Session& s, const TreeShape& t, const double* G, const doub
         EXAFAC_TRY(z_leaf<256>(s, t, G, U, J, p, order, dv, col, st));
     } else {
         EXAFAC_TRY(z_leaf<512>(s, t, G, U, J, p, order, dv, col, st));
+    }
+    if (t.F > 1) {
+        zq_place_kernel<<<(unsigned)std::min<int64_t>(J, 152 * 4), kPlaceThreads, 0, st>>>(s.R, t, G, U, b, dv, s.N, col,
+                                                                                         s.samples);
+        count_launch();
     }
     EXAFAC_CHECK_LAUNCH();
     return EXAFAC_OK;
