@@ -245,89 +245,122 @@ __global__ void syev_kernel(int R, const double* __restrict__ A, int64_t a_strid
 //      outputs.  X that is not orthonormal to 4 R eps, or a value that is not
 //      finite, starts the sweeps from A as before.
 // Measured (GB300, a batch of 3, launches included): R = 25 / 64 / 100 / 128:
-// 0.24 / 0.69 / 2.2 / 2.9 ms (the FP64 sweeps alone 0.88 / 5.2 / 17.6 / 35.9),
+// 0.20 / 0.57 / 1.9 / 2.5 ms (the FP64 sweeps alone 0.88 / 5.2 / 17.6 / 35.9),
 // |A v - lambda v| <= 6e-16 |A| against 5e-15 .. 3e-14, a 92-fold near-null
 // cluster at R = 100 11 against 26 ms.
 // ---------------------------------------------------------------------------
 constexpr int kRefineSteps = 4;
 constexpr int kJacobi32MaxSweeps = 10;
 
-// Cyclic Jacobi in FP32 on the full symmetric matrix a (Re x Re, shared), v
-// (Re x Re, shared) <- V^T (row i = eigenvector i).  A pair rotates while
-// |a_pq| > max(2^-22 sqrt|a_pp a_qq|, floor).  A round's rotations act on
-// disjoint pairs, so the two-sided update is independent 2 x 2 blocks.
-struct Jacobi32Smem {
-    float2 cs[kMaxRank / 2];
-    int2 pq[kMaxRank / 2];
-    int flag;
-};
+// Cyclic Jacobi in FP32 on the full symmetric matrix a (Re x Re, shared; two
+// buffers of it), v (Re x Re, shared) <- V^T (row i = eigenvector i).  A pair
+// rotates while |a_pq| > max(2^-22 sqrt|a_pp a_qq|, floor).  A round's
+// rotations act on disjoint pairs, so the two-sided update is independent 2 x
+// 2 blocks J_i^T a_ij J_j: a warp per pair i, its lanes along j, then along
+// the rows of V^T.  A round is latency and shared memory's bandwidth (0.97 /
+// 1.06 / 2.07 us at R = 25 / 64 / 100 with the angles in one warp, a second
+// barrier and IEEE divisions; 0.6 / 0.77 / 1.75 us as it is): every
+// warp forms all the angles itself, a pair (kPairs of them) per lane, and the
+// blocks go from one buffer to the other, so that one barrier remains.  The
+// rotations need no more than FP32's approximate quotients (the refinement
+// makes the vectors orthonormal).
 __device__ __forceinline__ bool jacobi32_rotates(float apq, float app, float aqq, float floor) {
-    return fabsf(apq) > fmaxf(0x1p-22f * sqrtf(fabsf(app) * fabsf(aqq)), floor);
+    return fabsf(apq) > floor && apq * apq > 0x1p-44f * fabsf(app * aqq);
 }
-__device__ void jacobi32_block(int R, float* a, float* v, float floor, Jacobi32Smem* sm) {
+template <int kPairs>
+__device__ void jacobi32_sweeps(int R, float* cur, float* nxt, float* v, float floor, int* flag) {
     const int Re = R + (R & 1), m = Re - 1, np = Re / 2, ld = Re;
-    const int tid = threadIdx.x, nt = blockDim.x;
+    const int tid = threadIdx.x, nt = blockDim.x, w = tid >> 5, nw = nt >> 5, lane = tid & 31;
     for (int e = tid; e < Re * Re; e += nt) v[e] = e / Re == e % Re ? 1.0f : 0.0f;
     __syncthreads();
     for (int sweep = 0; sweep < kJacobi32MaxSweeps && R > 1; sweep++) {
-        if (tid == 0) sm->flag = 0;
+        if (tid == 0) *flag = 0;
         __syncthreads();
         bool any = false;  // a look at every pair: a converged matrix ends here
-        for (int i = tid >> 5; i < R && !any; i += nt >> 5)
-            for (int j = i + 1 + (tid & 31); j < R; j += 32)
-                any = any || jacobi32_rotates(a[i * ld + j], a[i * ld + i], a[j * ld + j], floor);
-        if (any) sm->flag = 1;
+        for (int i = w; i < R && !any; i += nw)
+            for (int j = i + 1 + lane; j < R; j += 32)
+                any = any || jacobi32_rotates(cur[i * ld + j], cur[i * ld + i], cur[j * ld + j], floor);
+        if (any) *flag = 1;
         __syncthreads();
-        if (!sm->flag) break;
+        if (!*flag) break;
         for (int t = 0; t < m; t++) {
-            if (tid < np) {
-                int p, q;
-                rr_pair(t, tid, m, p, q);
-                float c = 1.0f, s = 0.0f;
-                const float apq = a[p * ld + q], app = a[p * ld + p], aqq = a[q * ld + q];
-                if (q < R && jacobi32_rotates(apq, app, aqq, floor)) {
-                    const float tau = (aqq - app) / (2.0f * apq);
-                    const float tt = copysignf(1.0f, tau) / (fabsf(tau) + sqrtf(fmaf(tau, tau, 1.0f)));
-                    c = rsqrtf(fmaf(tt, tt, 1.0f));
-                    s = tt * c;
-                }
-                sm->cs[tid] = make_float2(c, s);
-                sm->pq[tid] = make_int2(p, q);
-            }
-            __syncthreads();
-            // the 2 x 2 blocks J_i^T a_ij J_j, and the rows of V^T: a warp per
-            // pair i, its lanes along j and along the row
-            for (int i = tid >> 5; i < np; i += nt >> 5) {
-                const float2 ri = sm->cs[i];
-                const int2 pi = sm->pq[i];
-                float* rp = a + pi.x * ld;
-                float* rq = a + pi.y * ld;
-                for (int j = tid & 31; j < np; j += 32) {
-                    const float2 rj = sm->cs[j];
-                    if (ri.y == 0.0f && rj.y == 0.0f) continue;
-                    const int2 pj = sm->pq[j];
-                    const float pp = rp[pj.x], pqv = rp[pj.y], qp = rq[pj.x], qq = rq[pj.y];
-                    const float l0 = ri.x * pp - ri.y * qp, l1 = ri.x * pqv - ri.y * qq;
-                    const float m0 = ri.y * pp + ri.x * qp, m1 = ri.y * pqv + ri.x * qq;
-                    rp[pj.x] = rj.x * l0 - rj.y * l1;
-                    rp[pj.y] = rj.y * l0 + rj.x * l1;
-                    rq[pj.x] = rj.x * m0 - rj.y * m1;
-                    rq[pj.y] = rj.y * m0 + rj.x * m1;
-                }
-                if (ri.y == 0.0f) continue;
-                float* vp = v + pi.x * ld;
-                float* vq = v + pi.y * ld;
-                for (int r = tid & 31; r < Re; r += 32) {
-                    const float x = vp[r], y = vq[r];
-                    vp[r] = ri.x * x - ri.y * y;
-                    vq[r] = ri.y * x + ri.x * y;
+            float c[kPairs], s[kPairs];
+            int p[kPairs], q[kPairs];
+            bool rot = false;
+#pragma unroll
+            for (int h = 0; h < kPairs; h++) {
+                const int j = lane + 32 * h;
+                c[h] = 1.0f;
+                s[h] = 0.0f;
+                p[h] = q[h] = 0;
+                if (j < np) {  // rr_pair without the divisions
+                    const int x = t + j, y = t - j;
+                    const int u = j == 0 ? 0 : 1 + (x >= m ? x - m : x), z = 1 + (y < 0 ? y + m : y);
+                    p[h] = u;  // in this order: consecutive over the lanes (banks)
+                    q[h] = z;
+                    const float apq = cur[p[h] * ld + q[h]], app = cur[p[h] * ld + p[h]], aqq = cur[q[h] * ld + q[h]];
+                    if (max(u, z) < R && jacobi32_rotates(apq, app, aqq, floor)) {
+                        const float tau = fmaxf(fminf(__fdividef(0.5f * (aqq - app), apq), 0x1p40f), -0x1p40f);
+                        const float k = fmaf(tau, tau, 1.0f);
+                        const float tt = copysignf(__fdividef(1.0f, fabsf(tau) + k * rsqrtf(k)), tau);
+                        c[h] = rsqrtf(fmaf(tt, tt, 1.0f));
+                        s[h] = tt * c[h];
+                        rot = true;
+                    }
                 }
             }
+            if (!__any_sync(0xffffffffu, rot)) continue;  // the same in every warp
+            for (int i = w; i < np; i += nw) {
+                const int from = i & 31;
+                const bool hi = kPairs > 1 && i >= 32;
+                const float ci = __shfl_sync(0xffffffffu, hi ? c[kPairs - 1] : c[0], from);
+                const float si = __shfl_sync(0xffffffffu, hi ? s[kPairs - 1] : s[0], from);
+                const int pi = __shfl_sync(0xffffffffu, hi ? p[kPairs - 1] : p[0], from);
+                const int qi = __shfl_sync(0xffffffffu, hi ? q[kPairs - 1] : q[0], from);
+                const float *rp = cur + pi * ld, *rq = cur + qi * ld;
+                float *wp = nxt + pi * ld, *wq = nxt + qi * ld;
+#pragma unroll
+                for (int h = 0; h < kPairs; h++) {
+                    if (lane + 32 * h < np) {
+                        const float pp = rp[p[h]], pqv = rp[q[h]], qp = rq[p[h]], qq = rq[q[h]];
+                        const float l0 = ci * pp - si * qp, l1 = ci * pqv - si * qq;
+                        const float m0 = si * pp + ci * qp, m1 = si * pqv + ci * qq;
+                        wp[p[h]] = c[h] * l0 - s[h] * l1;
+                        wp[q[h]] = s[h] * l0 + c[h] * l1;
+                        wq[p[h]] = c[h] * m0 - s[h] * m1;
+                        wq[q[h]] = s[h] * m0 + c[h] * m1;
+                    }
+                }
+                if (si == 0.0f) continue;
+                float *vp = v + pi * ld, *vq = v + qi * ld;
+#pragma unroll
+                for (int h = 0; h < 2 * kPairs; h++) {
+                    const int r = lane + 32 * h;
+                    if (r < Re) {
+                        const float x = vp[r], y = vq[r];
+                        vp[r] = ci * x - si * y;
+                        vq[r] = si * x + ci * y;
+                    }
+                }
+            }
             __syncthreads();
+            float* const done = nxt;
+            nxt = cur;
+            cur = done;
         }
         __syncthreads();  // flag is read by everyone before the next sweep clears it
     }
     __syncthreads();
+}
+// a: two buffers, then v, Re x Re floats each (jacobi32_bytes).
+__host__ __device__ __forceinline__ size_t jacobi32_bytes(int R) {
+    const size_t Re = R + (R & 1);
+    return 3 * Re * Re * sizeof(float);
+}
+__device__ void jacobi32_block(int R, float* a, float* v, float floor, int* flag) {
+    const int Re = R + (R & 1);
+    if (R <= 64) jacobi32_sweeps<1>(R, a, a + Re * Re, v, floor, flag);
+    else jacobi32_sweeps<2>(R, a, a + Re * Re, v, floor, flag);
 }
 
 // The power of two that brings mx into [1, 2); 0 when there is none to speak of.
@@ -358,12 +391,12 @@ __global__ void __launch_bounds__(512) jacobi32_kernel(int R, const double* __re
                                                        double* __restrict__ X, double* __restrict__ As,
                                                        int64_t scratch_stride) {
     extern __shared__ float j32[];
-    __shared__ Jacobi32Smem sm;
+    __shared__ int flag;
     __shared__ double red[32];
     const int Re = R + (R & 1);
     const int tid = threadIdx.x, nt = blockDim.x;
     float* a = j32;
-    float* v = a + Re * Re;
+    float* v = a + 2 * Re * Re;
     A += blockIdx.x * a_stride;
     X += blockIdx.x * scratch_stride;
     As += blockIdx.x * scratch_stride;
@@ -386,7 +419,7 @@ __global__ void __launch_bounds__(512) jacobi32_kernel(int R, const double* __re
         a[e] = (float)(x * sc);
     }
     __syncthreads();
-    jacobi32_block(R, a, v, 0x1p-22f, &sm);
+    jacobi32_block(R, a, v, 0x1p-22f, &flag);
     for (int e = tid; e < R * R; e += nt) X[e] = (double)v[(e % R) * Re + e / R];  // column j = eigenvector j
 }
 
@@ -462,7 +495,7 @@ __global__ void __launch_bounds__(512) refine_first_kernel(int R, const double* 
                                                            const double* __restrict__ G, double* __restrict__ E,
                                                            int64_t scratch_stride) {
     extern __shared__ float j32[];
-    __shared__ Jacobi32Smem sm;
+    __shared__ int flag;
     __shared__ double red[32];
     __shared__ int second;
     pdl_wait();
@@ -506,7 +539,7 @@ __global__ void __launch_bounds__(512) refine_first_kernel(int R, const double* 
     const double sc = scale_of(block_max(mx, red));
     if (sc == 0.0) return;
     float* a = j32;
-    float* v = a + Re * Re;
+    float* v = a + 2 * Re * Re;
     for (int e = tid; e < Re * Re; e += nt) {
         const int i = e / Re, j = e % Re;
         double x = 0.0;
@@ -514,7 +547,7 @@ __global__ void __launch_bounds__(512) refine_first_kernel(int R, const double* 
         a[e] = (float)(x * sc);
     }
     __syncthreads();
-    jacobi32_block(R, a, v, (float)(0x1p-22 * spread * sc), &sm);
+    jacobi32_block(R, a, v, (float)(0x1p-22 * spread * sc), &flag);
     for (int e = tid; e < R * R; e += nt) {
         const int i = e / R, j = e % R;
         E[e] = (double)v[j * Re + i] - (i == j ? 1.0 : 0.0);
@@ -1074,20 +1107,17 @@ __global__ void spd_pinv_packed_kernel(int R, const double* __restrict__ A, doub
 }
 
 // ---------------------------------------------------------------------------
-// The Cholesky inverse of one matrix over many blocks (32 < R <= 128), the same
-// operations in the same order as the one-block kernels above (and so the same
-// bits), spread where they are independent:
-//   chol_factor_kernel   one CTA: L, every element in a register of its owner
-//                        (a step: the pivot column's owners divide, all owners
-//                        of later columns take one FMA)
+// The Cholesky inverse of one matrix over many blocks (32 < R <= 128), spread
+// where its operations are independent:
+//   chol_factor_kernel   one CTA: L
 //   chol_columns_kernel  a block per column of L^{-1}, its rows' sums in the
 //                        threads, one finished row per step
 //   chol_gram_kernel     a block per row of L^{-T} L^{-1}
 // then the acceptance test with the Jacobi fallback in one CTA, and the Newton
 // step a block per row.  On one SM the FP64 pipe's ~1.8 operations per clock
 // and the ~64 cycles of each dependent one made them 0.13 / 0.25 / 0.87 ms at
-// R = 45 / 64 / 128; split, the factor takes 0.075 / 0.106 / 0.33 ms (a square
-// root and an FMA deep per column, so still latency), the columns 0.013 /
+// R = 45 / 64 / 128; split, the factor takes 0.047 / 0.061 /
+// 0.33 ms (twice that beside other FP64 kernels on its SM), the columns 0.013 /
 // 0.027 / 0.052 and the products and the test 0.013 each.  kFour: L^{-1} and
 // the products summed in four chains (sub_dot, gram_dot), as the packed
 // kernels do.  At R <= 32 the small kernels' one launch is the shorter.
@@ -1109,66 +1139,106 @@ size_t chol_scratch_doubles(int R) { return (size_t)R * (R + 1) / 2 + 2 * (size_
 
 constexpr int kFactorThreads = 512;
 
-template <int EPT>
+// 1 / d of a positive normal d: an FP32 reciprocal y of its mantissa (|e| <=
+// 2^-22, e = 1 - m y) and one step of the third-order iteration y (1 + e +
+// e^2) (Householder), three dependent FP64 operations of ~64 cycles; the
+// error is e^3 and the last rounding.
+__device__ __forceinline__ double pivot_reciprocal(double d) {
+    const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+    const int ex = (int)((hi >> 20) & 0x7ff);
+    if (ex < 3 || ex > 2040) return 1.0 / d;  // (a pivot that is not positive and finite stops the caller)
+    const double m = __hiloint2double((int)((hi & 0xfffffu) | 0x3ff00000u), (int)lo);
+    const float y0 = __fdividef(1.0f, __uint_as_float(0x3f800000u | ((hi & 0xfffffu) << 3) | (lo >> 29)));
+    const unsigned yb = __float_as_uint(y0);  // widened in integers
+    const double y = __hiloint2double((int)((yb >> 3) + (896u << 20)), (int)(yb << 29));
+    const double e = fma(-m, y, 1.0);
+    const double r = fma(y, fma(e, e, e), y);
+    return __hiloint2double(__double2hiint(r) - ((ex - 1023) << 20), __double2loint(r));
+}
+
+// L by columns, kTpc threads per column (row i of column j: thread i % kTpc),
+// every element in a register of its owner.  A step takes one barrier: the
+// pivot column's owners publish it unscaled, its diagonal's owner the pivot's
+// reciprocal, and the owners of the later columns take v_ij -= v_ik (v_jk /
+// d_k); the square roots and the division of the columns by them follow for
+// all columns at once.  With the root, its reciprocal and the division inside
+// the step it took 75 / 106 / 332 us at R = 45 / 64 / 128 (now 47 / 61 / 330: a
+// warp retires one FP64 instruction per 64 clocks and an SM one per 19, so at R
+// > 64 the updates themselves are the bound).
+template <int kTpc, int kSlots>
 __global__ void __launch_bounds__(kFactorThreads) chol_factor_kernel(int R, const double* __restrict__ A,
                                                                      double* __restrict__ scr) {
-    __shared__ double colv[2][kMaxRank];  // the pivot column (scaled), ping-pong
-    __shared__ double diag[2][3];         // the pivot, its square root and the root's reciprocal
+    __shared__ double colv[2][kMaxRank];  // the pivot column, ping-pong
+    __shared__ double rpiv[2];            // its pivot's reciprocal
+    for (int i = threadIdx.x; i < 2 * kMaxRank; i += kFactorThreads) colv[0][i] = 0.0;
+    __syncthreads();
     pdl_wait();
     pdl_trigger();
     const CholScratch c = chol_scratch(scr, R);
-    const int tid = threadIdx.x, P = R * (R + 1) / 2;
-    // element e of the lower triangle by columns: column j holds rows j .. R - 1
-    double v[EPT];
-    int ij[EPT];  // i | j << 16; j = 0xffff: none
+    const int j = threadIdx.x / kTpc, g = threadIdx.x % kTpc;
+    double v[kSlots];
 #pragma unroll
-    for (int m = 0; m < EPT; m++) {
-        const int e = tid + m * kFactorThreads;
-        int j = 0, start = 0;
-        while (j < R - 1 && e >= start + (R - j)) {
-            start += R - j;
-            j++;
+    for (int m = 0; m < kSlots; m++) {
+        const int i = kTpc * m + g;
+        v[m] = j < R && i >= j && i < R ? A[j * R + i] : 0.0;  // upper triangle of A
+    }
+    const int m0 = (int)((threadIdx.x & ~31u) / kTpc) / kTpc, m1 = (R + kTpc - 1) / kTpc;  // the warp's live slots
+    const bool diag = j < R && g == j % kTpc;
+    double dj = diag ? A[j * R + j] : 0.0;  // the diagonal element, ahead of its slot
+    auto publish = [&]() {
+#pragma unroll
+        for (int m = 0; m < kSlots; m++) {
+            const int i = kTpc * m + g;
+            if (i >= j && i < R) colv[j & 1][i] = v[m];
         }
-        const int i = j + (e - start);
-        ij[m] = e < P ? (i | (j << 16)) : (0xffff << 16);
-        v[m] = e < P ? A[j * R + i] : 0.0;  // upper triangle of A
+    };
+    if (j == 0) {
+        if (diag) rpiv[0] = pivot_reciprocal(dj);
+        publish();
     }
     int rank = R;
     for (int k = 0; k < R; k++) {
-        double* col = colv[k & 1];
-#pragma unroll
-        for (int m = 0; m < EPT; m++)
-            if (ij[m] == (k | (k << 16))) {  // its owner alone, two independent chains
-                diag[k & 1][0] = v[m];
-                diag[k & 1][1] = sqrt(v[m]);
-                diag[k & 1][2] = rsqrt(v[m]);
-            }
+        const double* col = colv[k & 1];
         __syncthreads();
-        const double d = diag[k & 1][0], lkk = diag[k & 1][1], y = diag[k & 1][2];
-        const long long bits = __double_as_longlong(d);
+        const long long bits = __double_as_longlong(col[k]);
         if (!(bits > 0 && bits < 0x7ff0000000000000ll)) {  // not a positive finite number: the same in every thread
             rank = k;
             break;
         }
-#pragma unroll
-        for (int m = 0; m < EPT; m++) {
-            if ((ij[m] >> 16) == k) {
-                const int i = ij[m] & 0xffff;
-                v[m] = i == k ? lkk : div_by(v[m], lkk, y);
-                col[i] = v[m];
+        if (j > k && j < R) {
+            const double cj = col[j], t = cj * rpiv[k & 1];
+            if (diag) {
+                dj = fma(-cj, t, dj);
+                if (j == k + 1) rpiv[j & 1] = pivot_reciprocal(dj);
             }
-        }
-        __syncthreads();
+            // rows in groups of four slots from the warp's first column's on (the
+            // others' are no part of L: col's slots are finite or unused)
 #pragma unroll
-        for (int m = 0; m < EPT; m++) {
-            const int i = ij[m] & 0xffff, j = ij[m] >> 16;
-            if (j > k && j < R) v[m] -= col[i] * col[j];
+            for (int q = 0; q < kSlots; q += 4) {
+                if (q + 3 >= m0 && q < m1) {
+                    double x[4];
+#pragma unroll
+                    for (int h = 0; h < 4; h++) x[h] = col[kTpc * (q + h) + g];
+#pragma unroll
+                    for (int h = 0; h < 4; h++) v[q + h] = fma(-x[h], t, v[q + h]);
+                }
+            }
+            if (j == k + 1) publish();
         }
     }
+    __syncthreads();
+    double* pivots = colv[0];
+    if (diag) pivots[j] = dj;
+    __syncthreads();
+    if (j < R) {
+        const double root = sqrt(pivots[j]), y = 1.0 / root;
 #pragma unroll
-    for (int m = 0; m < EPT; m++)
-        if ((ij[m] >> 16) < R) c.Lp[tri(ij[m] & 0xffff, ij[m] >> 16)] = v[m];
-    if (tid == 0) *c.rank = rank;
+        for (int m = 0; m < kSlots; m++) {
+            const int i = kTpc * m + g;
+            if (i >= j && i < R) c.Lp[tri(i, j)] = i == j ? root : div_by(v[m], root, y);
+        }
+    }
+    if (threadIdx.x == 0) *c.rank = rank;
 }
 
 template <bool kFour>
@@ -1337,7 +1407,7 @@ size_t pinv_smem_bytes(int R) {
 
 // L, L^{-1} (scr) and out = A^{-1} where the factorisation goes through.
 static int launch_chol_inverse(int R, const double* A, double* out, bool four, double* scr, cudaStream_t st) {
-    auto factor = R <= 64 ? chol_factor_kernel<5> : R <= 96 ? chol_factor_kernel<10> : chol_factor_kernel<17>;
+    auto factor = R <= 64 ? chol_factor_kernel<8, 8> : chol_factor_kernel<4, 32>;
     factor<<<1, kFactorThreads, 0, st>>>(R, A, scr);
     EXAFAC_CUDA_TRY(launch_dependent(four ? chol_columns_kernel<true> : chol_columns_kernel<false>, R, kMaxRank, 0, st, R,
                                      scr));
@@ -1449,16 +1519,15 @@ size_t syev_refine_doubles(int R, int batch) { return (size_t)batch * 6 * R * R;
 
 int launch_syev_refined(int R, const double* A, int64_t a_stride, int batch, double* V, double* lam, int64_t v_stride,
                         double* vt_scratch, double* scratch, cudaStream_t stream) {
-    const int Re = R + (R & 1);
     const int64_t R2 = (int64_t)R * R, ss = 6 * R2;
     double *X = scratch, *Xn = X + R2, *As = Xn + R2, *S = As + R2, *G = S + R2, *E = G + R2;
-    const size_t jsm = sizeof(float) * 2 * (size_t)Re * Re;
-    if (jsm > 48 * 1024) {
+    const size_t jsm = jacobi32_bytes(R);
+    if (jsm > 40 * 1024) {  // (the 48 KB of a launch without it include the static part)
         EXAFAC_CUDA_TRY(cudaFuncSetAttribute(jacobi32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jsm));
         EXAFAC_CUDA_TRY(
             cudaFuncSetAttribute(refine_first_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jsm));
     }
-    jacobi32_kernel<<<batch, R <= 32 ? 256 : 512, jsm, stream>>>(R, A, a_stride, X, As, ss);
+    jacobi32_kernel<<<batch, 512, jsm, stream>>>(R, A, a_stride, X, As, ss);
     count_launch();
     const dim3 grid((unsigned)R, (unsigned)batch);
     for (int it = 0; it <= kRefineSteps; it++) {
@@ -1467,7 +1536,7 @@ int launch_syev_refined(int R, const double* A, int64_t a_stride, int batch, dou
         count_launch();
         if (it == kRefineSteps) break;
         if (it == 0) {
-            EXAFAC_CUDA_TRY(launch_dependent(refine_first_kernel, (unsigned)batch, R <= 32 ? 256 : 512, jsm, stream, R,
+            EXAFAC_CUDA_TRY(launch_dependent(refine_first_kernel, (unsigned)batch, 512, jsm, stream, R,
                                              (const double*)S, (const double*)G, E, ss));
         } else {
             EXAFAC_CUDA_TRY(launch_dependent(refine_e_kernel, grid, 128, 0, stream, R, (const double*)S,

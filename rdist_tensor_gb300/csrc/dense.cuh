@@ -22,7 +22,7 @@ int launch_syev_refined(int R, const double* A, int64_t a_stride, int batch, dou
 // Symmetric pseudo-inverse (eigenvalues <= tol dropped) of one matrix:
 // Cholesky inverse when provably well conditioned, Jacobi otherwise.
 // scr (chol_scratch_doubles(R) doubles, 32 < R): spread over many blocks; null:
-// one CTA (for callers with vt_scratch only).  The same bits either way.
+// one CTA (for callers with vt_scratch only).
 size_t chol_scratch_doubles(int R);
 int launch_pinv(int R, const double* A, double* out, double tol, double* vt_scratch, cudaStream_t stream,
                 double* scr = nullptr);
