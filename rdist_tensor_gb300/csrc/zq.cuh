@@ -6,7 +6,7 @@
 namespace exafac {
 
 struct ZState {
-    int64_t* xi = nullptr;      // J x (R rounded up to 4): the descent's vector, fixed point
+    int64_t* xi = nullptr;      // J x (R rounded up to 4): the descent's vector, fixed point (pack_x)
     double2* lh = nullptr;      // (low, high) of the current descent
     double* rinv = nullptr;     // 1 / root mass (scaled units)
     float2* err = nullptr;      // error bounds of (low, high)
@@ -29,6 +29,7 @@ struct ZState {
     int64_t* pref64 = nullptr;  // per tile: prefix of tcount (more tiles than shared memory takes)
     int64_t* off[2] = {nullptr, nullptr};  // slot ranges of a level's nodes (ping-pong)
     int32_t* tree_exp = nullptr;           // 2 N + 1: exponent of each tree's root diagonal, and Phi's
+    uint4* nodes = nullptr;     // a level's left children as product operands (z_node_cap of them)
 };
 
 void zq_carve(Arena& a, ZState& b, int R, int64_t J, int64_t widest, int trees);

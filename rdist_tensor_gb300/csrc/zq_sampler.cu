@@ -180,12 +180,23 @@ __device__ __forceinline__ void load_x8(const long long* row, int k, int Rx, boo
     }
 }
 
-// The four digits of eight x values (fixed point) into the slices of the
-// operand, 16 bytes each.
+// A fixed-point entry X is kept as its rounding z4 to multiples of 2^23 (low
+// word; the four digits) and the rest, |xr| <= 2^22 (high word): X = 2^23 z4 +
+// xr.  Every level reads the entries and none needs 64-bit arithmetic.
+__device__ __forceinline__ long long pack_x(long long X) {
+    const int z4 = (int)((X + (1ll << 22)) >> 23);
+    const int xr = (int)((unsigned)X - ((unsigned)z4 << 23));
+    return (long long)(((unsigned long long)(unsigned)xr << 32) | (unsigned)z4);
+}
+__device__ __forceinline__ int x_z4(long long x) { return (int)x; }
+__device__ __forceinline__ int x_rest(long long x) { return (int)(x >> 32); }
+
+// The four digits of eight x values into the slices of the operand, 16 bytes
+// each.
 __device__ __forceinline__ void store_x_digits(unsigned char* dst, uint32_t xs, const long long (&X)[8]) {
     uint32_t t[8];
 #pragma unroll
-    for (int q = 0; q < 8; q++) t[q] = (uint32_t)(int)((X[q] + (1ll << 22)) >> 23) + 0x808080u;
+    for (int q = 0; q < 8; q++) t[q] = (uint32_t)x_z4(X[q]) + 0x808080u;
     uint32_t o[kZx][4];
 #pragma unroll
     for (int q = 0; q < 4; q++) {
@@ -245,12 +256,15 @@ __device__ __forceinline__ void store_a_digits(unsigned char* dst, uint32_t bs, 
 // R zero.  The row runs fastest over the threads (conflict-free stores).
 __device__ __forceinline__ void stage_x(unsigned char* A, const long long* __restrict__ xi, const int32_t* js, int n,
                                         int R, const ZShape& z) {
-    const int total = kZTile * (z.Rk / 8);
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
-        const int r = e & (kZTile - 1), k = 8 * (e / kZTile);
+    // lanes: eight rows, four 64-byte pieces of each (half the cache lines per
+    // load of a row per lane, the same conflict-free stores)
+    const int k8s = z.Rk / 8, quads = (k8s + 3) / 4, lane = threadIdx.x & 31;
+    for (int q = threadIdx.x >> 5; q < (kZTile / 8) * quads; q += blockDim.x >> 5) {
+        const int r = 8 * (q & (kZTile / 8 - 1)) + (lane & 7), k8 = 4 * (q / (kZTile / 8)) + (lane >> 3);
+        if (k8 >= k8s) continue;
         long long X[8];
-        load_x8(xi + (int64_t)js[r < n ? r : 0] * z_row(R), k, z_row(R), r < n, X);
-        store_x_digits(A + (uint32_t)(r >> 3) * z.sbo + (uint32_t)(k >> 3) * 128u + (uint32_t)(r & 7) * 16u, z.xs, X);
+        load_x8(xi + (int64_t)js[r < n ? r : 0] * z_row(R), 8 * k8, z_row(R), r < n, X);
+        store_x_digits(A + (uint32_t)(r >> 3) * z.sbo + (uint32_t)k8 * 128u + (uint32_t)(r & 7) * 16u, z.xs, X);
     }
 }
 
@@ -272,6 +286,23 @@ __device__ __forceinline__ void expand_node(unsigned char* B, const double* __re
         store_a_digits<kZa>(B + (uint32_t)(c >> 3) * z.sbo + (uint32_t)(k >> 3) * 128u + (uint32_t)(c & 7) * 16u, z.bs,
                             v, emax);
     }
+}
+
+// One chunk of a node's B operand in global memory, for bulk copies: eight
+// entries per item.
+__host__ __device__ __forceinline__ uint32_t z_chunk_bytes(const ZShape& z) { return kZa * z.bs; }
+__device__ __forceinline__ void expand_item(unsigned char* B, const double* __restrict__ g, int ch, int item, int R,
+                                            int emax, const ZShape& z) {
+    const int c = item & (kZCols - 1), k = 8 * (item / kZCols);
+    const int col = ch * kZCols + c;
+    double v[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        const int kk = k + q;
+        v[q] = (col < R && kk < R) ? __ldg(g + packed_index(R, min(kk, col), max(kk, col))) : 0.0;
+    }
+    store_a_digits<kZa>(B + (uint32_t)(c >> 3) * z.sbo + (uint32_t)(k >> 3) * 128u + (uint32_t)(c & 7) * 16u, z.bs, v,
+                        emax);
 }
 
 // Rows 32 ch .. + 31 of a leaf (its first rows live, else zero) as the B operand.
@@ -423,9 +454,8 @@ __device__ __forceinline__ void z_dot8(uint32_t taddr, const long long* xrow, in
         const int V = __float_as_int(v + 0.005859375f) - 0x3BC00000;  // units of 2^-31
         const int Pn = m0 * 256 + m1;                                  // units of 2^-8
         const int Qn = m2 * 128 + m3;                                  // units of 2^-23
-        const long long z4 = (X[q] + (1ll << 22)) >> 23;
-        const long long wi = 2 * X[q] - (z4 << 23);  // x0 + 2 xr
-        const int wh = (int)(wi >> 27), wl = (int)wi & 0x7ffffff;
+        // x0 + 2 xr = 2^27 wh + wl
+        const int z4 = x_z4(X[q]), wh = z4 >> 4, wl = ((z4 & 15) << 23) + 2 * x_rest(X[q]);
         s.Ph += (long long)Pn * wh;
         s.Pl += (long long)Pn * wl;
         s.Qh += (long long)Qn * wh;
@@ -443,11 +473,20 @@ __device__ __forceinline__ void z_dot8(uint32_t taddr, const long long* xrow, in
 // NT = 512 (R > 64, one block per SM): a chunk's products run beside the
 // previous chunk's read-back (two accumulator sets), and beside the next
 // chunk's expansion when a second node buffer fits (nb = 2).
+// nodes != null: the operands of the level's left children (of the root: MODE
+// 0), node by node in z_chunk_bytes chunks (zq_partition_kernel has expanded
+// them; lb the parents' first index), brought by bulk copies, the first one of
+// a run ahead of its use; null: each run expands its node here.
+// A run's sums are kept and a tile's masses and branches formed together: an
+// SM takes an FP64 instruction per 19 clocks whatever its active lanes, and
+// the ~14 of them per run cost as much as the products on levels with short
+// runs.
 template <int MODE, int NT>
 __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
-    zq_level_kernel(int R, int nb, TreeShape t, const double* __restrict__ G, const int32_t* __restrict__ tree_exp,
-                    int64_t J, ZState b, int p, const int32_t* __restrict__ order, const double* __restrict__ dv,
-                    DeviceStatus* status, uint32_t wait_polls) {
+    zq_level_kernel(int R, int nb, TreeShape t, const double* __restrict__ G, const unsigned char* __restrict__ nodes,
+                    int64_t lb, const int32_t* __restrict__ tree_exp, int64_t J, ZState b, int p,
+                    const int32_t* __restrict__ order, const double* __restrict__ dv, DeviceStatus* status,
+                    uint32_t wait_polls) {
     extern __shared__ __align__(128) unsigned char z_raw[];
     constexpr int NG = NT / 128;        // threads per slot in the read-back
     constexpr int CPT = kZCols / NG;    // columns of a chunk per thread
@@ -456,32 +495,36 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
     __shared__ int32_t cs[kZTile], js[kZTile];
     __shared__ uint32_t rmask[4];
     __shared__ long long part[NG][5][kZTile];
-    __shared__ int32_t flag_sm[kZTile];  // -1: not this block's, 0 right, 1 left (or stays)
     __shared__ int rs[kMaxRank];
-    __shared__ __align__(8) uint64_t bars[2];
+    __shared__ __align__(8) uint64_t bars[2];    // products
+    __shared__ __align__(8) uint64_t copied[2];  // node buffers
     __shared__ uint32_t tmem_base;
-    __shared__ int abort_flag;
     const ZShape z = z_shape(R);
     const int Rx = z_row(R);
     unsigned char* A = z_raw + ((128u - (smem_u32(z_raw) & 127u)) & 127u);
     unsigned char* Bb[2] = {A + kZx * z.xs, A + kZx * z.xs + (nb - 1) * kZa * z.bs};
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const int P = packed_size(R);
+    const bool pre = nodes != nullptr;
+    const uint32_t cbytes = z_chunk_bytes(z);
     if (w == 0) tmem_alloc(&tmem_base, kTmem);
     for (int a = tid; a < R; a += NT) rs[a] = packed_index(R, a, a);
     if (tid == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
+        for (int q = 0; q < 2; q++) {
+            mbar_init(&bars[q], 1);
+            mbar_init(&copied[q], 1);
+        }
         fence_mbar_init();
-        abort_flag = 0;
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base;
     const int emax = *tree_exp;
-    uint32_t phase[2] = {0, 0};
-    int64_t resident = -1;  // the node B holds (one-chunk ranks)
+    uint32_t phase[2] = {0, 0}, cphase[2] = {0, 0};
+    bool lost = false;     // a wait of this thread ran out
+    int64_t resident = -1; // the node B holds, or is being copied (one-chunk ranks)
+    bool aborted = false;
     const int row = (w & 3) * 32 + lane, grp = w >> 2;
     const uint32_t lane_base = tmem + ((uint32_t)((w & 3) * 32) << 16);
     const int64_t ntiles = (J + kZTile - 1) / kZTile;
@@ -495,12 +538,34 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
         for (int64_t q = (int64_t)blockIdx.x * NT + tid; q < ntiles; q += (int64_t)gridDim.x * NT) b.truns[p ^ 1][q] = 0;
     }
     const bool ok = emax < 2047;  // a tree with a non-finite root: every sample is marked at the root
-    // the chunk's products are done (every thread); a wait that ran out raises abort_flag
+    // the chunk's products are done (every thread)
     auto wait = [&](int q) {
-        if (!mbar_wait_limited(&bars[q], phase[q], wait_polls)) abort_flag = 1;
+        if (!mbar_wait_limited(&bars[q], phase[q], wait_polls)) lost = true;
         phase[q] ^= 1u;
         tc_fence_after();
     };
+    // thread 0: chunk ch of the left child of parent c into buffer q; the products of buffer q's chunk
+    auto fetch = [&](int q, int32_t c, int ch) {
+        const int64_t slot = MODE == 0 ? 0 : (int64_t)c - lb;
+        mbar_arrive_expect_tx(&copied[q], cbytes);
+        bulk_g2s(Bb[q], nodes + (slot * z.nch + ch) * cbytes, cbytes, &copied[q]);
+    };
+    auto issue = [&](int q, int set, bool fresh) {
+        if (fresh) {
+            if (!mbar_wait_limited(&copied[q], cphase[q], wait_polls)) {
+                lost = true;  // no products: the others' waits run out as well
+                return;
+            }
+            cphase[q] ^= 1u;
+        }
+        issue_chunk<kZa>(tmem + (uint32_t)(set * 256), A, Bb[q], z, &bars[set]);
+    };
+    // the chunk's columns of this thread
+    auto dots = [&](uint32_t acc, const long long* xrow, int ch, ZSums& sum) {
+#pragma unroll
+        for (int h = 0; h < CPT / 8; h++) z_dot8(acc + 8 * h, xrow, ch * kZCols + grp * CPT + 8 * h, Rx, sum);
+    };
+    auto stays = [&](int32_t c) { return MODE == 2 && tree_is_leaf(t, c); };
     for (; sh.count > 0 && sh.tile < ntiles; sh.tile++, sh.run = 0) {
         const int64_t s0 = sh.tile * kZTile;
         const int n = (int)min((int64_t)kZTile, J - s0);
@@ -508,6 +573,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
         float2 er = make_float2(0.f, 0.f);
         float e0 = 0.f, n1 = 0.f;
         int ex = 0;
+        int flag = -1;  // -1: not this block's, 0 right, 1 left (or stays), 2 summed
         if (tid < kZTile) {
             int32_t j = 0, c = -1;
             if (tid < n) {
@@ -525,125 +591,171 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
             }
             js[tid] = j;
             cs[tid] = c;
-            flag_sm[tid] = -1;
         }
         z_run_mask(cs, n, rmask);
-        stage_x(A, reinterpret_cast<const long long*>(b.xi), js, n, R, z);
         int i0 = 0;
         for (int q = 0; q < sh.run && i0 < n; q++) i0 = z_run_end(rmask, i0, n);
+        bool ahead = false;  // the next run's first chunk is on its way
+        if (pre && i0 < n && !stays(cs[i0]) && !(z.nch == 1 && resident == cs[i0])) {
+            if (tid == 0) fetch(0, cs[i0], 0);
+            ahead = true;
+        }
+        stage_x(A, reinterpret_cast<const long long*>(b.xi), js, n, R, z);
+        fence_proxy_async_smem();
+        tc_fence_before();
+        __syncthreads();
         for (; i0 < n && sh.count > 0; sh.count--) {  // runs of equal node (uniform over the block)
             const int32_t c = cs[i0];
             const int i1 = z_run_end(rmask, i0, n);
-            if (MODE == 2 && tree_is_leaf(t, c)) {  // stays
-                if (tid >= i0 && tid < i1) flag_sm[tid] = 1;
+            if (stays(c)) {
+                if (tid >= i0 && tid < i1) flag = 1;
                 i0 = i1;
                 continue;
             }
-            const int64_t g = MODE == 0 ? 0 : 2 * (int64_t)c + 1;
             ZSums sum = {0, 0, 0, 0, 0};
             const long long* xrow = reinterpret_cast<const long long*>(b.xi) + (int64_t)js[row < n ? row : 0] * Rx;
-            if (resident != g || z.nch > 1) expand_node(Bb[0], G + g * P, rs, 0, R, emax, z);
-            resident = g;
-            fence_proxy_async_smem();
-            tc_fence_before();
-            __syncthreads();
-            if (tid == 0) issue_chunk<kZa>(tmem, A, Bb[0], z, &bars[0]);
-            for (int ch = 0; ch < z.nch; ch++) {
-                const int cur = kPipe ? ch & 1 : 0;
-                const bool more = ch + 1 < z.nch;
-                const uint32_t acc = lane_base + (uint32_t)(cur * 256 + grp * CPT);
-                if (kPipe) {
+            if (pre) {
+                const bool held = z.nch == 1 && resident == c && !ahead;
+                if (tid == 0) {
+                    if (!held && !ahead) fetch(0, c, 0);
+                    if (nb == 2 && z.nch > 1) fetch(1, c, 1);
+                    issue(0, 0, !held);
+                }
+                ahead = false;
+                resident = c;
+                for (int ch = 0; ch < z.nch; ch++) {
+                    const int cur = kPipe ? ch & 1 : 0;
+                    const bool more = ch + 1 < z.nch;
+                    const uint32_t acc = lane_base + (uint32_t)(cur * 256 + grp * CPT);
+                    if (kPipe && nb == 2 && more && tid == 0) issue((ch + 1) & 1, cur ^ 1, true);
+                    wait(cur);
                     if (more) {
-                        if (nb == 1) wait(cur);
-                        expand_node(Bb[(ch + 1) & (nb - 1)], G + g * P, rs, ch + 1, R, emax, z);
-                        fence_proxy_async_smem();
+                        if (tid == 0) {
+                            if (kPipe && nb == 2) {
+                                if (ch + 2 < z.nch) fetch(ch & 1, c, ch + 2);
+                            } else {
+                                fetch(0, c, ch + 1);
+                                if (kPipe) issue(0, cur ^ 1, true);
+                            }
+                        }
+                    } else if (i1 < n && sh.count > 1 && cs[i1] != c && !stays(cs[i1])) {
+                        if (tid == 0) fetch(0, cs[i1], 0);
+                        ahead = true;
+                    }
+                    dots(acc, xrow, ch, sum);
+                    if (more) {  // the accumulators are read
                         tc_fence_before();
                         __syncthreads();
-                        if (tid == 0)
-                            issue_chunk<kZa>(tmem + (uint32_t)((cur ^ 1) * 256), A, Bb[(ch + 1) & (nb - 1)], z,
-                                             &bars[cur ^ 1]);
-                    }
-                    if (nb == 2 || !more) wait(cur);
-#pragma unroll
-                    for (int h = 0; h < CPT / 8; h++)
-                        z_dot8(acc + 8 * h, xrow, ch * kZCols + grp * CPT + 8 * h, Rx, sum);
-                } else {
-                    wait(0);
-#pragma unroll
-                    for (int h = 0; h < CPT / 8; h++)
-                        z_dot8(acc + 8 * h, xrow, ch * kZCols + grp * CPT + 8 * h, Rx, sum);
-                    if (more) {
-                        expand_node(Bb[0], G + g * P, rs, ch + 1, R, emax, z);
-                        fence_proxy_async_smem();
-                        tc_fence_before();
-                        __syncthreads();
-                        if (tid == 0) issue_chunk<kZa>(tmem, A, Bb[0], z, &bars[0]);
+                        if (!kPipe && tid == 0) issue(0, 0, true);
                     }
                 }
-            }
-            part[grp][0][row] = sum.Ph;
-            part[grp][1][row] = sum.Pl;
-            part[grp][2][row] = sum.Qh;
-            part[grp][3][row] = sum.Ql;
-            part[grp][4][row] = sum.V;
-            tc_fence_before();
-            __syncthreads();
-            if (abort_flag) break;
-            if (tid >= i0 && tid < i1) {
-                long long s5[5];
-#pragma unroll
-                for (int u = 0; u < 5; u++) {
-                    s5[u] = part[0][u][tid];
-#pragma unroll
-                    for (int gq = 1; gq < NG; gq++) s5[u] += part[gq][u][tid];
-                }
-                // weights: P 2^-8, Q 2^-23, V 2^-31; wh 2^-20, wl 2^-47
-                const double q = (double)s5[0] * 0x1p-28 + (double)s5[1] * 0x1p-55 + (double)s5[2] * 0x1p-43 +
-                                 (double)s5[3] * 0x1p-70 + (double)s5[4] * 0x1p-51;
-                const int32_t j = js[tid];
-                if (MODE == 0) {
-                    const double E = z_bound(n1, R);
-                    const double e = E / q;
-                    const bool good = ok && ex < 2047 && q > 0.0 && e < 0x1p-10;
-                    b.rinv[j] = good ? 1.0 / q : 0.0;
-                    const float ef = __double2float_ru(e + 0x1p-50);
-                    b.e0[j] = good ? ef : 1.0f;
-                    b.err[j] = make_float2(good ? ef : 1.0f, good ? ef : 1.0f);
-                    if (!good) z_mark(b.redo, b.redo_list, b.redo_count, j);
-                } else {
-                    const double cutoff = low + q * rinv;
-                    const float ec = (er.x + e0) * 1.0001f + 0x1p-50f;
-                    const bool left = d <= cutoff;
-                    if (!(fabs(d - cutoff) > (double)ec)) z_mark(b.redo, b.redo_list, b.redo_count, j);
-                    b.node[j] = left ? 2 * (int64_t)c + 1 : 2 * (int64_t)c + 2;
-                    if (left) {
-                        b.lh[j].y = cutoff;
-                        b.err[j].y = ec;
+            } else {
+                const int64_t g = MODE == 0 ? 0 : 2 * (int64_t)c + 1;
+                if (resident != c || z.nch > 1) expand_node(Bb[0], G + g * P, rs, 0, R, emax, z);
+                resident = c;
+                fence_proxy_async_smem();
+                tc_fence_before();
+                __syncthreads();
+                if (tid == 0) issue_chunk<kZa>(tmem, A, Bb[0], z, &bars[0]);
+                for (int ch = 0; ch < z.nch; ch++) {
+                    const int cur = kPipe ? ch & 1 : 0;
+                    const bool more = ch + 1 < z.nch;
+                    const uint32_t acc = lane_base + (uint32_t)(cur * 256 + grp * CPT);
+                    if (kPipe) {
+                        if (more) {
+                            if (nb == 1) wait(cur);
+                            expand_node(Bb[(ch + 1) & (nb - 1)], G + g * P, rs, ch + 1, R, emax, z);
+                            fence_proxy_async_smem();
+                            tc_fence_before();
+                            __syncthreads();
+                            if (tid == 0)
+                                issue_chunk<kZa>(tmem + (uint32_t)((cur ^ 1) * 256), A, Bb[(ch + 1) & (nb - 1)], z,
+                                                 &bars[cur ^ 1]);
+                        }
+                        if (nb == 2 || !more) wait(cur);
+                        dots(acc, xrow, ch, sum);
                     } else {
-                        b.lh[j].x = cutoff;
-                        b.err[j].x = ec;
+                        wait(0);
+                        dots(acc, xrow, ch, sum);
+                        if (more) {
+                            expand_node(Bb[0], G + g * P, rs, ch + 1, R, emax, z);
+                            fence_proxy_async_smem();
+                            tc_fence_before();
+                            __syncthreads();
+                            if (tid == 0) issue_chunk<kZa>(tmem, A, Bb[0], z, &bars[0]);
+                        }
                     }
-                    flag_sm[tid] = left ? 1 : 0;
                 }
             }
-            __syncthreads();  // part, and the accumulators and node buffers for the next run
+            if (row >= i0 && row < i1) {
+                part[grp][0][row] = sum.Ph;
+                part[grp][1][row] = sum.Pl;
+                part[grp][2][row] = sum.Qh;
+                part[grp][3][row] = sum.Ql;
+                part[grp][4][row] = sum.V;
+            }
+            if (tid >= i0 && tid < i1) flag = 2;
+            tc_fence_before();
+            // part, and the accumulators and node buffers for the next run
+            if (__syncthreads_or(lost)) {
+                aborted = true;
+                break;
+            }
             i0 = i1;
         }
-        if (abort_flag) break;
-        __syncthreads();
+        if (aborted) break;
+        if (tid < kZTile && flag == 2) {
+            long long s5[5];
+#pragma unroll
+            for (int u = 0; u < 5; u++) {
+                s5[u] = part[0][u][tid];
+#pragma unroll
+                for (int gq = 1; gq < NG; gq++) s5[u] += part[gq][u][tid];
+            }
+            // weights: P 2^-8, Q 2^-23, V 2^-31; wh 2^-20, wl 2^-47
+            const double q = (double)s5[0] * 0x1p-28 + (double)s5[1] * 0x1p-55 + (double)s5[2] * 0x1p-43 +
+                             (double)s5[3] * 0x1p-70 + (double)s5[4] * 0x1p-51;
+            const int32_t j = js[tid], c = cs[tid];
+            if (MODE == 0) {
+                const double E = z_bound(n1, R);
+                const double e = E / q;
+                const bool good = ok && ex < 2047 && q > 0.0 && e < 0x1p-10;
+                b.rinv[j] = good ? 1.0 / q : 0.0;
+                const float ef = __double2float_ru(e + 0x1p-50);
+                b.e0[j] = good ? ef : 1.0f;
+                b.err[j] = make_float2(good ? ef : 1.0f, good ? ef : 1.0f);
+                if (!good) z_mark(b.redo, b.redo_list, b.redo_count, j);
+            } else {
+                const double cutoff = low + q * rinv;
+                const float ec = (er.x + e0) * 1.0001f + 0x1p-50f;
+                const bool left = d <= cutoff;
+                if (!(fabs(d - cutoff) > (double)ec)) z_mark(b.redo, b.redo_list, b.redo_count, j);
+                b.node[j] = left ? 2 * (int64_t)c + 1 : 2 * (int64_t)c + 2;
+                if (left) {
+                    b.lh[j].y = cutoff;
+                    b.err[j].y = ec;
+                } else {
+                    b.lh[j].x = cutoff;
+                    b.err[j].x = ec;
+                }
+                flag = left ? 1 : 0;
+            }
+        }
         if (MODE != 0 && tid < kZTile) {
-            const uint32_t bits = __ballot_sync(0xffffffffu, flag_sm[tid] > 0);
+            const uint32_t bits = __ballot_sync(0xffffffffu, flag > 0);
             if (lane == 0 && bits) {
                 atomicOr(b.mask[p] + 4 * sh.tile + w, bits);
                 atomicAdd(b.tcount[p] + sh.tile, __popc(bits));
             }
         }
-        __syncthreads();
     }
     __syncthreads();
-    if (abort_flag) {  // the tiles left out keep clear flags: the partition keeps their order
-        if (tid == 0) report(status, EXAFAC_ERR_TIMEOUT, 23, blockIdx.x, 0);
-        // the MMAs in flight may still complete (bounded)
+    if (aborted) {  // the tiles left out keep clear flags: the partition keeps their order
+        if (tid == 0) {
+            report(status, EXAFAC_ERR_TIMEOUT, 23, blockIdx.x, 0);
+            // the copies and MMAs in flight may still complete (bounded)
+            for (int q = 0; q < 2; q++) mbar_wait_limited(&copied[q], cphase[q], wait_polls);
+        }
         if (tid == 0) mbar_wait_limited(&bars[0], phase[0] ^ 1u, wait_polls);
         if (tid == 32) mbar_wait_limited(&bars[1], phase[1] ^ 1u, wait_polls);
         tc_fence_before();
@@ -881,7 +993,7 @@ __global__ void __launch_bounds__(kPlaceThreads)
             if (lane == 0) diag_exp = z_leaf_exp(e);
         }
         const long long* X = reinterpret_cast<const long long*>(b.xi) + (int64_t)j * z_row(R);
-        for (int a = tid; a < R; a += kPlaceThreads) xs[a] = (double)X[a] * 0x1p-47;
+        for (int a = tid; a < R; a += kPlaceThreads) xs[a] = (double)(((long long)x_z4(X[a]) << 23) + x_rest(X[a])) * 0x1p-47;
         __syncthreads();
         const int emax = diag_exp;
         const double scale = scalbn(1.0, max(min(1028 - emax, 1000), -1000));
@@ -981,7 +1093,8 @@ __device__ __forceinline__ void tile_prefix(const int32_t* __restrict__ tcount, 
 // Within its parent's slot range a slot whose flag is set (went left, or
 // stayed at a leaf) keeps its order among those, before the others; the
 // children's slot ranges (coff) and their runs per tile follow, and the next
-// level's flags are cleared.  Every block
+// level's flags are cleared, and the next level's left children are expanded
+// into `nodes` (where it takes them: nx_nl > 0).  Every block
 // forms the tiles' prefix in shared memory (up to kZPrefSmem tiles), or reads
 // pref64 (more).  lb: the parents' first node index, nl their number.
 __global__ void __launch_bounds__(512)
@@ -989,8 +1102,22 @@ __global__ void __launch_bounds__(512)
                         uint32_t* __restrict__ mask_next, int32_t* __restrict__ tcount_next,
                         int32_t* __restrict__ truns_next, const int64_t* __restrict__ pref64, int64_t lb, int64_t nl, const int32_t* __restrict__ order,
                         const int64_t* __restrict__ node, const int64_t* __restrict__ off,
-                        int32_t* __restrict__ order2, int64_t* __restrict__ coff) {
+                        int32_t* __restrict__ order2, int64_t* __restrict__ coff, int R, const double* __restrict__ G,
+                        const int32_t* __restrict__ tree_exp, int64_t node_count, int64_t nx_lb, int64_t nx_nl,
+                        unsigned char* __restrict__ nodes) {
     extern __shared__ int32_t z_pref[];
+    if (nx_nl > 0) {
+        const ZShape z = z_shape(R);
+        const int emax = *tree_exp, items = kZCols * (z.Rk / 8);
+        const int64_t all = nx_nl * z.nch * items;
+        for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < all; q += (int64_t)gridDim.x * blockDim.x) {
+            const int64_t at = q / items;  // node and chunk
+            const int64_t g = 2 * (nx_lb + at / z.nch) + 1;
+            if (g < node_count)
+                expand_item(nodes + at * z_chunk_bytes(z), G + g * packed_size(R), (int)(at % z.nch), (int)(q - at * items),
+                            R, emax, z);
+        }
+    }
     if (!pref64) tile_prefix(tcount, ntiles, z_pref);
     auto SL = [&](int64_t s) -> int64_t {
         const int64_t tile = s >> 7;
@@ -1037,12 +1164,29 @@ __global__ void __launch_bounds__(512)
 
 // Largest diagonal exponent of a tree's root, plus one (the entries of the
 // tree's nodes are bounded by their diagonals, those by the root's; one more
-// bit for rounding).
-__global__ void zq_tree_exp_kernel(int R, const double* __restrict__ root, int32_t* __restrict__ out) {
-    int e = 0;
-    for (int a = threadIdx.x; a < R; a += 32) e = max(e, bexp(root[packed_index(R, a, a)]));
-    e = __reduce_max_sync(0xffffffffu, e);
-    if (threadIdx.x == 0) *out = e >= 2047 ? 2047 : e + 1;
+// bit for rounding).  nodes != null: blockIdx.x = node and chunk of the root
+// and its left child, which the block expands.
+__global__ void __launch_bounds__(256) zq_tree_exp_kernel(int R, const double* __restrict__ root,
+                                                          int32_t* __restrict__ out, int64_t node_count,
+                                                          unsigned char* __restrict__ nodes) {
+    __shared__ int top;
+    if (threadIdx.x < 32) {
+        int e = 0;
+        for (int a = threadIdx.x; a < R; a += 32) e = max(e, bexp(root[packed_index(R, a, a)]));
+        e = __reduce_max_sync(0xffffffffu, e);
+        if (threadIdx.x == 0) {
+            top = e >= 2047 ? 2047 : e + 1;
+            if (blockIdx.x == 0) *out = top;
+        }
+    }
+    __syncthreads();
+    if (!nodes) return;
+    const ZShape z = z_shape(R);
+    const int64_t g = blockIdx.x / z.nch;
+    if (g >= node_count) return;
+    for (int q = threadIdx.x; q < kZCols * (z.Rk / 8); q += blockDim.x)
+        expand_item(nodes + (int64_t)blockIdx.x * z_chunk_bytes(z), root + g * packed_size(R), blockIdx.x % z.nch, q, R,
+                    top, z);
 }
 
 // The vector of the next descent in fixed point, a warp per sample, and the
@@ -1083,7 +1227,7 @@ __global__ void zq_vector_kernel(int R, int64_t J, double* __restrict__ h, const
             const int c = lane + 32 * q;
             if (c < z_row(R)) {  // (x is zero past R)
                 const long long f = e < 2047 ? fix47_rn(x[q], e) : 0ll;
-                reinterpret_cast<long long*>(b.xi)[j * z_row(R) + c] = f;
+                reinterpret_cast<long long*>(b.xi)[j * z_row(R) + c] = pack_x(f);
                 n1 += (float)((int)(llabs(f) >> 24) + 1) * 0x1p-23f;
             }
         }
@@ -1188,7 +1332,8 @@ __global__ void __launch_bounds__(NT, 1)
             int hi[8];
 #pragma unroll
             for (int q = 0; q < 8; q++) {
-                const long long t = ((X[q] + (1ll << 14)) >> 15) + 0x80808080ll;  // units of 2^-32
+                const long long t = (long long)x_z4(X[q]) * 256 + ((x_rest(X[q]) + (1 << 14)) >> 15) +
+                                    0x80808080ll;  // units of 2^-32
                 lo[q] = (uint32_t)t;
                 hi[q] = (int)(t >> 32);
             }
@@ -1296,9 +1441,8 @@ __global__ void __launch_bounds__(NT, 1)
                     const float g6 = (g5 - (t5 - 0x1.8p-15f)) + (f[6] + f[7]);
                     const int W = __float_as_int(g6 + 0x1.8p-23f) - 0x34400000;
                     const int Pn = m0 * 256 + m1, Qn = m2 * 128 + m3, Tn = m4 * 256 + m5;
-                    const long long z5 = (X[q] + (1ll << 14)) >> 15;
-                    const long long wi = 2 * X[q] - (z5 << 15);
-                    const int wh = (int)(wi >> 27), wl = (int)wi & 0x7ffffff;
+                    const int z4 = x_z4(X[q]), xr = x_rest(X[q]), k5 = (xr + (1 << 14)) >> 15;
+                    const int wh = z4 >> 4, wl = ((z4 & 15) << 23) + 2 * xr - (k5 << 15);
                     sum[0] += (long long)Pn * wh;
                     sum[1] += (long long)Pn * wl;
                     sum[2] += (long long)Qn * wh;
@@ -1363,6 +1507,20 @@ __global__ void __launch_bounds__(NT, 1)
 // 2^22 of them is the size from which the breadth-first form was no slower.
 bool sts_zq_wanted(int R, int64_t J) { return J * (int64_t)packed_size(R) >= (1ll << 22); }
 
+// The levels whose nodes are expanded once into global memory: those with at
+// most half as many parents as tiles (each is then read twice or more), within
+// 32 MB.  R = 64, J = 2^18: a level 135 -> 114 us (the runs' scattered reads of
+// the packed node were half of its L1 wavefronts).  A node of one chunk (R <=
+// 32) is expanded by one item per thread and kept from tile to tile: there the
+// partition's extra work was the larger (a sweep at R = 25 4.65 against 4.71 ms).
+constexpr size_t kZNodeBytes = 32u << 20;
+static bool z_expands(int R) { return R > kZCols; }
+static int64_t z_node_cap(int R, int64_t J) {
+    const ZShape z = z_shape(R);
+    const int64_t fit = (int64_t)(kZNodeBytes / ((size_t)z.nch * z_chunk_bytes(z)));
+    return std::max<int64_t>(2, std::min<int64_t>(ceil_div(J, kZTile) / 2, fit));
+}
+
 void zq_carve(Arena& a, ZState& b, int R, int64_t J, int64_t widest, int trees) {
     b.xi = a.take<int64_t>(J * z_row(R));
     b.lh = a.take<double2>(J);
@@ -1390,6 +1548,8 @@ void zq_carve(Arena& a, ZState& b, int R, int64_t J, int64_t widest, int trees) 
     b.off[0] = a.take<int64_t>(2 * widest + 2);
     b.off[1] = a.take<int64_t>(2 * widest + 2);
     b.tree_exp = a.take<int32_t>(trees + 1);
+    const ZShape z = z_shape(R);
+    if (z_expands(R)) b.nodes = a.take<uint4>(z_node_cap(R, J) * z.nch * z_chunk_bytes(z) / sizeof(uint4));
 }
 
 static unsigned z_grid(int64_t work) {
@@ -1397,8 +1557,8 @@ static unsigned z_grid(int64_t work) {
 }
 
 template <int MODE, int NT>
-static int z_level(Session& s, const TreeShape& t, const double* G, const int32_t* ex, int64_t J, int p,
-                   const int32_t* order, const double* dv, cudaStream_t st) {
+static int z_level(Session& s, const TreeShape& t, const double* G, const unsigned char* nodes, int64_t lb,
+                   const int32_t* ex, int64_t J, int p, const int32_t* order, const double* dv, cudaStream_t st) {
     // a second node buffer where one block per SM runs and it fits beside the
     // 22 KB of static shared memory
     const size_t two = z_smem(s.R, 2 * kZa);
@@ -1407,16 +1567,16 @@ static int z_level(Session& s, const TreeShape& t, const double* G, const int32_
     EXAFAC_CUDA_TRY(cudaFuncSetAttribute(zq_level_kernel<MODE, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem));
     const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(J, kZTile), NT == 256 ? 304 : 152);
-    zq_level_kernel<MODE, NT><<<blocks, NT, smem, st>>>(s.R, nb, t, G, ex, J, s.zq, p, order, dv, s.status,
-                                                        s.wait_polls ? s.wait_polls : kSpinLimit);
+    zq_level_kernel<MODE, NT><<<blocks, NT, smem, st>>>(s.R, nb, t, G, nodes, lb, ex, J, s.zq, p, order, dv,
+                                                        s.status, s.wait_polls ? s.wait_polls : kSpinLimit);
     count_launch();
     return EXAFAC_OK;
 }
 template <int MODE>
-static int z_level_any(Session& s, const TreeShape& t, const double* G, const int32_t* ex, int64_t J, int p,
-                       const int32_t* order, const double* dv, cudaStream_t st) {
-    return s.R <= 64 ? z_level<MODE, 256>(s, t, G, ex, J, p, order, dv, st)
-                     : z_level<MODE, 512>(s, t, G, ex, J, p, order, dv, st);
+static int z_level_any(Session& s, const TreeShape& t, const double* G, const unsigned char* nodes, int64_t lb,
+                       const int32_t* ex, int64_t J, int p, const int32_t* order, const double* dv, cudaStream_t st) {
+    return s.R <= 64 ? z_level<MODE, 256>(s, t, G, nodes, lb, ex, J, p, order, dv, st)
+                     : z_level<MODE, 512>(s, t, G, nodes, lb, ex, J, p, order, dv, st);
 }
 template <int NT>
 static int z_leaf(Session& s, const TreeShape& t, const double* G, const double* U, int64_t J, int p,
@@ -1435,9 +1595,12 @@ static int z_descend(Session& s, const TreeShape& t, const double* G, const doub
                      int col, int tree, cudaStream_t st) {
     ZState& b = s.zq;
     int32_t* ex = b.tree_exp + tree;
-    zq_tree_exp_kernel<<<1, 32, 0, st>>>(s.R, G, ex);
+    const ZShape z = z_shape(s.R);
+    unsigned char* nodes = z_expands(s.R) ? reinterpret_cast<unsigned char*>(b.nodes) : nullptr;
+    const int64_t cap = nodes ? z_node_cap(s.R, J) : 0;
+    zq_tree_exp_kernel<<<nodes ? (unsigned)(2 * z.nch) : 1u, 256, 0, st>>>(s.R, G, ex, t.node_count, nodes);
     count_launch();
-    EXAFAC_TRY(z_level_any<0>(s, t, G, ex, J, 0, nullptr, dv, st));
+    EXAFAC_TRY(z_level_any<0>(s, t, G, nodes, 0, ex, J, 0, nullptr, dv, st));
     const int64_t ntiles = ceil_div(J, kZTile);
     const bool in_smem = ntiles <= kZPrefSmem;
     const size_t psm = in_smem ? sizeof(int32_t) * (ntiles + 1) : 0;
@@ -1451,15 +1614,18 @@ static int z_descend(Session& s, const TreeShape& t, const double* G, const doub
     for (int64_t lvl = 0; lvl <= t.lfill_level; lvl++) {
         const bool is_tail = lvl == t.lfill_level;
         if (is_tail && !tail) break;
-        if (is_tail) EXAFAC_TRY(z_level_any<2>(s, t, G, ex, J, p, order, dv, st));
-        else EXAFAC_TRY(z_level_any<1>(s, t, G, ex, J, p, order, dv, st));
+        // the root's left child lies after the root in `nodes`
+        const unsigned char* at = nl > cap || !nodes ? nullptr : nodes + (lvl == 0 ? (size_t)z.nch * z_chunk_bytes(z) : 0);
+        if (is_tail) EXAFAC_TRY(z_level_any<2>(s, t, G, at, lb, ex, J, p, order, dv, st));
+        else EXAFAC_TRY(z_level_any<1>(s, t, G, at, lb, ex, J, p, order, dv, st));
         if (is_tail && t.F <= 1) break;  // the leaf index needs no order
         if (!in_smem)
             EXAFAC_TRY(scan_exclusive_u32_to_i64(reinterpret_cast<const uint32_t*>(b.tcount[p]), b.pref64, ntiles,
                                                  b.pref64 + ntiles, s.scan_sc, st));
         zq_partition_kernel<<<(unsigned)std::min<int64_t>(ceil_div(J, 512), 152 * 2), 512, psm, st>>>(
             J, (int)ntiles, b.mask[p], b.tcount[p], b.mask[p ^ 1], b.tcount[p ^ 1], b.truns[p ^ 1],
-            in_smem ? nullptr : b.pref64, lb, nl, order, b.node, b.off[p], b.order[p], b.off[p ^ 1]);
+            in_smem ? nullptr : b.pref64, lb, nl, order, b.node, b.off[p], b.order[p], b.off[p ^ 1], s.R, G, ex,
+            t.node_count, 2 * lb + 1, lvl + 1 < t.lfill_level + (tail ? 1 : 0) && 2 * nl <= cap ? 2 * nl : 0, nodes);
         count_launch();
         order = b.order[p];
         p ^= 1;
@@ -1506,7 +1672,7 @@ int sts_draw_zq(Session& s, int n, int64_t J, const double* uni, cudaStream_t st
         zq_vector_kernel<2><<<vgrid, 256, 0, st>>>(R, J, h, s.F.U[k], s.samples, N, k, s.dims[k], b, s.status);
         count_launch();
     }
-    zq_tree_exp_kernel<<<1, 32, 0, st>>>(R, s.PhiP, b.tree_exp + 2 * N);
+    zq_tree_exp_kernel<<<1, 256, 0, st>>>(R, s.PhiP, b.tree_exp + 2 * N, 0, nullptr);
     count_launch();
     const size_t smem = zw_smem(R);
     const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(J, kZTile), 152);
