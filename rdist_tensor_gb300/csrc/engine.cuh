@@ -205,6 +205,9 @@ int sts_rebuild_tree(Session& s, int k, cudaStream_t st);
 // ---- step kernels (step_kernels.cu)
 int dedup(Session& s, int n, int64_t J, cudaStream_t st);
 int design_gram(Session& s, int n, int64_t J, cudaStream_t st);
+// The FP64 form's design rows and their Gram from digit products (gramq.cu).
+bool design_digits_wanted(int R, int64_t J);
+int design_gram_digits(Session& s, int n, int64_t J, int64_t* nblk, cudaStream_t st);
 int design_pinv(Session& s, cudaStream_t st);
 int gram_rows(Session& s, const double* A, int64_t rows, const uint32_t* rowlist, const int64_t* count_dev,
               double* out_full, cudaStream_t st);

@@ -271,9 +271,12 @@ __global__ void design_kernel(int N, int n, int R, const int64_t* __restrict__ j
                               const double* __restrict__ wd, FactorPtrs f, double* __restrict__ D,
                               double* __restrict__ part) {
     extern __shared__ double sm[];
+    __shared__ double root[kGramRows];  // (a square root per element was a quarter of the kernel)
     const int P = packed_size(R);
     const int64_t ju = *ju_dev;
     const int64_t base = (int64_t)blockIdx.x * kGramRows;
+    if (threadIdx.x < kGramRows) root[threadIdx.x] = base + threadIdx.x < ju ? sqrt(wd[base + threadIdx.x]) : 0.0;
+    __syncthreads();
     for (int e = threadIdx.x; e < kGramRows * R; e += blockDim.x) {
         int lr = e / R, c = e % R;
         int64_t j = base + lr;
@@ -284,7 +287,7 @@ __global__ void design_kernel(int N, int n, int R, const int64_t* __restrict__ j
                 if (k == n) continue;
                 d *= f.U[k][(int64_t)sd[j * N + k] * R + c];
             }
-            const double sw = sqrt(wd[j]);
+            const double sw = root[lr];
             d *= sw;
             v = d;
             D[j * R + c] = d * sw;
@@ -614,8 +617,12 @@ int design_gram(Session& s, int n, int64_t J, cudaStream_t st) {
         EXAFAC_CHECK_LAUNCH();
         return EXAFAC_OK;
     }
-    design_kernel<<<(unsigned)nblk, 128, sizeof(double) * kGramRows * R, st>>>(s.N, n, R, s.counters + 0, s.sd, s.wd,
-                                                                               factor_ptrs(s), s.D, s.part); count_launch();
+    if (design_digits_wanted(R, J)) {
+        EXAFAC_TRY(design_gram_digits(s, n, J, &nblk, st));
+    } else {
+        design_kernel<<<(unsigned)nblk, 128, sizeof(double) * kGramRows * R, st>>>(s.N, n, R, s.counters + 0, s.sd, s.wd,
+                                                                                   factor_ptrs(s), s.D, s.part); count_launch();
+    }
     gram_reduce_kernel<<<packed_size(R), 256, 0, st>>>(s.part, nblk, R, s.dgram); count_launch();
     EXAFAC_CHECK_LAUNCH();
     return EXAFAC_OK;
