@@ -574,6 +574,27 @@ __global__ void sts_draw_kernel(int N, int n, int R, int G, int S, int64_t J, St
     }
 }
 
+// The weights of the samples list[0 .. *list_count) from their h (rows of
+// hrows), as sts_draw_kernel<double> forms them.
+__global__ void sts_weight_list_kernel(int R, int G, int S, int64_t J, const double* __restrict__ hrows,
+                                       const double* __restrict__ PhiP, double* __restrict__ weights,
+                                       const int32_t* __restrict__ list, const int32_t* __restrict__ list_count) {
+    extern __shared__ __align__(16) unsigned char stsdyn[];
+    double *h, *sh, *q;
+    int gi;
+    const SampleGroup<double> grp = sample_group<double>(stsdyn, R, G, h, sh, q, gi);
+    const int64_t todo = *list_count;
+    for (int64_t q0 = (int64_t)blockIdx.x * S + gi; q0 < todo; q0 += (int64_t)gridDim.x * S) {
+        const int64_t i = list[q0];
+        for (int r = grp.tg; r < R; r += grp.nthreads()) h[r] = hrows[i * R + r];
+        grp.sync();
+        grp.build_z(R, h);
+        const double hq = grp.quad(packed_size(R), PhiP);
+        if (grp.tg == 0) weights[i] = hq > 0.0 ? (double)R / (hq * (double)J) : 0.0;
+        grp.sync();
+    }
+}
+
 int sts_refresh_f32(Session& s, int k, cudaStream_t st) {
     if (s.cfg.sampler != EXAFAC_SAMPLER_STS_CP || s.cfg.precision == EXAFAC_PREC_FP64) return EXAFAC_OK;
     EXAFAC_TRY(narrow_copy(s.F.U[k], s.Uf[k], s.dims[k] * s.R, st));
@@ -633,6 +654,15 @@ int sts_draw(Session& s, int n, int64_t J, const double* uni, cudaStream_t st) {
         const int32_t *list = nullptr, *count = nullptr;
         if (s.zq.xi && sts_zq_wanted(s.R, J)) {
             EXAFAC_TRY(sts_draw_zq(s, n, J, uni, st));
+            int G, S;
+            sample_group_shape(s.R, sizeof(double), G, S);
+            const size_t smem = (size_t)S * sample_group_bytes(s.R, sizeof(double));
+            if (smem > 48 * 1024)
+                EXAFAC_CUDA_TRY(
+                    cudaFuncSetAttribute(sts_weight_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            sts_weight_list_kernel<<<(unsigned)std::max<int64_t>(std::min<int64_t>(ceil_div(J, S), 152 * 4), 1), S * G * 32,
+                                     smem, st>>>(s.R, G, S, J, s.D, s.PhiP, s.weights, s.zq.near_list, s.zq.near_count);
+            count_launch();
             list = s.zq.redo_list;
             count = s.zq.redo_count;
         }

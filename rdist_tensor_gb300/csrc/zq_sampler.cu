@@ -1223,8 +1223,11 @@ __global__ void zq_leaf1_kernel(TreeShape t, int64_t J, ZState b, int N, int col
 // chunks of 16 columns): the dropped part is below R 4 2^-50 of n1 in the
 // scaled units, under FP64's rounding of the depth-first sum, whose R^2 / 2
 // products and sums per sample took 3.1 ms at R = 64, J = 2^18.  A sample
-// whose form is not positive, not finite, or cancels (the bound above 2^-45 of
-// it) is marked.
+// whose form is not positive or not finite is marked; one whose form cancels
+// (the bound above 2^-42 of it) gets the depth-first kernel's own sum from h
+// (sts_weight_list_kernel).  As a decomposition converges that is a tenth of the
+// samples, and drawing them again whole took 1.1 ms a step at R = 100 with four
+// modes, 6 ms at R = 66 with three.
 constexpr int kWx = 5, kWa = 8, kWCols = 16;
 
 static size_t zw_smem(int R) {
@@ -1427,11 +1430,12 @@ __global__ void __launch_bounds__(NT, 1)
                               ((double)s6[2] * 0x1p-43 + (double)s6[0] * 0x1p-28));
             const int64_t j = s0 + tid;
             const int ex = b.ex[j];
-            const bool good = q > 0.0 && ex < 2047 && emax < 2047 &&
-                              (double)b.n1[j] * (double)R * 0x1p-48 + (double)R * (double)R * 0x1p-57 < q * 0x1p-45;
+            const bool usable = q > 0.0 && ex < 2047 && emax < 2047;
+            const bool good = usable && (double)b.n1[j] * (double)R * 0x1p-48 + (double)R * (double)R * 0x1p-57 < q * 0x1p-42;
             const double hq = scalbn(q, 2 * ex + emax - 3084);
             weights[j] = good ? (double)R / (hq * (double)J) : 0.0;
-            if (!good) z_mark(b.redo, b.redo_list, b.redo_count, (int32_t)j);
+            if (!usable) z_mark(b.redo, b.redo_list, b.redo_count, (int32_t)j);
+            else if (!good) b.near_list[atomicAdd(b.near_count, 1)] = (int32_t)j;
         }
         __syncthreads();
     }
