@@ -657,6 +657,8 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
             i0 = i1;
         }
         if (aborted) break;
+        // runs that stay take no barrier: everyone is done with cs before the next tile's replaces it
+        if (MODE == 2) __syncthreads();
         if (tid < kZTile && flag == 2) {
             long long s5[5];
 #pragma unroll

@@ -3,7 +3,7 @@ cores, marked samples drawn again depth first) against the CPU oracle's
 depth-first draws: samples equal, weights to 1e-12 (the bound of the other
 draw tests), at the edges of the tiles and ranks: odd ranks, ranks below and
 above a 32-column chunk and the 64-column switch, one-leaf trees, partial
-leaves, a last tile of one sample, heavy-tailed rows, and zero columns."""
+leaves, a last tile of one sample, heavy-tailed and skewed rows, and zero columns."""
 import numpy as np
 import pytest
 
@@ -19,6 +19,7 @@ CASES = [
     ((140, 70, 300), 65, 4097, "sparse"),
     ((400, 99, 201), 100, 2048, "heavy"),
     ((300, 128, 129), 128, 2049, "gaussian"),
+    ((17811, 97, 611), 58, 20001, "skewed"),
 ]
 
 
@@ -34,6 +35,8 @@ def test_draws_match_oracle(oracle_mod, dims, R, J, kind):
         U = rng.standard_normal((d, R))
         if kind == "heavy":
             U *= np.exp(2.0 * rng.standard_normal((d, 1)))
+        if kind == "skewed":  # the rare rows' tiles of the tail level: long sequences of leaves that stay
+            U *= (1.0 + np.arange(d))[:, None] ** -0.55
         if kind == "sparse":
             U *= rng.random((d, R)) < 0.3
         factors.append(np.ascontiguousarray(U / np.sqrt((U * U).sum(axis=0))))
