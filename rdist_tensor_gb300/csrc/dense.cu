@@ -254,8 +254,8 @@ __global__ void syev_kernel(int R, const double* __restrict__ A, int64_t a_strid
 //      left (a cluster, eigenvalues below FP32's resolution), then the sorted
 //      outputs.  X that is not orthonormal to 4 R eps, or a value that is not
 //      finite, starts the sweeps from A as before.
-// Measured (GB300, a batch of 3, launches included): R = 25 / 64 / 100 / 128:
-// 0.20 / 0.57 / 1.9 / 2.5 ms (the FP64 sweeps alone 0.88 / 5.2 / 17.6 / 35.9),
+// Measured (GB300, one to three matrices a call, launches included): R = 25 / 64 /
+// 100: 0.21 / 0.56 / 1.8 ms (the FP64 sweeps alone 0.88 / 5.2 / 17.6),
 // |A v - lambda v| <= 6e-16 |A| against 5e-15 .. 3e-14, a 92-fold near-null
 // cluster at R = 100 11 against 26 ms.
 // ---------------------------------------------------------------------------

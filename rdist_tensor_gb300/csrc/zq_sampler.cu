@@ -42,7 +42,7 @@
 // and from FP64 dots where that bound leaves it open (zq_place_kernel).
 //
 // Measured (GB300), draws of a step: R = 64, J = 2^18, three 2000-row modes:
-// 55.8 -> 7.9 ms; R = 25, J = 65536: 4.3 -> 1.4 ms.
+// 55.8 -> 4.1 ms; R = 25, J = 65536: 4.3 -> 0.8 ms.
 #include "digits.cuh"
 #include "engine.cuh"
 #include "prims.cuh"
