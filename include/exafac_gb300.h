@@ -259,6 +259,11 @@ int exafac_als_sweeps(exafac_als_t s, int64_t J, int32_t count, const double* un
  * pass publish no status, so the waits on it run out; -1 turns this off. */
 int exafac_als_set_wait_limit(exafac_als_t s, uint32_t polls, int64_t withhold_tile);
 
+/* Test hook: the number of blocks of the FP64 form's breadth-first STS-CP draw
+ * kernels (0 = the default, one wave of the chip).  The draws do not depend on
+ * it, nor on the order in which the blocks run. */
+int exafac_als_set_draw_blocks(exafac_als_t s, int32_t blocks);
+
 /* Copies the last step's counters to the host (synchronises). */
 int exafac_als_step_info(exafac_als_t s, exafac_step_info* out, void* stream);
 

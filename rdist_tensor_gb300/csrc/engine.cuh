@@ -178,6 +178,9 @@ struct Session {
     // a tile of the first digit pass that publishes no status.
     uint32_t wait_polls = kSpinLimit;
     int64_t withhold_tile = -1;
+    // Test hook (exafac_als_set_draw_blocks): blocks of the FP64 form's
+    // breadth-first draw kernels, 0 = one wave of the chip.
+    int64_t draw_blocks = 0;
 };
 
 // ---- sampler kernels (sampler_kernels.cu)

@@ -724,6 +724,17 @@ extern "C" int exafac_als_set_wait_limit(exafac_als_t h, uint32_t polls, int64_t
     return EXAFAC_OK;
 }
 
+extern "C" int exafac_als_set_draw_blocks(exafac_als_t h, int32_t blocks) {
+    EXAFAC_ARG(h != nullptr, "null session");
+    EXAFAC_ARG(blocks >= 0, "blocks must be >= 0");
+    h->s.draw_blocks = blocks;
+    if (h->sweep_exec) {  // the captured sweep holds the old grid
+        cudaGraphExecDestroy(h->sweep_exec);
+        h->sweep_exec = nullptr;
+    }
+    return EXAFAC_OK;
+}
+
 extern "C" int exafac_als_estimated_fit(exafac_als_t h, int64_t Z, const uint32_t* zero_idx, uint64_t seed,
                                         double* fit, int64_t* kept, void* stream) {
     EXAFAC_ARG(h && h->s.initialized, "session not initialised");

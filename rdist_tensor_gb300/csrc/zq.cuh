@@ -25,7 +25,7 @@ struct ZState {
     // of two consecutive levels (ping-pong), per tile of 128 slots:
     uint32_t* mask[2] = {nullptr, nullptr};   // 4 words: went left (or stayed)
     int32_t* tcount[2] = {nullptr, nullptr};  // flags set
-    int32_t* truns[2] = {nullptr, nullptr};   // runs of equal node, less one
+    uint32_t* runs[2] = {nullptr, nullptr};   // 4 words: a run of equal node starts here (bit 0 of a tile clear)
     int64_t* pref64 = nullptr;  // per tile: prefix of tcount (more tiles than shared memory takes)
     int64_t* off[2] = {nullptr, nullptr};  // slot ranges of a level's nodes (ping-pong)
     int32_t* tree_exp = nullptr;           // 2 N + 1: exponent of each tree's root diagonal, and Phi's

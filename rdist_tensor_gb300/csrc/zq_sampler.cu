@@ -303,23 +303,30 @@ __device__ __forceinline__ double z_bound(float n1, int R) {
 // at the same node) costs its node's expansion and products whatever its
 // length, and the runs are spread unevenly over the tiles (skewed modes: the
 // tiles of the rare rows hold up to 128), so every block takes the same number
-// of runs: runs [first, first + count) in slot order, found from the per-tile
-// run counts.  With equal numbers of tiles the slowest block took 3.9 ms on a
-// tail level of a Zipf mode, with equal numbers of runs 0.2 ms.
+// of runs: runs [first, first + count) in slot order, found from the tiles'
+// run starts (a bit per slot, ZState::runs).  With equal numbers of tiles the
+// slowest block took 3.9 ms on a tail level of a Zipf mode, with equal numbers
+// of runs 0.2 ms.  A tile's runs may belong to several blocks, in any order of
+// time: a block takes the starts from the bits, which no level changes, and
+// reads and writes the nodes of its own slots only.
 struct ZShare {
     int64_t tile;   // first tile
     int run;        // first run within it
     int64_t count;  // runs
 };
 template <int NT>
-__device__ __forceinline__ ZShare z_share(const int32_t* __restrict__ truns, int64_t ntiles) {
+__device__ __forceinline__ ZShare z_share(const uint32_t* __restrict__ runs, int64_t ntiles) {
     __shared__ long long wsum[NT / 32];
     __shared__ long long found[2];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int64_t per = (ntiles + NT - 1) / NT;
     const int64_t a = min(ntiles, per * tid), e = min(ntiles, a + per);
-    long long sum = e - a;
-    for (int64_t q = a; q < e; q++) sum += __ldg(truns + q);
+    auto count = [&](int64_t q) {
+        const uint4 m = __ldg(reinterpret_cast<const uint4*>(runs) + q);
+        return 1 + (__popc(m.x) + __popc(m.y)) + (__popc(m.z) + __popc(m.w));
+    };
+    long long sum = 0;
+    for (int64_t q = a; q < e; q++) sum += count(q);
     long long inc = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -341,7 +348,7 @@ __device__ __forceinline__ ZShare z_share(const int32_t* __restrict__ truns, int
     if (first >= before && first < before + sum) {
         long long at = before;
         for (int64_t q = a; q < e; q++) {
-            const long long r = 1 + __ldg(truns + q);
+            const long long r = count(q);
             if (first < at + r) {
                 found[0] = q;
                 found[1] = first - at;
@@ -358,18 +365,7 @@ __device__ __forceinline__ ZShare z_share(const int32_t* __restrict__ truns, int
     return s;
 }
 
-// Run starts of the tile's nodes cs[0 .. n) as a bit mask (threads < 128;
-// cs[-1] differs); two block barriers.
-__device__ __forceinline__ void z_run_mask(const int32_t* cs, int n, uint32_t* rmask) {
-    const int tid = threadIdx.x;
-    __syncthreads();
-    if (tid < kZTile) {
-        const bool start = tid < n && (tid == 0 || cs[tid] != cs[tid - 1]);
-        const uint32_t m = __ballot_sync(0xffffffffu, start);
-        if ((tid & 31) == 0) rmask[tid >> 5] = m;
-    }
-    __syncthreads();
-}
+// The end of the run that slot i0 belongs to, from the tile's run starts.
 __device__ __forceinline__ int z_run_end(const uint32_t* rmask, int i0, int n) {
     for (int q = (i0 + 1) >> 5; q < 4; q++) {
         uint32_t bits = rmask[q];
@@ -377,6 +373,18 @@ __device__ __forceinline__ int z_run_end(const uint32_t* rmask, int i0, int n) {
         if (bits) return min(n, (q << 5) + __ffs(bits) - 1);
     }
     return n;
+}
+// The block's slots [first, last) of the tile: `count` runs from run `run` on.
+__device__ __forceinline__ int2 z_run_slots(const uint32_t* rmask, int run, int64_t count, int n) {
+    int first = 0;
+    for (int q = 0; q < run && first < n; q++) first = z_run_end(rmask, first, n);
+    const int all = 1 + (__popc(rmask[0]) + __popc(rmask[1])) + (__popc(rmask[2]) + __popc(rmask[3]));
+    int last = n;
+    if (count < all - run) {
+        last = first;
+        for (int64_t q = 0; q < count; q++) last = z_run_end(rmask, last, n);
+    }
+    return make_int2(first, last);
 }
 
 // One chunk's read-back, columns c0 .. c0 + 7 of the node: the five integer
@@ -421,8 +429,8 @@ __device__ __forceinline__ void z_dot8(uint32_t taddr, const long long* xrow, in
 // MODE 1: a level: the left child's mass and the branch.
 // MODE 2: the tail level: as MODE 1; samples already at a leaf stay.
 // The branch flags of a tile's slots are set in mask[p], their count added to
-// tcount[p] (both zero before); truns[p] holds the runs per tile less one,
-// truns[p ^ 1] is cleared for the partition that follows.
+// tcount[p] (both zero before); runs[p] holds the tiles' run starts, runs[p ^ 1]
+// is cleared for the partition that follows.
 // NT = 512 (R > 64, one block per SM): a chunk's products run beside the
 // previous chunk's read-back (two accumulator sets), and beside the next
 // chunk's expansion when a second node buffer fits (nb = 2).
@@ -487,8 +495,9 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
         sh.run = 0;
         sh.count = ntiles * (blockIdx.x + 1) / gridDim.x - sh.tile;
     } else {
-        sh = z_share<NT>(b.truns[p], ntiles);
-        for (int64_t q = (int64_t)blockIdx.x * NT + tid; q < ntiles; q += (int64_t)gridDim.x * NT) b.truns[p ^ 1][q] = 0;
+        sh = z_share<NT>(b.runs[p], ntiles);
+        for (int64_t q = (int64_t)blockIdx.x * NT + tid; q < ntiles; q += (int64_t)gridDim.x * NT)
+            reinterpret_cast<uint4*>(b.runs[p ^ 1])[q] = make_uint4(0u, 0u, 0u, 0u);
     }
     const bool ok = emax < 2047;  // a tree with a non-finite root: every sample is marked at the root
     // the chunk's products are done (every thread)
@@ -527,10 +536,14 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
         float e0 = 0.f, n1 = 0.f;
         int ex = 0;
         int flag = -1;  // -1: not this block's, 0 right, 1 left (or stays), 2 summed
+        if (tid < 4) rmask[tid] = MODE == 0 ? 0u : b.runs[p][4 * sh.tile + tid];
+        __syncthreads();
+        const int2 own = z_run_slots(rmask, sh.run, sh.count, n);
+        int i0 = own.x;
         if (tid < kZTile) {
             int32_t j = 0, c = -1;
-            if (tid < n) {
-                j = order ? order[s0 + tid] : (int32_t)(s0 + tid);
+            if (tid < n) j = order ? order[s0 + tid] : (int32_t)(s0 + tid);
+            if (tid >= own.x && tid < own.y) {
                 c = MODE == 0 ? 0 : (int32_t)b.node[j];
                 ex = b.ex[j];
                 n1 = b.n1[j];
@@ -545,11 +558,9 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
             js[tid] = j;
             cs[tid] = c;
         }
-        z_run_mask(cs, n, rmask);
-        int i0 = 0;
-        for (int q = 0; q < sh.run && i0 < n; q++) i0 = z_run_end(rmask, i0, n);
+        __syncthreads();
         bool ahead = false;  // the next run's first chunk is on its way
-        if (pre && i0 < n && !stays(cs[i0]) && !(z.nch == 1 && resident == cs[i0])) {
+        if (pre && i0 < own.y && !stays(cs[i0]) && !(z.nch == 1 && resident == cs[i0])) {
             if (tid == 0) fetch(0, cs[i0], 0);
             ahead = true;
         }
@@ -557,7 +568,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
         fence_proxy_async_smem();
         tc_fence_before();
         __syncthreads();
-        for (; i0 < n && sh.count > 0; sh.count--) {  // runs of equal node (uniform over the block)
+        for (; i0 < own.y; sh.count--) {  // runs of equal node (uniform over the block)
             const int32_t c = cs[i0];
             const int i1 = z_run_end(rmask, i0, n);
             if (stays(c)) {
@@ -591,7 +602,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
                                 if (kPipe) issue(0, cur ^ 1, true);
                             }
                         }
-                    } else if (i1 < n && sh.count > 1 && cs[i1] != c && !stays(cs[i1])) {
+                    } else if (i1 < own.y && !stays(cs[i1])) {
                         if (tid == 0) fetch(0, cs[i1], 0);
                         ahead = true;
                     }
@@ -770,7 +781,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
     uint32_t phase = 0;
     const int row = (w & 3) * 32 + lane, grp = w >> 2;
     const int64_t ntiles = (J + kZTile - 1) / kZTile;
-    ZShare sh = z_share<NT>(b.truns[p], ntiles);
+    ZShare sh = z_share<NT>(b.runs[p], ntiles);
     for (; sh.count > 0 && sh.tile < ntiles; sh.tile++, sh.run = 0) {
         const int64_t s0 = sh.tile * kZTile;
         const int n = (int)min((int64_t)kZTile, J - s0);
@@ -779,11 +790,11 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
             js[tid] = j;
             cs[tid] = tid < n ? (int32_t)b.node[j] : -1;
         }
-        z_run_mask(cs, n, rmask);
+        if (tid < 4) rmask[tid] = b.runs[p][4 * sh.tile + tid];
+        __syncthreads();
         stage_x(A, reinterpret_cast<const long long*>(b.xi), js, n, R, z);
-        int i0 = 0;
-        for (int q = 0; q < sh.run && i0 < n; q++) i0 = z_run_end(rmask, i0, n);
-        for (; i0 < n && sh.count > 0; sh.count--) {
+        const int2 own = z_run_slots(rmask, sh.run, sh.count, n);
+        for (int i0 = own.x; i0 < own.y; sh.count--) {
             const int32_t c = cs[i0];
             const int i1 = z_run_end(rmask, i0, n);
             if (!tree_is_leaf(t, c)) {  // only after a wait that ran out: not placed
@@ -1047,7 +1058,7 @@ __device__ __forceinline__ void tile_prefix(const int32_t* __restrict__ tcount, 
 // before slot s, is the tile's prefix plus the bits below s of its mask.
 // Within its parent's slot range a slot whose flag is set (went left, or
 // stayed at a leaf) keeps its order among those, before the others; the
-// children's slot ranges (coff) and their runs per tile follow, and the next
+// children's slot ranges (coff) and their run starts follow, and the next
 // level's flags are cleared, and the next level's left children are expanded
 // into `nodes` (where it takes them: nx_nl > 0).  Every block
 // forms the tiles' prefix in shared memory (up to kZPrefSmem tiles), or reads
@@ -1055,7 +1066,7 @@ __device__ __forceinline__ void tile_prefix(const int32_t* __restrict__ tcount, 
 __global__ void __launch_bounds__(512)
     zq_partition_kernel(int64_t J, int ntiles, const uint32_t* __restrict__ mask, const int32_t* __restrict__ tcount,
                         uint32_t* __restrict__ mask_next, int32_t* __restrict__ tcount_next,
-                        int32_t* __restrict__ truns_next, const int64_t* __restrict__ pref64, int64_t lb, int64_t nl, const int32_t* __restrict__ order,
+                        uint32_t* __restrict__ runs_next, const int64_t* __restrict__ pref64, int64_t lb, int64_t nl, const int32_t* __restrict__ order,
                         const int64_t* __restrict__ node, const int64_t* __restrict__ off,
                         int32_t* __restrict__ order2, int64_t* __restrict__ coff, int R, const double* __restrict__ G,
                         const int32_t* __restrict__ tree_exp, int64_t node_count, int64_t nx_lb, int64_t nx_nl,
@@ -1108,8 +1119,8 @@ __global__ void __launch_bounds__(512)
         coff[2 * i + 1] = mid;
         if (i == 0) coff[2 * nl] = J;
         // a child that begins inside a tile begins one more run there
-        if (mid > start && (start & 127)) atomicAdd(truns_next + (start >> 7), 1);
-        if (end > mid && (mid & 127)) atomicAdd(truns_next + (mid >> 7), 1);
+        if (mid > start && (start & 127)) atomicOr(runs_next + (start >> 5), 1u << (start & 31));
+        if (end > mid && (mid & 127)) atomicOr(runs_next + (mid >> 5), 1u << (mid & 31));
     }
     for (int64_t q = first; q < ntiles; q += step) {
         reinterpret_cast<uint4*>(mask_next)[q] = make_uint4(0u, 0u, 0u, 0u);
@@ -1200,7 +1211,7 @@ __global__ void zq_vector_kernel(int R, int64_t J, double* __restrict__ h, const
                 const int64_t tile = j >> 7;
                 reinterpret_cast<uint4*>(b.mask[0])[tile] = make_uint4(0u, 0u, 0u, 0u);
                 b.tcount[0][tile] = 0;
-                b.truns[0][tile] = 0;
+                reinterpret_cast<uint4*>(b.runs[0])[tile] = make_uint4(0u, 0u, 0u, 0u);
             }
             if (j == 0) {
                 b.off[0][0] = 0;
@@ -1501,7 +1512,7 @@ void zq_carve(Arena& a, ZState& b, int R, int64_t J, int64_t widest, int trees) 
     for (int q = 0; q < 2; q++) {
         b.mask[q] = a.take<uint32_t>(4 * ceil_div(J, kZTile));
         b.tcount[q] = a.take<int32_t>(ceil_div(J, kZTile) + 4);
-        b.truns[q] = a.take<int32_t>(ceil_div(J, kZTile) + 4);
+        b.runs[q] = a.take<uint32_t>(4 * ceil_div(J, kZTile));
     }
     b.pref64 = a.take<int64_t>(ceil_div(J, kZTile) + 1);
     b.off[0] = a.take<int64_t>(2 * widest + 2);
@@ -1515,6 +1526,12 @@ static unsigned z_grid(int64_t work) {
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(work, 256), 152 * 16));
 }
 
+// One wave of the chip (or the test hook's number of blocks: the draws are the
+// same for any).
+static unsigned z_blocks(const Session& s, int64_t J, int64_t wave) {
+    return (unsigned)(s.draw_blocks > 0 ? s.draw_blocks : std::min(ceil_div(J, kZTile), wave));
+}
+
 template <int MODE, int NT>
 static int z_level(Session& s, const TreeShape& t, const double* G, const unsigned char* nodes, int64_t lb,
                    const int32_t* ex, int64_t J, int p, const int32_t* order, const double* dv, cudaStream_t st) {
@@ -1525,7 +1542,7 @@ static int z_level(Session& s, const TreeShape& t, const double* G, const unsign
     const size_t smem = nb == 2 ? two : z_smem(s.R, kZa);
     EXAFAC_CUDA_TRY(cudaFuncSetAttribute(zq_level_kernel<MODE, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem));
-    const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(J, kZTile), NT == 256 ? 304 : 152);
+    const unsigned blocks = z_blocks(s, J, NT == 256 ? 304 : 152);
     zq_level_kernel<MODE, NT><<<blocks, NT, smem, st>>>(s.R, nb, t, G, nodes, lb, ex, J, s.zq, p, order, dv,
                                                         s.status, s.wait_polls ? s.wait_polls : kSpinLimit);
     count_launch();
@@ -1542,7 +1559,7 @@ static int z_leaf(Session& s, const TreeShape& t, const double* G, const double*
                   const int32_t* order, const double* dv, int col, cudaStream_t st) {
     const size_t smem = z_smem(s.R, kZu);
     EXAFAC_CUDA_TRY(cudaFuncSetAttribute(zq_leaf_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(J, kZTile), NT == 256 ? 304 : 152);
+    const unsigned blocks = z_blocks(s, J, NT == 256 ? 304 : 152);
     zq_leaf_kernel<NT><<<blocks, NT, smem, st>>>(s.R, t, G, U, J, s.zq, p, order, dv, s.N, col, s.samples, s.status,
                                                  s.wait_polls ? s.wait_polls : kSpinLimit);
     count_launch();
@@ -1582,7 +1599,7 @@ static int z_descend(Session& s, const TreeShape& t, const double* G, const doub
             EXAFAC_TRY(scan_exclusive_u32_to_i64(reinterpret_cast<const uint32_t*>(b.tcount[p]), b.pref64, ntiles,
                                                  b.pref64 + ntiles, s.scan_sc, st));
         zq_partition_kernel<<<(unsigned)std::min<int64_t>(ceil_div(J, 512), 152 * 2), 512, psm, st>>>(
-            J, (int)ntiles, b.mask[p], b.tcount[p], b.mask[p ^ 1], b.tcount[p ^ 1], b.truns[p ^ 1],
+            J, (int)ntiles, b.mask[p], b.tcount[p], b.mask[p ^ 1], b.tcount[p ^ 1], b.runs[p ^ 1],
             in_smem ? nullptr : b.pref64, lb, nl, order, b.node, b.off[p], b.order[p], b.off[p ^ 1], s.R, G, ex,
             t.node_count, 2 * lb + 1, lvl + 1 < t.lfill_level + (tail ? 1 : 0) && 2 * nl <= cap ? 2 * nl : 0, nodes);
         count_launch();
