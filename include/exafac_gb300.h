@@ -256,7 +256,11 @@ int exafac_als_sweeps(exafac_als_t s, int64_t J, int32_t count, const double* un
  * `polls` polls (0 = the default, 2^22, about half a second) and the step then
  * reports EXAFAC_ERR_TIMEOUT through exafac_als_step_info.device_status, with
  * no hits processed.  withhold_tile >= 0 makes that tile of the first digit
- * pass publish no status, so the waits on it run out; -1 turns this off. */
+ * pass publish no status, so the waits on it run out; -1 turns this off.
+ * site << 32 | tile does the same to the tensor-core products of the FP64
+ * form: site 23 / 24 / 25 the levels, the leaf stage and the weights of the
+ * breadth-first STS-CP draws (a tile is 128 samples; the samples not drawn by
+ * then are row 0 with weight 0), 26 the design Gram (a tile is 64 rows). */
 int exafac_als_set_wait_limit(exafac_als_t s, uint32_t polls, int64_t withhold_tile);
 
 /* Test hook: the number of blocks of the FP64 form's breadth-first STS-CP draw

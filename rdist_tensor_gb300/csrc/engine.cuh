@@ -174,10 +174,14 @@ struct Session {
     float* Df = nullptr;          // Jmax x f32_row_stride(R) design rows (mixed forms)
 
     uint64_t seed = 0x5eed;  // Philox key; the stream counter is counters[kRngSlot] on the device
-    // Look-back waits of the row sort: poll limit, and (test hook, -1 = off)
-    // a tile of the first digit pass that publishes no status.
+    // Device-side waits: poll limit, and (test hook, -1 = off) site << 32 |
+    // tile, a tile whose waits run out: site 0 the row sort's first digit pass
+    // (no status published), 23 .. 26 as report() numbers them (no products).
     uint32_t wait_polls = kSpinLimit;
     int64_t withhold_tile = -1;
+    int64_t withheld(int site) const {
+        return (withhold_tile >> 32) == site ? withhold_tile & 0xffffffffll : (int64_t)-1;
+    }
     // Test hook (exafac_als_set_draw_blocks): blocks of the FP64 form's
     // breadth-first draw kernels, 0 = one wave of the chip.
     int64_t draw_blocks = 0;

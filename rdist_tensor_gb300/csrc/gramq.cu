@@ -48,7 +48,7 @@ static size_t gq_smem(int R) {
 __global__ void __launch_bounds__(kGqThreads, 1)
     design_digits_kernel(int N, int n, int R, const int64_t* __restrict__ ju_dev, const uint32_t* __restrict__ sd,
                          const double* __restrict__ wd, FactorPtrs f, double* __restrict__ D, double* __restrict__ part,
-                         DeviceStatus* status, uint32_t wait_polls) {
+                         DeviceStatus* status, uint32_t wait_polls, int64_t withhold) {
     extern __shared__ __align__(128) unsigned char gq_raw[];
     __shared__ uint32_t at[kMaxModes][kGqRows];  // the rows' indices
     __shared__ double sw[kGqRows];
@@ -73,6 +73,7 @@ __global__ void __launch_bounds__(kGqThreads, 1)
     const int64_t ntiles = (live + kGqRows - 1) / kGqRows;
     uint32_t phase = 0;
     bool lost = false, dead = false;
+    bool flight = false;  // thread 0: products on their way
     // entry (a, b): a = tensor memory lane, b in this thread's 16 columns of each pass
     const int a = (w & 3) * 32 + lane, grp = w >> 2;
     const int cpt = g.nb / 4;
@@ -171,7 +172,8 @@ __global__ void __launch_bounds__(kGqThreads, 1)
         for (int pass = 0; pass < 2; pass++) {
             if (pass >= g.passes) break;
             const int b0 = pass * kGqCols, nb = min(g.nb, g.Rp - b0);
-            if (tid == 0) {
+            if (tid == 0 && tile != withhold) {
+                flight = true;
                 tc_fence_after();
                 const uint32_t idesc = umma_idesc_bf16(128, nb);
                 for (int i = 0; i < kGqDigits; i++)
@@ -182,8 +184,12 @@ __global__ void __launch_bounds__(kGqThreads, 1)
                                       idesc, (i > 0 || ks > 0) ? 1u : 0u);
                 umma_commit(&bar);
             }
-            if (!mbar_wait_limited(&bar, phase, wait_polls)) lost = true;
-            phase ^= 1u;
+            if (mbar_wait_limited(&bar, phase, wait_polls)) {
+                phase ^= 1u;
+                flight = false;
+            } else {
+                lost = true;
+            }
             tc_fence_after();
             const double sa = scale[a];
 #pragma unroll
@@ -223,7 +229,7 @@ __global__ void __launch_bounds__(kGqThreads, 1)
     if (dead) {
         if (tid == 0) {
             report(status, EXAFAC_ERR_TIMEOUT, 26, blockIdx.x, 0);
-            mbar_wait_limited(&bar, phase ^ 1u, wait_polls);
+            if (flight) mbar_wait_limited(&bar, phase, kSpinLimit);
         }
     }
 #pragma unroll
@@ -256,7 +262,8 @@ int design_gram_digits(Session& s, int n, int64_t J, int64_t* nblk, cudaStream_t
         cudaFuncSetAttribute(design_digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     *nblk = std::max<int64_t>(1, std::min<int64_t>(ceil_div(J, kGqRows), 152));
     design_digits_kernel<<<(unsigned)*nblk, kGqThreads, smem, st>>>(s.N, n, s.R, s.counters + 0, s.sd, s.wd, f, s.D, s.part,
-                                                                    s.status, s.wait_polls ? s.wait_polls : kSpinLimit);
+                                                                    s.status, s.wait_polls ? s.wait_polls : kSpinLimit,
+                                                                    s.withheld(26));
     count_launch();
     EXAFAC_CHECK_LAUNCH();
     return EXAFAC_OK;

@@ -556,13 +556,13 @@ static int sort_keys(Session& s, int n, bool packed, cudaStream_t st) {
             EXAFAC_CUDA_TRY(launch_dependent(os_downsweep_kernel<uint64_t, IT>, kHsDownGridPacked, kHsThreads, smem, st,
                                              s.counters, cap, s.hit_key[src], s.pay64[src], p, s.os_aux, s.os_status,
                                              s.hit_key[dst], s.pay64[dst], s.status, s.wait_polls,
-                                             p == 0 ? s.withhold_tile : (int64_t)-1));
+                                             p == 0 ? s.withheld(0) : (int64_t)-1));
         } else {
             const size_t smem = (sizeof(uint32_t) + sizeof(uint32_t)) * kHsTile;
             EXAFAC_CUDA_TRY(launch_dependent(os_downsweep_kernel<uint32_t, kHsItems>, kHsDownGrid, kHsThreads, smem, st,
                                              s.counters, cap, s.hit_key[src], p == 0 ? nullptr : s.hit_pay[src], p,
                                              s.os_aux, s.os_status, s.hit_key[dst], s.hit_pay[dst], s.status,
-                                             s.wait_polls, p == 0 ? s.withhold_tile : (int64_t)-1));
+                                             s.wait_polls, p == 0 ? s.withheld(0) : (int64_t)-1));
         }
         count_launch();
         EXAFAC_CHECK_LAUNCH();

@@ -22,6 +22,7 @@ struct ZState {
     int32_t* redo_count = nullptr;  // 1
     int32_t* near_list = nullptr;   // leaf reached, its row within the FP32 stage's bound of another (later: FP64 weight)
     int32_t* near_count = nullptr;  // 1
+    int32_t* lost = nullptr;        // 1: a wait of this draw ran out, its later kernels do nothing
     // of two consecutive levels (ping-pong), per tile of 128 slots:
     uint32_t* mask[2] = {nullptr, nullptr};   // 4 words: went left (or stayed)
     int32_t* tcount[2] = {nullptr, nullptr};  // flags set

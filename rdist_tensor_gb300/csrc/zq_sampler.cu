@@ -294,6 +294,13 @@ __device__ __forceinline__ void z_mark(int32_t* redo, int32_t* list, int32_t* co
     if (atomicExch(redo + j, 1) == 0) list[atomicAdd(count, 1)] = j;
 }
 
+// A wait of this draw ran out (ZState::lost): the draw's later kernels return
+// at once, every sample that is not drawn yet takes row 0 and no weight.  The
+// caller sees EXAFAC_ERR_TIMEOUT.  Every thread of the block calls.
+__device__ __forceinline__ bool z_lost(const ZState& b) {
+    return __syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile int32_t*>(b.lost) != 0);
+}
+
 // E of the header, in the scaled units.
 __device__ __forceinline__ double z_bound(float n1, int R) {
     return (double)n1 * ((double)R * 4.6 * 0x1p-34 + 1.7 * 0x1p-32) + (double)R * (double)R * 0x1p-44;
@@ -447,8 +454,9 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
     zq_level_kernel(int R, int nb, TreeShape t, const double* __restrict__ G, const unsigned char* __restrict__ nodes,
                     int64_t lb, const int32_t* __restrict__ tree_exp, int64_t J, ZState b, int p,
                     const int32_t* __restrict__ order, const double* __restrict__ dv, DeviceStatus* status,
-                    uint32_t wait_polls) {
+                    uint32_t wait_polls, int64_t withhold) {
     extern __shared__ __align__(128) unsigned char z_raw[];
+    if (z_lost(b)) return;
     constexpr int NG = NT / 128;        // threads per slot in the read-back
     constexpr int CPT = kZCols / NG;    // columns of a chunk per thread
     constexpr bool kPipe = NT == 512;
@@ -484,6 +492,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
     const int emax = *tree_exp;
     uint32_t phase[2] = {0, 0}, cphase[2] = {0, 0};
     bool lost = false;     // a wait of this thread ran out
+    uint32_t flight = 0;   // thread 0: bit q a copy into buffer q, bit 2 + q products of set q
     int64_t resident = -1; // the node B holds, or is being copied (one-chunk ranks)
     bool aborted = false;
     const int row = (w & 3) * 32 + lane, grp = w >> 2;
@@ -502,24 +511,36 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
     const bool ok = emax < 2047;  // a tree with a non-finite root: every sample is marked at the root
     // the chunk's products are done (every thread)
     auto wait = [&](int q) {
-        if (!mbar_wait_limited(&bars[q], phase[q], wait_polls)) lost = true;
-        phase[q] ^= 1u;
+        if (mbar_wait_limited(&bars[q], phase[q], wait_polls)) {
+            phase[q] ^= 1u;
+            flight &= ~(4u << q);
+        } else {
+            lost = true;
+        }
         tc_fence_after();
     };
-    // thread 0: chunk ch of the left child of parent c into buffer q; the products of buffer q's chunk
+    // thread 0: chunk ch of the left child of parent c into buffer q; the products of buffer q's
+    // chunk into accumulator set `set`, after its copy (fresh).  Nothing more once a wait ran out
+    // (the others' waits run out as well), nor for the tile of the wait-limit test hook.
     auto fetch = [&](int q, int32_t c, int ch) {
+        if (lost) return;
+        flight |= 1u << q;
         const int64_t slot = MODE == 0 ? 0 : (int64_t)c - lb;
         mbar_arrive_expect_tx(&copied[q], cbytes);
         bulk_g2s(Bb[q], nodes + (slot * z.nch + ch) * cbytes, cbytes, &copied[q]);
     };
     auto issue = [&](int q, int set, bool fresh) {
+        if (lost) return;
         if (fresh) {
             if (!mbar_wait_limited(&copied[q], cphase[q], wait_polls)) {
-                lost = true;  // no products: the others' waits run out as well
+                lost = true;
                 return;
             }
             cphase[q] ^= 1u;
+            flight &= ~(1u << q);
         }
+        if (sh.tile == withhold) return;
+        flight |= 4u << set;
         issue_chunk<kZa>(tmem + (uint32_t)(set * 256), A, Bb[q], z, &bars[set]);
     };
     // the chunk's columns of this thread
@@ -620,7 +641,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
                 fence_proxy_async_smem();
                 tc_fence_before();
                 __syncthreads();
-                if (tid == 0) issue_chunk<kZa>(tmem, A, Bb[0], z, &bars[0]);
+                if (tid == 0) issue(0, 0, false);
                 for (int ch = 0; ch < z.nch; ch++) {
                     const int cur = kPipe ? ch & 1 : 0;
                     const bool more = ch + 1 < z.nch;
@@ -632,9 +653,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
                             fence_proxy_async_smem();
                             tc_fence_before();
                             __syncthreads();
-                            if (tid == 0)
-                                issue_chunk<kZa>(tmem + (uint32_t)((cur ^ 1) * 256), A, Bb[(ch + 1) & (nb - 1)], z,
-                                                 &bars[cur ^ 1]);
+                            if (tid == 0) issue((ch + 1) & (nb - 1), cur ^ 1, false);
                         }
                         if (nb == 2 || !more) wait(cur);
                         dots(acc, xrow, ch, sum);
@@ -646,7 +665,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
                             fence_proxy_async_smem();
                             tc_fence_before();
                             __syncthreads();
-                            if (tid == 0) issue_chunk<kZa>(tmem, A, Bb[0], z, &bars[0]);
+                            if (tid == 0) issue(0, 0, false);
                         }
                     }
                 }
@@ -716,17 +735,19 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
         }
     }
     __syncthreads();
-    if (aborted) {  // the tiles left out keep clear flags: the partition keeps their order
-        if (tid == 0) {
+    if (tid == 0) {
+        if (aborted) {
             report(status, EXAFAC_ERR_TIMEOUT, 23, blockIdx.x, 0);
-            // the copies and MMAs in flight may still complete (bounded)
-            for (int q = 0; q < 2; q++) mbar_wait_limited(&copied[q], cphase[q], wait_polls);
+            *b.lost = 1;
         }
-        if (tid == 0) mbar_wait_limited(&bars[0], phase[0] ^ 1u, wait_polls);
-        if (tid == 32) mbar_wait_limited(&bars[1], phase[1] ^ 1u, wait_polls);
-        tc_fence_before();
-        __syncthreads();
+        // the copies and products in flight (after a wait that ran out only)
+        for (int q = 0; q < 2; q++) {
+            if (flight & (1u << q)) mbar_wait_limited(&copied[q], cphase[q], kSpinLimit);
+            if (flight & (4u << q)) mbar_wait_limited(&bars[q], phase[q], kSpinLimit);
+        }
     }
+    tc_fence_before();
+    __syncthreads();
     if (w == 0) {
         tc_fence_after();
         tmem_dealloc(tmem, kTmem);
@@ -750,8 +771,9 @@ template <int NT>
 __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
     zq_leaf_kernel(int R, TreeShape t, const double* __restrict__ G, const double* __restrict__ U, int64_t J, ZState b,
                    int p, const int32_t* __restrict__ order, const double* __restrict__ dv, int N, int col,
-                   uint32_t* __restrict__ samples, DeviceStatus* status, uint32_t wait_polls) {
+                   uint32_t* __restrict__ samples, DeviceStatus* status, uint32_t wait_polls, int64_t withhold) {
     extern __shared__ __align__(128) unsigned char z_raw[];
+    if (z_lost(b)) return;
     constexpr int NG = NT / 128;
     constexpr int CPT = kZCols / NG;
     constexpr int NS = (NT == 256 ? 2 : 4);  // chunks (leaf rows / 32) at most
@@ -779,6 +801,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
     tc_fence_after();
     const uint32_t tmem = tmem_base;
     uint32_t phase = 0;
+    bool flight = false;  // thread 0: products on their way
     const int row = (w & 3) * 32 + lane, grp = w >> 2;
     const int64_t ntiles = (J + kZTile - 1) / kZTile;
     ZShare sh = z_share<NT>(b.runs[p], ntiles);
@@ -797,14 +820,6 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
         for (int i0 = own.x; i0 < own.y; sh.count--) {
             const int32_t c = cs[i0];
             const int i1 = z_run_end(rmask, i0, n);
-            if (!tree_is_leaf(t, c)) {  // only after a wait that ran out: not placed
-                if (tid >= i0 && tid < i1) {
-                    z_mark(b.redo, b.redo_list, b.redo_count, js[tid]);
-                    samples[(int64_t)js[tid] * N + col] = 0u;
-                }
-                i0 = i1;
-                continue;
-            }
             const int64_t leaf = tree_leaf_idx(t, c);
             const int rows = (int)min((int64_t)F, t.n - leaf * F);
             const double* Ub = U + leaf * F * R;
@@ -825,9 +840,16 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
                     fence_proxy_async_smem();
                     tc_fence_before();
                     __syncthreads();
-                    if (tid == 0) issue_chunk<kZu>(tmem, A, B, z, &bar);
-                    if (!mbar_wait_limited(&bar, phase, wait_polls)) abort_flag = 1;
-                    phase ^= 1u;
+                    if (tid == 0 && sh.tile != withhold) {
+                        issue_chunk<kZu>(tmem, A, B, z, &bar);
+                        flight = true;
+                    }
+                    if (mbar_wait_limited(&bar, phase, wait_polls)) {
+                        phase ^= 1u;
+                        flight = false;
+                    } else {
+                        abort_flag = 1;
+                    }
                     tc_fence_after();
                     float ps = 0.0f;
 #pragma unroll
@@ -918,7 +940,8 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
     if (abort_flag) {
         if (tid == 0) {
             report(status, EXAFAC_ERR_TIMEOUT, 24, blockIdx.x, 0);
-            mbar_wait_limited(&bar, phase ^ 1u, wait_polls);
+            *b.lost = 1;
+            if (flight) mbar_wait_limited(&bar, phase, kSpinLimit);
         }
         tc_fence_before();
         __syncthreads();
@@ -945,6 +968,7 @@ __global__ void __launch_bounds__(kPlaceThreads)
     __shared__ double xs[kMaxRank], sq[kMaxLeafRows];
     __shared__ int diag_exp;
     const int tid = threadIdx.x, lane = tid & 31, P = packed_size(R), F = (int)t.F;
+    if (z_lost(b)) return;
     const int count = *b.near_count;
     for (int q = blockIdx.x; q < count; q += gridDim.x) {
         const int32_t j = b.near_list[q];
@@ -1070,8 +1094,9 @@ __global__ void __launch_bounds__(512)
                         const int64_t* __restrict__ node, const int64_t* __restrict__ off,
                         int32_t* __restrict__ order2, int64_t* __restrict__ coff, int R, const double* __restrict__ G,
                         const int32_t* __restrict__ tree_exp, int64_t node_count, int64_t nx_lb, int64_t nx_nl,
-                        unsigned char* __restrict__ nodes) {
+                        unsigned char* __restrict__ nodes, const int32_t* __restrict__ lost) {
     extern __shared__ int32_t z_pref[];
+    if (*lost) return;  // (no level runs beside this kernel: the same in every thread)
     if (nx_nl > 0) {
         const ZShape z = z_shape(R);
         const int emax = *tree_exp, items = kZCols * (z.Rk / 8);
@@ -1101,16 +1126,12 @@ __global__ void __launch_bounds__(512)
         const int32_t j = order ? order[s] : (int32_t)s;
         const int64_t c = node[j];
         const int64_t i = (c >= lb + nl ? (c - 1) / 2 : c) - lb;
-        if (i < 0 || i >= nl) {  // only after a wait that ran out
-            order2[s] = j;
-            continue;
-        }
         const int64_t start = off[i], end = off[i + 1];
         const int64_t at0 = SL(start), at = SL(s);
         const bool fl = (__ldg(mask + 4 * (s >> 7) + ((s & 127) >> 5)) >> (s & 31)) & 1u;
         const int64_t before = at - at0;
         const int64_t pos = fl ? start + before : start + (SL(end) - at0) + ((s - start) - before);
-        if (pos >= 0 && pos < J) order2[pos] = j;
+        order2[pos] = j;
     }
     for (int64_t i = first; i < nl; i += step) {
         const int64_t start = off[i], end = off[i + 1];
@@ -1160,11 +1181,17 @@ __global__ void __launch_bounds__(256) zq_tree_exp_kernel(int R, const double* _
 // KIND 0: h = 1.  KIND 1: x = h * E[v].  KIND 2: h *= U[row], x = h.
 template <int KIND>
 __global__ void zq_vector_kernel(int R, int64_t J, double* __restrict__ h, const double* __restrict__ M,
-                                 const uint32_t* __restrict__ samples, int N, int col, int64_t rows, ZState b,
+                                 uint32_t* __restrict__ samples, int N, int col, int64_t rows, ZState b,
                                  DeviceStatus* status) {
     const int lane = threadIdx.x & 31;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const bool lost = KIND != 0 && *b.lost != 0;
     for (int64_t j = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < J; j += nw) {
+        if (lost) {
+            if (lane == 0) samples[j * N + col] = 0u;
+            if (j == 0 && lane == 0) *b.near_count = 0;
+            continue;
+        }
         double x[4];
         int64_t r = 0;
         if (KIND != 0) {
@@ -1206,6 +1233,7 @@ __global__ void zq_vector_kernel(int R, int64_t J, double* __restrict__ h, const
             b.pick[j] = -1;
             if (KIND == 0) b.redo[j] = 0;
             if (KIND == 0 && j == 0) *b.redo_count = 0;
+            if (KIND == 0 && j == 0) *b.lost = 0;
             if (j == 0) *b.near_count = 0;
             if ((j & 127) == 0) {
                 const int64_t tile = j >> 7;
@@ -1223,6 +1251,7 @@ __global__ void zq_vector_kernel(int R, int64_t J, double* __restrict__ h, const
 
 // The eigen tree's leaves: the leaf's index (F = 1).
 __global__ void zq_leaf1_kernel(TreeShape t, int64_t J, ZState b, int N, int col, uint32_t* __restrict__ samples) {
+    if (*b.lost) return;
     for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < J; j += (int64_t)gridDim.x * blockDim.x) {
         const int64_t v = tree_leaf_idx(t, b.node[j]);
         samples[j * N + col] = (uint32_t)v;
@@ -1258,8 +1287,12 @@ __device__ __forceinline__ void tmem_ld4_nowait(uint32_t taddr, uint32_t (&r)[4]
 template <int NT>
 __global__ void __launch_bounds__(NT, 1)
     zq_weight_kernel(int R, int64_t J, ZState b, const double* __restrict__ PhiP, const int32_t* __restrict__ phi_exp,
-                     double* __restrict__ weights, DeviceStatus* status, uint32_t wait_polls) {
+                     double* __restrict__ weights, DeviceStatus* status, uint32_t wait_polls, int64_t withhold) {
     extern __shared__ __align__(128) unsigned char z_raw[];
+    if (z_lost(b)) {
+        for (int64_t j = (int64_t)blockIdx.x * NT + threadIdx.x; j < J; j += (int64_t)gridDim.x * NT) weights[j] = 0.0;
+        return;
+    }
     constexpr int NG = NT / 128;
     constexpr int CPT = kWCols / NG;  // columns per thread: 8 or 4, in groups of 4
     __shared__ long long part[NG][7][kZTile];
@@ -1286,6 +1319,7 @@ __global__ void __launch_bounds__(NT, 1)
     const uint32_t tmem = tmem_base;
     const int emax = *phi_exp;
     uint32_t phase = 0;
+    bool flight = false;  // thread 0: products on their way
     const int row = (w & 3) * 32 + lane, grp = w >> 2;
     const int nch = (R + kWCols - 1) / kWCols;
     const int64_t ntiles = (J + kZTile - 1) / kZTile;
@@ -1359,7 +1393,8 @@ __global__ void __launch_bounds__(NT, 1)
             fence_proxy_async_smem();
             tc_fence_before();
             __syncthreads();
-            if (tid == 0) {
+            if (tid == 0 && tile != withhold) {
+                flight = true;
                 tc_fence_after();
 #pragma unroll
                 for (int i = 0; i < kWx; i++) {
@@ -1370,8 +1405,12 @@ __global__ void __launch_bounds__(NT, 1)
                 }
                 umma_commit(&bar);
             }
-            if (!mbar_wait_limited(&bar, phase, wait_polls)) abort_flag = 1;
-            phase ^= 1u;
+            if (mbar_wait_limited(&bar, phase, wait_polls)) {
+                phase ^= 1u;
+                flight = false;
+            } else {
+                abort_flag = 1;
+            }
             tc_fence_after();
 #pragma unroll
             for (int h = 0; h < CPT / 4; h++) {
@@ -1425,7 +1464,11 @@ __global__ void __launch_bounds__(NT, 1)
             __syncthreads();  // the accumulators and B are free for the next chunk
             if (abort_flag) break;
         }
-        if (abort_flag) break;
+        if (abort_flag) {  // this tile and the block's later ones
+            for (int64_t q = tile; q < ntiles; q += gridDim.x)
+                if (tid < kZTile && q * kZTile + tid < J) weights[q * kZTile + tid] = 0.0;
+            break;
+        }
 #pragma unroll
         for (int u = 0; u < 7; u++) part[grp][u][row] = sum[u];
         __syncthreads();
@@ -1456,7 +1499,7 @@ __global__ void __launch_bounds__(NT, 1)
     if (abort_flag) {
         if (tid == 0) {
             report(status, EXAFAC_ERR_TIMEOUT, 25, blockIdx.x, 0);
-            mbar_wait_limited(&bar, phase ^ 1u, wait_polls);
+            if (flight) mbar_wait_limited(&bar, phase, kSpinLimit);
         }
         tc_fence_before();
         __syncthreads();
@@ -1509,6 +1552,7 @@ void zq_carve(Arena& a, ZState& b, int R, int64_t J, int64_t widest, int trees) 
     b.redo_count = a.take<int32_t>(1);
     b.near_list = a.take<int32_t>(J);
     b.near_count = a.take<int32_t>(1);
+    b.lost = a.take<int32_t>(1);
     for (int q = 0; q < 2; q++) {
         b.mask[q] = a.take<uint32_t>(4 * ceil_div(J, kZTile));
         b.tcount[q] = a.take<int32_t>(ceil_div(J, kZTile) + 4);
@@ -1544,7 +1588,8 @@ static int z_level(Session& s, const TreeShape& t, const double* G, const unsign
                                          (int)smem));
     const unsigned blocks = z_blocks(s, J, NT == 256 ? 304 : 152);
     zq_level_kernel<MODE, NT><<<blocks, NT, smem, st>>>(s.R, nb, t, G, nodes, lb, ex, J, s.zq, p, order, dv,
-                                                        s.status, s.wait_polls ? s.wait_polls : kSpinLimit);
+                                                        s.status, s.wait_polls ? s.wait_polls : kSpinLimit,
+                                                        MODE == 0 ? -1 : s.withheld(23));
     count_launch();
     return EXAFAC_OK;
 }
@@ -1561,7 +1606,7 @@ static int z_leaf(Session& s, const TreeShape& t, const double* G, const double*
     EXAFAC_CUDA_TRY(cudaFuncSetAttribute(zq_leaf_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const unsigned blocks = z_blocks(s, J, NT == 256 ? 304 : 152);
     zq_leaf_kernel<NT><<<blocks, NT, smem, st>>>(s.R, t, G, U, J, s.zq, p, order, dv, s.N, col, s.samples, s.status,
-                                                 s.wait_polls ? s.wait_polls : kSpinLimit);
+                                                 s.wait_polls ? s.wait_polls : kSpinLimit, s.withheld(24));
     count_launch();
     return EXAFAC_OK;
 }
@@ -1601,7 +1646,8 @@ static int z_descend(Session& s, const TreeShape& t, const double* G, const doub
         zq_partition_kernel<<<(unsigned)std::min<int64_t>(ceil_div(J, 512), 152 * 2), 512, psm, st>>>(
             J, (int)ntiles, b.mask[p], b.tcount[p], b.mask[p ^ 1], b.tcount[p ^ 1], b.runs[p ^ 1],
             in_smem ? nullptr : b.pref64, lb, nl, order, b.node, b.off[p], b.order[p], b.off[p ^ 1], s.R, G, ex,
-            t.node_count, 2 * lb + 1, lvl + 1 < t.lfill_level + (tail ? 1 : 0) && 2 * nl <= cap ? 2 * nl : 0, nodes);
+            t.node_count, 2 * lb + 1, lvl + 1 < t.lfill_level + (tail ? 1 : 0) && 2 * nl <= cap ? 2 * nl : 0, nodes,
+            b.lost);
         count_launch();
         order = b.order[p];
         p ^= 1;
@@ -1655,7 +1701,7 @@ int sts_draw_zq(Session& s, int n, int64_t J, const double* uni, cudaStream_t st
     EXAFAC_CUDA_TRY(
         cudaFuncSetAttribute(zq_weight_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     zq_weight_kernel<512><<<blocks, 512, smem, st>>>(R, J, b, s.PhiP, b.tree_exp + 2 * N, s.weights, s.status,
-                                                     s.wait_polls ? s.wait_polls : kSpinLimit);
+                                                     s.wait_polls ? s.wait_polls : kSpinLimit, s.withheld(25));
     count_launch();
     EXAFAC_CHECK_LAUNCH();
     return EXAFAC_OK;
