@@ -106,6 +106,12 @@ int exafac_quad_forms_f32(int32_t R, int64_t J, const float* X_dev, const int64_
 int exafac_syev(int32_t R, const double* A_dev, double* V_dev, double* lambda_dev, void* workspace_dev,
                 size_t workspace_bytes, void* stream);
 
+/* The same decomposition from an FP32 start refined in FP64 over many blocks
+ * (the FP64 form's STS-CP sampling matrices). */
+int exafac_syev_refined(int32_t R, const double* A_dev, double* V_dev, double* lambda_dev, void* workspace_dev,
+                        size_t workspace_bytes, void* stream);
+size_t exafac_syev_refined_workspace_bytes(int32_t R);
+
 /* compute_pinv_square (common.h:405-443): symmetric pseudo-inverse dropping
  * eigenvalues <= tol (the reference uses 1e-11).  out_dev is full symmetric. */
 int exafac_pinv_square(int32_t R, const double* A_dev, double* out_dev, double tol, void* workspace_dev,

@@ -56,6 +56,8 @@ SIGNATURES = {
     "exafac_quad_forms_f32": (ctypes.c_int, [_I32, _I64, _P, _P, _P, _P, _I32, _P]),
     "exafac_tree_build_f32": (ctypes.c_int, [_I64, _I32, _I32, _P, _P, _P]),
     "exafac_syev": (ctypes.c_int, [_I32, _P, _P, _P, _P, _SZ, _P]),
+    "exafac_syev_refined": (ctypes.c_int, [_I32, _P, _P, _P, _P, _SZ, _P]),
+    "exafac_syev_refined_workspace_bytes": (_SZ, [_I32]),
     "exafac_pinv_square": (ctypes.c_int, [_I32, _P, _P, ctypes.c_double, _P, _SZ, _P]),
     "exafac_dense_workspace_bytes": (_SZ, [_I32]),
     "exafac_pinv_square_static": (ctypes.c_int, [_I32, _P, _P, ctypes.c_double, _P]),

@@ -56,7 +56,7 @@ __device__ __forceinline__ bool jacobi_rotates(int R, double apq, double app, do
 
 // Sweeps until no pair rotates.  A sweep starts by looking at every pair at
 // once, so a matrix that is already diagonal (the end of every call, and the
-// usual start after syev_refine) costs one pass instead of Re - 1 rounds.
+// usual start of syev_finish_kernel) costs one pass instead of Re - 1 rounds.
 __device__ void jacobi_sweeps(int R, double* a, double* vt, double* rc, double* rs, int* flag, double null = 0.0) {
     const int Re = R + (R & 1);
     const int m = Re - 1;
@@ -234,7 +234,7 @@ __global__ void syev_kernel(int R, const double* __restrict__ A, int64_t a_strid
 // start, refined in FP64.
 //
 // The FP64 Jacobi takes ~10 sweeps of ~6 R^3 FP64 operations on one SM (GB300
-// retires ~1.7 of them per clock per SM): 0.87 / 5.2 / 19 ms a call at R = 25 /
+// retires ~1.7 of them per clock per SM): 0.85 / 5.1 / 17 ms a call at R = 25 /
 // 64 / 100, which was 15 to 52 % of an FP64 STS-CP sweep.  Here
 //   1. jacobi32_kernel: the sweeps in FP32 (shared memory, one CTA a matrix);
 //   2. kRefineSteps refinement steps of the eigenvector matrix X in FP64
@@ -245,21 +245,30 @@ __global__ void syev_kernel(int R, const double* __restrict__ A, int64_t a_strid
 //      quotient is no small rotation (equal eigenvalues).  S is taken
 //      symmetric (its upper triangle), which keeps E_ij + E_ji = r_ij to
 //      rounding and so X orthonormal.  The error squares per step; the
-//      products run on R blocks.  Where a quotient is no small rotation in
-//      the first step (eigenvalues closer than FP32 resolves beside the
-//      largest), that step is a second FP32 Jacobi, on S less those pairs'
-//      mean eigenvalue, whose block FP64 has resolved by then: E = V - I;
+//      products run on R blocks.  Eigenvalues closer than FP32 resolves
+//      beside the largest get a second FP32 Jacobi in the first step, cluster
+//      by cluster at the clusters' own scales (refine_first_kernel).  How
+//      large a rotation counts as small falls from step to step, and the last
+//      step is r / 2 alone: a pair that no step resolves leaves X orthonormal;
 //   3. syev_finish_kernel: the FP64 Jacobi sweeps on S with X as the start,
 //      so the result meets the same convergence criterion whatever the steps
 //      left (a cluster, eigenvalues below FP32's resolution), then the sorted
 //      outputs.  X that is not orthonormal to 4 R eps, or a value that is not
-//      finite, starts the sweeps from A as before.
-// Measured (GB300, one to three matrices a call, launches included): R = 25 / 64 /
-// 100: 0.21 / 0.56 / 1.8 ms (the FP64 sweeps alone 0.88 / 5.2 / 17.6),
-// |A v - lambda v| <= 6e-16 |A| against 5e-15 .. 3e-14, a 92-fold near-null
-// cluster at R = 100 11 against 26 ms.
+//      finite, starts the sweeps from A.
+// Measured (GB300, one matrix, launches included), the FP64 sweeps alone ->
+// this: Grams of random factors at R = 25 / 64 / 100 0.85 / 5.1 / 17 -> 0.19 /
+// 0.52 / 1.6 ms, |A v - lambda v| 5e-15 .. 3e-14 -> 3e-16 |A|.  Clusters: the
+// chains of converged factors at R = 25 / 58 0.86 .. 1.2 / 3.9 .. 5.9 -> 0.19 ..
+// 0.28 / 0.41 .. 0.95 ms (with one mean for all clusters, rotations up to 2^-5
+// in every step and no orthonormalising one X was given up: 1.1 .. 1.4 / 4.3 ..
+// 6.4); 1 + 10^-u, u uniform in 0 .. 16, at R = 64 8.2 -> 2.7; half the spectrum
+// null at R = 64 37 -> 4.2; I but for rounding at R = 64 0.03 -> 0.21.
+// Below kRefineMinRank the FP64 sweeps alone are faster: R = 4 / 5 0.05 / 0.08
+// against 0.05 / 0.065 ms.
 // ---------------------------------------------------------------------------
+constexpr int kRefineMinRank = 5;
 constexpr int kRefineSteps = 4;
+constexpr double kRefineLimit[kRefineSteps] = {0x1p-5, 0x1p-8, 0x1p-18, 0.0};
 constexpr int kJacobi32MaxSweeps = 10;
 
 // Cyclic Jacobi in FP32 on the full symmetric matrix a (Re x Re, shared; two
@@ -415,13 +424,16 @@ __global__ void __launch_bounds__(512) jacobi32_kernel(int R, const double* __re
     for (int i = 0; i < R; i++) tr += A[i * R + i];
     const double mu = tr / R;
     double mx = 0.0;
+    bool turns = false;
     for (int e = tid; e < R * R; e += nt) {
         const int i = e / R, j = e % R;
         const double x = i <= j ? A[i * R + j] : A[j * R + i];
+        turns = turns || (i < j && jacobi_rotates(R, x, A[i * R + i], A[j * R + j]));
         As[e] = x;
         mx = fmax(mx, fabs(i == j ? x - mu : x));
     }
-    const double sc = scale_of(block_max(mx, red));
+    // (a matrix with no pair to rotate, as of factors with orthogonal columns: X = I)
+    const double sc = __syncthreads_or(turns) ? scale_of(block_max(mx, red)) : 0.0;
     for (int e = tid; e < Re * Re; e += nt) {
         const int i = e / Re, j = e % Re;
         double x = 0.0;
@@ -447,7 +459,7 @@ __device__ __forceinline__ double dot4(const double* x, const double* __restrict
     return (s0 + s1) + (s2 + s3);
 }
 
-// Row i (blockIdx.x) of S = X^T A X and G = X^T X of matrix blockIdx.y.
+// Row i (blockIdx.x) of S = X^T A X (unless null) and G = X^T X of matrix blockIdx.y.
 __global__ void __launch_bounds__(128) refine_forms_kernel(int R, const double* __restrict__ As,
                                                            const double* __restrict__ X, double* __restrict__ S,
                                                            double* __restrict__ G, int64_t scratch_stride) {
@@ -458,10 +470,10 @@ __global__ void __launch_bounds__(128) refine_forms_kernel(int R, const double* 
     const int64_t o = (int64_t)blockIdx.y * scratch_stride;
     if (j < R) xi[j] = X[o + (int64_t)j * R + i];
     __syncthreads();
-    if (j < R) ti[j] = dot4(xi, As + o + j, R, R);
+    if (j < R && S) ti[j] = dot4(xi, As + o + j, R, R);
     __syncthreads();
     if (j < R) {
-        S[o + (int64_t)i * R + j] = dot4(ti, X + o + j, R, R);
+        if (S) S[o + (int64_t)i * R + j] = dot4(ti, X + o + j, R, R);
         G[o + (int64_t)i * R + j] = dot4(xi, X + o + j, R, R);
     }
 }
@@ -474,15 +486,16 @@ __device__ __forceinline__ double3 refine_quotient(int R, const double* S, const
     const double g = G[i * R + j];
     return make_double3(sij - lj * g, lj - li, fmax(fabs(sij - lj * g), fabs(sij - li * g)));
 }
-// A quotient that is a small rotation, and one that says something: between
-// close eigenvalues (lmax: the largest) a numerator at the rounding of S
-// would turn X by noise / gap in every step, whose square X's orthonormality
-// loses again; those pairs are left to the Jacobi sweeps.
-__device__ __forceinline__ bool small_rotation(double3 q, double lmax) {
-    return q.z < 0x1p-5 * fabs(q.y) && (q.z > 0x1p-48 * lmax || fabs(q.y) > 0x1p-23 * lmax);
+// A quotient that is a small rotation (up to `limit`), and one that says
+// something: between close eigenvalues (lmax: the largest) a numerator at the
+// rounding of S would turn X by noise / gap; those pairs are left to the
+// Jacobi sweeps.
+__device__ __forceinline__ bool small_rotation(double3 q, double lmax, double limit) {
+    return q.z < limit * fabs(q.y) && (q.z > 0x1p-48 * lmax || fabs(q.y) > 0x1p-23 * lmax);
 }
 
-__global__ void __launch_bounds__(128) refine_e_kernel(int R, const double* __restrict__ S,
+// limit 0: the orthonormalising step, E = r / 2 (S is not read).
+__global__ void __launch_bounds__(128) refine_e_kernel(int R, double limit, const double* __restrict__ S,
                                                        const double* __restrict__ G, double* __restrict__ E,
                                                        int64_t scratch_stride) {
     pdl_wait();
@@ -490,77 +503,121 @@ __global__ void __launch_bounds__(128) refine_e_kernel(int R, const double* __re
     __shared__ double red[32];
     const int i = blockIdx.x, j = threadIdx.x;
     const int64_t o = (int64_t)blockIdx.y * scratch_stride;
-    const double lmax = block_max(j < R ? fabs(S[o + j * R + j]) : 0.0, red);
+    const double lmax = limit > 0.0 ? block_max(j < R ? fabs(S[o + j * R + j]) : 0.0, red) : 0.0;
     if (j >= R) return;
     double e = 0.5 * ((i == j ? 1.0 : 0.0) - G[o + i * R + j]);
-    if (i != j) {
+    if (i != j && limit > 0.0) {
         const double3 q = refine_quotient(R, S + o, G + o, i, j);
-        if (small_rotation(q, lmax)) e = q.x / q.y;
+        if (small_rotation(q, lmax, limit)) e = q.x / q.y;
     }
     E[o + i * R + j] = e;
 }
 
-// The first step's E, a CTA per matrix.
-__global__ void __launch_bounds__(512) refine_first_kernel(int R, const double* __restrict__ S,
+// The first step's E, a CTA per matrix.  The pairs whose rotation is not small
+// link their indices to clusters; each cluster's block of X^T (A - m I) X = S -
+// m G, m the mean of its eigenvalues, is diagonalised by an FP32 Jacobi at its
+// own scale (so that clusters anywhere in the spectrum gain FP32's 24 bits in
+// their own spread): X <- X (I + E0) V with E0 the small rotations between the
+// clusters and r / 2 inside them.
+__global__ void __launch_bounds__(512) refine_first_kernel(int R, double limit, const double* __restrict__ S,
                                                            const double* __restrict__ G, double* __restrict__ E,
                                                            int64_t scratch_stride) {
     extern __shared__ float j32[];
     __shared__ int flag;
     __shared__ double red[32];
-    __shared__ int second;
+    __shared__ unsigned near[kMaxRank][kMaxRank / 32];  // the pairs whose rotation is not small
+    __shared__ int cluster[kMaxRank];                   // the least index of the cluster
+    __shared__ double lam[kMaxRank], mean[kMaxRank];    // mean: by cluster; NaN for a cluster of one
+    __shared__ int top[kMaxRank];                       // by cluster: high word of its block's largest entry
     pdl_wait();
     const int Re = R + (R & 1);
     const int tid = threadIdx.x, nt = blockDim.x;
     S += blockIdx.x * scratch_stride;
     G += blockIdx.x * scratch_stride;
     E += blockIdx.x * scratch_stride;
-    if (tid == 0) second = 0;
-    __syncthreads();
-    // the pairs whose rotation is not small: how many, their mean eigenvalue
-    // and the spread among them
-    const double lmax = block_max(tid < R ? fabs(S[tid * R + tid]) : 0.0, red);
-    double cnt = 0.0, mean = 0.0, spread = 0.0;
+    for (int e = tid; e < kMaxRank * (kMaxRank / 32); e += nt) near[0][e] = 0u;
+    const double lmax = block_max(tid < R ? fabs(S[tid * R + tid]) : 0.0, red);  // (its barriers: near is clear)
+    bool any = false;
     for (int e = tid; e < R * R; e += nt) {
         const int i = e / R, j = e % R;
         double v = 0.5 * ((i == j ? 1.0 : 0.0) - G[e]);
         if (i != j) {
             const double3 q = refine_quotient(R, S, G, i, j);
-            if (small_rotation(q, lmax)) {
+            if (small_rotation(q, lmax, limit)) {
                 v = q.x / q.y;
-            } else if (i < j && jacobi_rotates(R, S[e], S[i * R + i], S[j * R + j])) {
-                cnt += 1.0;
-                mean += 0.5 * (S[i * R + i] + S[j * R + j]);
-                spread = fmax(spread, fmax(fabs(q.y), fabs(S[e])));
+            } else if (jacobi_rotates(R, q.z, S[i * R + i], S[j * R + j])) {
+                atomicOr(&near[i][j >> 5], 1u << (j & 31));
+                any = true;
             }
         }
         E[e] = v;
     }
-    if (cnt > 0.0) second = 1;
-    __syncthreads();
-    if (!second) return;
-    cnt = block_sum(cnt, red);
-    mean = block_sum(mean, red) / cnt;
-    spread = block_max(spread, red);
-    double mx = 0.0;
-    for (int e = tid; e < R * R; e += nt) {
-        const int i = e / R, j = e % R;
-        mx = fmax(mx, fabs(i == j ? S[e] - mean : S[i <= j ? e : j * R + i]));
+    if (!__syncthreads_or(any)) return;
+    if (tid < R) {
+        cluster[tid] = tid;
+        top[tid] = 0;
+        lam[tid] = S[tid * R + tid] / G[tid * R + tid];
     }
-    const double sc = scale_of(block_max(mx, red));
-    if (sc == 0.0) return;
+    for (bool moved = true; moved;) {  // the least index along the links
+        __syncthreads();
+        int c = 0;
+        if (tid < R) {
+            c = cluster[tid];
+            for (int w = 0; w < kMaxRank / 32; w++)
+                for (unsigned bits = near[tid][w]; bits; bits &= bits - 1) c = min(c, cluster[32 * w + __ffs(bits) - 1]);
+            c = cluster[c];
+        }
+        __syncthreads();
+        moved = tid < R && c != cluster[tid];
+        if (moved) cluster[tid] = c;
+        moved = __syncthreads_or(moved);
+    }
+    if (tid < R) {
+        double sum = 0.0;
+        int n = 0;
+        for (int k = tid; k < R; k++) {
+            if (cluster[k] != tid) continue;
+            sum += lam[k];
+            n++;
+        }
+        mean[tid] = n > 1 ? sum / n : __longlong_as_double(0x7ff8000000000000ll);
+    }
+    __syncthreads();
+    auto block = [&](int i, int j) {  // of one cluster
+        const int u = min(i, j) * R + max(i, j);
+        return S[u] - mean[cluster[i]] * G[u];
+    };
+    for (int e = tid; e < R * R; e += nt) {
+        const int i = e / R, j = e % R, c = cluster[i];
+        if (c != cluster[j]) continue;
+        const double x = fabs(block(i, j));
+        if (x < 0x1p1000) atomicMax(&top[c], __double2hiint(x));  // (false for the NaN of a single index)
+    }
+    __syncthreads();
     float* a = j32;
     float* v = a + 2 * Re * Re;
     for (int e = tid; e < Re * Re; e += nt) {
         const int i = e / Re, j = e % Re;
         double x = 0.0;
-        if (i < R && j < R) x = (i <= j ? S[i * R + j] : S[j * R + i]) - (i == j ? mean : 0.0);
-        a[e] = (float)(x * sc);
+        if (i < R && j < R && cluster[i] == cluster[j]) {
+            const double sc = scale_of(__hiloint2double(top[cluster[i]], 0));
+            if (sc > 0.0) x = block(i, j) * sc;
+        }
+        a[e] = (float)x;
     }
     __syncthreads();
-    jacobi32_block(R, a, v, (float)(0x1p-22 * spread * sc), &flag);
+    jacobi32_block(R, a, v, 0x1p-22f, &flag);
+    // E = (I + E0) V - I; E0 to FP32 like V, transposed into the Jacobi's buffer
     for (int e = tid; e < R * R; e += nt) {
-        const int i = e / R, j = e % R;
-        E[e] = (double)v[j * Re + i] - (i == j ? 1.0 : 0.0);
+        const int i = e / R, k = e % R;
+        a[k * Re + i] = (float)(cluster[i] == cluster[k] ? 0.5 * ((i == k ? 1.0 : 0.0) - G[e]) : E[e]);
+    }
+    __syncthreads();
+    for (int e = tid; e < R * R; e += nt) {
+        const int i = e % R, j = e / R;
+        float acc = 0.0f;
+        for (int k = 0; k < R; k++) acc = fmaf(a[k * Re + i], v[j * Re + k], acc);
+        E[i * R + j] = (double)v[j * Re + i] - (i == j ? 1.0 : 0.0) + (double)acc;
     }
 }
 
@@ -1529,6 +1586,7 @@ size_t syev_refine_doubles(int R, int batch) { return (size_t)batch * 6 * R * R;
 
 int launch_syev_refined(int R, const double* A, int64_t a_stride, int batch, double* V, double* lam, int64_t v_stride,
                         double* vt_scratch, double* scratch, cudaStream_t stream) {
+    if (R < kRefineMinRank) return launch_syev(R, A, a_stride, batch, V, lam, v_stride, nullptr, 0.0, vt_scratch, stream);
     const int64_t R2 = (int64_t)R * R, ss = 6 * R2;
     double *X = scratch, *Xn = X + R2, *As = Xn + R2, *S = As + R2, *G = S + R2, *E = G + R2;
     const size_t jsm = jacobi32_bytes(R);
@@ -1541,15 +1599,16 @@ int launch_syev_refined(int R, const double* A, int64_t a_stride, int batch, dou
     count_launch();
     const dim3 grid((unsigned)R, (unsigned)batch);
     for (int it = 0; it <= kRefineSteps; it++) {
+        const double limit = it < kRefineSteps ? kRefineLimit[it] : 1.0;
         EXAFAC_CUDA_TRY(launch_dependent(refine_forms_kernel, grid, 128, 0, stream, R, (const double*)As,
-                                         (const double*)X, S, G, ss));
+                                         (const double*)X, limit > 0.0 ? S : (double*)nullptr, G, ss));
         count_launch();
         if (it == kRefineSteps) break;
         if (it == 0) {
-            EXAFAC_CUDA_TRY(launch_dependent(refine_first_kernel, (unsigned)batch, 512, jsm, stream, R,
+            EXAFAC_CUDA_TRY(launch_dependent(refine_first_kernel, (unsigned)batch, 512, jsm, stream, R, limit,
                                              (const double*)S, (const double*)G, E, ss));
         } else {
-            EXAFAC_CUDA_TRY(launch_dependent(refine_e_kernel, grid, 128, 0, stream, R, (const double*)S,
+            EXAFAC_CUDA_TRY(launch_dependent(refine_e_kernel, grid, 128, 0, stream, R, limit, (const double*)S,
                                              (const double*)G, E, ss));
         }
         count_launch();
@@ -1815,6 +1874,20 @@ extern "C" int exafac_syev(int32_t R, const double* A, double* V, double* lam, v
     EXAFAC_ARG(A && V && lam && workspace, "exafac_syev: null pointer");
     EXAFAC_ARG(workspace_bytes >= exafac_dense_workspace_bytes(R), "exafac_syev: workspace too small");
     return launch_syev(R, A, 0, 1, V, lam, 0, nullptr, 0.0, (double*)workspace, (cudaStream_t)stream);
+}
+
+extern "C" size_t exafac_syev_refined_workspace_bytes(int32_t R) {
+    if (R < 1 || R > kMaxRank) return 0;
+    return sizeof(double) * (syev_scratch_doubles(R, 1) + syev_refine_doubles(R, 1));
+}
+
+extern "C" int exafac_syev_refined(int32_t R, const double* A, double* V, double* lam, void* workspace,
+                                   size_t workspace_bytes, void* stream) {
+    EXAFAC_ARG(R >= 1 && R <= kMaxRank, "exafac_syev_refined: R out of range");
+    EXAFAC_ARG(A && V && lam && workspace, "exafac_syev_refined: null pointer");
+    EXAFAC_ARG(workspace_bytes >= exafac_syev_refined_workspace_bytes(R), "exafac_syev_refined: workspace too small");
+    double* vt = (double*)workspace;
+    return launch_syev_refined(R, A, 0, 1, V, lam, 0, vt, vt + syev_scratch_doubles(R, 1), (cudaStream_t)stream);
 }
 
 extern "C" int exafac_pinv_square(int32_t R, const double* A, double* out, double tol, void* workspace,
