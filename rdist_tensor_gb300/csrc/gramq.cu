@@ -10,9 +10,22 @@
 // of the digits i and j with i + j <= 7 accumulate by weight i + j in tensor
 // memory, at most 8 x 64 products of below 2^14, exact integers.  The eight
 // weights are put together in 64-bit integers, scaled back and added to an
-// FP64 total per entry, once per tile.  The dropped weights are below 2^-55 of
-// the columns' largest products, an eighth of the rounding of the FMA that
-// they replace.  A column with a value that is not finite makes its entries NaN.
+// FP64 total per entry, once per tile.
+//
+// Error of an entry and tile, in the scaled units (the columns' largest values
+// are 2^5 to 2^6): the cut of x' to 2^-56 on both sides 64 x 2 x 2^6 x 2^-56 =
+// 2^-43, the dropped weights (i + j >= 8) 64 x 7.1 x 2^14 x 2^-64 = 2^-41.2, the
+// cut of the sum 2^-44: together below 2^-40.6, that is 2^-50.6 of the product of
+// the two columns' largest values in the tile.  64 FMAs may lose 64^2 / 2 x
+// 2^-53 = 2^-42 of it.  An entry all of whose products are far smaller than that
+// (columns that are large in different rows) keeps fewer bits than an FMA sum
+// would; the inverse takes no harm, since a Cholesky factor's own error is a
+// rounding of sqrt(G_aa G_bb) in every entry.
+//
+// A tile with a value above 2^877, infinite or NaN, or with values below 2^-895
+// (a group of eight rows of a column, not all zero), is summed in FP64: products
+// would overflow on the way, infinities have no digits, and a column of
+// subnormals does not scale to 2^5.
 // Measured (GB300): R = 64, J = 2^18: 1270 -> 436 us; R = 100, J = 100003, four modes:
 // 970 -> 180 us (and their partial sums' reduction 65 -> 10 us).
 #include "digits.cuh"
@@ -24,6 +37,7 @@ constexpr int kGqRows = 64;     // rows of a tile (the products' K)
 constexpr int kGqDigits = 8;
 constexpr int kGqThreads = 512;
 constexpr int kGqCols = 64;     // columns per pass: 8 weights of them fill tensor memory
+constexpr int kGqMinExp = 128, kGqMaxExp = 1900;  // biased exponents between which a tile goes by digits
 
 struct GqShape {
     int Rp, nb, passes;   // R padded to 16, columns per pass, passes
@@ -95,6 +109,7 @@ __global__ void __launch_bounds__(kGqThreads, 1)
         __syncthreads();
         // column a, rows 8 kc .. + 7 per item, the column fastest
         double v[2][8];
+        bool fp64 = false;
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const int e = tid + u * kGqThreads, kc = e / g.Rp, c = e - kc * g.Rp;
@@ -127,13 +142,44 @@ __global__ void __launch_bounds__(kGqThreads, 1)
                 for (int q = 0; q < 8; q++) v[u][q] = 0.0;
             }
             if (top > 0) atomicMax(&ecol[buf][c], top);  // (c < R here)
+            long long bits = 0;
+#pragma unroll
+            for (int q = 0; q < 8; q++) bits |= __double_as_longlong(v[u][q]);
+            fp64 = fp64 || top > kGqMaxExp || (top < kGqMinExp && bits << 1 != 0);
         }
-        __syncthreads();
+        fp64 = __syncthreads_or(fp64);
         if (tid < kMaxRank) {
             // the accumulators' integers are in units of 2^-44 of the scaled columns' products
-            const int e = ecol[buf][tid];
-            scale[tid] = e >= 2047 ? __longlong_as_double(0x7ff8000000000000ll) : scalbn(1.0, e - 1028 - 22);
+            scale[tid] = scalbn(1.0, ecol[buf][tid] - 1028 - 22);
             ecol[buf ^ 1][tid] = 0;
+        }
+        if (fp64) {  // in FP64, the rows in shared memory where the digits go
+            double* x = reinterpret_cast<double*>(X);
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const int e = tid + u * kGqThreads, kc = e / g.Rp, c = e - kc * g.Rp;
+                if (kc >= 8) continue;
+#pragma unroll
+                for (int q = 0; q < 8; q++) x[(8 * kc + q) * g.Rp + c] = v[u][q];
+            }
+            __syncthreads();
+#pragma unroll
+            for (int pass = 0; pass < 2; pass++)
+#pragma unroll
+                for (int q = 0; q < 16; q++) {
+                    const int b = pass * kGqCols + grp * cpt + q;
+                    if (pass < g.passes && q < cpt && a < R && b <= a) {
+                        // the smaller column 2^600 larger where its products would be subnormal
+                        const int lo = ecol[buf][a] <= ecol[buf][b] ? a : b, hi = a + b - lo;
+                        const bool up = ecol[buf][lo] < 400;
+                        double sum = 0.0;
+                        for (int r = 0; r < nr; r++)
+                            sum = fma(x[r * g.Rp + lo] * (up ? 0x1p600 : 1.0), x[r * g.Rp + hi], sum);
+                        total[pass][q] = fma(sum, up ? 0x1p-600 : 1.0, total[pass][q]);
+                    }
+                }
+            __syncthreads();
+            continue;
         }
 #pragma unroll
         for (int u = 0; u < 2; u++) {
@@ -143,7 +189,7 @@ __global__ void __launch_bounds__(kGqThreads, 1)
             uint32_t lo[8], hi[8];
 #pragma unroll
             for (int q = 0; q < 8; q++) {
-                const long long t = (emax < 2047 ? fix56(v[u][q], emax) : 0ll) + 0x80808080808080ll;
+                const long long t = fix56(v[u][q], emax) + 0x80808080808080ll;
                 lo[q] = (uint32_t)t;
                 hi[q] = (uint32_t)(t >> 32);
             }
