@@ -283,6 +283,10 @@ int exafac_als_step_info(exafac_als_t s, exafac_step_info* out, void* stream);
 int exafac_als_last_dedup(exafac_als_t s, const uint32_t** samples_dev, const double** weights_dev,
                           const double** design_gram_dev, const double** design_pinv_dev);
 
+/* The same for the last STS-CP draw: Phi, packed by rows of its upper triangle
+ * [R (R + 1) / 2]; a sample's weight is R / (J h^T Phi h). */
+int exafac_als_last_phi(exafac_als_t s, const double** phi_packed_dev);
+
 /* ---------------------------------------------------------------------------
  * Generalized CP on sampled entries.  No counterpart in the reference: these
  * are the forward and adjoint of a sampled-MTTKRP torch.autograd.Function

@@ -772,3 +772,10 @@ extern "C" int exafac_als_last_dedup(exafac_als_t h, const uint32_t** samples, c
     if (pinv) *pinv = s.dpinv;
     return EXAFAC_OK;
 }
+
+extern "C" int exafac_als_last_phi(exafac_als_t h, const double** phi) {
+    EXAFAC_ARG(h && phi, "null argument");
+    EXAFAC_ARG(h->s.cfg.sampler == EXAFAC_SAMPLER_STS_CP, "exafac_als_last_phi: not an STS-CP session");
+    *phi = h->s.PhiP;
+    return EXAFAC_OK;
+}

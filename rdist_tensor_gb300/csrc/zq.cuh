@@ -7,6 +7,7 @@ namespace exafac {
 
 struct ZState {
     int64_t* xi = nullptr;      // J x (R rounded up to 4): the descent's vector, fixed point (pack_x)
+    int8_t* rest = nullptr;     // J x (R rounded up to 4): h less its fixed point, 256ths of a unit
     double2* lh = nullptr;      // (low, high) of the current descent
     double* rinv = nullptr;     // 1 / root mass (scaled units)
     float2* err = nullptr;      // error bounds of (low, high)

@@ -111,6 +111,19 @@ __device__ __forceinline__ long long fix47_rn(double v, int emax) {
     return b < 0 ? -(long long)m : (long long)m;
 }
 
+// What fix47_rn leaves off v, in 256ths of its unit: the eight bits below the
+// last one, as a signed number where they rounded it up (rounded themselves).
+__device__ __forceinline__ int fix47_rest(double v, int emax) {
+    const long long b = __double_as_longlong(v);
+    const int e = (int)((b >> 52) & 0x7ff);
+    unsigned long long m = (unsigned long long)b & 0xfffffffffffffull;
+    if (e) m |= 1ull << 52;
+    const int s = max(max(emax, 1) - max(e, 1), 0);
+    const uint32_t f = s >= 32 ? (s < 96 ? (uint32_t)(m >> (s - 32)) : 0u) : (uint32_t)(m << (32 - s));
+    const int r = min(((int)f >> 24) + (int)((f >> 23) & 1u), 127);
+    return b < 0 ? -r : r;
+}
+
 // Rows of the fixed-point vectors are padded with zeros to a multiple of 4
 // (32 bytes), so that a thread's eight values are two 32-byte loads: with
 // 8-byte loads of 32 different rows the level kernel took 3.3 times the
@@ -1221,6 +1234,7 @@ __global__ void zq_vector_kernel(int R, int64_t J, double* __restrict__ h, const
             if (c < z_row(R)) {  // (x is zero past R)
                 const long long f = e < 2047 ? fix47_rn(x[q], e) : 0ll;
                 reinterpret_cast<long long*>(b.xi)[j * z_row(R) + c] = pack_x(f);
+                if (KIND == 2) b.rest[j * z_row(R) + c] = (int8_t)(e < 2047 ? fix47_rest(x[q], e) : 0);
                 n1 += (float)((int)(llabs(f) >> 24) + 1) * 0x1p-23f;
             }
         }
@@ -1262,14 +1276,23 @@ __global__ void zq_leaf1_kernel(TreeShape t, int64_t J, ZState b, int N, int col
 // ---- the weights R / (J h^T Phi h)
 //
 // The same products with five digits of h and eight of Phi (weights <= 7, in
-// chunks of 16 columns): the dropped part is below R 4 2^-50 of n1 in the
-// scaled units, under FP64's rounding of the depth-first sum, whose R^2 / 2
-// products and sums per sample took 3.1 ms at R = 64, J = 2^18.  A sample
-// whose form is not positive or not finite is marked; one whose form cancels
-// (the bound above 2^-42 of it) gets the depth-first kernel's own sum from h
-// (sts_weight_list_kernel).  As a decomposition converges that is a tenth of the
-// samples, and drawing them again whole took 1.1 ms a step at R = 100 with four
-// modes, 6 ms at R = 66 with three.
+// chunks of 16 columns), in place of R^2 / 2 FP64 products and sums per sample,
+// which took 3.1 ms at R = 64, J = 2^18.  What the fixed point of h leaves off
+// (up to 2^-48 of the scaled units, more than FP64 where the entries of h differ
+// by decades) is kept to 256ths of its unit (ZState::rest) and added in FP32 to
+// first order, 2 sum_c Y_c (h - x)_c.  The
+// digits and the cut of Phi that are dropped are below R 4 2^-50 of n1; an FP64
+// sum's own rounding is some 2^-53 of sum |h_a Phi_ab h_b|, of which sum_c
+// Phi_cc h_c^2 is a part.  A sample whose bound is above 2^-42 of its form or
+// above 2^-46 of that diagonal part gets the depth-first kernel's own sum from h
+// (sts_weight_list_kernel); one whose form is not positive or not finite is
+// marked.  Against exact arithmetic, the largest error of a dozen samples, FP64
+// sums -> digits: Grams of random factors at R = 64 3e-16 -> 2e-17, nearly
+// collinear columns (Phi_cc to 170) at R = 100 9e-15 -> 2.4e-15, small h where Phi
+// is large (three decades) 2.2e-16 -> 2.2e-16 (6e-15 without the diagonal's test).
+// As a decomposition converges up to a tenth of the samples go to FP64; drawing
+// them again whole took 1.1 ms a step at R = 100 with four modes, 6 ms at R = 66
+// with three.
 constexpr int kWx = 5, kWa = 8, kWCols = 16;
 
 static size_t zw_smem(int R) {
@@ -1296,7 +1319,9 @@ __global__ void __launch_bounds__(NT, 1)
     constexpr int NG = NT / 128;
     constexpr int CPT = kWCols / NG;  // columns per thread: 8 or 4, in groups of 4
     __shared__ long long part[NG][7][kZTile];
+    __shared__ float2 fpart[NG][kZTile];
     __shared__ int rs[kMaxRank];
+    __shared__ float diag[kMaxRank];  // Phi_cc in the scaled units
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_base;
     __shared__ int abort_flag;
@@ -1318,6 +1343,8 @@ __global__ void __launch_bounds__(NT, 1)
     tc_fence_after();
     const uint32_t tmem = tmem_base;
     const int emax = *phi_exp;
+    for (int c = tid; c < kMaxRank; c += NT)  // (read after the barriers of the first chunk)
+        diag[c] = c < R ? (float)scalbn(PhiP[packed_index(R, c, c)], 1028 - emax) : 0.0f;
     uint32_t phase = 0;
     bool flight = false;  // thread 0: products on their way
     const int row = (w & 3) * 32 + lane, grp = w >> 2;
@@ -1356,7 +1383,10 @@ __global__ void __launch_bounds__(NT, 1)
                 *reinterpret_cast<uint4*>(dst + d * z.xs) = make_uint4(o[d][0], o[d][1], o[d][2], o[d][3]);
         }
         long long sum[7] = {0, 0, 0, 0, 0, 0, 0};  // P, Q, T times the high and low parts of x0 + 2 xr, W times the high
-        const long long* xrow = xi + (s0 + (row < n ? row : 0)) * Rx;
+        float rest = 0.0f, dsum = 0.0f;  // sum_c Y_c (h - x)_c in units of 2^-55, sum_c Phi_cc x_c^2
+        const int64_t jrow = s0 + (row < n ? row : 0);
+        const long long* xrow = xi + jrow * Rx;
+        const uint32_t* rrow = reinterpret_cast<const uint32_t*>(b.rest + jrow * Rx);
         for (int ch = 0; ch < nch; ch++) {
             for (int e = tid; e < kWCols * (z.Rk / 8); e += NT) {  // Phi's columns, the column fastest
                 const int c = e & (kWCols - 1), k = 8 * (e / kWCols);
@@ -1420,10 +1450,13 @@ __global__ void __launch_bounds__(NT, 1)
                 for (int q = 0; q < kWa; q++)
                     tmem_ld4_nowait(tmem + ((uint32_t)((w & 3) * 32) << 16) + (uint32_t)(kWCols * q + cc), a[q]);
                 long long X[4] = {0, 0, 0, 0};
-                if (ch * kWCols + cc < Rx)
+                uint32_t r4 = 0x80808080u;  // the four rests, plus 128 each
+                if (ch * kWCols + cc < Rx) {
                     asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
                                  : "=l"(X[0]), "=l"(X[1]), "=l"(X[2]), "=l"(X[3])
                                  : "l"(xrow + ch * kWCols + cc));
+                    r4 ^= __ldg(rrow + (ch * kWCols + cc) / 4);
+                }
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                 for (int q = 0; q < kWa; q++)
@@ -1458,6 +1491,9 @@ __global__ void __launch_bounds__(NT, 1)
                     sum[4] += (long long)Tn * wh;
                     sum[5] += (long long)Tn * wl;
                     sum[6] += (long long)W * wh;
+                    const float x = (float)z4 * 0x1p-24f;
+                    rest = fmaf((f[0] + f[1]) + f[2], digit_f<0>(r4, q), rest);
+                    dsum = fmaf(diag[ch * kWCols + cc + q] * x, x, dsum);
                 }
             }
             tc_fence_before();
@@ -1471,9 +1507,16 @@ __global__ void __launch_bounds__(NT, 1)
         }
 #pragma unroll
         for (int u = 0; u < 7; u++) part[grp][u][row] = sum[u];
+        fpart[grp][row] = make_float2(rest, dsum);
         __syncthreads();
         if (tid < n) {
             long long s6[7];
+            float2 fs = fpart[0][tid];
+#pragma unroll
+            for (int gq = 1; gq < NG; gq++) {
+                fs.x += fpart[gq][tid].x;
+                fs.y += fpart[gq][tid].y;
+            }
 #pragma unroll
             for (int u = 0; u < 7; u++) {
                 s6[u] = part[0][u][tid];
@@ -1481,13 +1524,15 @@ __global__ void __launch_bounds__(NT, 1)
                 for (int gq = 1; gq < NG; gq++) s6[u] += part[gq][u][tid];
             }
             // P 2^-8, Q 2^-23, T 2^-38, W 2^-46; the parts of x0 + 2 xr 2^-20, 2^-47
-            const double q = (((double)s6[5] * 0x1p-85 + (double)s6[6] * 0x1p-66) + (double)s6[4] * 0x1p-58) +
+            const double q = ((((double)fs.x * 0x1p-54 + (double)s6[5] * 0x1p-85) + (double)s6[6] * 0x1p-66) +
+                              (double)s6[4] * 0x1p-58) +
                              (((double)s6[3] * 0x1p-70 + (double)s6[1] * 0x1p-55) +
                               ((double)s6[2] * 0x1p-43 + (double)s6[0] * 0x1p-28));
             const int64_t j = s0 + tid;
             const int ex = b.ex[j];
             const bool usable = q > 0.0 && ex < 2047 && emax < 2047;
-            const bool good = usable && (double)b.n1[j] * (double)R * 0x1p-48 + (double)R * (double)R * 0x1p-57 < q * 0x1p-42;
+            const double err = (double)b.n1[j] * (double)R * 0x1p-48 + (double)R * (double)R * 0x1p-57;
+            const bool good = usable && err < q * 0x1p-42 && err < (double)fs.y * 0x1p-46;
             const double hq = scalbn(q, 2 * ex + emax - 3084);
             weights[j] = good ? (double)R / (hq * (double)J) : 0.0;
             if (!usable) z_mark(b.redo, b.redo_list, b.redo_count, (int32_t)j);
@@ -1536,6 +1581,7 @@ static int64_t z_node_cap(int R, int64_t J) {
 
 void zq_carve(Arena& a, ZState& b, int R, int64_t J, int64_t widest, int trees) {
     b.xi = a.take<int64_t>(J * z_row(R));
+    b.rest = a.take<int8_t>(J * z_row(R));
     b.lh = a.take<double2>(J);
     b.rinv = a.take<double>(J);
     b.err = a.take<float2>(J);
