@@ -8,7 +8,7 @@ namespace exafac {
 
 constexpr uint32_t kNoRow = 0xffffffffu;  // rows are < 2^32 - 1
 constexpr int kLongSpan = 256;             // chunks from which an FP64 row takes a whole block
-constexpr int kMaxLongSpans = 64;          // of them kept per block; more are summed by their warps
+constexpr int kLongBatch = 8;               // chunks a warp looks at before the block sums the long rows among them
 
 // Crossing rows, one warp per chunk c0 whose last row continues: the row's
 // carries carry_last[c0] + sum over c in (c0, c1] of carry_first[c], c1 the
@@ -19,7 +19,8 @@ constexpr int kMaxLongSpans = 64;          // of them kept per block; more are s
 // (almost every row): lane = column, chunks summed in order.  Longer spans
 // (the hot rows): lane l sums chunks c0+1+l, c0+1+l+32, ... over all 32 padded
 // columns, then a butterfly reduce-scatter leaves column l's total in lane l.
-// Both orders are fixed, so results are reproducible run to run.
+// FP64 spans of more than kLongSpan chunks take the whole block.  The order of
+// a row's sum depends on its span alone, so results are reproducible run to run.
 // carry_seg != null: Mc is compact and the row's output index is carry_seg[c0].
 template <typename TA, int kChunk, int CB = 1>  // CB column blocks of 32 (carry stride 32 CB)
 __global__ void __launch_bounds__(256) segfix_kernel(int R, int ldm, const int64_t* __restrict__ counters, int64_t cap,
@@ -39,14 +40,10 @@ __global__ void __launch_bounds__(256) segfix_kernel(int R, int ldm, const int64
     const unsigned full = 0xffffffffu;
     constexpr bool kBlockSpans = sizeof(TA) == 8;
     __shared__ int nlong;
-    __shared__ int64_t longs[kBlockSpans ? kMaxLongSpans : 1][2];
-    if (kBlockSpans) {
-        if (threadIdx.x == 0) nlong = 0;
-        __syncthreads();
-    }
-    for (int64_t c0 = warp; c0 < nchunks; c0 += nwarps) {
+    __shared__ int64_t longs[kBlockSpans ? 8 * kLongBatch : 1][2];
+    auto one = [&](int64_t c0) {
         const uint32_t row = carry_row[c0];
-        if (row == kNoRow) continue;
+        if (row == kNoRow) return;
         const int64_t out = carry_seg ? (int64_t)carry_seg[c0] : (int64_t)row;
         int64_t c1 = c0;
         if (seg_start) {
@@ -81,19 +78,15 @@ __global__ void __launch_bounds__(256) segfix_kernel(int R, int ldm, const int64
                 for (int64_t m = c0 + 1; m <= c1; m++) v += carry_first[m * (32 * CB) + col];
                 Mc[out * ldm + col] = v;
             }
-            continue;
+            return;
         }
         if (kBlockSpans && c1 - c0 > kLongSpan) {  // a hot row: left to the whole block, below
-            int at = 0;
-            if (lane == 0) at = atomicAdd(&nlong, 1);
-            at = __shfl_sync(full, at, 0);
-            if (at < kMaxLongSpans) {
-                if (lane == 0) {
-                    longs[at][0] = c0;
-                    longs[at][1] = c1;
-                }
-                continue;
+            if (lane == 0) {
+                const int at = atomicAdd(&nlong, 1);
+                longs[at][0] = c0;
+                longs[at][1] = c1;
             }
+            return;
         }
         for (int cb = 0; cb < CB; cb++) {
             TA acc[32];
@@ -118,45 +111,57 @@ __global__ void __launch_bounds__(256) segfix_kernel(int R, int ldm, const int64
             if (col < R) Mc[out * ldm + col] = carry_last[c0 * (32 * CB) + col] + acc[0];
             else if (col < ldm) Mc[out * ldm + col] = TA(0);
         }
+    };
+    if (!kBlockSpans) {
+        for (int64_t c0 = warp; c0 < nchunks; c0 += nwarps) one(c0);
+        return;
     }
-    if (!kBlockSpans) return;
-    // FP64 spans of more than kLongSpan chunks (rows of thousands of hits), by
-    // the whole block: warp w sums the chunks c0 + 1 + w, + 8, ... with lane =
-    // column, the warps' sums are added in warp order (one warp took 0.9 ms
-    // over the hottest row of 1e7 Zipf nonzeros, the block 0.05)
-    __syncthreads();
+    // A block's warps look at kLongBatch chunks each, then the block sums the
+    // long rows among them: warp w takes the chunks c0 + 1 + w, + 8, ... with
+    // lane = column, the warps' sums are added in warp order (one warp took 0.9
+    // ms over the hottest row of 1e7 Zipf nonzeros, the block 0.05)
     __shared__ TA wsum[8][32];
     const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int todo = min(nlong, kMaxLongSpans);
-    for (int q = 0; q < todo; q++) {
-        const int64_t c0 = longs[q][0], c1 = longs[q][1];
-        const int64_t out = carry_seg ? (int64_t)carry_seg[c0] : (int64_t)carry_row[c0];
-        for (int cb = 0; cb < CB; cb++) {
-            TA s[8];
-#pragma unroll
-            for (int k = 0; k < 8; k++) s[k] = TA(0);
-            int64_t m = c0 + 1 + w;
-            for (; m + 7 * nw <= c1; m += 8 * nw) {
-                TA v[8];
-#pragma unroll
-                for (int k = 0; k < 8; k++) v[k] = carry_first[(m + k * nw) * (32 * CB) + 32 * cb + lane];
-#pragma unroll
-                for (int k = 0; k < 8; k++) s[k] += v[k];
-            }
-            for (; m <= c1; m += nw) s[0] += carry_first[m * (32 * CB) + 32 * cb + lane];
-            wsum[w][lane] = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
-            __syncthreads();
-            const int col = 32 * cb + lane;
-            if (w == 0 && col < ldm) {
-                TA v = TA(0);
-                if (col < R) {
-                    v = carry_last[c0 * (32 * CB) + col];
-                    for (int k = 0; k < nw; k++) v += wsum[k][lane];
-                }
-                Mc[out * ldm + col] = v;
-            }
-            __syncthreads();
+    for (int64_t b0 = (int64_t)blockIdx.x * nw; b0 < nchunks; b0 += kLongBatch * nwarps) {
+        if (threadIdx.x == 0) nlong = 0;
+        __syncthreads();
+        for (int k = 0; k < kLongBatch; k++) {
+            const int64_t c0 = b0 + w + k * nwarps;
+            if (c0 < nchunks) one(c0);
         }
+        __syncthreads();
+        const int todo = nlong;
+        for (int q = 0; q < todo; q++) {
+            const int64_t c0 = longs[q][0], c1 = longs[q][1];
+            const int64_t out = carry_seg ? (int64_t)carry_seg[c0] : (int64_t)carry_row[c0];
+            for (int cb = 0; cb < CB; cb++) {
+                TA s[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) s[k] = TA(0);
+                int64_t m = c0 + 1 + w;
+                for (; m + 7 * nw <= c1; m += 8 * nw) {
+                    TA v[8];
+#pragma unroll
+                    for (int k = 0; k < 8; k++) v[k] = carry_first[(m + k * nw) * (32 * CB) + 32 * cb + lane];
+#pragma unroll
+                    for (int k = 0; k < 8; k++) s[k] += v[k];
+                }
+                for (; m <= c1; m += nw) s[0] += carry_first[m * (32 * CB) + 32 * cb + lane];
+                wsum[w][lane] = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+                __syncthreads();
+                const int col = 32 * cb + lane;
+                if (w == 0 && col < ldm) {
+                    TA v = TA(0);
+                    if (col < R) {
+                        v = carry_last[c0 * (32 * CB) + col];
+                        for (int k = 0; k < nw; k++) v += wsum[k][lane];
+                    }
+                    Mc[out * ldm + col] = v;
+                }
+                __syncthreads();
+            }
+        }
+        __syncthreads();  // nlong is read
     }
 }
 
