@@ -209,6 +209,10 @@ class FusedAdam:
                   0.0 if self.lower is None else float(self.lower), _stream())
 
 
+# What a step's fused objective stands in for.
+_EXPRESSION = (sampled_model, loss_values, SampledCPModel, EPS)
+
+
 class GCP:
     """Gradient-based GCP of a sparse tensor with stratified entry sampling,
     fused Adam steps, and (for the Poisson and Bernoulli losses) nonnegative
@@ -256,12 +260,14 @@ class GCP:
     def _step_objective(self, idx, x, w) -> torch.Tensor:
         """``objective`` of a step's own sample: the fused loss (3 launches
         forward and backward where the torch expression takes 19) when the
-        sample and the objective are this class's and the sample's type is the
-        factors'; an overridden objective or sampler, an empty sample and an
-        unknown loss take the expression."""
+        sample, the objective and what it is made of are this module's and the
+        sample's type is the factors'; an overridden objective or sampler, a
+        replaced ``sampled_model``, ``SampledCPModel``, ``loss_values`` or
+        ``EPS``, an empty sample and an unknown loss take the expression."""
         cls = type(self)
         own = (cls.objective is GCP.objective and cls.step_sample is GCP.step_sample
-               and "objective" not in self.__dict__ and "step_sample" not in self.__dict__)
+               and "objective" not in self.__dict__ and "step_sample" not in self.__dict__
+               and (sampled_model, loss_values, SampledCPModel, EPS) == _EXPRESSION)
         if own and self.loss in _LOSSES and idx.shape[0] > 0 and x.dtype == self.factors[0].dtype:
             return SampledLoss.apply(self.loss, idx, x, w, *self.factors)
         return self.objective(idx, x, w)
