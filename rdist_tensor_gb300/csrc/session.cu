@@ -84,11 +84,11 @@ static void carve(Session& s) {
         } else {
             s.eigscr = a.take<double>((int64_t)syev_refine_doubles(R, std::max(N - 1, 1)));
         }
-        if (s.cfg.precision == EXAFAC_PREC_FP64 && sts_zq_wanted(R, J)) {
-            int64_t widest = std::max<int64_t>(s.etree.leaf_count, 1);
-            for (int k = 0; k < N; k++) widest = std::max<int64_t>(widest, s.rtree[k].leaf_count);
+        int64_t widest = std::max<int64_t>(s.etree.leaf_count, 1);
+        for (int k = 0; k < N; k++) widest = std::max<int64_t>(widest, s.rtree[k].leaf_count);
+        // (the breadth-first kernels hold a node in 32 bits)
+        if (s.cfg.precision == EXAFAC_PREC_FP64 && sts_zq_wanted(R, J) && widest <= (int64_t)1 << 30)
             zq_carve(a, s.zq, R, J, widest, 2 * N);
-        }
     }
     s.cdf_total = a.take<double>(N);
     s.gram = a.take<double>((int64_t)N * R2);
