@@ -705,7 +705,7 @@ __device__ void newton_refine(int R, const double* __restrict__ A, double* __res
 }
 
 __global__ void spd_pinv_kernel(int R, const double* __restrict__ A, double* __restrict__ out, double tol,
-                                double* vt_scratch, int refine, int fast) {
+                                double* vt_scratch) {
     extern __shared__ double smem[];
     __shared__ int fail;
     __shared__ double fro;
@@ -713,10 +713,6 @@ __global__ void spd_pinv_kernel(int R, const double* __restrict__ A, double* __r
     double* L = smem;
     double* Li = smem + R * R;
     const int tid = threadIdx.x, nt = blockDim.x;
-    if (!fast) {  // the Cholesky buffers do not fit in shared memory
-        syev_block(R, A, nullptr, nullptr, out, tol, vt_scratch, smem);
-        return;
-    }
     for (int e = tid; e < R * R; e += nt) {
         int i = e / R, j = e % R;
         L[e] = (i <= j) ? A[i * R + j] : A[j * R + i];
@@ -773,14 +769,10 @@ __global__ void spd_pinv_kernel(int R, const double* __restrict__ A, double* __r
         }
         __syncthreads();
         const double bound = 1.0 / sqrt(fro);
-        if (isfinite(fro) && bound > 10.0 * tol) {
-            if (refine) newton_refine(R, A, out, smem);
-            return;
-        }
+        if (isfinite(fro) && bound > 10.0 * tol) return;
         __syncthreads();
     }
     syev_block(R, A, nullptr, nullptr, out, tol, vt_scratch, smem);
-    if (refine) newton_refine(R, A, out, smem);
 }
 
 // R <= 32: the symmetric sweep operator (Gauss-Jordan with diagonal pivots,
@@ -1042,9 +1034,9 @@ __device__ __forceinline__ int tri(int i, int j) { return i * (i + 1) / 2 + j; }
 // a / b from y ~ 1 / b: the quotient's exact residual, multiplied back
 // (Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000 processor", 1990): the correctly rounded a / b when y is the
-// rounded reciprocal, and for a y within an ulp of it unless a / b lies within
-// 2^-52 ulp of a midpoint.  Three dependent FP64 operations (~64 cycles each)
-// where the division itself takes some 700 cycles.
+// rounded reciprocal, and for a y within two ulps of it unless a / b lies
+// within 2^-49 ulp of a midpoint.  Three dependent FP64 operations (~64 cycles
+// each) where the division itself takes some 700 cycles.
 __device__ __forceinline__ double div_by(double a, double b, double y) {
     const double q = a * y;
     return fma(fma(-q, b, a), y, q);
@@ -1080,31 +1072,8 @@ __device__ __forceinline__ double gram_dot(const double* Li, int a, int b, int k
     return (s0 + s1) + (s2 + s3);
 }
 
-__device__ void newton_refine_global(int R, const double* __restrict__ A, double* __restrict__ out,
-                                     double* __restrict__ scratch) {
-    double* X = scratch;
-    double* T = scratch + (size_t)R * R;
-    __syncthreads();
-    for (int e = threadIdx.x; e < R * R; e += blockDim.x) X[e] = out[e];
-    __syncthreads();
-    for (int e = threadIdx.x; e < R * R; e += blockDim.x) {  // T = A X
-        const int i = e / R, j = e % R;
-        double acc = 0.0;
-        for (int k = 0; k < R; k++) acc = fma(i <= k ? A[i * R + k] : A[k * R + i], X[k * R + j], acc);
-        T[e] = acc;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < R * R; e += blockDim.x) {  // out = 2X - X T
-        const int i = e / R, j = e % R;
-        double acc = 0.0;
-        for (int k = 0; k < R; k++) acc = fma(X[i * R + k], T[k * R + j], acc);
-        out[e] = 2.0 * X[e] - acc;
-    }
-    __syncthreads();
-}
-
 __global__ void spd_pinv_packed_kernel(int R, const double* __restrict__ A, double* __restrict__ out, double tol,
-                                       double* vt_scratch, int refine) {
+                                       double* vt_scratch) {
     extern __shared__ double smem[];
     __shared__ int fail;
     __shared__ double fro_w[32];  // per-warp parts, summed in warp order
@@ -1163,14 +1132,10 @@ __global__ void spd_pinv_packed_kernel(int R, const double* __restrict__ A, doub
         double fro = 0.0;
         for (int q = 0; q < (nt + 31) / 32; q++) fro += fro_w[q];
         const double bound = 1.0 / sqrt(fro);
-        if (isfinite(fro) && bound > 10.0 * tol) {  // the same in every thread
-            if (refine) newton_refine_global(R, A, out, vt_scratch);
-            return;
-        }
+        if (isfinite(fro) && bound > 10.0 * tol) return;  // the same in every thread
         __syncthreads();
     }
     syev_block(R, A, nullptr, nullptr, out, tol, vt_scratch, smem);
-    if (refine) newton_refine_global(R, A, out, vt_scratch);
 }
 
 // ---------------------------------------------------------------------------
@@ -1459,18 +1424,12 @@ __global__ void newton_update_kernel(int R, const double* __restrict__ T, double
     }
 }
 
-// Shared memory of the Cholesky path (L, L^{-1}, and the Newton step's
-// third matrix).  The Cholesky path in full matrices is used when its buffers
-// fit under kPinvSmemCap (R <= 92); larger ranks take the packed kernel.
+// Shared memory of the one-CTA Cholesky path (L, L^{-1}, and at R <= 32 the
+// Newton step's third matrix).  The path in full matrices is used when three
+// of them fit under kPinvSmemCap (R <= 92); larger ranks take the packed kernel.
 static size_t chol_smem_bytes(int R) { return sizeof(double) * 3 * (size_t)R * R; }
 static size_t chol_packed_smem_bytes(int R) { return sizeof(double) * 2 * (size_t)(R * (R + 1) / 2); }
 constexpr size_t kPinvSmemCap = 200 * 1024;
-
-size_t pinv_smem_bytes(int R) {
-    size_t jac = syev_smem_bytes(R);
-    if (chol_smem_bytes(R) > kPinvSmemCap) return jac;
-    return std::max(chol_smem_bytes(R), jac);
-}
 
 // L, L^{-1} (scr) and out = A^{-1} where the factorisation goes through.
 static int launch_chol_inverse(int R, const double* A, double* out, bool four, double* scr, cudaStream_t st) {
@@ -1515,26 +1474,12 @@ static int launch_pinv_impl(int R, const double* A, double* out, double tol, dou
         EXAFAC_CHECK_LAUNCH();
         return EXAFAC_OK;
     }
-    const int fast = chol_smem_bytes(R) <= kPinvSmemCap;
-    if (!fast) {
-        const size_t smem = std::max(chol_packed_smem_bytes(R), syev_smem_bytes(R));
-        EXAFAC_CUDA_TRY(
-            cudaFuncSetAttribute(spd_pinv_packed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        spd_pinv_packed_kernel<<<1, 512, smem, stream>>>(R, A, out, tol, vt_scratch, 0);
-        count_launch();
-        if (refine) {
-            newton_residual_kernel<<<R, 128, 0, stream>>>(R, A, out, vt_scratch);
-            count_launch();
-            newton_update_kernel<<<R, 128, 0, stream>>>(R, vt_scratch, out);
-            count_launch();
-        }
-        EXAFAC_CHECK_LAUNCH();
-        return EXAFAC_OK;
-    }
-    size_t smem = pinv_smem_bytes(R);
-    if (smem > 48 * 1024)
-        EXAFAC_CUDA_TRY(cudaFuncSetAttribute(spd_pinv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    spd_pinv_kernel<<<1, R <= 32 ? 256 : 512, smem, stream>>>(R, A, out, tol, vt_scratch, fast ? refine : 0, fast);
+    // one CTA, for the entry points without that scratch (no Newton step)
+    const bool packed = chol_smem_bytes(R) > kPinvSmemCap;
+    auto kernel = packed ? spd_pinv_packed_kernel : spd_pinv_kernel;
+    const size_t smem = std::max(packed ? chol_packed_smem_bytes(R) : chol_smem_bytes(R), syev_smem_bytes(R));
+    EXAFAC_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<1, 512, smem, stream>>>(R, A, out, tol, vt_scratch);
     count_launch();
     EXAFAC_CHECK_LAUNCH();
     return EXAFAC_OK;

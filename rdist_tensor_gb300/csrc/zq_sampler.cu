@@ -454,10 +454,11 @@ __device__ __forceinline__ void z_dot8(uint32_t taddr, const long long* xrow, in
 // NT = 512 (R > 64, one block per SM): a chunk's products run beside the
 // previous chunk's read-back (two accumulator sets), and beside the next
 // chunk's expansion when a second node buffer fits (nb = 2).
-// nodes != null: the operands of the level's left children (of the root: MODE
-// 0), node by node in z_chunk_bytes chunks (zq_partition_kernel has expanded
-// them; lb the parents' first index), brought by bulk copies, the first one of
-// a run ahead of its use; null: each run expands its node here.
+// nodes != null (R > 32, two chunks or more): the operands of the level's left
+// children (of the root: MODE 0), node by node in z_chunk_bytes chunks
+// (zq_partition_kernel has expanded them; lb the parents' first index), brought
+// by bulk copies, the first one of a run ahead of its use; null: each run
+// expands its node here.
 // A run's sums are kept and a tile's masses and branches formed together: an
 // SM takes an FP64 instruction per 19 clocks whatever its active lanes, and
 // the ~14 of them per run cost as much as the products on levels with short
@@ -506,7 +507,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
     uint32_t phase[2] = {0, 0}, cphase[2] = {0, 0};
     bool lost = false;     // a wait of this thread ran out
     uint32_t flight = 0;   // thread 0: bit q a copy into buffer q, bit 2 + q products of set q
-    int64_t resident = -1; // the node B holds, or is being copied (one-chunk ranks)
+    int64_t resident = -1; // the node B holds (one-chunk ranks)
     bool aborted = false;
     const int row = (w & 3) * 32 + lane, grp = w >> 2;
     const uint32_t lane_base = tmem + ((uint32_t)((w & 3) * 32) << 16);
@@ -594,7 +595,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
         }
         __syncthreads();
         bool ahead = false;  // the next run's first chunk is on its way
-        if (pre && i0 < own.y && !stays(cs[i0]) && !(z.nch == 1 && resident == cs[i0])) {
+        if (pre && i0 < own.y && !stays(cs[i0])) {
             if (tid == 0) fetch(0, cs[i0], 0);
             ahead = true;
         }
@@ -613,14 +614,12 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
             ZSums sum = {0, 0, 0, 0, 0};
             const long long* xrow = reinterpret_cast<const long long*>(b.xi) + (int64_t)js[row < n ? row : 0] * Rx;
             if (pre) {
-                const bool held = z.nch == 1 && resident == c && !ahead;
                 if (tid == 0) {
-                    if (!held && !ahead) fetch(0, c, 0);
-                    if (nb == 2 && z.nch > 1) fetch(1, c, 1);
-                    issue(0, 0, !held);
+                    if (!ahead) fetch(0, c, 0);
+                    if (nb == 2) fetch(1, c, 1);
+                    issue(0, 0, true);
                 }
                 ahead = false;
-                resident = c;
                 for (int ch = 0; ch < z.nch; ch++) {
                     const int cur = kPipe ? ch & 1 : 0;
                     const bool more = ch + 1 < z.nch;
@@ -1307,17 +1306,17 @@ __device__ __forceinline__ void tmem_ld4_nowait(uint32_t taddr, uint32_t (&r)[4]
                  : "memory");
 }
 
-template <int NT>
-__global__ void __launch_bounds__(NT, 1)
+constexpr int kWThreads = 512;
+__global__ void __launch_bounds__(kWThreads, 1)
     zq_weight_kernel(int R, int64_t J, ZState b, const double* __restrict__ PhiP, const int32_t* __restrict__ phi_exp,
                      double* __restrict__ weights, DeviceStatus* status, uint32_t wait_polls, int64_t withhold) {
     extern __shared__ __align__(128) unsigned char z_raw[];
     if (z_lost(b)) {
-        for (int64_t j = (int64_t)blockIdx.x * NT + threadIdx.x; j < J; j += (int64_t)gridDim.x * NT) weights[j] = 0.0;
+        for (int64_t j = (int64_t)blockIdx.x * kWThreads + threadIdx.x; j < J; j += (int64_t)gridDim.x * kWThreads)
+            weights[j] = 0.0;
         return;
     }
-    constexpr int NG = NT / 128;
-    constexpr int CPT = kWCols / NG;  // columns per thread: 8 or 4, in groups of 4
+    constexpr int NG = kWThreads / 128;  // threads per slot in the read-back, four columns each
     __shared__ long long part[NG][7][kZTile];
     __shared__ float2 fpart[NG][kZTile];
     __shared__ int rs[kMaxRank];
@@ -1332,7 +1331,7 @@ __global__ void __launch_bounds__(NT, 1)
     unsigned char* B = A + kWx * z.xs;
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     if (w == 0) tmem_alloc(&tmem_base, 128);
-    for (int a = tid; a < R; a += NT) rs[a] = packed_index(R, a, a);
+    for (int a = tid; a < R; a += kWThreads) rs[a] = packed_index(R, a, a);
     if (tid == 0) {
         mbar_init(&bar, 1);
         fence_mbar_init();
@@ -1343,7 +1342,7 @@ __global__ void __launch_bounds__(NT, 1)
     tc_fence_after();
     const uint32_t tmem = tmem_base;
     const int emax = *phi_exp;
-    for (int c = tid; c < kMaxRank; c += NT)  // (read after the barriers of the first chunk)
+    for (int c = tid; c < kMaxRank; c += kWThreads)  // (read after the barriers of the first chunk)
         diag[c] = c < R ? (float)scalbn(PhiP[packed_index(R, c, c)], 1028 - emax) : 0.0f;
     uint32_t phase = 0;
     bool flight = false;  // thread 0: products on their way
@@ -1354,7 +1353,7 @@ __global__ void __launch_bounds__(NT, 1)
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int64_t s0 = tile * kZTile;
         const int n = (int)min((int64_t)kZTile, J - s0);
-        for (int e = tid; e < kZTile * (z.Rk / 8); e += NT) {  // h, the row fastest
+        for (int e = tid; e < kZTile * (z.Rk / 8); e += kWThreads) {  // h, the row fastest
             const int r = e & (kZTile - 1), k = 8 * (e / kZTile);
             long long X[8];
             load_x8(xi + (s0 + (r < n ? r : 0)) * Rx, k, Rx, r < n, X);
@@ -1388,7 +1387,7 @@ __global__ void __launch_bounds__(NT, 1)
         const long long* xrow = xi + jrow * Rx;
         const uint32_t* rrow = reinterpret_cast<const uint32_t*>(b.rest + jrow * Rx);
         for (int ch = 0; ch < nch; ch++) {
-            for (int e = tid; e < kWCols * (z.Rk / 8); e += NT) {  // Phi's columns, the column fastest
+            for (int e = tid; e < kWCols * (z.Rk / 8); e += kWThreads) {  // Phi's columns, the column fastest
                 const int c = e & (kWCols - 1), k = 8 * (e / kWCols);
                 const int col = ch * kWCols + c;
                 const int rc = col < R ? rs[col] : 0;
@@ -1442,59 +1441,56 @@ __global__ void __launch_bounds__(NT, 1)
                 abort_flag = 1;
             }
             tc_fence_after();
+            const int cc = 4 * grp;
+            uint32_t a[kWa][4];
 #pragma unroll
-            for (int h = 0; h < CPT / 4; h++) {
-                const int cc = grp * CPT + 4 * h;
-                uint32_t a[kWa][4];
+            for (int q = 0; q < kWa; q++)
+                tmem_ld4_nowait(tmem + ((uint32_t)((w & 3) * 32) << 16) + (uint32_t)(kWCols * q + cc), a[q]);
+            long long X[4] = {0, 0, 0, 0};
+            uint32_t r4 = 0x80808080u;  // the four rests, plus 128 each
+            if (ch * kWCols + cc < Rx) {
+                asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+                             : "=l"(X[0]), "=l"(X[1]), "=l"(X[2]), "=l"(X[3])
+                             : "l"(xrow + ch * kWCols + cc));
+                r4 ^= __ldg(rrow + (ch * kWCols + cc) / 4);
+            }
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int q = 0; q < kWa; q++)
-                    tmem_ld4_nowait(tmem + ((uint32_t)((w & 3) * 32) << 16) + (uint32_t)(kWCols * q + cc), a[q]);
-                long long X[4] = {0, 0, 0, 0};
-                uint32_t r4 = 0x80808080u;  // the four rests, plus 128 each
-                if (ch * kWCols + cc < Rx) {
-                    asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
-                                 : "=l"(X[0]), "=l"(X[1]), "=l"(X[2]), "=l"(X[3])
-                                 : "l"(xrow + ch * kWCols + cc));
-                    r4 ^= __ldg(rrow + (ch * kWCols + cc) / 4);
-                }
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            for (int q = 0; q < kWa; q++)
+                asm volatile("" : "+r"(a[q][0]), "+r"(a[q][1]), "+r"(a[q][2]), "+r"(a[q][3]));
 #pragma unroll
-                for (int q = 0; q < kWa; q++)
-                    asm volatile("" : "+r"(a[q][0]), "+r"(a[q][1]), "+r"(a[q][2]), "+r"(a[q][3]));
+            for (int q = 0; q < 4; q++) {
+                float f[kWa];
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    float f[kWa];
-#pragma unroll
-                    for (int u = 0; u < kWa; u++) f[u] = __uint_as_float(a[u][q]);
-                    // integers of the weights 0, 1, 2; weight 3 to 2^-23, weight
-                    // 4 to 2^-30; their (exact) rests with weight 5 to 2^-38;
-                    // that rest with the weights 6 and 7 to 2^-46
-                    const int m0 = __float_as_int(f[0] + 12582912.0f) - 0x4B400000;
-                    const int m1 = __float_as_int(f[1] + 49152.0f) - 0x47400000;
-                    const int m2 = __float_as_int(f[2] + 192.0f) - 0x43400000;
-                    const float t3 = f[3] + 1.5f;
-                    const int m3 = __float_as_int(t3) - 0x3FC00000;
-                    const float t4 = f[4] + 0x1.8p-7f;
-                    const int m4 = __float_as_int(t4) - 0x3C400000;
-                    const float g5 = ((f[3] - (t3 - 1.5f)) + (f[4] - (t4 - 0x1.8p-7f))) + f[5];
-                    const float t5 = g5 + 0x1.8p-15f;
-                    const int m5 = __float_as_int(t5) - 0x38400000;
-                    const float g6 = (g5 - (t5 - 0x1.8p-15f)) + (f[6] + f[7]);
-                    const int W = __float_as_int(g6 + 0x1.8p-23f) - 0x34400000;
-                    const int Pn = m0 * 256 + m1, Qn = m2 * 128 + m3, Tn = m4 * 256 + m5;
-                    const int z4 = x_z4(X[q]), xr = x_rest(X[q]), k5 = (xr + (1 << 14)) >> 15;
-                    const int wh = z4 >> 4, wl = ((z4 & 15) << 23) + 2 * xr - (k5 << 15);
-                    sum[0] += (long long)Pn * wh;
-                    sum[1] += (long long)Pn * wl;
-                    sum[2] += (long long)Qn * wh;
-                    sum[3] += (long long)Qn * wl;
-                    sum[4] += (long long)Tn * wh;
-                    sum[5] += (long long)Tn * wl;
-                    sum[6] += (long long)W * wh;
-                    const float x = (float)z4 * 0x1p-24f;
-                    rest = fmaf((f[0] + f[1]) + f[2], digit_f<0>(r4, q), rest);
-                    dsum = fmaf(diag[ch * kWCols + cc + q] * x, x, dsum);
-                }
+                for (int u = 0; u < kWa; u++) f[u] = __uint_as_float(a[u][q]);
+                // integers of the weights 0, 1, 2; weight 3 to 2^-23, weight
+                // 4 to 2^-30; their (exact) rests with weight 5 to 2^-38;
+                // that rest with the weights 6 and 7 to 2^-46
+                const int m0 = __float_as_int(f[0] + 12582912.0f) - 0x4B400000;
+                const int m1 = __float_as_int(f[1] + 49152.0f) - 0x47400000;
+                const int m2 = __float_as_int(f[2] + 192.0f) - 0x43400000;
+                const float t3 = f[3] + 1.5f;
+                const int m3 = __float_as_int(t3) - 0x3FC00000;
+                const float t4 = f[4] + 0x1.8p-7f;
+                const int m4 = __float_as_int(t4) - 0x3C400000;
+                const float g5 = ((f[3] - (t3 - 1.5f)) + (f[4] - (t4 - 0x1.8p-7f))) + f[5];
+                const float t5 = g5 + 0x1.8p-15f;
+                const int m5 = __float_as_int(t5) - 0x38400000;
+                const float g6 = (g5 - (t5 - 0x1.8p-15f)) + (f[6] + f[7]);
+                const int W = __float_as_int(g6 + 0x1.8p-23f) - 0x34400000;
+                const int Pn = m0 * 256 + m1, Qn = m2 * 128 + m3, Tn = m4 * 256 + m5;
+                const int z4 = x_z4(X[q]), xr = x_rest(X[q]), k5 = (xr + (1 << 14)) >> 15;
+                const int wh = z4 >> 4, wl = ((z4 & 15) << 23) + 2 * xr - (k5 << 15);
+                sum[0] += (long long)Pn * wh;
+                sum[1] += (long long)Pn * wl;
+                sum[2] += (long long)Qn * wh;
+                sum[3] += (long long)Qn * wl;
+                sum[4] += (long long)Tn * wh;
+                sum[5] += (long long)Tn * wl;
+                sum[6] += (long long)W * wh;
+                const float x = (float)z4 * 0x1p-24f;
+                rest = fmaf((f[0] + f[1]) + f[2], digit_f<0>(r4, q), rest);
+                dsum = fmaf(diag[ch * kWCols + cc + q] * x, x, dsum);
             }
             tc_fence_before();
             __syncthreads();  // the accumulators and B are free for the next chunk
@@ -1745,8 +1741,8 @@ int sts_draw_zq(Session& s, int n, int64_t J, const double* uni, cudaStream_t st
     const size_t smem = zw_smem(R);
     const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(J, kZTile), 152);
     EXAFAC_CUDA_TRY(
-        cudaFuncSetAttribute(zq_weight_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    zq_weight_kernel<512><<<blocks, 512, smem, st>>>(R, J, b, s.PhiP, b.tree_exp + 2 * N, s.weights, s.status,
+        cudaFuncSetAttribute(zq_weight_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    zq_weight_kernel<<<blocks, kWThreads, smem, st>>>(R, J, b, s.PhiP, b.tree_exp + 2 * N, s.weights, s.status,
                                                      s.wait_polls ? s.wait_polls : kSpinLimit, s.withheld(25));
     count_launch();
     EXAFAC_CHECK_LAUNCH();
