@@ -434,9 +434,9 @@ def run_gcp(args, w):
            "steps_run": warmup + steps, "optimizer_ms_per_step": opt_ms,
            "optimizer_bytes_per_step": 7 * 4 * sum(int(d) for d in dims) * R,
            "optimizer_gbs": 7 * 4 * sum(int(d) for d in dims) * R / (opt_ms * 1e-3) / 1e9,
-           "step_kernels_of_this_library": "gcp_sample_kernel, cp_model_kernel, cp_adjoint_kernel, "
-                                           "adam_step_kernel (Adam fused with the projection); the loss terms and "
-                                           "their derivative are torch elementwise ops under autograd"}
+           "step_kernels_of_this_library": "gcp_sample_kernel, cp_loss_kernel (model, loss and derivative), "
+                                           "zero_list_kernel, cp_adjoint_kernel, adam_step_kernel (Adam fused "
+                                           "with the projection)"}
     line = {"metric": GCP_METRIC, "value": value, "unit": "steps/s", "n_gpus": ws, "steps": steps,
             "warmup": warmup, "ms_per_step": 1000.0 * elapsed / steps, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f32",

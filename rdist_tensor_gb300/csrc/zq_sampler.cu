@@ -1279,19 +1279,18 @@ __global__ void zq_leaf1_kernel(TreeShape t, int64_t J, ZState b, int N, int col
 // which took 3.1 ms at R = 64, J = 2^18.  What the fixed point of h leaves off
 // (up to 2^-48 of the scaled units, more than FP64 where the entries of h differ
 // by decades) is kept to 256ths of its unit (ZState::rest) and added in FP32 to
-// first order, 2 sum_c Y_c (h - x)_c.  The
-// digits and the cut of Phi that are dropped are below R 4 2^-50 of n1; an FP64
-// sum's own rounding is some 2^-53 of sum |h_a Phi_ab h_b|, of which sum_c
-// Phi_cc h_c^2 is a part.  A sample whose bound is above 2^-42 of its form or
-// above 2^-46 of that diagonal part gets the depth-first kernel's own sum from h
-// (sts_weight_list_kernel); one whose form is not positive or not finite is
-// marked.  Against exact arithmetic, the largest error of a dozen samples, FP64
-// sums -> digits: Grams of random factors at R = 64 3e-16 -> 2e-17, nearly
-// collinear columns (Phi_cc to 170) at R = 100 9e-15 -> 2.4e-15, small h where Phi
-// is large (three decades) 2.2e-16 -> 2.2e-16 (6e-15 without the diagonal's test).
-// As a decomposition converges up to a tenth of the samples go to FP64; drawing
-// them again whole took 1.1 ms a step at R = 100 with four modes, 6 ms at R = 66
-// with three.
+// first order, 2 sum_c Y_c (h - x)_c.  The digits and the cut of Phi that are
+// dropped are below R 4 2^-50 of n1; an FP64 sum's own rounding is some 2^-53 of
+// sum |h_a Phi_ab h_b|, of which sum_c Phi_cc h_c^2 is a part.  A sample whose
+// bound is above 2^-42 of its form or above 2^-46 of that diagonal part gets the
+// depth-first kernel's own sum from h (sts_weight_list_kernel); one whose form
+// is not positive or not finite is marked.  Against exact arithmetic, the
+// largest error of a dozen samples, FP64 sums -> digits: Grams of random
+// factors at R = 64 3e-16 -> 2e-17, nearly collinear columns (Phi_cc to 170) at
+// R = 100 9e-15 -> 2.4e-15, small h where Phi is large (three decades) 2.2e-16
+// -> 2.2e-16 (6e-15 without the diagonal's test). As a decomposition converges
+// up to a tenth of the samples go to FP64; drawing them again whole took 1.1 ms
+// a step at R = 100 with four modes, 6 ms at R = 66 with three.
 constexpr int kWx = 5, kWa = 8, kWCols = 16;
 
 static size_t zw_smem(int R) {
