@@ -18,7 +18,9 @@ CASES = [((3001, 700), 64, 4096, 4096, (0, 1)),
          ((5003, 120, 77, 300, 64), 33, 9001, 9001, (0, 2, 4)),
          ((901, 120, 77), 58, 4097, 50000, (0, 1)),
          ((900, 120, 300), 100, 1000, 4097, (2,)),
-         ((4001, 120, 90), 3, (1 << 21) + 77, (1 << 21) + 77, (1,))]
+         ((4001, 120, 90), 3, (1 << 21) + 77, (1 << 21) + 77, (1,)),
+         ((301, 1, 70), 2, 1500000, 1500000, (0, 2)),
+         ((130, 77), 1, (1 << 22) + 5, (1 << 22) + 5, (1,))]
 
 
 @pytest.mark.parametrize("dims,R,J,Jmax,modes", CASES)
