@@ -231,6 +231,16 @@ inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 bl
     return launch_dependent_if(true, kernel, grid, block, smem, st, args...);
 }
 
+// Lets a kernel's launches take all the dynamic shared memory that a block can
+// have beside its static part.  The limit is state of the process, shared by
+// every thread's sessions: set to one launch's size it could fall below what
+// another thread, at another rank, was about to launch with.
+cudaError_t allow_smem_of(const void* kernel);
+template <typename K>
+inline cudaError_t allow_smem(K* kernel) {
+    return allow_smem_of(reinterpret_cast<const void*>(kernel));
+}
+
 // Number of bits needed to hold coordinates in [0, dim).
 inline int bits_for(int64_t dim) {
     int b = 0;

@@ -1451,8 +1451,7 @@ static int launch_pinv_impl(int R, const double* A, double* out, double tol, dou
         EXAFAC_TRY(launch_chol_inverse(R, A, out, four, scr, stream));
         const size_t smem = syev_smem_bytes(R);
         if (smem > 48 * 1024)
-            EXAFAC_CUDA_TRY(
-                cudaFuncSetAttribute(chol_accept_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            EXAFAC_CUDA_TRY(allow_smem(chol_accept_kernel));
         EXAFAC_CUDA_TRY(launch_dependent(chol_accept_kernel, 1, 512, smem, stream, R, A, out, tol, scr, vt_scratch));
         count_launch();
         if (refine && four) {
@@ -1478,7 +1477,7 @@ static int launch_pinv_impl(int R, const double* A, double* out, double tol, dou
     const bool packed = chol_smem_bytes(R) > kPinvSmemCap;
     auto kernel = packed ? spd_pinv_packed_kernel : spd_pinv_kernel;
     const size_t smem = std::max(packed ? chol_packed_smem_bytes(R) : chol_smem_bytes(R), syev_smem_bytes(R));
-    EXAFAC_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    EXAFAC_CUDA_TRY(allow_smem(kernel));
     kernel<<<1, 512, smem, stream>>>(R, A, out, tol, vt_scratch);
     count_launch();
     EXAFAC_CHECK_LAUNCH();
@@ -1518,7 +1517,7 @@ int launch_syev(int R, const double* A, int64_t a_stride, int batch, double* V, 
                 double* pinv, double tol, double* vt_scratch, cudaStream_t stream) {
     size_t smem = syev_smem_bytes(R);
     if (smem > 48 * 1024) {
-        EXAFAC_CUDA_TRY(cudaFuncSetAttribute(syev_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        EXAFAC_CUDA_TRY(allow_smem(syev_kernel));
     }
     int threads = R <= 32 ? 256 : 512;
     syev_kernel<<<batch, threads, smem, stream>>>(R, A, a_stride, V, lam, v_stride, pinv, tol, vt_scratch); count_launch();
@@ -1536,9 +1535,8 @@ int launch_syev_refined(int R, const double* A, int64_t a_stride, int batch, dou
     double *X = scratch, *Xn = X + R2, *As = Xn + R2, *S = As + R2, *G = S + R2, *E = G + R2;
     const size_t jsm = jacobi32_bytes(R);
     if (jsm > 40 * 1024) {  // (the 48 KB of a launch without it include the static part)
-        EXAFAC_CUDA_TRY(cudaFuncSetAttribute(jacobi32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jsm));
-        EXAFAC_CUDA_TRY(
-            cudaFuncSetAttribute(refine_first_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jsm));
+        EXAFAC_CUDA_TRY(allow_smem(jacobi32_kernel));
+        EXAFAC_CUDA_TRY(allow_smem(refine_first_kernel));
     }
     jacobi32_kernel<<<batch, 512, jsm, stream>>>(R, A, a_stride, X, As, ss);
     count_launch();
@@ -1564,8 +1562,7 @@ int launch_syev_refined(int R, const double* A, int64_t a_stride, int batch, dou
     }
     const size_t smem = syev_smem_bytes(R);
     if (smem > 48 * 1024)
-        EXAFAC_CUDA_TRY(
-            cudaFuncSetAttribute(syev_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        EXAFAC_CUDA_TRY(allow_smem(syev_finish_kernel));
     EXAFAC_CUDA_TRY(launch_dependent(syev_finish_kernel, (unsigned)batch, R <= 32 ? 256 : 512, smem, stream, R, A,
                                      a_stride, (const double*)X, (const double*)S, (const double*)G, ss, V, lam,
                                      v_stride, vt_scratch));
@@ -1786,16 +1783,14 @@ int launch_sts_factors_chol(int N, int n, int R, double tol, double* chain, doub
     EXAFAC_TRY(launch_chol_inverse(R, A, Phi, true, scr, stream));
     const size_t smem = syev_smem_bytes(R);
     if (smem > 48 * 1024)
-        EXAFAC_CUDA_TRY(
-            cudaFuncSetAttribute(sts_phi_accept_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        EXAFAC_CUDA_TRY(allow_smem(sts_phi_accept_kernel));
     EXAFAC_CUDA_TRY(launch_dependent(sts_phi_accept_kernel, 1, 512, smem, stream, N, R, A, tol, E, Phi, V, lam, vt, scr));
     EXAFAC_CUDA_TRY(launch_dependent(sts_phi_rows_kernel, R, kMaxRank, 0, stream, N, n, R, chain, E, (const double*)Phi,
                                      PhiP, scr));
     add_launches(2);
     const size_t fsm = sizeof(double) * (size_t)(R * (R + 1) / 2);
     if (fsm > 48 * 1024)
-        EXAFAC_CUDA_TRY(
-            cudaFuncSetAttribute(sts_chain_chol_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsm));
+        EXAFAC_CUDA_TRY(allow_smem(sts_chain_chol_kernel));
     if (N > 1) {
         sts_chain_chol_kernel<<<N, 512, fsm, stream>>>(N, n, R, chain, E);
         count_launch();

@@ -304,8 +304,7 @@ int design_gram_digits(Session& s, int n, int64_t J, int64_t* nblk, cudaStream_t
     FactorPtrs f;
     for (int k = 0; k < kMaxModes; k++) f.U[k] = k < s.N ? s.F.U[k] : nullptr;
     const size_t smem = gq_smem(s.R);
-    EXAFAC_CUDA_TRY(
-        cudaFuncSetAttribute(design_digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    EXAFAC_CUDA_TRY(allow_smem(design_digits_kernel));
     *nblk = std::max<int64_t>(1, std::min<int64_t>(ceil_div(J, kGqRows), 152));
     design_digits_kernel<<<(unsigned)*nblk, kGqThreads, smem, st>>>(s.N, n, s.R, s.counters + 0, s.sd, s.wd, f, s.D, s.part,
                                                                     s.status, s.wait_polls ? s.wait_polls : kSpinLimit,

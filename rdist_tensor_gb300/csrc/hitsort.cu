@@ -551,8 +551,7 @@ static int sort_keys(Session& s, int n, bool packed, cudaStream_t st) {
         if (packed) {
             constexpr int IT = kHsItemsPacked;
             const size_t smem = (sizeof(uint64_t) + sizeof(uint32_t)) * kHsThreads * IT;
-            EXAFAC_CUDA_TRY(cudaFuncSetAttribute(os_downsweep_kernel<uint64_t, IT>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            EXAFAC_CUDA_TRY(allow_smem(os_downsweep_kernel<uint64_t, IT>));
             EXAFAC_CUDA_TRY(launch_dependent(os_downsweep_kernel<uint64_t, IT>, kHsDownGridPacked, kHsThreads, smem, st,
                                              s.counters, cap, s.hit_key[src], s.pay64[src], p, s.os_aux, s.os_status,
                                              s.hit_key[dst], s.pay64[dst], s.status, s.wait_polls,

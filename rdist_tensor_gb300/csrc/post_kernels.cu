@@ -926,8 +926,7 @@ __global__ void __launch_bounds__(kSolveWarps * 32, 4) normlev_f32_kernel(int R,
 template <int KC>
 static int launch_solve_f32(Session& s, int n, cudaStream_t st) {
     const size_t smem = MmaShape<KC>::kSmem;
-    EXAFAC_CUDA_TRY(
-        cudaFuncSetAttribute(solve_gram_mma_kernel<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    EXAFAC_CUDA_TRY(allow_smem(solve_gram_mma_kernel<KC>));
     // follows segfix, unless a dense factor was cleared in between
     EXAFAC_CUDA_TRY(launch_dependent_if(!s.dense[n], solve_gram_mma_kernel<KC>, kMmaBlocks, kMmaWarps * 32, smem, st,
                                         s.R, s.counters, reinterpret_cast<const float*>(s.Mc), s.dpinv, s.Uc, s.part,
@@ -965,14 +964,12 @@ static int solve_typed(Session& s, int n, cudaStream_t st) {
     const TA* Mc = reinterpret_cast<const TA*>(s.Mc);
     if (Q <= 9) {
         const size_t smem = solve_gram_smem<TA, 9>();
-        EXAFAC_CUDA_TRY(
-            cudaFuncSetAttribute(solve_gram_kernel<TA, 9>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        EXAFAC_CUDA_TRY(allow_smem(solve_gram_kernel<TA, 9>));
         solve_gram_kernel<TA, 9><<<kSolveBlocks, kSolveWarps * 32, smem, st>>>(R, s.counters, s.touched, Mc, s.dpinv,
                                                                                 s.F.U[n], s.part);
     } else {
         const size_t smem = solve_gram_smem<TA, 17>();
-        EXAFAC_CUDA_TRY(
-            cudaFuncSetAttribute(solve_gram_kernel<TA, 17>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        EXAFAC_CUDA_TRY(allow_smem(solve_gram_kernel<TA, 17>));
         solve_gram_kernel<TA, 17><<<kSolveBlocks, kSolveWarps * 32, smem, st>>>(R, s.counters, s.touched, Mc,
                                                                                  s.dpinv, s.F.U[n], s.part);
     }

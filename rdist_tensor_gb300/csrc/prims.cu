@@ -419,10 +419,8 @@ int radix_sort_pairs(int64_t count, int bits, int kw, const uint64_t* lo_in, con
         EXAFAC_CUDA_TRY(cudaMemcpyAsync(pay_out, pay_in, sizeof(uint32_t) * count, cudaMemcpyDeviceToDevice, s));
         return EXAFAC_OK;
     }
-    EXAFAC_CUDA_TRY(cudaFuncSetAttribute(radix_scatter_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)radix_smem<true>()));
-    EXAFAC_CUDA_TRY(cudaFuncSetAttribute(radix_scatter_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)radix_smem<false>()));
+    EXAFAC_CUDA_TRY(allow_smem(radix_scatter_kernel<true>));
+    EXAFAC_CUDA_TRY(allow_smem(radix_scatter_kernel<false>));
     for (int p = 0; p < passes; p++) {
         // Destination alternates so the final pass lands in *_out.
         const bool to_out = ((passes - 1 - p) % 2) == 0;

@@ -128,8 +128,7 @@ int arls_build_cdf(Session& s, int k, const uint32_t* list, const int64_t* count
     if (n <= kExactCdfMax) {
         const size_t smem = sizeof(double) * n;
         if (smem > 48 * 1024)
-            EXAFAC_CUDA_TRY(cudaFuncSetAttribute(cdf_sequential_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)smem));
+            EXAFAC_CUDA_TRY(allow_smem(cdf_sequential_kernel));
         cdf_sequential_kernel<<<1, 256, smem, st>>>(w, n, s.cdf[k], s.cdf_total + k, nullptr, count_dev);
         count_launch();
     } else {
@@ -180,7 +179,7 @@ int arls_leverage(Session& s, int k, bool all_rows, const double* pinv, cudaStre
     const int warps = 8;
     size_t smem = sizeof(double) * ((size_t)R * (R | 1) + warps * R);
     if (smem > 48 * 1024)
-        EXAFAC_CUDA_TRY(cudaFuncSetAttribute(leverage_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        EXAFAC_CUDA_TRY(allow_smem(leverage_kernel));
     int64_t rows = all_rows ? s.dims[k] : s.dims[k];
     int blocks = (int)std::min<int64_t>(ceil_div(rows, warps), 152 * 16);
     leverage_kernel<<<blocks, warps * 32, smem, st>>>(R, s.F.U[k], pinv, s.dims[k], all_rows ? nullptr : s.touched,
@@ -635,7 +634,7 @@ static int sts_draw_launch(Session& s, int n, int64_t J, const double* uni, cons
     sample_group_shape(s.R, sizeof(T), G, S);
     const size_t smem = (size_t)S * sample_group_bytes(s.R, sizeof(T));
     if (smem > 48 * 1024)
-        EXAFAC_CUDA_TRY(cudaFuncSetAttribute(sts_draw_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        EXAFAC_CUDA_TRY(allow_smem(sts_draw_kernel<T>));
     const int64_t blocks = std::max<int64_t>(std::min<int64_t>(ceil_div(J, S), 152 * (list ? 4 : 32)), 1);
     sts_draw_kernel<T><<<(unsigned)blocks, S * G * 32, smem, st>>>(N, n, s.R, G, S, J, m, s.etree, eigG, E, PhiP, uni,
                                                                    s.samples, s.weights, s.status, list, list_count);
@@ -659,8 +658,7 @@ int sts_draw(Session& s, int n, int64_t J, const double* uni, cudaStream_t st) {
             sample_group_shape(s.R, sizeof(double), G, S);
             const size_t smem = (size_t)S * sample_group_bytes(s.R, sizeof(double));
             if (smem > 48 * 1024)
-                EXAFAC_CUDA_TRY(
-                    cudaFuncSetAttribute(sts_weight_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                EXAFAC_CUDA_TRY(allow_smem(sts_weight_list_kernel));
             sts_weight_list_kernel<<<(unsigned)std::max<int64_t>(std::min<int64_t>(ceil_div(J, S), 152 * 4), 1), S * G * 32,
                                      smem, st>>>(s.R, G, S, J, s.D, s.PhiP, s.weights, s.zq.near_list, s.zq.near_count);
             count_launch();

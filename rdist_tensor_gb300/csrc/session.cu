@@ -9,7 +9,9 @@
 #include <cmath>
 #include <cstring>
 #include <deque>
+#include <mutex>
 #include <new>
+#include <unordered_map>
 #include <vector>
 
 #include "dense.cuh"
@@ -24,6 +26,29 @@ void set_error(const std::string& msg) { g_last_error = msg; }
 static std::atomic<long long> g_launches{0};
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 void add_launches(long long n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
+
+cudaError_t allow_smem_of(const void* kernel) {
+    static std::mutex mu;
+    static std::unordered_map<const void*, int> limits;  // by kernel: what its static part leaves
+    int limit = -1;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        const auto it = limits.find(kernel);
+        if (it != limits.end()) limit = it->second;
+    }
+    if (limit < 0) {
+        int dev = 0, most = 0;
+        cudaFuncAttributes a;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
+        if (e != cudaSuccess) return e;
+        limit = most - (int)a.sharedSizeBytes;
+        std::lock_guard<std::mutex> lock(mu);
+        limits[kernel] = limit;
+    }
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+}
 
 static int64_t next_pow2(int64_t x) {
     int64_t p = 1;

@@ -584,8 +584,7 @@ template <int kRound, int RP>
 static int launch_design_wide(Session& s, int n, cudaStream_t st) {
     const size_t smem = sizeof(float) * 32 * (RP + 8) + sizeof(double) * packed_size(RP);
     if (smem > 48 * 1024)
-        EXAFAC_CUDA_TRY(cudaFuncSetAttribute(design_mma_wide_kernel<kRound, RP>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        EXAFAC_CUDA_TRY(allow_smem(design_mma_wide_kernel<kRound, RP>));
     design_mma_wide_kernel<kRound, RP><<<kDesignBlocks, kDesignWarps * 32, smem, st>>>(
         s.N, n, s.R, s.counters + 0, s.sd, s.wd, factor_ptrs(s), s.Df, s.part);
     count_launch();
@@ -749,8 +748,7 @@ int spmm_solve_into(Session& s, int n, const double* Phi, double* out, cudaStrea
     const int warps = 8;
     size_t smem = sizeof(double) * ((size_t)R * R + warps * R);
     if (smem > 48 * 1024)
-        EXAFAC_CUDA_TRY(
-            cudaFuncSetAttribute(spmm_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        EXAFAC_CUDA_TRY(allow_smem(spmm_solve_kernel));
     spmm_solve_kernel<<<grid_cap(s.dims[n], warps * 32), warps * 32, smem, st>>>(
         R, s.counters, s.touched, s.seg_start, s.pay_sorted, s.ex_j, s.ex_val, s.D, Phi, out); count_launch();
     EXAFAC_CHECK_LAUNCH();
@@ -1029,8 +1027,7 @@ int matmul_rows_sym(Session& s, const double* M, const double* Phi, double* U, i
     const int R = s.R, warps = 8;
     size_t smem = sizeof(double) * ((size_t)R * R + warps * R);
     if (smem > 48 * 1024)
-        EXAFAC_CUDA_TRY(
-            cudaFuncSetAttribute(matmul_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        EXAFAC_CUDA_TRY(allow_smem(matmul_rows_kernel));
     matmul_rows_kernel<<<grid_cap(rows, warps), warps * 32, smem, st>>>(R, rows, M, Phi, U); count_launch();
     EXAFAC_CHECK_LAUNCH();
     return EXAFAC_OK;

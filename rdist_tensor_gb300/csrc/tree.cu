@@ -289,8 +289,7 @@ int launch_tree_build(const TreeShape& t, int R, const double* U, double* G, cud
     while (groups > 1 && sizeof(double) * groups * t.F * R > 160 * 1024) groups /= 2;
     const size_t smem = align_up(2 * P * sizeof(unsigned short), 16) + sizeof(double) * groups * t.F * R;
     if (smem > 48 * 1024) {
-        EXAFAC_CUDA_TRY(
-            cudaFuncSetAttribute(tree_leaf_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        EXAFAC_CUDA_TRY(allow_smem(tree_leaf_gram_kernel));
     }
     const int64_t sets = ceil_div(t.leaf_count, (int64_t)groups);
     // fewer sets of leaves than two blocks per SM: each split in parts of one
@@ -317,15 +316,13 @@ int launch_tree_build_f32(const TreeShape& t, int R, const float* U, double* G, 
     const int P = packed_size(R);
     if (R >= 32 && t.F > 1 && t.F <= 128) {
         const size_t smem = 2 * sizeof(float) * 128 * (size_t)((t.F + 15) & ~15) + 1024;
-        EXAFAC_CUDA_TRY(
-            cudaFuncSetAttribute(tree_leaf_gram_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        EXAFAC_CUDA_TRY(allow_smem(tree_leaf_gram_tc_kernel));
         const int blocks = (int)std::min<int64_t>(t.leaf_count, 152);
         tree_leaf_gram_tc_kernel<<<blocks, kLeafTcThreads, smem, stream>>>(t, R, U, G, status, polls);
     } else {
         const size_t smem = sizeof(float) * t.F * R;
         if (smem > 48 * 1024)
-            EXAFAC_CUDA_TRY(
-                cudaFuncSetAttribute(tree_leaf_gram_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            EXAFAC_CUDA_TRY(allow_smem(tree_leaf_gram_f32_kernel));
         const int blocks = (int)std::min<int64_t>(t.leaf_count, 152 * 4);
         tree_leaf_gram_f32_kernel<<<blocks, 128, smem, stream>>>(t, R, U, G);
     }
@@ -356,7 +353,7 @@ int launch_tree_sample(const TreeShape& t, int R, const double* G, const double*
     sample_group_shape(R, sizeof(double), Gw, S);
     const size_t smem = (size_t)S * sample_group_bytes(R, sizeof(double));
     if (smem > 48 * 1024)
-        EXAFAC_CUDA_TRY(cudaFuncSetAttribute(tree_sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        EXAFAC_CUDA_TRY(allow_smem(tree_sample_kernel));
     int64_t blocks = (J + S - 1) / S;
     if (blocks > 152 * 32) blocks = 152 * 32;
     if (blocks < 1) blocks = 1;

@@ -432,8 +432,7 @@ static int wide_solve(Session& s, int n, cudaStream_t st) {
     const bool f32 = std::is_same<T, float>::value;
     const int ldm = f32 ? f32_row_stride(s.R) : s.R;
     const size_t smem = wide_solve_smem<T, CB>();
-    EXAFAC_CUDA_TRY(
-        cudaFuncSetAttribute(solve_gram_wide_kernel<T, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    EXAFAC_CUDA_TRY(allow_smem(solve_gram_wide_kernel<T, CB>));
     EXAFAC_CUDA_TRY(launch_dependent_if(!s.dense[n], solve_gram_wide_kernel<T, CB>, kWideSolveBlocks,
                                         kWideWarps * 32, smem, st, s.R, ldm, s.counters, s.touched,
                                         reinterpret_cast<const T*>(s.Mc), s.dpinv, s.F.U[n],
@@ -452,8 +451,7 @@ static int wide_normalize(Session& s, int n, bool arls, cudaStream_t st) {
     if (arls) EXAFAC_TRY(launch_pinv(R, s.ngram, s.upinv, 1e-11, s.vt, st, s.cholscr));
     constexpr int RP = 32 * CB;
     const size_t smem = sizeof(double) * ((arls ? (size_t)RP * RP : 0) + (size_t)kWideWarps * RP);
-    EXAFAC_CUDA_TRY(
-        cudaFuncSetAttribute(normalize_wide_kernel<T, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    EXAFAC_CUDA_TRY(allow_smem(normalize_wide_kernel<T, CB>));
     normalize_wide_kernel<T, CB><<<152 * 4, kWideWarps * 32, smem, st>>>(
         R, f32 ? f32_row_stride(R) : R, s.counters, s.touched, f32 ? reinterpret_cast<const T*>(s.Uc) : nullptr,
         s.F.sigma, arls ? s.upinv : nullptr, reinterpret_cast<int*>(s.counters + 6), s.F.U[n],

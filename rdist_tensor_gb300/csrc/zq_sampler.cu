@@ -1625,8 +1625,7 @@ static int z_level(Session& s, const TreeShape& t, const double* G, const unsign
     const size_t two = z_smem(s.R, 2 * kZa);
     const int nb = NT == 512 && two <= 200 * 1024 ? 2 : 1;
     const size_t smem = nb == 2 ? two : z_smem(s.R, kZa);
-    EXAFAC_CUDA_TRY(cudaFuncSetAttribute(zq_level_kernel<MODE, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
+    EXAFAC_CUDA_TRY(allow_smem(zq_level_kernel<MODE, NT>));
     const unsigned blocks = z_blocks(s, J, NT == 256 ? 304 : 152);
     zq_level_kernel<MODE, NT><<<blocks, NT, smem, st>>>(s.R, nb, t, G, nodes, lb, ex, J, s.zq, p, order, dv,
                                                         s.status, s.wait_polls ? s.wait_polls : kSpinLimit,
@@ -1644,7 +1643,7 @@ template <int NT>
 static int z_leaf(Session& s, const TreeShape& t, const double* G, const double* U, int64_t J, int p,
                   const int32_t* order, const double* dv, int col, cudaStream_t st) {
     const size_t smem = z_smem(s.R, kZu);
-    EXAFAC_CUDA_TRY(cudaFuncSetAttribute(zq_leaf_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    EXAFAC_CUDA_TRY(allow_smem(zq_leaf_kernel<NT>));
     const unsigned blocks = z_blocks(s, J, NT == 256 ? 304 : 152);
     zq_leaf_kernel<NT><<<blocks, NT, smem, st>>>(s.R, t, G, U, J, s.zq, p, order, dv, s.N, col, s.samples, s.status,
                                                  s.wait_polls ? s.wait_polls : kSpinLimit, s.withheld(24));
@@ -1667,8 +1666,7 @@ static int z_descend(Session& s, const TreeShape& t, const double* G, const doub
     const bool in_smem = ntiles <= kZPrefSmem;
     const size_t psm = in_smem ? sizeof(int32_t) * (ntiles + 1) : 0;
     if (psm > 40 * 1024)  // (the 48 KB of a launch without it include the static part)
-        EXAFAC_CUDA_TRY(
-            cudaFuncSetAttribute(zq_partition_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
+        EXAFAC_CUDA_TRY(allow_smem(zq_partition_kernel));
     const bool tail = t.node_count > t.nodes_upto_lfill;
     const int32_t* order = nullptr;
     int p = 0;  // parity of the level
@@ -1739,8 +1737,7 @@ int sts_draw_zq(Session& s, int n, int64_t J, const double* uni, cudaStream_t st
     count_launch();
     const size_t smem = zw_smem(R);
     const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(J, kZTile), 152);
-    EXAFAC_CUDA_TRY(
-        cudaFuncSetAttribute(zq_weight_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    EXAFAC_CUDA_TRY(allow_smem(zq_weight_kernel));
     zq_weight_kernel<<<blocks, kWThreads, smem, st>>>(R, J, b, s.PhiP, b.tree_exp + 2 * N, s.weights, s.status,
                                                      s.wait_polls ? s.wait_polls : kSpinLimit, s.withheld(25));
     count_launch();
