@@ -27,7 +27,7 @@ static std::atomic<long long> g_launches{0};
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 void add_launches(long long n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
-cudaError_t allow_smem_of(const void* kernel) {
+cudaError_t allow_smem_of(const void* kernel) try {
     static std::mutex mu;
     static std::unordered_map<const void*, int> limits;  // by kernel: what its static part leaves
     int limit = -1;
@@ -48,6 +48,8 @@ cudaError_t allow_smem_of(const void* kernel) {
         limits[kernel] = limit;
     }
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+} catch (...) {  // (no exception leaves a C entry)
+    return cudaErrorMemoryAllocation;
 }
 
 static int64_t next_pow2(int64_t x) {
